@@ -368,8 +368,8 @@ def fourier_values(n: int, seed: int, dev, k: int = 32):
     return out.float().contiguous()
 
 
-GRAD_KERNELS = ["mc_signs", "mc_count", "mc_scan", "mc_emit", "mc_backward", "dc_classify", "dc_intersect",
-                "dc_solve", "dc_quads", "dc_weld", "dc_backward"]
+GRAD_KERNELS = ["mc_signs", "mc_count", "mc_scan", "mc_emit", "mc_fix", "mc_backward", "dc_classify",
+                "dc_intersect", "dc_solve", "dc_quads", "dc_weld", "dc_backward"]
 
 
 def run_grad(args, wl, rank, world) -> dict | None:

@@ -1,6 +1,6 @@
 // Dense-grid marching cubes on sm_103a.
 //
-// Four launches on one stream, nothing read back by the host:
+// Five launches on one stream, nothing read back by the host:
 //   1. mc_signs   streams the grid once (one warp per row, 16 coalesced
 //                 128-byte loads in flight per warp) into a sign bitmap,
 //                 1 bit per point.  This is the only pass over all values.
@@ -19,9 +19,10 @@
 //                 vertex indices by rank).  Vertices that can share a position
 //                 with another edge's (t within tau of 0 or 1) go through a small
 //                 hash that counts exact coincidences.
-//   The last emit CTA to finish does the fix-up when the emit kernel found
-//   coinciding vertices: it merges them by exact position, drops faces that
-//   became degenerate and compacts vertices and faces, keeping their order.
+//   5. mc_fix     returns at once unless the emit found coinciding vertices; then
+//                 merges them by exact position, drops faces that became
+//                 degenerate and compacts vertices and faces in place, keeping
+//                 their order.
 //
 // Equivalence with the reference (src/mc/mc.cu:17-68): the reference emits the
 // triangles of active cells in ascending cell id, drops triangles with two equal
@@ -98,26 +99,31 @@ struct McWs {
     unsigned long long* vlist;  // vertex entries [capV]: pw | axis << 32 | bit << 34 | slot << 39
     unsigned long long* clist;  // cell entries [capF]: pw | bit << 32 | case << 37 | face offset << 45
     uint32_t* foff;             // per word with faces: segment-local face offset
-    unsigned long long* ctr;    // [0] list size [1] snaps [2] barrier count [3] barrier gen [4] V' [5] F'
-                                // [6] unused [7] scan ticket [8] merges [9] small hash full
-                                // [10] cell entries [11] emit CTAs done
+    unsigned long long* ctr;    // [0] list size [1] snaps [4] V [5] F (before the fix-up) [7] scan ticket
+                                // [8] merges [9] small hash full [10] cell entries [12] fix-up ticket
+                                // [13] fix-up tiles done; the rest unused
     unsigned long long* state;  // look-back state per segment (follows ctr; zeroed with it)
     uint32_t* small;            // SMALL_HC entries after the states (zeroed with them)
     float* gc;                  // grid coordinates [nx + ny + nz] (x, then y, then z)
     uint32_t* snaps;            // snapped vertex slots [capV]
     uint32_t* table;            // position hash of snapped vertices [HC]
-    uint32_t* used;             // vertex used bits [capV / 32 + 1]
-    uint32_t* newidx;           // compacted vertex index [capV]
-    int32_t* ftmp;              // compacted faces [capF, 3]
-    float* vtmp;                // compacted vertices [capV, 3]
+    uint32_t* moved;            // fix-up: bitmap of the merged vertices [capV / 32 + 1]
+    uint32_t* newidx;           // fix-up: a merged vertex's representative, then new indices [capV]
+    unsigned long long* fstate; // fix-up: look-back states of its face tiles (region of capF * 12 bytes)
+    uint32_t* vbits;            // fix-up: two more bitmaps, then the look-back states of its vertex tiles
+                                // (region of capV * 12 bytes)
     long long nBlk;             // segments at most (SEG_MIN point words each)
     uint32_t HC;
     size_t total;
 };
 
 constexpr uint32_t SMALL_HC = 1u << 15;  // merge-detection hash of emit (entries: vertex + 1, 0 = empty)
+constexpr uint32_t SMALL_PROBES = 256;
 constexpr int NCTR = 16;
 constexpr int WPT = 4;                       // point words per count thread
+constexpr int FIX_THREADS = 512;
+constexpr int FIX_PER = 4;                   // rows per thread of a fix-up tile
+constexpr int FIX_TILE = FIX_THREADS * FIX_PER;
 constexpr uint32_t SEG_MIN = 128 * WPT;      // words per segment (one scan entry) with 128-thread count CTAs
 
 inline size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
@@ -155,10 +161,11 @@ McWs carve(int nx, int ny, int nz, long long capV, long long capF, uint8_t* base
     w.gc = reinterpret_cast<float*>(take(size_t(nx + ny + nz) * 4));
     w.snaps = reinterpret_cast<uint32_t*>(take(size_t(capV) * 4));
     w.table = reinterpret_cast<uint32_t*>(take(size_t(w.HC) * 4));
-    w.used = reinterpret_cast<uint32_t*>(take(size_t(capV / 32 + 1) * 4));
+    w.moved = reinterpret_cast<uint32_t*>(take(size_t(capV / 32 + 1) * 4));
     w.newidx = reinterpret_cast<uint32_t*>(take(size_t(capV) * 4));
-    w.ftmp = reinterpret_cast<int32_t*>(take(size_t(capF) * 12));
-    w.vtmp = reinterpret_cast<float*>(take(size_t(capV) * 12));
+    // the fix-up needs far less of these two, whose sizes are part of the workspace's
+    w.fstate = reinterpret_cast<unsigned long long*>(take(size_t(capF) * 12));
+    w.vbits = reinterpret_cast<uint32_t*>(take(size_t(capV) * 12));
     w.total = o + 256;  // room to align the base
     return w;
 }
@@ -301,8 +308,10 @@ __device__ __forceinline__ uint32_t phash(uint32_t a, uint32_t b, uint32_t c) {
     h ^= h >> 12;
     return h;
 }
+// Equal positions; q is read through L2 (another CTA of the launch may have
+// written it).
 __device__ __forceinline__ bool same_pos(const float* p, const float* q) {
-    return p[0] == q[0] && p[1] == q[1] && p[2] == q[2];
+    return p[0] == __ldcg(q) && p[1] == __ldcg(q + 1) && p[2] == __ldcg(q + 2);
 }
 
 // Position of the k-th (from 0) set bit of m; m has more than k set bits.
@@ -687,6 +696,8 @@ __global__ void __launch_bounds__(SCAN_THREADS) mc_scan(unsigned long long* blk,
                 const unsigned long long V = pv + ta, F = pf + tb;
                 counts[0] = (long long)V;
                 counts[1] = (long long)F;
+                ctr[4] = V;
+                ctr[5] = F;
                 if ((long long)V > capV || (long long)F > capF || V >= LB_MASK31 || F >= LB_MASK31)
                     atomicCAS(status, 0, int(ISO_ERR_OVERFLOW));
             }
@@ -741,7 +752,6 @@ struct EmitArgs {
     int* status;
     long long capV, capF;
     unsigned nbv;  // CTAs with the vertex role; the rest emit faces
-    McWs w;        // for the fix-up
     long long* vedge;  // optional: each vertex's grid edge
 };
 
@@ -782,19 +792,25 @@ __device__ void emit_vertices(const McGrid& g, const EmitArgs& a, unsigned bi, u
         vo[1] = py;
         vo[2] = pz;
         if (a.vedge) a.vedge[vi] = 3 * ia + ax;
-        if (!(t >= g.tau && t <= 1.0f - g.tau) || (px == xa && py == ya && pz == za) ||
-            (px == xb && py == yb && pz == zb)) {
+        // (a position with a NaN equals none)
+        if ((!(t >= g.tau && t <= 1.0f - g.tau) || (px == xa && py == ya && pz == za) ||
+             (px == xb && py == yb && pz == zb)) &&
+            px == px && py == py && pz == pz) {
             // a candidate for sharing its position: list it, and look for an
-            // equal position among the candidates so far
+            // equal position among the candidates so far.  A slot keeps the
+            // smallest vertex of its position (the fix-up's representative).
             const unsigned long long sidx = atomicAdd(ctr + 1, 1ull);
             if ((long long)sidx < capV) snaps[sidx] = vi;
             __threadfence();  // the position is visible before the hash entry
+            const float pos[3] = {px, py, pz};
             uint32_t h = phash(pbits(px), pbits(py), pbits(pz)) & (SMALL_HC - 1u);
             bool placed = false;
-            for (uint32_t probe = 0; probe < SMALL_HC; ++probe, h = (h + 1) & (SMALL_HC - 1u)) {
+            // past SMALL_PROBES the table counts as full: the fix-up builds its own
+            for (uint32_t probe = 0; probe < SMALL_PROBES; ++probe, h = (h + 1) & (SMALL_HC - 1u)) {
                 const uint32_t cur = atomicCAS(&small[h], 0u, vi + 1u);
                 if (cur == 0u) { placed = true; break; }
-                if (same_pos(vo, vout + 3ll * (cur - 1u))) {
+                if (same_pos(pos, vout + 3ll * (cur - 1u))) {
+                    atomicMin(&small[h], vi + 1u);
                     atomicAdd(ctr + 8, 1ull);
                     placed = true;
                     break;
@@ -869,157 +885,280 @@ __device__ void emit_faces(const McGrid& g, const EmitArgs& a, unsigned bi, unsi
     }
 }
 
-__device__ void fixup_block(const McWs& w, float* vout, int32_t* fout, long long* counts, int* status,
-                            long long capV, long long* vedge);
-
 template <int EMIT_THREADS>
 __global__ void __launch_bounds__(EMIT_THREADS) mc_emit(const McGrid g, const EmitArgs a) {
-    __shared__ int last;
     iso::grid_wait();
     if (a.counts[0] > a.capV || a.counts[1] > a.capF || a.counts[0] > 0x7fffffffll) return;
     if (blockIdx.x < a.nbv) emit_vertices<EMIT_THREADS>(g, a, blockIdx.x, a.nbv);
     else emit_faces<EMIT_THREADS>(g, a, blockIdx.x - a.nbv, gridDim.x - a.nbv);
-    // the last CTA to finish sees every vertex and face; it does the fix-up if
-    // the emit found coinciding positions
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(a.ctr + 11, 1ull) == gridDim.x - 1;
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    if (a.ctr[1] == 0 || (a.ctr[8] == 0 && a.ctr[9] == 0)) return;
-    fixup_block(a.w, a.vout, a.fout, a.counts, a.status, a.capV, a.vedge);
 }
 
 // ---------------------------------------------------------------------------
-// 4. fix-up: run by the last CTA of mc_emit to finish, and only when some vertex
-// positions coincide (found by the emit kernel's small hash).  It merges the
-// candidates by exact position (smallest index wins, as a sorted weld keeps the
-// first), drops faces that became degenerate and compacts vertices and faces,
-// keeping their order.  One CTA: these inputs are rare (values exactly at the
-// level on grid points, or grids near float resolution).
+// 5. fix-up: when some vertex positions coincide (found by the emit's small
+// hash; a value within FP32 rounding of the level at one grid point is enough,
+// and a generic field on a fine grid has a few), merges the candidates by exact
+// position (smallest index wins, as a sorted weld keeps the first), drops faces
+// that became degenerate and vertices that no face uses any more, and compacts
+// vertices and faces in place, keeping their order.
+//
+// One launch, its work cut into tiles that CTAs take by ticket, phase after
+// phase; a tile waits (bounded) until the tiles of the phases before its own
+// are done, so it only ever waits on tickets that running CTAs hold, and the
+// launch needs no co-residency:
+//   0  clear the bitmaps and look-back states (and the position table)
+//   1  (small hash full) candidates into the position table
+//   2  each candidate's representative; `moved` bits of those that have another
+//   3  faces: representatives for vertices, degenerate ones dropped (their
+//      vertices become `suspect`: only those can be left without a face), the
+//      rest compacted in place (look-back over tiles)
+//   4  kept faces mark the suspects that they use
+//   5  vertices: those neither moved nor left without a face, compacted in
+//      place (look-back); their new indices
+//   6  faces take the new indices
+// Compaction in place: a tile's rows move to indices no higher than their own,
+// and it writes only after every tile before it has published its count, for
+// which that tile has read its rows.
+// It is bound by latency (six dependent phases of L2 traffic, about 100 MB for
+// 1.6 M faces).  The fix-up by one CTA that it replaces was a serial chain of a
+// block scan per 256 rows: 29.5 ms for a 512^3 sphere's 0.8 M vertices.
 
-__device__ __forceinline__ bool face_keep(const int32_t* f) {
-    return f[0] != f[1] && f[0] != f[2] && f[1] != f[2];
-}
+struct FixArgs {
+    McWs w;
+    float* vout;
+    int32_t* fout;
+    long long* vedge;
+    long long* counts;
+    int* status;
+    long long capV, capF;
+};
 
-// Exclusive block scan of one count; total in `total`.
-__device__ __forceinline__ uint32_t block_excl(uint32_t x, uint32_t& total, uint32_t* sm) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    uint32_t inc = x;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const uint32_t u = __shfl_up_sync(~0u, inc, d);
-        if (lane >= d) inc += u;
-    }
-    if (lane == 31) sm[warp] = inc;
-    __syncthreads();
-    if (warp == 0) {
-        uint32_t y = lane < nwarps ? sm[lane] : 0u;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t u = __shfl_up_sync(~0u, y, d);
-            if (lane >= d) y += u;
-        }
-        sm[lane] = y;
-    }
-    __syncthreads();
-    const uint32_t ex = (warp ? sm[warp - 1] : 0u) + inc - x;
-    total = sm[31];
-    __syncthreads();
-    return ex;
-}
+__device__ __forceinline__ bool bit_of(const uint32_t* bits, uint32_t i) { return (bits[i >> 5] >> (i & 31u)) & 1u; }
+__device__ __forceinline__ void set_bit(uint32_t* bits, uint32_t i) { atomicOr(&bits[i >> 5], 1u << (i & 31u)); }
 
-// Smallest index of a snapped vertex at vertex v's position, or v.
-__device__ uint32_t rep_of(const McWs& w, const float* vout, uint32_t v) {
-    const float* p = vout + 3ll * v;
-    const uint32_t mask = w.HC - 1;
+// Smallest candidate at vertex v's position, or v.
+__device__ __forceinline__ uint32_t fix_rep(const McWs& w, const float* vout, uint32_t v, bool big) {
+    const float p[3] = {__ldcg(vout + 3ll * v), __ldcg(vout + 3ll * v + 1), __ldcg(vout + 3ll * v + 2)};
+    const uint32_t mask = big ? w.HC - 1u : SMALL_HC - 1u;
     uint32_t h = phash(pbits(p[0]), pbits(p[1]), pbits(p[2])) & mask;
     for (uint32_t probe = 0; probe <= mask; ++probe, h = (h + 1) & mask) {
-        const uint32_t j = w.table[h];
+        const uint32_t j = big ? __ldcg(w.table + h) : __ldcg(w.small + h) - 1u;
         if (j == 0xffffffffu) break;
         if (same_pos(p, vout + 3ll * j)) return j;
     }
     return v;
 }
 
-__device__ void fixup_block(const McWs& w, float* vout, int32_t* fout, long long* counts, int* status,
-                            long long capV, long long* vedge) {
-    __shared__ uint32_t sm[32];
-    const long long V = counts[0], F = counts[1];
-    const long long nsnap = min((long long)w.ctr[1], capV);
-    const uint32_t mask = w.HC - 1;
-    const int T = blockDim.x, tid = threadIdx.x;
-    for (long long i = tid; i < w.HC; i += T) w.table[i] = 0xffffffffu;
-    for (long long i = tid; i < V / 32 + 1; i += T) w.used[i] = 0u;
+// Candidate v into the position table; the smallest index wins.
+__device__ __forceinline__ void fix_insert(const McWs& w, const float* vout, uint32_t v, int* status) {
+    const float p[3] = {__ldcg(vout + 3ll * v), __ldcg(vout + 3ll * v + 1), __ldcg(vout + 3ll * v + 2)};
+    const uint32_t mask = w.HC - 1u;
+    uint32_t h = phash(pbits(p[0]), pbits(p[1]), pbits(p[2])) & mask;
+    for (uint32_t probe = 0; probe <= mask; ++probe, h = (h + 1) & mask) {
+        const uint32_t cur = atomicCAS(&w.table[h], 0xffffffffu, v);
+        if (cur == 0xffffffffu) return;
+        if (same_pos(p, vout + 3ll * cur)) {
+            atomicMin(&w.table[h], v);
+            return;
+        }
+    }
+    atomicCAS(status, 0, int(ISO_ERR_OVERFLOW));
+}
+
+// Ordered compaction of a tile's kept rows (row k * FIX_THREADS + tid of the tile
+// for k < FIX_PER): to[k] <- the row's index among all kept rows.  Call with
+// every row read: the tile's count is published here.
+__device__ __forceinline__ void fix_place(const bool* keep, unsigned long long* state, uint32_t tile, int* status,
+                                          uint32_t (*wcnt)[FIX_THREADS / 32], unsigned long long* pre_s,
+                                          unsigned long long* to) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t bal[FIX_PER];
+#pragma unroll
+    for (int k = 0; k < FIX_PER; ++k) {
+        bal[k] = __ballot_sync(~0u, keep[k]);
+        if (lane == 0) wcnt[k][warp] = __popc(bal[k]);
+    }
     __syncthreads();
-    // candidates into the position hash; the smallest index wins
-    for (long long s = tid; s < nsnap; s += T) {
-        const uint32_t v = w.snaps[s];
-        const float* p = vout + 3ll * v;
-        uint32_t h = phash(pbits(p[0]), pbits(p[1]), pbits(p[2])) & mask;
-        bool done = false;
-        for (uint32_t probe = 0; probe <= mask && !done; ++probe, h = (h + 1) & mask) {
-            const uint32_t cur = atomicCAS(&w.table[h], 0xffffffffu, v);
-            if (cur == 0xffffffffu) { done = true; break; }
-            if (same_pos(p, vout + 3ll * cur)) {
-                atomicMin(&w.table[h], v);
-                done = true;
+    uint32_t before[FIX_PER], run = 0;
+#pragma unroll
+    for (int k = 0; k < FIX_PER; ++k) {
+        uint32_t mine = 0;
+        for (int q = 0; q < FIX_THREADS / 32; ++q) {
+            if (q == warp) mine = run;
+            run += wcnt[k][q];
+        }
+        before[k] = mine + __popc(bal[k] & ((1u << lane) - 1u));
+    }
+    if (warp == 0) {
+        unsigned long long e = 0, unused = 0;
+        __threadfence();  // the tile's reads come before its count
+        lb_tile(state, tile, run, 0, e, unused, status);
+        __threadfence();
+        if (lane == 0) *pre_s = e;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < FIX_PER; ++k) to[k] = *pre_s + before[k];
+}
+
+__global__ void __launch_bounds__(FIX_THREADS) mc_fix(const FixArgs a) {
+    __shared__ uint32_t wcnt[FIX_PER][FIX_THREADS / 32];
+    __shared__ unsigned long long pre_s, ticket_s;
+    __shared__ int ok_s;
+    iso::grid_wait();
+    const McWs& w = a.w;
+    unsigned long long* ctr = w.ctr;
+    const unsigned long long nsnap = min(ctr[1], (unsigned long long)a.capV);
+    if (nsnap == 0 || (ctr[8] == 0 && ctr[9] == 0)) return;
+    const bool big = ctr[9] != 0;
+    const uint32_t V = uint32_t(ctr[4]), F = uint32_t(ctr[5]);
+    const int tid = threadIdx.x;
+    const uint32_t nb = V / 32 + 1;
+    uint32_t *moved = w.moved, *suspect = w.vbits, *used = w.vbits + nb;
+    const uint32_t ntF = (F + FIX_TILE - 1) / FIX_TILE, ntV = (V + FIX_TILE - 1) / FIX_TILE;
+    const uint32_t ntS = uint32_t((nsnap + FIX_TILE - 1) / FIX_TILE);
+    unsigned long long *fst = w.fstate, *vst = reinterpret_cast<unsigned long long*>(w.vbits + 2 * (size_t)nb);
+    constexpr uint32_t CLEAR = 16 * FIX_TILE;  // words per tile of phase 0
+    const uint32_t nv = 2 * nb + 2 * ntV;  // words of vbits in use
+    const unsigned long long nclear = (unsigned long long)nb + nv + 2 * ntF + (big ? w.HC : 0u);
+    // first ticket of each phase
+    unsigned long long s[8];
+    s[0] = 0;
+    s[1] = s[0] + (nclear + CLEAR - 1) / CLEAR;
+    s[2] = s[1] + (big ? ntS : 0u);
+    s[3] = s[2] + ntS;
+    s[4] = s[3] + ntF;
+    s[5] = s[4] + ntF;
+    s[6] = s[5] + ntV;
+    s[7] = s[6] + (ntF ? ntF : 1u);
+    for (;;) {
+        if (tid == 0) {
+            const unsigned long long t = atomicAdd(ctr + 12, 1ull);
+            ticket_s = t;
+            ok_s = 1;
+            if (t < s[7]) {
+                unsigned long long need = 0;  // tiles of the phases before this ticket's
+#pragma unroll
+                for (int p = 1; p < 7; ++p)
+                    if (t >= s[p]) need = s[p];
+                uint32_t spins = 0;
+                while (*(volatile unsigned long long*)(ctr + 13) < need) {
+                    if (++spins > ISO_SPIN_LIMIT) {
+                        atomicCAS(a.status, 0, int(ISO_ERR_TIMEOUT));
+                        ok_s = 0;
+                        break;
+                    }
+                    __nanosleep(20);
+                }
+                __threadfence();
             }
         }
-        if (!done) atomicCAS(status, 0, int(ISO_ERR_OVERFLOW));
-    }
-    __syncthreads();
-    // faces: merge, keep the non-degenerate ones in order, mark their vertices
-    uint32_t fn = 0;
-    for (long long base = 0; base < F; base += T) {
-        const long long f = base + tid;
-        uint32_t keep = 0;
-        int32_t v3[3] = {0, 0, 0};
-        if (f < F) {
-#pragma unroll
-            for (int k = 0; k < 3; ++k) v3[k] = int32_t(rep_of(w, vout, uint32_t(fout[3 * f + k])));
-            keep = face_keep(v3);
-        }
-        uint32_t tot;
-        const uint32_t ex = block_excl(keep, tot, sm);
-        if (keep) {
-            int32_t* o = w.ftmp + 3ll * (fn + ex);
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                o[k] = v3[k];
-                atomicOr(&w.used[uint32_t(v3[k]) >> 5], 1u << (uint32_t(v3[k]) & 31u));
+        __syncthreads();
+        const unsigned long long t = ticket_s;
+        if (t >= s[7] || !ok_s) return;
+        if (t < s[1]) {
+            for (unsigned long long i = t * CLEAR + tid; i < min(nclear, (t + 1) * CLEAR); i += FIX_THREADS) {
+                unsigned long long j = i;
+                if (j < nb) { moved[j] = 0u; continue; }
+                j -= nb;
+                if (j < nv) { w.vbits[j] = 0u; continue; }
+                j -= nv;
+                if (j < 2 * ntF) reinterpret_cast<uint32_t*>(fst)[j] = 0u;
+                else w.table[j - 2 * ntF] = 0xffffffffu;
             }
+        } else if (t < s[3]) {
+            const bool insert = t < s[2];
+            const unsigned long long b0 = (t - (insert ? s[1] : s[2])) * FIX_TILE;
+            for (unsigned long long i = b0 + tid; i < min(nsnap, b0 + FIX_TILE); i += FIX_THREADS) {
+                const uint32_t v = w.snaps[i];
+                if (insert) {
+                    fix_insert(w, a.vout, v, a.status);
+                } else {
+                    const uint32_t r = fix_rep(w, a.vout, v, big);
+                    if (r != v) {
+                        w.newidx[v] = r;
+                        set_bit(moved, v);
+                    }
+                }
+            }
+        } else if (t < s[4]) {
+            const uint32_t tile = uint32_t(t - s[3]);
+            int32_t v3[FIX_PER][3];
+            bool keep[FIX_PER];
+#pragma unroll
+            for (int k = 0; k < FIX_PER; ++k) {
+                const uint32_t f = tile * FIX_TILE + k * FIX_THREADS + tid;
+#pragma unroll
+                for (int q = 0; q < 3; ++q) v3[k][q] = f < F ? __ldcg(a.fout + 3ull * f + q) : 0;
+            }
+#pragma unroll
+            for (int k = 0; k < FIX_PER; ++k) {
+                const uint32_t f = tile * FIX_TILE + k * FIX_THREADS + tid;
+                keep[k] = false;
+                if (f >= F) continue;
+#pragma unroll
+                for (int q = 0; q < 3; ++q)
+                    if (bit_of(moved, uint32_t(v3[k][q]))) v3[k][q] = int32_t(__ldcg(w.newidx + v3[k][q]));
+                keep[k] = v3[k][0] != v3[k][1] && v3[k][0] != v3[k][2] && v3[k][1] != v3[k][2];
+                if (!keep[k]) {
+#pragma unroll
+                    for (int q = 0; q < 3; ++q) set_bit(suspect, uint32_t(v3[k][q]));
+                }
+            }
+            unsigned long long to[FIX_PER];
+            fix_place(keep, fst, tile, a.status, wcnt, &pre_s, to);
+#pragma unroll
+            for (int k = 0; k < FIX_PER; ++k)
+                if (keep[k]) {
+                    int32_t* o = a.fout + 3 * to[k];
+                    o[0] = v3[k][0]; o[1] = v3[k][1]; o[2] = v3[k][2];
+                }
+        } else if (t < s[5] || t >= s[6]) {
+            const bool mark = t < s[5];
+            const uint32_t Fk = ntF ? uint32_t((__ldcg(fst + ntF - 1) >> 31) & LB_MASK31) : 0u;  // faces kept
+            const unsigned long long b0 = 3ull * FIX_TILE * (t - (mark ? s[4] : s[6]));
+#pragma unroll 4
+            for (int k = 0; k < 3 * FIX_PER; ++k) {
+                const unsigned long long i = b0 + k * FIX_THREADS + tid;
+                if (i >= 3ull * Fk) continue;
+                const uint32_t v = uint32_t(__ldcg(a.fout + i));
+                if (!mark) a.fout[i] = int32_t(__ldcg(w.newidx + v));
+                else if (bit_of(suspect, v) && !bit_of(used, v)) set_bit(used, v);
+            }
+            if (t == s[6] && tid == 0) {
+                a.counts[0] = ntV ? (long long)((__ldcg(vst + ntV - 1) >> 31) & LB_MASK31) : 0;
+                a.counts[1] = Fk;
+            }
+        } else {
+            const uint32_t tile = uint32_t(t - s[5]);
+            float p[FIX_PER][3];
+            long long e[FIX_PER];
+            bool keep[FIX_PER];
+#pragma unroll
+            for (int k = 0; k < FIX_PER; ++k) {
+                const uint32_t v = tile * FIX_TILE + k * FIX_THREADS + tid;
+                keep[k] = v < V && F && !bit_of(moved, v) && !(bit_of(suspect, v) && !bit_of(used, v));
+                e[k] = 0;
+                if (!keep[k]) continue;
+#pragma unroll
+                for (int q = 0; q < 3; ++q) p[k][q] = __ldcg(a.vout + 3ull * v + q);
+                if (a.vedge) e[k] = __ldcg(a.vedge + v);
+            }
+            unsigned long long to[FIX_PER];
+            fix_place(keep, vst, tile, a.status, wcnt, &pre_s, to);
+#pragma unroll
+            for (int k = 0; k < FIX_PER; ++k)
+                if (keep[k]) {
+                    w.newidx[tile * FIX_TILE + k * FIX_THREADS + tid] = uint32_t(to[k]);
+                    float* o = a.vout + 3 * to[k];
+                    o[0] = p[k][0]; o[1] = p[k][1]; o[2] = p[k][2];
+                    if (a.vedge) a.vedge[to[k]] = e[k];
+                }
         }
-        fn += tot;
-    }
-    __syncthreads();
-    // vertices still used, in order
-    uint32_t vn = 0;
-    for (long long base = 0; base < V; base += T) {
-        const long long v = base + tid;
-        const uint32_t u = v < V ? (w.used[v >> 5] >> (v & 31)) & 1u : 0u;
-        // edges move in place: every read of this window precedes the scan's
-        // barriers, and a vertex never moves to a higher index
-        const long long ev = (u && vedge) ? vedge[v] : 0;
-        uint32_t tot;
-        const uint32_t ex = block_excl(u, tot, sm);
-        if (u) {
-            const uint32_t j = vn + ex;
-            if (vedge) vedge[j] = ev;
-            w.newidx[v] = j;
-            w.vtmp[3ll * j] = vout[3 * v];
-            w.vtmp[3ll * j + 1] = vout[3 * v + 1];
-            w.vtmp[3ll * j + 2] = vout[3 * v + 2];
+        __syncthreads();
+        if (tid == 0) {
+            __threadfence();
+            atomicAdd(ctr + 13, 1ull);
         }
-        vn += tot;
-    }
-    __syncthreads();
-    for (long long j = tid; j < 3ll * vn; j += T) vout[j] = w.vtmp[j];
-    for (long long j = tid; j < 3ll * fn; j += T) fout[j] = int32_t(w.newidx[w.ftmp[j]]);
-    if (tid == 0) {
-        counts[0] = vn;
-        counts[1] = fn;
     }
 }
 
@@ -1089,10 +1228,17 @@ int launch_emit(const McParams& p, const McGrid& g, const McWs& w, cudaStream_t 
     const long long nbv = std::max<long long>(1, std::min(want(p.capV), resident / 3));
     const long long nbf = std::max<long long>(1, std::min(want(p.capF), resident - nbv));
     EmitArgs a{p.vals, w.S, w.info, w.blk, w.foff, w.vlist, w.clist, w.ctr, w.snaps, w.small,
-               p.vout, p.fout, p.counts, p.status, p.capV, p.capF, unsigned(nbv), w, p.vedge};
+               p.vout, p.fout, p.counts, p.status, p.capV, p.capF, unsigned(nbv), p.vedge};
     {
         iso::ProfScope ps("mc_emit", st);
         iso::launch_pdl(mc_emit<EMIT_THREADS>, unsigned(nbv + nbf), EMIT_THREADS, st, g, a);
+        if (cudaGetLastError() != cudaSuccess) return iso::fail_code(ISO_ERR_CUDA);
+    }
+    {
+        iso::ProfScope ps("mc_fix", st);
+        const FixArgs f{w, p.vout, p.fout, p.vedge, p.counts, p.status, p.capV, p.capF};
+        const long long tiles = std::max<long long>(1, (std::max(p.capV, p.capF) + FIX_TILE - 1) / FIX_TILE);
+        iso::launch_pdl(mc_fix, unsigned(std::min<long long>(tiles, sms)), unsigned(FIX_THREADS), st, f);
         if (cudaGetLastError() != cudaSuccess) return iso::fail_code(ISO_ERR_CUDA);
     }
     return 0;

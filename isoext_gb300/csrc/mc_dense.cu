@@ -122,6 +122,7 @@ constexpr uint32_t SMALL_PROBES = 256;
 constexpr int NCTR = 16;
 constexpr int WPT = 4;                       // point words per count thread
 constexpr int FIX_THREADS = 512;
+constexpr int FIX_CTAS = 3;                  // resident fix-up CTAs per SM
 constexpr int FIX_PER = 4;                   // rows per thread of a fix-up tile
 constexpr int FIX_TILE = FIX_THREADS * FIX_PER;
 constexpr uint32_t SEG_MIN = 128 * WPT;      // words per segment (one scan entry) with 128-thread count CTAs
@@ -752,6 +753,7 @@ struct EmitArgs {
     int* status;
     long long capV, capF;
     unsigned nbv;  // CTAs with the vertex role; the rest emit faces
+    McWs w;        // what the fix-up needs cleared
     long long* vedge;  // optional: each vertex's grid edge
 };
 
@@ -885,10 +887,37 @@ __device__ void emit_faces(const McGrid& g, const EmitArgs& a, unsigned bi, unsi
     }
 }
 
+// What the fix-up of V vertices and F faces keeps in the workspace.
+struct FixLayout {
+    uint32_t nb;        // words of a bitmap over the vertices
+    uint32_t ntF, ntV;  // tiles of faces and of vertices
+    uint32_t *moved, *suspect, *used;
+    unsigned long long *fst, *vst;  // look-back states of the face and vertex tiles
+    __device__ __forceinline__ FixLayout(const McWs& w, uint32_t V, uint32_t F) {
+        nb = V / 32 + 1;
+        ntF = (F + FIX_TILE - 1) / FIX_TILE;
+        ntV = (V + FIX_TILE - 1) / FIX_TILE;
+        moved = w.moved;
+        suspect = w.vbits;
+        used = w.vbits + nb;
+        fst = w.fstate;
+        vst = reinterpret_cast<unsigned long long*>(w.vbits + 2 * (size_t)nb);
+    }
+    __device__ __forceinline__ uint32_t vwords() const { return 2 * nb + 2 * ntV; }  // suspect, used, vst
+};
+
 template <int EMIT_THREADS>
 __global__ void __launch_bounds__(EMIT_THREADS) mc_emit(const McGrid g, const EmitArgs a) {
     iso::grid_wait();
     if (a.counts[0] > a.capV || a.counts[1] > a.capF || a.counts[0] > 0x7fffffffll) return;
+    // the fix-up's bitmaps and look-back states (half a byte per vertex)
+    {
+        const FixLayout l(a.w, uint32_t(a.counts[0]), uint32_t(a.counts[1]));
+        const uint32_t step = gridDim.x * EMIT_THREADS, i0 = blockIdx.x * EMIT_THREADS + threadIdx.x;
+        for (uint32_t i = i0; i < l.nb; i += step) l.moved[i] = 0u;
+        for (uint32_t i = i0; i < l.vwords(); i += step) l.suspect[i] = 0u;
+        for (uint32_t i = i0; i < l.ntF; i += step) l.fst[i] = 0ull;
+    }
     if (blockIdx.x < a.nbv) emit_vertices<EMIT_THREADS>(g, a, blockIdx.x, a.nbv);
     else emit_faces<EMIT_THREADS>(g, a, blockIdx.x - a.nbv, gridDim.x - a.nbv);
 }
@@ -905,8 +934,7 @@ __global__ void __launch_bounds__(EMIT_THREADS) mc_emit(const McGrid g, const Em
 // phase; a tile waits (bounded) until the tiles of the phases before its own
 // are done, so it only ever waits on tickets that running CTAs hold, and the
 // launch needs no co-residency:
-//   0  clear the bitmaps and look-back states (and the position table)
-//   1  (small hash full) candidates into the position table
+//   0, 1  (small hash full) clear the position table; candidates into it
 //   2  each candidate's representative; `moved` bits of those that have another
 //   3  faces: representatives for vertices, degenerate ones dropped (their
 //      vertices become `suspect`: only those can be left without a face), the
@@ -918,9 +946,13 @@ __global__ void __launch_bounds__(EMIT_THREADS) mc_emit(const McGrid g, const Em
 // Compaction in place: a tile's rows move to indices no higher than their own,
 // and it writes only after every tile before it has published its count, for
 // which that tile has read its rows.
-// It is bound by latency (six dependent phases of L2 traffic, about 100 MB for
-// 1.6 M faces).  The fix-up by one CTA that it replaces was a serial chain of a
-// block scan per 256 rows: 29.5 ms for a 512^3 sphere's 0.8 M vertices.
+// It is bound by latency: five dependent phases of L2 traffic, a few us each
+// however small the mesh, about 100 MB for 1.6 M faces.  The fix-up by one CTA
+// that it replaces was a serial chain of a block scan per 256 rows: 29.5 ms for
+// a 512^3 sphere's 0.8 M vertices, against 61 us, and 3.4 ms against 31 us for
+// 0.1 M.  Three CTAs per SM (one: 149 us, two: 85 us at the time), tickets taken
+// ahead, and the emit clearing the bitmaps instead of a phase of their own
+// (76 -> 61 us) gave the last factor of two.
 
 struct FixArgs {
     McWs w;
@@ -1000,9 +1032,9 @@ __device__ __forceinline__ void fix_place(const bool* keep, unsigned long long* 
     for (int k = 0; k < FIX_PER; ++k) to[k] = *pre_s + before[k];
 }
 
-__global__ void __launch_bounds__(FIX_THREADS) mc_fix(const FixArgs a) {
+__global__ void __launch_bounds__(FIX_THREADS, FIX_CTAS) mc_fix(const FixArgs a) {
     __shared__ uint32_t wcnt[FIX_PER][FIX_THREADS / 32];
-    __shared__ unsigned long long pre_s, ticket_s;
+    __shared__ unsigned long long pre_s, ticket_s[2];
     __shared__ int ok_s;
     iso::grid_wait();
     const McWs& w = a.w;
@@ -1012,14 +1044,12 @@ __global__ void __launch_bounds__(FIX_THREADS) mc_fix(const FixArgs a) {
     const bool big = ctr[9] != 0;
     const uint32_t V = uint32_t(ctr[4]), F = uint32_t(ctr[5]);
     const int tid = threadIdx.x;
-    const uint32_t nb = V / 32 + 1;
-    uint32_t *moved = w.moved, *suspect = w.vbits, *used = w.vbits + nb;
-    const uint32_t ntF = (F + FIX_TILE - 1) / FIX_TILE, ntV = (V + FIX_TILE - 1) / FIX_TILE;
-    const uint32_t ntS = uint32_t((nsnap + FIX_TILE - 1) / FIX_TILE);
-    unsigned long long *fst = w.fstate, *vst = reinterpret_cast<unsigned long long*>(w.vbits + 2 * (size_t)nb);
+    const FixLayout l(w, V, F);  // cleared by the emit
+    uint32_t *moved = l.moved, *suspect = l.suspect, *used = l.used;
+    unsigned long long *fst = l.fst, *vst = l.vst;
+    const uint32_t ntF = l.ntF, ntV = l.ntV, ntS = uint32_t((nsnap + FIX_TILE - 1) / FIX_TILE);
     constexpr uint32_t CLEAR = 16 * FIX_TILE;  // words per tile of phase 0
-    const uint32_t nv = 2 * nb + 2 * ntV;  // words of vbits in use
-    const unsigned long long nclear = (unsigned long long)nb + nv + 2 * ntF + (big ? w.HC : 0u);
+    const unsigned long long nclear = big ? w.HC : 0u;
     // first ticket of each phase
     unsigned long long s[8];
     s[0] = 0;
@@ -1030,41 +1060,40 @@ __global__ void __launch_bounds__(FIX_THREADS) mc_fix(const FixArgs a) {
     s[5] = s[4] + ntF;
     s[6] = s[5] + ntV;
     s[7] = s[6] + (ntF ? ntF : 1u);
-    for (;;) {
-        if (tid == 0) {
-            const unsigned long long t = atomicAdd(ctr + 12, 1ull);
-            ticket_s = t;
-            ok_s = 1;
-            if (t < s[7]) {
-                unsigned long long need = 0;  // tiles of the phases before this ticket's
+    // a CTA takes its next ticket while it works on one, and reports a tile done
+    // while it goes on to the next: both atomics are off its critical path
+    if (tid == 0) ticket_s[0] = atomicAdd(ctr + 12, 1ull);
+    __syncthreads();
+    unsigned long long t = ticket_s[0], met = 0;  // tiles known to be done
+    for (int buf = 1;; buf ^= 1) {
+        if (t >= s[7]) return;
+        unsigned long long need = 0;  // tiles of the phases before this ticket's
 #pragma unroll
-                for (int p = 1; p < 7; ++p)
-                    if (t >= s[p]) need = s[p];
+        for (int p = 1; p < 7; ++p)
+            if (t >= s[p]) need = s[p];
+        if (need > met) {
+            met = need;
+            if (tid == 0) {
+                int ok = 1;
                 uint32_t spins = 0;
                 while (*(volatile unsigned long long*)(ctr + 13) < need) {
                     if (++spins > ISO_SPIN_LIMIT) {
                         atomicCAS(a.status, 0, int(ISO_ERR_TIMEOUT));
-                        ok_s = 0;
+                        ok = 0;
                         break;
                     }
                     __nanosleep(20);
                 }
                 __threadfence();
+                ok_s = ok;
             }
+            __syncthreads();
+            if (!ok_s) return;
         }
-        __syncthreads();
-        const unsigned long long t = ticket_s;
-        if (t >= s[7] || !ok_s) return;
+        if (tid == 0) ticket_s[buf] = atomicAdd(ctr + 12, 1ull);
         if (t < s[1]) {
-            for (unsigned long long i = t * CLEAR + tid; i < min(nclear, (t + 1) * CLEAR); i += FIX_THREADS) {
-                unsigned long long j = i;
-                if (j < nb) { moved[j] = 0u; continue; }
-                j -= nb;
-                if (j < nv) { w.vbits[j] = 0u; continue; }
-                j -= nv;
-                if (j < 2 * ntF) reinterpret_cast<uint32_t*>(fst)[j] = 0u;
-                else w.table[j - 2 * ntF] = 0xffffffffu;
-            }
+            for (unsigned long long i = t * CLEAR + tid; i < min(nclear, (t + 1) * CLEAR); i += FIX_THREADS)
+                w.table[i] = 0xffffffffu;
         } else if (t < s[3]) {
             const bool insert = t < s[2];
             const unsigned long long b0 = (t - (insert ? s[1] : s[2])) * FIX_TILE;
@@ -1116,13 +1145,25 @@ __global__ void __launch_bounds__(FIX_THREADS) mc_fix(const FixArgs a) {
             const bool mark = t < s[5];
             const uint32_t Fk = ntF ? uint32_t((__ldcg(fst + ntF - 1) >> 31) & LB_MASK31) : 0u;  // faces kept
             const unsigned long long b0 = 3ull * FIX_TILE * (t - (mark ? s[4] : s[6]));
-#pragma unroll 4
+            uint32_t v[3 * FIX_PER];
+#pragma unroll
             for (int k = 0; k < 3 * FIX_PER; ++k) {
                 const unsigned long long i = b0 + k * FIX_THREADS + tid;
-                if (i >= 3ull * Fk) continue;
-                const uint32_t v = uint32_t(__ldcg(a.fout + i));
-                if (!mark) a.fout[i] = int32_t(__ldcg(w.newidx + v));
-                else if (bit_of(suspect, v) && !bit_of(used, v)) set_bit(used, v);
+                v[k] = i < 3ull * Fk ? uint32_t(__ldcg(a.fout + i)) : 0u;
+            }
+            if (mark) {
+#pragma unroll
+                for (int k = 0; k < 3 * FIX_PER; ++k)
+                    if (b0 + k * FIX_THREADS + tid < 3ull * Fk && bit_of(suspect, v[k]) && !bit_of(used, v[k]))
+                        set_bit(used, v[k]);
+            } else {
+#pragma unroll
+                for (int k = 0; k < 3 * FIX_PER; ++k) v[k] = __ldcg(w.newidx + v[k]);
+#pragma unroll
+                for (int k = 0; k < 3 * FIX_PER; ++k) {
+                    const unsigned long long i = b0 + k * FIX_THREADS + tid;
+                    if (i < 3ull * Fk) a.fout[i] = int32_t(v[k]);
+                }
             }
             if (t == s[6] && tid == 0) {
                 a.counts[0] = ntV ? (long long)((__ldcg(vst + ntV - 1) >> 31) & LB_MASK31) : 0;
@@ -1159,6 +1200,7 @@ __global__ void __launch_bounds__(FIX_THREADS) mc_fix(const FixArgs a) {
             __threadfence();
             atomicAdd(ctr + 13, 1ull);
         }
+        t = ticket_s[buf];
     }
 }
 
@@ -1228,7 +1270,7 @@ int launch_emit(const McParams& p, const McGrid& g, const McWs& w, cudaStream_t 
     const long long nbv = std::max<long long>(1, std::min(want(p.capV), resident / 3));
     const long long nbf = std::max<long long>(1, std::min(want(p.capF), resident - nbv));
     EmitArgs a{p.vals, w.S, w.info, w.blk, w.foff, w.vlist, w.clist, w.ctr, w.snaps, w.small,
-               p.vout, p.fout, p.counts, p.status, p.capV, p.capF, unsigned(nbv), p.vedge};
+               p.vout, p.fout, p.counts, p.status, p.capV, p.capF, unsigned(nbv), w, p.vedge};
     {
         iso::ProfScope ps("mc_emit", st);
         iso::launch_pdl(mc_emit<EMIT_THREADS>, unsigned(nbv + nbf), EMIT_THREADS, st, g, a);
@@ -1238,7 +1280,7 @@ int launch_emit(const McParams& p, const McGrid& g, const McWs& w, cudaStream_t 
         iso::ProfScope ps("mc_fix", st);
         const FixArgs f{w, p.vout, p.fout, p.vedge, p.counts, p.status, p.capV, p.capF};
         const long long tiles = std::max<long long>(1, (std::max(p.capV, p.capF) + FIX_TILE - 1) / FIX_TILE);
-        iso::launch_pdl(mc_fix, unsigned(std::min<long long>(tiles, sms)), unsigned(FIX_THREADS), st, f);
+        iso::launch_pdl(mc_fix, unsigned(std::min<long long>(tiles, (long long)sms * FIX_CTAS)), unsigned(FIX_THREADS), st, f);
         if (cudaGetLastError() != cudaSuccess) return iso::fail_code(ISO_ERR_CUDA);
     }
     return 0;

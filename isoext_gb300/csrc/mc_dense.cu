@@ -4,20 +4,18 @@
 //   1. mc_signs   streams the grid once (one warp per row, 16 coalesced
 //                 128-byte loads in flight per warp) into a sign bitmap,
 //                 1 bit per point.  This is the only pass over all values.
-//   2. mc_count   one CTA per segment of 1024 point words, from the bitmap alone
-//                 (16.8 MB at 512^3): crossed-edge masks along x, y and z, active
-//                 cells (their triangle counts spread over the lanes of a warp);
-//                 segment-local vertex offsets per word; words with vertices or
-//                 faces are appended to a list (one atomic per warp).  Words
-//                 wholly inside or outside take an early exit.
-//   3. mc_scan    segment (V, F) sums to offsets: CTAs over chunks of 4096
+//   2. mc_count   one CTA per segment of 256 to 1024 point words, from the bitmap
+//                 alone (16.8 MB at 512^3): the words near the surface, listed;
+//                 their crossed-edge masks, active cells and triangle counts,
+//                 bit-parallel; vertex and cell entry lists.  On grids of few
+//                 segments its last CTA scans their sums.
+//   3. mc_scan    (more segments) (V, F) sums to offsets: CTAs over chunks of 1024
 //                 segments chained by decoupled look-back; totals and the
 //                 capacity check.
-//   4. mc_emit    warp-cooperative over the listed words: each lane takes one
-//                 vertex (position at its slot; values are read only at crossed
-//                 edges), then one active cell (faces at the word's face offset,
-//                 vertex indices by rank).  Vertices that can share a position
-//                 with another edge's (t within tau of 0 or 1) go through a small
+//   4. mc_emit    one thread per vertex entry (position at its slot; values are
+//                 read only at crossed edges) and per cell entry (its faces, vertex
+//                 indices by rank).  Vertices that can share a position with
+//                 another edge's (t within tau of 0 or 1) go through a small
 //                 hash that counts exact coincidences.
 //   5. mc_fix     returns at once unless the emit found coinciding vertices; then
 //                 merges them by exact position, drops faces that became
@@ -97,9 +95,9 @@ struct McWs {
     uint32_t* info;             // per word: segment-local vertex offset | popc(ex) << 20 | popc(ey) << 26
     unsigned long long* blk;    // per segment of words: (V, F) sums, then exclusive offsets
     unsigned long long* vlist;  // vertex entries [capV]: pw | axis << 32 | bit << 34 | slot << 39
-    unsigned long long* clist;  // cell entries [capF]: pw | bit << 32 | case << 37 | face offset << 45
-    uint32_t* foff;             // per word with faces: segment-local face offset
-    unsigned long long* ctr;    // [0] list size [1] snaps [4] V [5] F (before the fix-up) [7] scan ticket
+    unsigned long long* clist;  // cell entries [capF]: pw | bit << 32 | the word's segment-local face offset << 37
+    unsigned long long* blk2;   // blk of grids cut into more than nBlk segments
+    unsigned long long* ctr;    // [0] list size [1] snaps [4] V [5] F (before the fix-up) [6] count CTAs done [7] scan ticket
                                 // [8] merges [9] small hash full [10] cell entries [12] fix-up ticket
                                 // [13] fix-up tiles done; the rest unused
     unsigned long long* state;  // look-back state per segment (follows ctr; zeroed with it)
@@ -120,12 +118,12 @@ struct McWs {
 constexpr uint32_t SMALL_HC = 1u << 15;  // merge-detection hash of emit (entries: vertex + 1, 0 = empty)
 constexpr uint32_t SMALL_PROBES = 256;
 constexpr int NCTR = 16;
-constexpr int WPT = 4;                       // point words per count thread
+constexpr int WPT_MAX = 4;                   // point words per count thread (1 on small grids)
 constexpr int FIX_THREADS = 512;
 constexpr int FIX_CTAS = 3;                  // resident fix-up CTAs per SM
 constexpr int FIX_PER = 4;                   // rows per thread of a fix-up tile
 constexpr int FIX_TILE = FIX_THREADS * FIX_PER;
-constexpr uint32_t SEG_MIN = 128 * WPT;      // words per segment (one scan entry) with 128-thread count CTAs
+constexpr uint32_t SEG_MIN = 128 * WPT_MAX;  // words per segment (one scan entry) of 128-thread count CTAs
 
 inline size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
 
@@ -155,7 +153,7 @@ McWs carve(int nx, int ny, int nz, long long capV, long long capF, uint8_t* base
     w.blk = reinterpret_cast<unsigned long long*>(take(size_t(w.nBlk + 1) * 16));
     w.vlist = reinterpret_cast<unsigned long long*>(take(size_t(capV) * 8));
     w.clist = reinterpret_cast<unsigned long long*>(take(size_t(capF) * 8));
-    w.foff = reinterpret_cast<uint32_t*>(take(size_t(PW) * 4));
+    w.blk2 = reinterpret_cast<unsigned long long*>(take(size_t(PW) * 4));
     w.ctr = reinterpret_cast<unsigned long long*>(take(zeroed_bytes(w.nBlk)));  // + states + small hash
     w.state = w.ctr ? w.ctr + NCTR : nullptr;
     w.small = w.ctr ? reinterpret_cast<uint32_t*>(w.state + w.nBlk) : nullptr;
@@ -230,19 +228,58 @@ __device__ __forceinline__ uint32_t active_cells(const Words& d, uint32_t zm) {
     return (o & ~a) & zm;
 }
 
-// Case number of the cell at bit b: corner k = 4dx + 2dy + dz.
-__device__ __forceinline__ uint32_t cell_case(const Words& d, int b) {
+// The 8 corner words of a word's cells: c[k] = corner k = 4dx + 2dy + dz.
+__device__ __forceinline__ void corner_words(const Words& d, uint32_t* c) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        c[2 * k] = d.s[k >> 1][k & 1][0];
+        c[2 * k + 1] = up1(d.s[k >> 1][k & 1][0], d.s[k >> 1][k & 1][1]);
+    }
+}
+__device__ __forceinline__ uint32_t case_at(const uint32_t* c, int b) {
     uint32_t cs = 0;
 #pragma unroll
-    for (int dx = 0; dx < 2; ++dx)
-#pragma unroll
-        for (int dy = 0; dy < 2; ++dy) {
-            const uint32_t lo = d.s[dx][dy][0];
-            const uint32_t hi = up1(lo, d.s[dx][dy][1]);
-            cs |= ((lo >> b) & 1u) << (4 * dx + 2 * dy);
-            cs |= ((hi >> b) & 1u) << (4 * dx + 2 * dy + 1);
-        }
+    for (int k = 0; k < 8; ++k) cs |= ((c[k] >> b) & 1u) << k;
     return cs;
+}
+
+// Cells whose crossed edges may form more than one loop: a face whose diagonal
+// corners pair up, or two opposite corners against the other six.  Every other
+// active cell has one polygon, so its table has (crossed edges - 2) triangles;
+// both tables hold to this (checked over all cases).
+__device__ __forceinline__ uint32_t many_loops(const uint32_t* c) {
+    uint32_t m = 0;
+    const int f[6][4] = {{0, 1, 3, 2}, {4, 5, 7, 6}, {0, 1, 5, 4}, {2, 3, 7, 6}, {0, 2, 6, 4}, {1, 3, 7, 5}};
+#pragma unroll
+    for (int q = 0; q < 6; ++q)
+        m |= ~(c[f[q][0]] ^ c[f[q][2]]) & ~(c[f[q][1]] ^ c[f[q][3]]) & (c[f[q][0]] ^ c[f[q][1]]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        uint32_t all = ~0u, any = 0u;
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (k != i && k != 7 - i) {
+                all &= c[k];
+                any |= c[k];
+            }
+        m |= (c[i] & c[7 - i] & ~any) | (~c[i] & ~c[7 - i] & all);
+    }
+    return m;
+}
+
+// Triangles of the active cells `cells` of a word, by popcounts: crossed edges
+// minus two per cell, and the table's own number where a cell may have several
+// loops.  ntri(case): the table.
+template <typename Ntri>
+__device__ __forceinline__ uint32_t word_faces(const uint32_t* c, uint32_t cells, const Ntri& ntri) {
+    uint32_t multi = many_loops(c) & cells;
+    const uint32_t one = cells & ~multi;
+    uint32_t n = 0;
+#pragma unroll
+    for (int e = 0; e < 12; ++e) n += __popc((c[iso_edge_corner(2 * e)] ^ c[iso_edge_corner(2 * e + 1)]) & one);
+    n -= 2u * __popc(one);
+    for (; multi; multi &= multi - 1) n += ntri(case_at(c, __ffs(multi) - 1));
+    return n;
 }
 
 // Block-wide exclusive scan of two counts; totals in ta, tb.
@@ -278,10 +315,9 @@ __device__ __forceinline__ void block_scan2(uint32_t a, uint32_t b, uint32_t& ea
 }
 
 // ---------------------------------------------------------------------------
-// 2. count: one CTA per segment of CNT_THREADS * WPT point words (the CTA size
-// is a launch parameter, "mc.count_threads"): per-word vertex entries,
-// per-cell entries, and the segment's (V, F) sums, which mc_scan turns into
-// offsets.
+// 2. count: one CTA per segment of T * WPT point words (T is a launch parameter,
+// "mc.count_threads"): per-word vertex offsets, vertex and cell entries, and the
+// segments' (V, F) sums turned into offsets.
 
 // Segment holding point word pw.
 __device__ __forceinline__ uint32_t seg_of(const McGrid& g, uint32_t pw) { return pw >> g.lgseg; }
@@ -292,13 +328,6 @@ __device__ __forceinline__ void word_xyw(const McGrid& g, uint32_t pw, int& x, i
     w = int(pw - row * uint32_t(g.NW));
     x = int(fdiv(row, g.dNY));
     y = int(row - uint32_t(x) * uint32_t(g.ny));
-}
-
-__device__ __forceinline__ void advance(const McGrid& g, int& x, int& y, int& w) {
-    if (++w == g.NW) {
-        w = 0;
-        if (++y == g.ny) { y = 0; ++x; }
-    }
 }
 
 __device__ __forceinline__ uint32_t pbits(float f) { return __float_as_uint(f == 0.0f ? 0.0f : f); }
@@ -315,52 +344,109 @@ __device__ __forceinline__ bool same_pos(const float* p, const float* q) {
     return p[0] == __ldcg(q) && p[1] == __ldcg(q + 1) && p[2] == __ldcg(q + 2);
 }
 
-// Position of the k-th (from 0) set bit of m; m has more than k set bits.
-__device__ __forceinline__ int nth_set(uint32_t m, int k) {
-    int base = 0;
-#pragma unroll
-    for (int s = 16; s >= 1; s >>= 1) {
-        const uint32_t low = m & ((1u << s) - 1u);
-        const int c = __popc(low);
-        if (k >= c) { k -= c; m >>= s; base += s; }
-        else m = low;
-    }
-    return base;
+// Totals of the scan: the counts, and whether they fit.
+__device__ __forceinline__ void mc_totals(unsigned long long V, unsigned long long F, unsigned long long* ctr,
+                                          long long* counts, int* status, long long capV, long long capF) {
+    counts[0] = (long long)V;
+    counts[1] = (long long)F;
+    ctr[4] = V;
+    ctr[5] = F;
+    if ((long long)V > capV || (long long)F > capF || V >= LB_MASK31 || F >= LB_MASK31)
+        atomicCAS(status, 0, int(ISO_ERR_OVERFLOW));
 }
 
-// Lane whose inclusive prefix first exceeds j (prefixes nondecreasing, j < total).
-__device__ __forceinline__ int owner_of(uint32_t incl, uint32_t j) {
-    int lo = 0;
+// Segments that the last count CTA scans by itself, per thread.  Up to 4 T
+// segments this saves the launch of mc_scan (4 us); the count's CTAs then each
+// take a fence and an atomic on one counter before they end, which costs more
+// than the launch from 2048 segments on (15 -> 22 us at 2048, 48 -> 60 us at 4096).
+constexpr int SCAN_LAST = 4;
+
+template <int T>
+__device__ void scan_segments(unsigned long long* blk, uint32_t nseg, unsigned long long* ctr, long long* counts,
+                              int* status, long long capV, long long capF, uint32_t* sm) {
+    const uint32_t per = (nseg + T - 1) / T;  // at most SCAN_LAST
+    const uint32_t s0 = threadIdx.x * per;
+    uint32_t a[SCAN_LAST], b[SCAN_LAST], sa = 0, sb = 0;
 #pragma unroll
-    for (int s = 16; s >= 1; s >>= 1) {
-        const uint32_t pv = __shfl_sync(~0u, incl, lo + s - 1);
-        if (pv <= j) lo += s;
+    for (int k = 0; k < SCAN_LAST; ++k) {
+        const bool in = k < per && s0 + k < nseg;
+        const ulonglong2 v = in ? __ldcg(reinterpret_cast<const ulonglong2*>(blk) + s0 + k) : make_ulonglong2(0, 0);
+        a[k] = uint32_t(v.x);
+        b[k] = uint32_t(v.y);
+        sa += a[k];
+        sb += b[k];
     }
-    return lo;
+    // totals beyond 32 bits: summed in 64 (the offsets then are not used)
+    unsigned long long wa = sa, wb = sb;
+#pragma unroll
+    for (int d = 16; d >= 1; d >>= 1) {
+        wa += __shfl_xor_sync(~0u, wa, d);
+        wb += __shfl_xor_sync(~0u, wb, d);
+    }
+    __shared__ unsigned long long tot[2][T / 32];
+    if ((threadIdx.x & 31) == 0) {
+        tot[0][threadIdx.x >> 5] = wa;
+        tot[1][threadIdx.x >> 5] = wb;
+    }
+    uint32_t ea, eb, ta, tb;
+    block_scan2<T>(sa, sb, ea, eb, ta, tb, sm);
+    if (threadIdx.x == 0) {
+        unsigned long long V = 0, F = 0;
+        for (int q = 0; q < T / 32; ++q) {
+            V += tot[0][q];
+            F += tot[1][q];
+        }
+        mc_totals(V, F, ctr, counts, status, capV, capF);
+    }
+#pragma unroll
+    for (int k = 0; k < SCAN_LAST; ++k) {
+        if (k < per && s0 + k < nseg)
+            reinterpret_cast<ulonglong2*>(blk)[s0 + k] = make_ulonglong2(ea, eb);
+        ea += a[k];
+        eb += b[k];
+    }
 }
 
-template <int CNT_THREADS>
-__global__ void __launch_bounds__(CNT_THREADS) mc_count(const McGrid g, const float amin0, const float amin1,
+// One CTA's segment: T threads of WPT words each.
+// First every thread tells which of its words may hold a crossing: most words
+// and their grid neighbours are all inside or all outside.  The others, a few
+// percent, are listed in order, and from there on a thread takes one of them at
+// a time: the crossed-edge masks, the active cells and the number of their
+// triangles (word_faces), all bit-parallel; a block scan of the three counts; and
+// the entries of the warp's crossed edges and active cells, laid out in order in
+// shared memory (a lane walks its word's set bits) so that they leave in
+// coalesced stores.  A cell's entry carries its word's face offset; the emit adds
+// the triangles of the cells before it in the word.
+// Bound by instruction issue near the surface and by latency elsewhere, not by
+// bytes (the bitmap is in L2).  A lane per active cell for its case and triangle
+// count, spread over the owning warp only, as before, took 48 us at 512^3 and 16 to
+// 40 at 256^3 (a warp along the surface alone with its cells); this takes 39 and
+// 14 to 19.  The same without the list of words (every lane its own four words'
+// masks, a quarter of the lanes near the surface) took 49.
+constexpr int CQ = 512;  // entries a warp lays out at a time
+
+template <int T, int WPT>
+__global__ void __launch_bounds__(T, 1280 / T) mc_count(const McGrid g, const float amin0, const float amin1,
                                                         const float amin2, const float size0, const float size1,
                                                         const float size2, const uint32_t* __restrict__ S,
-                                                        uint32_t* __restrict__ info,
-                                                        unsigned long long* __restrict__ blk,
+                                                        uint32_t* __restrict__ info, unsigned long long* blk,
                                                         unsigned long long* __restrict__ vlist,
                                                         unsigned long long* __restrict__ clist,
-                                                        uint32_t* __restrict__ foff, unsigned long long* ctr,
-                                                        float* __restrict__ gc, const uint32_t nseg,
-                                                        const long long capV, const long long capF) {
-    constexpr uint32_t SEG = CNT_THREADS * WPT;  // words of the segment
+                                                        unsigned long long* ctr, float* __restrict__ gc,
+                                                        const uint32_t nseg, const long long capV,
+                                                        const long long capF, long long* counts, int* status) {
+    constexpr uint32_t SEG = T * WPT;  // words of the segment
+    constexpr int NW = T / 32;
     __shared__ uint32_t sm[64];
-    __shared__ uint32_t nfs[SEG];  // faces of each word of the segment
-    __shared__ uint32_t wcell[CNT_THREADS / 32], wvert[CNT_THREADS / 32];
-    __shared__ unsigned long long cbase_s, vbase_s;
-    __shared__ uint32_t nt4[64];  // triangle counts of the 256 cases, 4 per word
-    __shared__ uint32_t vmask[3 * WPT][CNT_THREADS];  // x, y, z edge masks of each thread's words
-    __shared__ uint32_t rows[4][WPT + 1][CNT_THREADS];  // sign words of rows (dx, dy), words k = 0..4
+    __shared__ unsigned long long cbase_s, vbase_s, wsum[NW];
+    __shared__ uint32_t bsum[NW];
+    __shared__ uint16_t list[SEG];  // words that may hold a crossing
+    __shared__ uint32_t fofs[T];    // face offset of each thread's word
+    __shared__ uint16_t queue[NW][CQ];
+    __shared__ int last_s;
     iso::grid_wait();
     // grid coordinates (include/utils.cuh:62-80), read by the emit kernel
-    const uint32_t gid = blockIdx.x * CNT_THREADS + threadIdx.x;
+    const uint32_t gid = blockIdx.x * T + threadIdx.x;
     const uint32_t ncoord = uint32_t(g.nx + g.ny + g.nz);
     if (gid < ncoord) {
         if (gid < uint32_t(g.nx)) gc[gid] = iso::grid_coord(gid, g.nx, amin0, size0, g.fma);
@@ -371,292 +457,187 @@ __global__ void __launch_bounds__(CNT_THREADS) mc_count(const McGrid g, const fl
     if (seg >= nseg) return;  // CTAs past the segments only write coordinates
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t sxw = uint32_t(g.ny) * uint32_t(g.NW), syw = uint32_t(g.NW);
-    const bool vec = (g.NW & 3) == 0;  // rows start on 16-byte boundaries
-    const uint32_t pw0 = seg * SEG + threadIdx.x * WPT;
-#pragma unroll
-    for (int k = 0; k < WPT; ++k) nfs[threadIdx.x * WPT + k] = 0u;
-    if (threadIdx.x < 64) {
-        const uint8_t* t = ISO_NTRI + g.method * 256 + 4 * threadIdx.x;
-        nt4[threadIdx.x] = uint32_t(t[0]) | (uint32_t(t[1]) << 8) | (uint32_t(t[2]) << 16) | (uint32_t(t[3]) << 24);
-    }
-    // bitmap words pw0 .. pw0 + 3 of the rows (x, y), (x, y+1), (x+1, y), (x+1, y+1)
-    uint32_t r[2][2][WPT];
-    int x = 0, y = 0, w = 0;
-    if (pw0 < g.PW) word_xyw(g, pw0, x, y, w);
-#pragma unroll
-    for (int dx = 0; dx < 2; ++dx)
-#pragma unroll
-        for (int dy = 0; dy < 2; ++dy) {
-            const uint32_t q = pw0 + dx * sxw + dy * syw;
-            if (vec && pw0 + WPT <= g.PW && q + WPT <= g.PW) {
-                const uint4 v4 = __ldg(reinterpret_cast<const uint4*>(S + q));
-                r[dx][dy][0] = v4.x; r[dx][dy][1] = v4.y; r[dx][dy][2] = v4.z; r[dx][dy][3] = v4.w;
-            } else {
-#pragma unroll
-                for (int k = 0; k < WPT; ++k) r[dx][dy][k] = (q + k < g.PW) ? __ldg(S + q + k) : 0u;
-            }
-        }
-    // word pw0 + 4 of each row: the next lane's first word, or a load
-    uint32_t nx4[2][2];
-#pragma unroll
-    for (int dx = 0; dx < 2; ++dx)
-#pragma unroll
-        for (int dy = 0; dy < 2; ++dy) {
-            nx4[dx][dy] = __shfl_down_sync(~0u, r[dx][dy][0], 1);
-            if (lane == 31) {
-                const uint32_t q = pw0 + WPT + dx * sxw + dy * syw;
-                nx4[dx][dy] = q < g.PW ? __ldg(S + q) : 0u;
-            }
-        }
-    uint32_t nv[WPT], cxy[WPT], act[WPT];
-#pragma unroll
-    for (int k = 0; k < WPT; ++k) { nv[k] = 0; cxy[k] = 0; act[k] = 0; }
-    // Most words lie wholly inside or outside the surface: the word and its
-    // grid neighbours' words are all 0 or all ~0, and nothing crosses.  A warp
-    // whose 128 words are all like that skips the rest.
-    bool quiet_all;
+    uint32_t nbusy = 0;  // words of the segment that may hold a crossing
     {
-        // conservative: all 20 loaded words equal, and all 0 or all ~0 (words at
-        // the grid's edges may fail it and take the exact path)
-        const uint32_t u = r[0][0][0];
-        uint32_t diff = 0;
+        const bool vec = WPT == 4 && (g.NW & 3) == 0;  // rows start on 16-byte boundaries
+        const uint32_t pw0 = seg * SEG + threadIdx.x * WPT;
+        // a word is quiet when it, the words at the same place of the rows (x, y+1),
+        // (x+1, y), (x+1, y+1) and the words after these four are all 0 or all ~0
+        // (conservative: at the grid's edges the rows are not neighbours)
+        uint32_t lo[WPT], hi[WPT];  // AND and OR of the four rows' words
 #pragma unroll
-        for (int dx = 0; dx < 2; ++dx)
-#pragma unroll
-            for (int dy = 0; dy < 2; ++dy) {
-                diff |= nx4[dx][dy] ^ u;
-#pragma unroll
-                for (int k = 0; k < WPT; ++k) diff |= r[dx][dy][k] ^ u;
-            }
-        quiet_all = (u == 0u || u == ~0u) && diff == 0u;
-    }
-    const bool warp_quiet = __all_sync(~0u, quiet_all);
-    if (!warp_quiet) {
-        // the cells of these words read their corners from here
+        for (int k = 0; k < WPT; ++k) { lo[k] = ~0u; hi[k] = 0u; }
+        uint32_t nlo = ~0u, nhi = 0u;  // of the words after the thread's last
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
+            const uint32_t p = pw0 + (q >> 1) * sxw + (q & 1) * syw;
+            uint32_t v[WPT];
+            if (vec && pw0 + WPT <= g.PW && p + WPT <= g.PW) {
+                const uint4 v4 = __ldg(reinterpret_cast<const uint4*>(S + p));
+                const uint32_t t[4] = {v4.x, v4.y, v4.z, v4.w};
 #pragma unroll
-            for (int k = 0; k < WPT; ++k) rows[q][k][threadIdx.x] = r[q >> 1][q & 1][k];
-            rows[q][WPT][threadIdx.x] = nx4[q >> 1][q & 1];
+                for (int k = 0; k < WPT; ++k) v[k] = t[k];
+            } else {
+#pragma unroll
+                for (int k = 0; k < WPT; ++k) v[k] = p + k < g.PW ? __ldg(S + p + k) : 0u;
+            }
+            uint32_t nx = __shfl_down_sync(~0u, v[0], 1);
+            if (lane == 31) nx = p + WPT < g.PW ? __ldg(S + p + WPT) : 0u;
+            nlo &= nx;
+            nhi |= nx;
+#pragma unroll
+            for (int k = 0; k < WPT; ++k) { lo[k] &= v[k]; hi[k] |= v[k]; }
         }
+        uint32_t m = 0;
 #pragma unroll
         for (int k = 0; k < WPT; ++k) {
-            if (pw0 + k < g.PW) {
-                Words d;
-                d.x = x; d.y = y; d.w = w;
-                d.hasx = x < g.nx - 1;
-                d.hasy = y < g.ny - 1;
-                const bool nxt = w + 1 < g.NW;
-#pragma unroll
-                for (int dx = 0; dx < 2; ++dx)
-#pragma unroll
-                    for (int dy = 0; dy < 2; ++dy) {
-                        const bool ok = (dx == 0 || d.hasx) && (dy == 0 || d.hasy);
-                        d.s[dx][dy][0] = ok ? r[dx][dy][k] : 0u;
-                        d.s[dx][dy][1] = (ok && nxt) ? (k + 1 < WPT ? r[dx][dy][(k + 1) % WPT] : nx4[dx][dy]) : 0u;
-                    }
-                const uint32_t zm = zmask(g, w);
-                const uint32_t ex = d.hasx ? (d.s[0][0][0] ^ d.s[1][0][0]) : 0u;
-                const uint32_t ey = d.hasy ? (d.s[0][0][0] ^ d.s[0][1][0]) : 0u;
-                const uint32_t ez = ez_of(d.s[0][0][0], d.s[0][0][1], zm);
-                nv[k] = __popc(ex) + __popc(ey) + __popc(ez);
-                cxy[k] = (uint32_t(__popc(ex)) << 20) | (uint32_t(__popc(ey)) << 26);
-                act[k] = active_cells(d, zm);
-                vmask[3 * k][threadIdx.x] = ex;
-                vmask[3 * k + 1][threadIdx.x] = ey;
-                vmask[3 * k + 2][threadIdx.x] = ez;
-                advance(g, x, y, w);
-            }
+            const uint32_t l = lo[k] & (k + 1 < WPT ? lo[(k + 1) % WPT] : nlo);
+            const uint32_t h = hi[k] | (k + 1 < WPT ? hi[(k + 1) % WPT] : nhi);
+            if (l != ~0u && h != 0u && pw0 + k < g.PW) m |= 1u << k;
         }
-    }
-    // nfs cleared.  A segment whose warps are all quiet has no crossed edge and
-    // no active cell: its sums are 0, and no cell reads its words' vertex
-    // offsets (a cell's edges lie in words with crossings), so it stops here.
-    if (!__syncthreads_or(!warp_quiet)) {
-        if (threadIdx.x == 0) {
-            blk[2 * seg] = 0ull;
-            blk[2 * seg + 1] = 0ull;
-        }
-        return;
-    }
-    uint32_t sv = 0;
-#pragma unroll
-    for (int k = 0; k < WPT; ++k) sv += nv[k];
-    // active cells, one per lane of the warp: triangle counts, and a cell entry
-    // with the cell's face offset within its word (cells of a word come in bit
-    // order: a segmented scan over the lanes plus the word's faces of earlier rounds)
-    {
-        const uint32_t na = __popc(act[0]) + __popc(act[1]) + __popc(act[2]) + __popc(act[3]);
-        uint32_t incl = na, vsum = sv;
+        const uint32_t mine = __popc(m);
+        uint32_t inc = mine;
 #pragma unroll
         for (int dd = 1; dd < 32; dd <<= 1) {
-            const uint32_t t = __shfl_up_sync(~0u, incl, dd);
-            if (lane >= dd) incl += t;
-            vsum += __shfl_xor_sync(~0u, vsum, dd);
+            const uint32_t t = __shfl_up_sync(~0u, inc, dd);
+            if (lane >= dd) inc += t;
         }
-        const uint32_t total = __shfl_sync(~0u, incl, 31);
-        // the CTA's cell entries and vertex entries are allocated at once: warp
-        // offsets, one atomic each, both in flight together
-        if (lane == 0) {
-            wcell[warp] = total;
-            wvert[warp] = vsum;
-        }
+        if (lane == 31) bsum[warp] = inc;
         __syncthreads();
-        if (threadIdx.x == 0) {
-            uint32_t run = 0;
-            for (int q = 0; q < CNT_THREADS / 32; ++q) {
-                const uint32_t c = wcell[q];
-                wcell[q] = run;
-                run += c;
-            }
-            cbase_s = run ? atomicAdd(ctr + 10, (unsigned long long)run) : 0ull;
-        } else if (threadIdx.x == 32) {
-            uint32_t run = 0;
-            for (int q = 0; q < CNT_THREADS / 32; ++q) run += wvert[q];
-            vbase_s = run ? atomicAdd(ctr, (unsigned long long)run) : 0ull;
+        uint32_t at = inc - mine;
+#pragma unroll
+        for (int q = 0; q < NW; ++q) {
+            at += q < warp ? bsum[q] : 0u;
+            nbusy += bsum[q];
         }
-        __syncthreads();
-        const unsigned long long wbase = cbase_s + wcell[warp];
-        for (uint32_t rr = 0; rr < total; rr += 32) {
-            const uint32_t j = rr + lane;
-            const int o = owner_of(incl, j);
-            const uint32_t oexcl = __shfl_sync(~0u, incl - na, o);
-            uint32_t oa[WPT];
-#pragma unroll
-            for (int k = 0; k < WPT; ++k) oa[k] = __shfl_sync(~0u, act[k], o);
-            const bool valid = j < total;
-            uint32_t wid = 0xffffffffu, ntc = 0, cs = 0, pw = 0;
-            int b = 0;
-            if (valid) {
-                int kk = int(j - oexcl), k = 0;
-                uint32_t m = oa[0];
-#pragma unroll
-                for (int q = 0; q < WPT - 1; ++q) {
-                    const int c = __popc(m);
-                    if (kk >= c) { kk -= c; m = oa[q + 1]; k = q + 1; }
-                    else break;
-                }
-                b = nth_set(m, kk);
-                const uint32_t ot = uint32_t(warp * 32 + o);
-                wid = ot * WPT + uint32_t(k);
-                pw = seg * SEG + wid;
-                // corners from the owner's row words (an active cell has rows
-                // x + 1 and y + 1, and z + 1 in word w + 1 only at bit 31)
-                Words d;
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    d.s[q >> 1][q & 1][0] = rows[q][k][ot];
-                    d.s[q >> 1][q & 1][1] = rows[q][k + 1][ot];
-                }
-                cs = cell_case(d, b);
-                ntc = (nt4[cs >> 2] >> (8 * (cs & 3))) & 0xffu;
+        for (; m; m &= m - 1) list[at++] = uint16_t(threadIdx.x * WPT + __ffs(m) - 1);
+    }
+    // A segment without such words has no crossed edge and no active cell: its
+    // sums are 0, and no cell reads its words' vertex offsets (a cell's edges lie
+    // in words with crossings).
+    uint32_t tv = 0, tf = 0;  // edges and faces of the rounds so far
+    for (uint32_t r0 = 0; r0 < nbusy; r0 += T) {
+        __syncthreads();  // the list; the shared arrays of the round before
+        uint32_t e3[3] = {0u, 0u, 0u}, act = 0, nf = 0, pw = 0;
+        const uint32_t i = r0 + threadIdx.x;
+        if (i < nbusy) {
+            pw = seg * SEG + list[i];
+            int x, y, w;
+            word_xyw(g, pw, x, y, w);
+            Words d;
+            load_words(g, S, pw, x, y, w, d);
+            const uint32_t zm = zmask(g, w);
+            e3[0] = d.hasx ? (d.s[0][0][0] ^ d.s[1][0][0]) : 0u;
+            e3[1] = d.hasy ? (d.s[0][0][0] ^ d.s[0][1][0]) : 0u;
+            e3[2] = ez_of(d.s[0][0][0], d.s[0][0][1], zm);
+            act = active_cells(d, zm);
+            if (act) {
+                uint32_t c[8];
+                corner_words(d, c);
+                nf = word_faces(c, act, [&](uint32_t cs) { return uint32_t(ISO_NTRI[g.method * 256 + cs]); });
             }
-            uint32_t sc = ntc;
-#pragma unroll
-            for (int dd = 1; dd < 32; dd <<= 1) {
-                const uint32_t t = __shfl_up_sync(~0u, sc, dd);
-                if (lane >= dd) sc += t;
-            }
-            const uint32_t prev_wid = __shfl_up_sync(~0u, wid, 1);
-            const uint32_t next_wid = __shfl_down_sync(~0u, wid, 1);
-            const uint32_t heads = __ballot_sync(~0u, valid && (lane == 0 || prev_wid != wid));
-            const int start = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
-            const uint32_t base = __shfl_sync(~0u, sc, start > 0 ? start - 1 : 0);
-            const uint32_t within_round = sc - ntc - (start > 0 ? base : 0u);
-            const uint32_t carry = valid ? nfs[wid] : 0u;
-            __syncwarp();
-            if (valid) {
-                const unsigned long long ci = wbase + j;
-                if ((long long)ci < capF)
-                    clist[ci] = (unsigned long long)pw | ((unsigned long long)b << 32) |
-                                ((unsigned long long)cs << 37) |
-                                ((unsigned long long)(carry + within_round) << 45);
-                const bool tail = lane == 31 || next_wid != wid;
-                if (tail) nfs[wid] = carry + within_round + ntc;
-            }
-            __syncwarp();
         }
-    }
-    __syncthreads();
-    uint32_t nf[WPT], sf = 0;
-#pragma unroll
-    for (int k = 0; k < WPT; ++k) {
-        nf[k] = nfs[threadIdx.x * WPT + k];
-        sf += nf[k];
-    }
-    uint32_t ev, ef, tv, tf;
-    block_scan2<CNT_THREADS>(sv, sf, ev, ef, tv, tf, sm);
-    // vertex entries: the CTA's block of entries (allocated above), each entry
-    // at the block base plus its segment-local slot (x edges, then y, then z of
-    // each word); one vertex per lane of the warp, so consecutive lanes store
-    // consecutive entries
-    const unsigned long long vb0 = vbase_s;
-    {
-        uint32_t incl = sv;
+        const uint32_t cx = __popc(e3[0]), cy = __popc(e3[1]);
+        const uint32_t nv = cx + cy + __popc(e3[2]), na = __popc(act);
+        // active cells (at most 32 T), edges (from bit 20) and faces (from 40)
+        const unsigned long long mine = (unsigned long long)na | ((unsigned long long)nv << 20) |
+                                        ((unsigned long long)nf << 40);
+        unsigned long long inc = mine;
 #pragma unroll
         for (int dd = 1; dd < 32; dd <<= 1) {
-            const uint32_t t = __shfl_up_sync(~0u, incl, dd);
-            if (lane >= dd) incl += t;
+            const unsigned long long t = __shfl_up_sync(~0u, inc, dd);
+            if (lane >= dd) inc += t;
         }
-        const uint32_t total = __shfl_sync(~0u, incl, 31);
-        for (uint32_t rr = 0; rr < total; rr += 32) {
-            const uint32_t j = rr + lane;
-            const int o = owner_of(incl, j);
-            const uint32_t oexcl = __shfl_sync(~0u, incl - sv, o);
-            const uint32_t oev = __shfl_sync(~0u, ev, o);
-            uint32_t onv[WPT];
+        if (lane == 31) wsum[warp] = inc;
+        __syncthreads();
+        unsigned long long before = 0, all = 0;
 #pragma unroll
-            for (int k = 0; k < WPT; ++k) onv[k] = __shfl_sync(~0u, nv[k], o);
-            if (j < total) {
-                uint32_t kk = j - oexcl, slot = oev + kk;
-                int k = 0;
-#pragma unroll
-                for (int q = 0; q < WPT - 1; ++q) {
-                    if (k == q && kk >= onv[q]) { kk -= onv[q]; k = q + 1; }
+        for (int q = 0; q < NW; ++q) {
+            before += q < warp ? wsum[q] : 0ull;
+            all += wsum[q];
+        }
+        // the round's blocks of both lists, both atomics in flight together
+        const uint32_t ta = uint32_t(all) & 0xfffffu, te = uint32_t(all >> 20) & 0xfffffu;
+        if (threadIdx.x == 0) cbase_s = ta ? atomicAdd(ctr + 10, (unsigned long long)ta) : 0ull;
+        else if (threadIdx.x == 32) vbase_s = te ? atomicAdd(ctr, (unsigned long long)te) : 0ull;
+        const unsigned long long ex = inc - mine;  // within the warp
+        if (nv) info[pw] = (tv + (uint32_t((before + ex) >> 20) & 0xfffffu)) | (cx << 20) | (cy << 26);
+        fofs[threadIdx.x] = tf + uint32_t((before + ex) >> 40);
+        __syncthreads();  // the list blocks; from here to the next round warps go their own ways
+        const unsigned long long wtot = __shfl_sync(~0u, inc, 31);
+        uint16_t* q = queue[warp];
+        // active cells in cell order: lane << 5 | bit
+        {
+            const uint32_t n = uint32_t(wtot) & 0xfffffu, c0 = uint32_t(ex) & 0xfffffu;
+            const unsigned long long base = cbase_s + (uint32_t(before) & 0xfffffu);
+            for (uint32_t q0 = 0; q0 < n; q0 += CQ) {
+                if (na && c0 < q0 + CQ && c0 + na > q0) {
+                    uint32_t j = c0 - q0;  // wraps below q0: not in this window
+                    for (uint32_t m = act; m; m &= m - 1, ++j)
+                        if (j < uint32_t(CQ)) q[j] = uint16_t((lane << 5) | (__ffs(m) - 1));
                 }
-                const uint32_t ot = uint32_t(warp * 32 + o);
-                const uint32_t m0 = vmask[3 * k][ot], m1 = vmask[3 * k + 1][ot], m2 = vmask[3 * k + 2][ot];
-                const uint32_t c0 = __popc(m0), c1 = __popc(m1);
-                int ax, bb;
-                if (kk < c0) { ax = 0; bb = nth_set(m0, int(kk)); }
-                else if (kk < c0 + c1) { ax = 1; bb = nth_set(m1, int(kk - c0)); }
-                else { ax = 2; bb = nth_set(m2, int(kk - c0 - c1)); }
-                const uint32_t pw = seg * SEG + ot * WPT + uint32_t(k);
-                const unsigned long long vb = vb0 + slot;
-                if ((long long)vb < capV)
-                    vlist[vb] = (unsigned long long)pw | ((unsigned long long)ax << 32) |
-                                ((unsigned long long)bb << 34) | ((unsigned long long)slot << 39);
+                __syncwarp();
+                for (uint32_t j = lane; j < min(uint32_t(CQ), n - q0); j += 32) {
+                    const uint32_t it = q[j], o = warp * 32 + (it >> 5);
+                    const unsigned long long ci = base + q0 + j;
+                    if ((long long)ci < capF)
+                        clist[ci] = (unsigned long long)(seg * SEG + list[r0 + o]) |
+                                    ((unsigned long long)(it & 31u) << 32) | ((unsigned long long)fofs[o] << 37);
+                }
+                __syncwarp();
             }
         }
-    }
-    if (vec && pw0 + WPT <= g.PW) {
-        *reinterpret_cast<uint4*>(info + pw0) =
-            make_uint4(ev | cxy[0], (ev + nv[0]) | cxy[1], (ev + nv[0] + nv[1]) | cxy[2],
-                       (ev + nv[0] + nv[1] + nv[2]) | cxy[3]);
-    }
+        // crossed edges in slot order (x edges, then y, then z of each word):
+        // lane << 7 | axis << 5 | bit
+        {
+            const uint32_t n = uint32_t(wtot >> 20) & 0xfffffu, v0 = uint32_t(ex >> 20) & 0xfffffu;
+            const uint32_t slot0 = uint32_t(before >> 20) & 0xfffffu;
+            const unsigned long long base = vbase_s + slot0;
+            for (uint32_t q0 = 0; q0 < n; q0 += CQ) {
+                if (nv && v0 < q0 + CQ && v0 + nv > q0) {
+                    uint32_t j = v0 - q0;
 #pragma unroll
-    for (int k = 0; k < WPT; ++k) {
-        const uint32_t pw = pw0 + k;
-        if (pw < g.PW) {
-            if (!(vec && pw0 + WPT <= g.PW)) info[pw] = ev | cxy[k];
-            if (nf[k]) foff[pw] = ef;
+                    for (int ax = 0; ax < 3; ++ax)
+                        for (uint32_t m = e3[ax]; m; m &= m - 1, ++j)
+                            if (j < uint32_t(CQ)) q[j] = uint16_t((lane << 7) | (ax << 5) | (__ffs(m) - 1));
+                }
+                __syncwarp();
+                for (uint32_t j = lane; j < min(uint32_t(CQ), n - q0); j += 32) {
+                    const uint32_t it = q[j];
+                    const unsigned long long vb = base + q0 + j;
+                    if ((long long)vb < capV)
+                        vlist[vb] = (unsigned long long)(seg * SEG + list[r0 + warp * 32 + (it >> 7)]) |
+                                    ((unsigned long long)((it >> 5) & 3u) << 32) |
+                                    ((unsigned long long)(it & 31u) << 34) |
+                                    ((unsigned long long)(tv + slot0 + q0 + j) << 39);
+                }
+                __syncwarp();
+            }
         }
-        ev += nv[k];
-        ef += nf[k];
+        tv += te;
+        tf += uint32_t(all >> 40);
     }
+    // the segment's sums; the last CTA turns them into offsets when it can
+    const bool scans = nseg <= uint32_t(SCAN_LAST * T);
     if (threadIdx.x == 0) {
-        blk[2 * seg] = tv;
-        blk[2 * seg + 1] = tf;
+        reinterpret_cast<ulonglong2*>(blk)[seg] = make_ulonglong2(tv, tf);
+        if (scans) {
+            __threadfence();
+            last_s = atomicAdd(ctr + 6, 1ull) == nseg - 1;
+            __threadfence();
+        }
     }
+    if (!scans) return;
+    __syncthreads();
+    if (last_s) scan_segments<T>(blk, nseg, ctr, counts, status, capV, capF, sm);
 }
 
 // ---------------------------------------------------------------------------
-// 3. scan of the per-segment (V, F) sums of mc_count into exclusive offsets:
-// CTAs take chunks of SCAN_PER * SCAN_THREADS segments in ticket order and chain
-// their totals by decoupled look-back.  The last chunk writes the totals and
-// checks the capacities.
+// 3. scan of the per-segment (V, F) sums of mc_count into exclusive offsets,
+// for grids of more segments than the last count CTA scans: CTAs take chunks of
+// SCAN_THREADS segments in ticket order and chain their totals by decoupled
+// look-back.  The last chunk writes the totals and checks the capacities.
 constexpr int SCAN_THREADS = 1024;
-constexpr int SCAN_PER = 1;
 
 __global__ void __launch_bounds__(SCAN_THREADS) mc_scan(unsigned long long* blk, uint32_t nseg,
                                                         unsigned long long* ctr, unsigned long long* state,
@@ -669,18 +650,11 @@ __global__ void __launch_bounds__(SCAN_THREADS) mc_scan(unsigned long long* blk,
     if (threadIdx.x == 0) chunk_s = uint32_t(atomicAdd(ctr + 7, 1ull));
     __syncthreads();
     const uint32_t chunk = chunk_s;
-    const uint32_t nchunk = (nseg + SCAN_PER * SCAN_THREADS - 1) / (SCAN_PER * SCAN_THREADS);
-    const uint32_t s0 = chunk * SCAN_PER * SCAN_THREADS + threadIdx.x * SCAN_PER;
-    uint32_t a[SCAN_PER], b[SCAN_PER], sa = 0, sb = 0;
-#pragma unroll
-    for (int k = 0; k < SCAN_PER; ++k) {
-        a[k] = s0 + k < nseg ? uint32_t(blk[2 * (s0 + k)]) : 0u;
-        b[k] = s0 + k < nseg ? uint32_t(blk[2 * (s0 + k) + 1]) : 0u;
-        sa += a[k];
-        sb += b[k];
-    }
+    const uint32_t nchunk = (nseg + SCAN_THREADS - 1) / SCAN_THREADS;
+    const uint32_t s = chunk * SCAN_THREADS + threadIdx.x;
+    const uint32_t a = s < nseg ? uint32_t(blk[2 * s]) : 0u, b = s < nseg ? uint32_t(blk[2 * s + 1]) : 0u;
     uint32_t ea, eb, ta, tb;
-    block_scan2<SCAN_THREADS>(sa, sb, ea, eb, ta, tb, sm);
+    block_scan2<SCAN_THREADS>(a, b, ea, eb, ta, tb, sm);
     if (threadIdx.x < 32) {
         unsigned long long pv = 0, pf = 0;
         if (chunk == 0) {
@@ -693,27 +667,13 @@ __global__ void __launch_bounds__(SCAN_THREADS) mc_scan(unsigned long long* blk,
         if (threadIdx.x == 0) {
             pre_s[0] = pv;
             pre_s[1] = pf;
-            if (chunk == nchunk - 1) {
-                const unsigned long long V = pv + ta, F = pf + tb;
-                counts[0] = (long long)V;
-                counts[1] = (long long)F;
-                ctr[4] = V;
-                ctr[5] = F;
-                if ((long long)V > capV || (long long)F > capF || V >= LB_MASK31 || F >= LB_MASK31)
-                    atomicCAS(status, 0, int(ISO_ERR_OVERFLOW));
-            }
+            if (chunk == nchunk - 1) mc_totals(pv + ta, pf + tb, ctr, counts, status, capV, capF);
         }
     }
     __syncthreads();
-    unsigned long long ov = pre_s[0] + ea, of = pre_s[1] + eb;
-#pragma unroll
-    for (int k = 0; k < SCAN_PER; ++k) {
-        if (s0 + k < nseg) {
-            blk[2 * (s0 + k)] = ov;
-            blk[2 * (s0 + k) + 1] = of;
-        }
-        ov += a[k];
-        of += b[k];
+    if (s < nseg) {
+        blk[2 * s] = pre_s[0] + ea;
+        blk[2 * s + 1] = pre_s[1] + eb;
     }
 }
 
@@ -741,7 +701,6 @@ struct EmitArgs {
     const uint32_t* S;
     const uint32_t* info;
     const unsigned long long* blk;
-    const uint32_t* foff;
     const unsigned long long* vlist;
     const unsigned long long* clist;
     unsigned long long* ctr;
@@ -823,22 +782,20 @@ __device__ void emit_vertices(const McGrid& g, const EmitArgs& a, unsigned bi, u
     }
 }
 
-// Face role: one thread per cell entry; CTA `bi` of `nb`.
+// Face role: one thread per cell entry; CTA `bi` of `nb`.  Bound by the latency of
+// its gathers: everything that a cell reads after its entry (the bitmap words,
+// the vertex offsets of the four words its edges start in, its segment's
+// offsets) is requested at once, so a cell costs two rounds of memory latency.
 template <int EMIT_THREADS>
 __device__ void emit_faces(const McGrid& g, const EmitArgs& a, unsigned bi, unsigned nb) {
     __shared__ unsigned long long tpk[256];  // packed triangle lists of the table
-    __shared__ uint16_t est[256];
     __shared__ uint32_t vid[12][EMIT_THREADS];
     const uint32_t* __restrict__ S = a.S;
     const uint32_t* __restrict__ info = a.info;
     const unsigned long long* __restrict__ blk = a.blk;
-    const uint32_t* __restrict__ foff = a.foff;
     const unsigned long long* __restrict__ clist = a.clist;
     int32_t* __restrict__ fout = a.fout;
-    for (int i = threadIdx.x; i < 256; i += EMIT_THREADS) {
-        tpk[i] = ISO_TRI_PACKED[g.method * 256 + i];
-        est[i] = ISO_EDGE_STATUS[i];
-    }
+    for (int i = threadIdx.x; i < 256; i += EMIT_THREADS) tpk[i] = ISO_TRI_PACKED[g.method * 256 + i];
     __syncthreads();
     const unsigned long long n = min(a.ctr[10], (unsigned long long)a.capF);
     const uint32_t sxw = uint32_t(g.ny) * uint32_t(g.NW);
@@ -848,33 +805,51 @@ __device__ void emit_faces(const McGrid& g, const EmitArgs& a, unsigned bi, unsi
         const unsigned long long e = clist[i];
         const uint32_t pw = uint32_t(e);
         const int b = int((e >> 32) & 31u);
-        const uint32_t cs = uint32_t((e >> 37) & 255u);
         int x, y, w;
         word_xyw(g, pw, x, y, w);
-        const unsigned long long fo = blk[2 * seg_of(g, pw) + 1] + foff[pw] + ((e >> 45) & 255u);
         Words d;
         load_words(g, S, pw, x, y, w, d);
+        // word w of the rows (dx, dy): vertex offset, and where its y and z edges start
+        uint32_t base[4], inf[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint32_t p = pw + uint32_t(q >> 1) * sxw + uint32_t(q & 1) * uint32_t(g.NW);
+            inf[q] = info[p];
+            base[q] = uint32_t(blk[2 * seg_of(g, p)]);
+        }
+        const unsigned long long fseg = blk[2 * seg_of(g, pw) + 1];
         const uint32_t zm = zmask(g, w);
-        const uint32_t es = est[cs];
-        const int hi = (b + 1) >> 5;  // the cell's z + 1 lies in word w + 1
+        uint32_t c[8];
+        corner_words(d, c);
+        const uint32_t cs = case_at(c, b);
+        const unsigned long long fo =
+            fseg + (e >> 37) + word_faces(c, active_cells(d, zm) & ((1u << b) - 1u),
+                                          [&](uint32_t q) { return uint32_t(tpk[q] >> 60); });
 #pragma unroll
         for (int k = 0; k < 12; ++k) {
-            if (!((es >> k) & 1u)) continue;
-            const int a = iso_edge_corner(2 * k), c = iso_edge_corner(2 * k + 1);
-            const int ax = (c - a) == 4 ? 0 : ((c - a) == 2 ? 1 : 2);
-            const int adx = a >> 2, ady = (a >> 1) & 1, adz = a & 1;
-            const int ww = adz ? hi : 0;
-            const int bit = (b + adz) & 31;
-            uint32_t m;
-            if (ax == 0) m = ww ? (d.s[0][ady][1] ^ d.s[1][ady][1]) : (d.s[0][ady][0] ^ d.s[1][ady][0]);
-            else if (ax == 1) m = ww ? (d.s[adx][0][1] ^ d.s[adx][1][1]) : (d.s[adx][0][0] ^ d.s[adx][1][0]);
-            else m = ez_of(d.s[adx][ady][0], d.s[adx][ady][1], zm);
-            const uint32_t q = pw + uint32_t(adx) * sxw + uint32_t(ady) * uint32_t(g.NW) + uint32_t(ww);
-            const uint32_t inf = info[q];
-            uint32_t off = uint32_t(blk[2 * seg_of(g, q)]) + (inf & 0xfffffu);
-            if (ax >= 1) off += (inf >> 20) & 63u;
-            if (ax == 2) off += (inf >> 26) & 63u;
-            vid[k][tid] = off + __popc(m & ((1u << bit) - 1u));
+            const int ca = iso_edge_corner(2 * k), cb = iso_edge_corner(2 * k + 1);
+            if (!(((cs >> ca) ^ (cs >> cb)) & 1u)) continue;
+            const int ax = (cb - ca) == 4 ? 0 : ((cb - ca) == 2 ? 1 : 2);
+            const int adx = ca >> 2, ady = (ca >> 1) & 1, adz = ca & 1, q = 2 * adx + ady;
+            uint32_t off, m, below;
+            if (adz && b == 31) {
+                // the edge's low end lies in word w + 1 (at its bit 0)
+                const uint32_t p = pw + uint32_t(adx) * sxw + uint32_t(ady) * uint32_t(g.NW) + 1u;
+                const uint32_t in1 = info[p];
+                off = uint32_t(blk[2 * seg_of(g, p)]) + (in1 & 0xfffffu);
+                if (ax == 1) off += (in1 >> 20) & 63u;
+                m = 0;
+                below = 0;
+            } else {
+                off = base[q] + (inf[q] & 0xfffffu);
+                if (ax >= 1) off += (inf[q] >> 20) & 63u;
+                if (ax == 2) off += (inf[q] >> 26) & 63u;
+                if (ax == 0) m = d.s[0][ady][0] ^ d.s[1][ady][0];
+                else if (ax == 1) m = d.s[adx][0][0] ^ d.s[adx][1][0];
+                else m = ez_of(d.s[adx][ady][0], d.s[adx][ady][1], zm);
+                below = (1u << (b + adz)) - 1u;
+            }
+            vid[k][tid] = off + __popc(m & below);
         }
         unsigned long long pk = tpk[cs];
         const int ntc = int(pk >> 60);
@@ -907,7 +882,7 @@ struct FixLayout {
 };
 
 template <int EMIT_THREADS>
-__global__ void __launch_bounds__(EMIT_THREADS) mc_emit(const McGrid g, const EmitArgs a) {
+__global__ void __launch_bounds__(EMIT_THREADS, 1280 / EMIT_THREADS) mc_emit(const McGrid g, const EmitArgs a) {
     iso::grid_wait();
     if (a.counts[0] > a.capV || a.counts[1] > a.capF || a.counts[0] > 0x7fffffffll) return;
     // the fix-up's bitmaps and look-back states (half a byte per vertex)
@@ -1258,6 +1233,16 @@ int sm_count() {
     return sms;
 }
 
+// Threads of a count CTA.
+int count_threads() { return iso::tune_get(iso::TUNE_MC_COUNT_THREADS) == 128 ? 128 : 256; }
+
+// Point words up to which a count thread takes one word instead of four: four
+// times as many CTAs, for grids whose CTAs of four words per thread would not
+// fill the GPU.  32^3 in one CTA of 1024 words took 21 us and takes 9 in four;
+// 128^3 15 and 10.  From 2^18 words on (200 x 330 x 143 and 256^3) the scan that
+// the last CTA then no longer does costs what the count gains: 13 + 4 against 16 us.
+constexpr long long FINE_PW = 1ll << 18;
+
 template <int EMIT_THREADS>
 int launch_emit(const McParams& p, const McGrid& g, const McWs& w, cudaStream_t st, int sms) {
     static int per = -1;
@@ -1269,7 +1254,7 @@ int launch_emit(const McParams& p, const McGrid& g, const McWs& w, cudaStream_t 
     const auto want = [&](long long cap) { return std::max<long long>(1, (cap + EMIT_THREADS - 1) / EMIT_THREADS); };
     const long long nbv = std::max<long long>(1, std::min(want(p.capV), resident / 3));
     const long long nbf = std::max<long long>(1, std::min(want(p.capF), resident - nbv));
-    EmitArgs a{p.vals, w.S, w.info, w.blk, w.foff, w.vlist, w.clist, w.ctr, w.snaps, w.small,
+    EmitArgs a{p.vals, w.S, w.info, w.blk, w.vlist, w.clist, w.ctr, w.snaps, w.small,
                p.vout, p.fout, p.counts, p.status, p.capV, p.capF, unsigned(nbv), w, p.vedge};
     {
         iso::ProfScope ps("mc_emit", st);
@@ -1288,21 +1273,23 @@ int launch_emit(const McParams& p, const McGrid& g, const McWs& w, cudaStream_t 
 
 int launch_count_emit(const McParams& p, const McGrid& g, const McWs& w, cudaStream_t st) {
     const int sms = sm_count();
+    const int ct = count_threads();
+    const uint32_t nseg = uint32_t((g.PW + (1ll << g.lgseg) - 1) >> g.lgseg);
     {
         iso::ProfScope ps("mc_count", st);
+        const bool fine = (1 << g.lgseg) == ct;  // one word per thread
         const long long ncoord = (long long)p.nx + p.ny + p.nz;
-        const int ct = 1 << (g.lgseg - 2);  // the count CTA's threads (WPT = 4 words each)
-        const long long nseg = (g.PW + (1ll << g.lgseg) - 1) >> g.lgseg;
         const long long grid = std::max<long long>(nseg, (ncoord + ct - 1) / ct);
-        iso::launch_pdl(ct == 128 ? mc_count<128> : mc_count<256>, unsigned(grid), unsigned(ct), st, g, p.amin[0],
-                        p.amin[1], p.amin[2], p.asize[0], p.asize[1], p.asize[2], w.S, w.info, w.blk, w.vlist, w.clist,
-                        w.foff, w.ctr, w.gc, uint32_t(nseg), p.capV, p.capF);
+        const auto kernel = fine ? (ct == 128 ? mc_count<128, 1> : mc_count<256, 1>)
+                                 : (ct == 128 ? mc_count<128, WPT_MAX> : mc_count<256, WPT_MAX>);
+        iso::launch_pdl(kernel, unsigned(grid), unsigned(ct), st, g, p.amin[0], p.amin[1], p.amin[2], p.asize[0],
+                        p.asize[1], p.asize[2], w.S, w.info, w.blk, w.vlist, w.clist, w.ctr, w.gc, nseg, p.capV, p.capF,
+                        p.counts, p.status);
         if (cudaGetLastError() != cudaSuccess) return iso::fail_code(ISO_ERR_CUDA);
     }
-    {
+    if (nseg > uint32_t(SCAN_LAST * ct)) {
         iso::ProfScope ps("mc_scan", st);
-        const uint32_t nseg = uint32_t((g.PW + (1ll << g.lgseg) - 1) >> g.lgseg);
-        const uint32_t nchunk = (nseg + SCAN_PER * SCAN_THREADS - 1) / (SCAN_PER * SCAN_THREADS);
+        const uint32_t nchunk = (nseg + SCAN_THREADS - 1) / SCAN_THREADS;
         iso::launch_pdl(mc_scan, nchunk, SCAN_THREADS, st, w.blk, nseg, w.ctr, w.state, p.counts, p.status, p.capV,
                    p.capF);
         if (cudaGetLastError() != cudaSuccess) return iso::fail_code(ISO_ERR_CUDA);
@@ -1364,7 +1351,7 @@ int mc_launch(const McParams& p, void* ws, size_t ws_bytes, cudaStream_t st) {
     const McWs w0 = carve(p.nx, p.ny, p.nz, p.capV, p.capF, nullptr);
     if (ws_bytes < w0.total) return iso::fail_code(ISO_ERR_WORKSPACE);
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(ws) + 255) & ~uintptr_t(255));
-    const McWs w = carve(p.nx, p.ny, p.nz, p.capV, p.capF, base);
+    McWs w = carve(p.nx, p.ny, p.nz, p.capV, p.capF, base);
     McGrid g;
     g.nx = p.nx; g.ny = p.ny; g.nz = p.nz;
     g.NW = (p.nz + 31) / 32;
@@ -1375,7 +1362,9 @@ int mc_launch(const McParams& p, void* ws, size_t ws_bytes, cudaStream_t st) {
     g.method = p.method;
     g.tau = snap_tau(p);
     g.fma = iso::arith_fma();
-    g.lgseg = iso::tune_get(iso::TUNE_MC_COUNT_THREADS) == 128 ? 9 : 10;
+    const bool fine = g.PW <= FINE_PW;
+    g.lgseg = (count_threads() == 128 ? 7 : 8) + (fine ? 0 : 2);
+    if (fine) w.blk = w.blk2;
     g.gc = w.gc;
     if (g.PW > 0xffffffffll) return iso::fail_code(ISO_ERR_ARG);
     {

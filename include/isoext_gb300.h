@@ -277,6 +277,17 @@ int iso_sparse_mc(const int *ids, const float *vals, long long n, int nx, int ny
                   const float *aabb_min, const float *aabb_max, float level, int method, float *vertices,
                   long long vertex_capacity, int *faces, long long face_capacity, void *workspace,
                   size_t workspace_bytes, long long *counts, int *status, void *stream);
+/* Sparse DC in one call with no host synchronisation: dual contouring without a
+ * caller intersection (normals from each cell's values), the mesh of the
+ * intersection, solve, quads and weld calls.  vertex_capacity bounds the active
+ * cells.  values 16-byte aligned.  counts (device int64[5]) <- (V, F, A, K, Q):
+ * vertices, faces, active cells, crossings, quads; status 6 when A or 2 Q exceed
+ * the capacities (retry with A, then 2 Q; Q is 0 while A does not fit). */
+size_t iso_sparse_dc_workspace_size(long long n, long long vertex_capacity, long long face_capacity);
+int iso_sparse_dc(const int *ids, const float *values, long long n, int nx, int ny, int nz,
+                  const float *aabb_min, const float *aabb_max, float level, float reg, float svd_tol,
+                  float *vertices, long long vertex_capacity, int *faces, long long face_capacity,
+                  void *workspace, size_t workspace_bytes, long long *counts, int *status, void *stream);
 /* Corner positions [m, 8, 3] of cell ids (get_points / get_points_by_cell_indices,
  * src/grid/sparse.cu:21-43). */
 int iso_sparse_points(const int *ids, long long m, int nx, int ny, int nz, const float *aabb_min,

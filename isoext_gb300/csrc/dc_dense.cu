@@ -1290,7 +1290,7 @@ __global__ void __launch_bounds__(256) dc_cell_quads(const uint8_t* __restrict__
 // Exclusive scan of per-block (u64, u64) sums in place, totals -> totals[0..1]
 // (used by the sparse-grid kernels).
 void iso_block_scan_launch(unsigned long long* blk, long long nblk, long long* totals, cudaStream_t st) {
-    dc_block_scan<<<1, 1024, 0, st>>>(blk, nblk, totals);
+    iso::launch_pdl(dc_block_scan, 1u, 1024u, st, blk, nblk, totals);
 }
 
 extern "C" {

@@ -898,6 +898,12 @@ __device__ bool cell_quad(const SpGrid& g, const int* ids, const float* vals, lo
     return true;
 }
 
+// A quad needs its owner active too (a repeated id stands for its first cell):
+// the searches for the rest of a band's cells, nine tenths of them, are left out.
+__device__ __forceinline__ bool may_own_quads(const int* ids, const uint32_t* rank, long long c) {
+    return rank[c] != 0xffffffffu || (c > 0 && ids[c - 1] == ids[c]);
+}
+
 __global__ void __launch_bounds__(SP_BLOCK) sp_quad_count(SpGrid g, const int* __restrict__ ids,
                                                           const float* __restrict__ vals, long long n,
                                                           const uint32_t* __restrict__ rank,
@@ -905,7 +911,7 @@ __global__ void __launch_bounds__(SP_BLOCK) sp_quad_count(SpGrid g, const int* _
     __shared__ uint32_t sm[33];
     const long long c = (long long)blockIdx.x * SP_BLOCK + threadIdx.x;
     uint32_t nq = 0;
-    if (c < n) {
+    if (c < n && may_own_quads(ids, rank, c)) {
         for (int ax = 2; ax >= 0; --ax) {
             long long q[4];
             bool out;
@@ -936,7 +942,7 @@ __global__ void __launch_bounds__(SP_BLOCK) sp_quad_emit(SpGrid g, const int* __
     uint32_t nq = 0;
     long long qs[3][4];
     bool outs[3], oks[3] = {false, false, false};
-    if (c < n) {
+    if (c < n && may_own_quads(ids, rank, c)) {
         for (int ax = 2; ax >= 0; --ax) {
             if (!cell_quad(g, ids, vals, n, c, ax, qs[ax], outs[ax])) continue;
             bool ok = true;

@@ -33,6 +33,9 @@ _ffi.register({
     "iso_sparse_points": ([_vp, _ll, _i, _i, _i, _fa, _fa, _vp, _vp], _i),
     "iso_sparse_filter_count": ([_vp, _ll, _f, _vp, _vp, _vp], _i),
     "iso_sparse_filter_write": ([_vp, _vp, _ll, _f, _vp, _vp, _vp], _i),
+    "iso_sparse_dc_workspace_size": ([_ll, _ll, _ll], _sz),
+    "iso_sparse_dc": ([_vp, _vp, _ll, _i, _i, _i, _fa, _fa, _f, _f, _f, _vp, _ll, _vp, _ll, _vp, _sz, _vp, _vp, _vp],
+                      _i),
     "iso_sparse_mc_workspace_size": ([_ll, _ll, _ll], _sz),
     "iso_sparse_mc": ([_vp, _vp, _ll, _i, _i, _i, _fa, _fa, _f, _i, _vp, _ll, _vp, _ll, _vp, _sz, _vp, _vp, _vp], _i),
 })
@@ -353,9 +356,51 @@ class SparseGrid(SparseGridBase):
     def _get_intersection(self, level: float, compute_normals: bool):
         return self._intersect(level, compute_normals)
 
+    def _dc_one_call(self, level, reg, svd_tol):
+        """iso_sparse_dc, sized from the last call on this grid (one
+        synchronisation; retries with exact capacities when they were small)."""
+        from .mc import _views
+
+        lib = _ffi.lib()
+        dev = self.device
+        n = self.get_num_cells()
+        st = _stream(dev)
+        sx, sy, sz, lo, hi = self._geom()
+        key = (n, float(level))
+        if getattr(self, "_dc_sizes", None) and key in self._dc_sizes:
+            a, q = self._dc_sizes[key]
+            cap_v, cap_f = a + a // 10 + 1024, 2 * q + (2 * q) // 10 + 1024
+        else:
+            # a band of a few cells on each side of the surface
+            cap_v = min(n, n // 4 + 4096)
+            cap_f = 2 * cap_v
+        for _ in range(3):
+            vout = torch.empty((cap_v, 3), dtype=torch.float32, device=dev)
+            fout = torch.empty((cap_f, 3), dtype=torch.int32, device=dev)
+            ws = torch.empty(int(lib.iso_sparse_dc_workspace_size(n, cap_v, cap_f)), dtype=torch.uint8, device=dev)
+            small = torch.zeros(8, dtype=torch.int64, device=dev)
+            _ffi.check(lib.iso_sparse_dc(_p(self._ids), _p(self._values), n, sx, sy, sz, lo, hi, float(level),
+                                         float(reg), float(svd_tol), _p(vout), cap_v, _p(fout), cap_f, _p(ws),
+                                         ws.numel(), _p(small), C.c_void_p(small.data_ptr() + 48), st))
+            h = small.cpu()
+            V, F, A, Q, status = int(h[0]), int(h[1]), int(h[2]), int(h[4]), int(h[6] & 0xFFFFFFFF)
+            if status == _ffi.ISO_ERR_OVERFLOW:
+                cap_f = 2 * Q + 1024 if A <= cap_v else max(cap_f, 2 * A + 1024)
+                cap_v = max(cap_v, A + 1024)
+                continue
+            if status:
+                raise RuntimeError(f"isoext_gb300: device error {status} in dual_contouring")
+            if not getattr(self, "_dc_sizes", None):
+                self._dc_sizes = {}
+            self._dc_sizes[key] = (A, Q)
+            return _views(vout, fout, V, F)
+        raise RuntimeError("isoext_gb300: dual_contouring output did not fit after resizing")
+
     def _dual_contouring(self, level, its, reg, svd_tol):
         from .dc import weld_dual
 
+        if its is None and min(self.shape) >= 2 and self.get_num_cells():
+            return self._dc_one_call(level, reg, svd_tol)
         lib = _ffi.lib()
         dev = self.device
         st = _stream(dev)

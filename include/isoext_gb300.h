@@ -121,6 +121,12 @@ int iso_mc_dense(const float *values, int nx, int ny, int nz, const float *aabb_
                  const float *aabb_max, float level, int method, float *vertices,
                  long long vertex_capacity, int *faces, long long face_capacity, void *workspace,
                  size_t workspace_bytes, long long *counts, int *status, void *stream);
+/* iso_mc_dense and a wait for the stream: sizes (HOST long long[3]) <- (V, F, device
+ * status).  The device counts and status are kept in the workspace. */
+int iso_mc_dense_sync(const float *values, int nx, int ny, int nz, const float *aabb_min, const float *aabb_max,
+                      float level, int method, float *vertices, long long vertex_capacity, int *faces,
+                      long long face_capacity, void *workspace, size_t workspace_bytes, long long *sizes,
+                      void *stream);
 
 /* Marching cubes with no caller workspace. This has NO counterpart in the
  * reference: isoext allocates per call.  It is for callers that cannot give
@@ -190,6 +196,12 @@ int iso_dc_dense(const float *values, int nx, int ny, int nz, const float *aabb_
                  const float *aabb_max, float level, float reg, float svd_tol, float *vertices,
                  long long vertex_capacity, int *faces, long long face_capacity, void *workspace,
                  size_t workspace_bytes, long long *counts, int *status, void *stream);
+/* iso_dc_dense and a wait for the stream: sizes (HOST long long[6]) <- (V, F, A, K, Q, device
+ * status).  vertex_capacity is at least 1. */
+int iso_dc_dense_sync(const float *values, int nx, int ny, int nz, const float *aabb_min, const float *aabb_max,
+                      float level, float reg, float svd_tol, float *vertices, long long vertex_capacity, int *faces,
+                      long long face_capacity, void *workspace, size_t workspace_bytes, long long *sizes,
+                      void *stream);
 /* iso_dc_dense, and (each optional) the active cell ids [vertex_capacity] and
  * their crossing offsets [vertex_capacity + 1] (isoext's Intersection cells
  * and offsets), and the active cell each vertex came from [vertex_capacity]:
@@ -277,6 +289,11 @@ int iso_sparse_mc(const int *ids, const float *vals, long long n, int nx, int ny
                   const float *aabb_min, const float *aabb_max, float level, int method, float *vertices,
                   long long vertex_capacity, int *faces, long long face_capacity, void *workspace,
                   size_t workspace_bytes, long long *counts, int *status, void *stream);
+/* iso_sparse_mc and a wait for the stream: sizes (HOST long long[4]) <- (V, F, F needed, device status). */
+int iso_sparse_mc_sync(const int *ids, const float *vals, long long n, int nx, int ny, int nz,
+                       const float *aabb_min, const float *aabb_max, float level, int method, float *vertices,
+                       long long vertex_capacity, int *faces, long long face_capacity, void *workspace,
+                       size_t workspace_bytes, long long *sizes, void *stream);
 /* Sparse DC in one call with no host synchronisation: dual contouring without a
  * caller intersection (normals from each cell's values), the mesh of the
  * intersection, solve, quads and weld calls.  vertex_capacity bounds the active
@@ -288,6 +305,12 @@ int iso_sparse_dc(const int *ids, const float *values, long long n, int nx, int 
                   const float *aabb_min, const float *aabb_max, float level, float reg, float svd_tol,
                   float *vertices, long long vertex_capacity, int *faces, long long face_capacity,
                   void *workspace, size_t workspace_bytes, long long *counts, int *status, void *stream);
+/* iso_sparse_dc and a wait for the stream: sizes (HOST long long[6]) <- (V, F, A, K, Q, device
+ * status).  vertex_capacity is at least 1. */
+int iso_sparse_dc_sync(const int *ids, const float *values, long long n, int nx, int ny, int nz,
+                       const float *aabb_min, const float *aabb_max, float level, float reg, float svd_tol,
+                       float *vertices, long long vertex_capacity, int *faces, long long face_capacity,
+                       void *workspace, size_t workspace_bytes, long long *sizes, void *stream);
 /* Corner positions [m, 8, 3] of cell ids (get_points / get_points_by_cell_indices,
  * src/grid/sparse.cu:21-43). */
 int iso_sparse_points(const int *ids, long long m, int nx, int ny, int nz, const float *aabb_min,

@@ -44,6 +44,8 @@ def _declare(lib: C.CDLL) -> None:
     lib.iso_mc_dense_workspace_size.restype = C.c_size_t
     lib.iso_mc_dense.argtypes = [_vp, _i, _i, _i, _fa, _fa, _f, _i, _vp, _ll, _vp, _ll, _vp,
                                  C.c_size_t, _vp, _vp, _vp]
+    lib.iso_mc_dense_sync.argtypes = [_vp, _i, _i, _i, _fa, _fa, _f, _i, _vp, _ll, _vp, _ll, _vp, C.c_size_t,
+                                      C.POINTER(_ll), _vp]
     lib.iso_set_arith.argtypes = [_i]
     lib.iso_get_arith.restype = _i
     lib.iso_axis_coords.argtypes = [_vp, _i, _f, _f, _vp]
@@ -163,8 +165,23 @@ def in_vertex_order(v, f):
     return v, f
 
 
+_F3 = C.c_float * 3
+
+
 def fvec3(xs) -> C.Array:
-    return (C.c_float * 3)(*[float(x) for x in xs])
+    x, y, z = xs
+    return _F3(float(x), float(y), float(z))
+
+
+def raw_stream(dev) -> int:
+    """The current stream's handle on a CUDA device (one with an index)."""
+    import torch
+
+    return torch._C._cuda_getCurrentRawStream(dev.index)
+
+
+# Host sizes of the iso_*_sync calls.
+Sizes3, Sizes4, Sizes6 = _ll * 3, _ll * 4, _ll * 6
 
 
 def profile_read(kernel: str | None) -> tuple[int, float]:

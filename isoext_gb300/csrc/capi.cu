@@ -43,6 +43,33 @@ int fail_code(int code) {
     return code;
 }
 
+namespace {
+struct Pinned {
+    long long* p = nullptr;
+    ~Pinned() {
+        if (p) cudaFreeHost(p);
+    }
+};
+}  // namespace
+
+long long* host_sizes() {
+    thread_local Pinned t;
+    if (!t.p && cudaHostAlloc(reinterpret_cast<void**>(&t.p), 16 * sizeof(long long), cudaHostAllocPortable) != cudaSuccess)
+        t.p = nullptr;
+    if (t.p) std::memset(t.p, 0, 16 * sizeof(long long));
+    return t.p;
+}
+
+int wait_sizes(const long long* pinned, int n, long long* out, cudaStream_t st) {
+    const cudaError_t e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) {
+        g_err = std::string("CUDA error: ") + cudaGetErrorString(e);
+        return ISO_ERR_CUDA;
+    }
+    for (int i = 0; i < n; ++i) out[i] = const_cast<const volatile long long*>(pinned)[i];
+    return ISO_OK;
+}
+
 // Tunables: sign-pass CTAs per SM (MC and DC sign bitmaps), threads per block of
 // the per-active-cell DC kernels, threads per block of the MC count kernel.
 std::atomic<int> g_tune[TUNE_KEYS] = {{32}, {128}, {256}};
@@ -142,15 +169,16 @@ namespace {
 int mc_dense_impl(const float* values, int nx, int ny, int nz, const float* aabb_min, const float* aabb_max,
                   float level, int method, float* vertices, long long vertex_capacity, int* faces,
                   long long face_capacity, void* workspace, size_t workspace_bytes, long long* counts,
-                  int* status, long long* vertex_edges, void* stream) {
+                  int* status, long long* vertex_edges, void* stream, long long* host = nullptr) {
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     if (!grid_ok(nx, ny, nz))
         return fail(ISO_ERR_ARG, "Number of points exceeds maximum value 2147483647 (max int)");
     if (method != 0 && method != 1) return fail(ISO_ERR_ARG, "method must be 0 (nagae) or 1 (lorensen)");
-    if (!counts || !status || !aabb_min || !aabb_max)
+    if (((!counts || !status) && !host) || !aabb_min || !aabb_max)
         return fail(ISO_ERR_ARG, "counts, status and the bounding box are required");
     if (vertex_capacity < 0 || face_capacity < 0) return fail(ISO_ERR_ARG, "negative capacity");
     if (nx < 2 || ny < 2 || nz < 2) {
+        if (host) return ISO_OK;  // the sizes are 0
         // no cells: empty mesh
         if (cudaMemsetAsync(counts, 0, 2 * sizeof(long long), st) != cudaSuccess)
             return fail(ISO_ERR_CUDA, "cudaMemsetAsync failed");
@@ -177,6 +205,7 @@ int mc_dense_impl(const float* values, int nx, int ny, int nz, const float* aabb
     p.capF = face_capacity;
     p.counts = counts;
     p.vedge = vertex_edges;
+    p.host = host;
     int rc = mc_launch(p, workspace, workspace_bytes, st);
     if (rc == ISO_ERR_WORKSPACE) return fail(rc, "workspace too small");
     if (rc) {
@@ -196,6 +225,19 @@ int iso_mc_dense(const float* values, int nx, int ny, int nz, const float* aabb_
                  size_t workspace_bytes, long long* counts, int* status, void* stream) {
     return mc_dense_impl(values, nx, ny, nz, aabb_min, aabb_max, level, method, vertices, vertex_capacity, faces,
                          face_capacity, workspace, workspace_bytes, counts, status, nullptr, stream);
+}
+
+int iso_mc_dense_sync(const float* values, int nx, int ny, int nz, const float* aabb_min, const float* aabb_max,
+                      float level, int method, float* vertices, long long vertex_capacity, int* faces,
+                      long long face_capacity, void* workspace, size_t workspace_bytes, long long* sizes,
+                      void* stream) {
+    if (!sizes) return fail(ISO_ERR_ARG, "sizes is null");
+    long long* host = iso::host_sizes();
+    if (!host) return fail(ISO_ERR_CUDA, "cudaHostAlloc failed");
+    const int rc = mc_dense_impl(values, nx, ny, nz, aabb_min, aabb_max, level, method, vertices, vertex_capacity,
+                                 faces, face_capacity, workspace, workspace_bytes, nullptr, nullptr, nullptr, stream,
+                                 host);
+    return rc ? rc : iso::wait_sizes(host, 3, sizes, reinterpret_cast<cudaStream_t>(stream));
 }
 
 int iso_mc_dense_edges(const float* values, int nx, int ny, int nz, const float* aabb_min,

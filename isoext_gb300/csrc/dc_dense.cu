@@ -1219,8 +1219,14 @@ __global__ void __launch_bounds__(256) dc_cell_quads(const uint8_t* __restrict__
                                                      const uint32_t* __restrict__ offA,
                                                      const float* __restrict__ dual,
                                                      const uint32_t* __restrict__ vmap,
-                                                     const long long* __restrict__ eff, int32_t* __restrict__ faces) {
+                                                     const long long* __restrict__ eff, int32_t* __restrict__ faces,
+                                                     const long long* __restrict__ counts,
+                                                     const int* __restrict__ status, long long* host) {
     iso::grid_wait();
+    if (host && blockIdx.x == 0 && threadIdx.x == 0) {  // the sizes and the status for the host
+        for (int k = 0; k < 5; ++k) host[k] = counts[k];
+        host[5] = *status;
+    }
     const long long a = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= eff[0]) return;
     const uint32_t cid = cell_ids[a];
@@ -1545,7 +1551,7 @@ struct DcDenseWs {
     DcWs d;
     unsigned long long* zero;  // cleared by the sign pass
     long long nzero;
-    long long* misc;           // [0..1] V  [4..7] eff
+    long long* misc;           // [0..1] V  [4..7] eff  [8..12] counts [13] status when the caller has none
     unsigned long long* wblk;  // weld: representatives per block of DC_BLOCK cells
     uint32_t *wsum, *csum;     // dc_cells: 4 words per warp, per CTA
     long long ntC, ntV;        // CTAs of the dc_cells kernels and of the weld
@@ -1588,6 +1594,12 @@ DcDenseWs carve_dense(void* ws, int nx, int ny, int nz, long long capA) {
 }
 }  // namespace
 
+static int dc_dense_impl(const float* values, int nx, int ny, int nz, const float* aabb_min, const float* aabb_max,
+                         float level, float reg, float svd_tol, float* vertices, long long vertex_capacity, int* faces,
+                         long long face_capacity, void* workspace, size_t workspace_bytes, long long* counts,
+                         int* status, int* cell_ids, int* cell_offsets, int* vertex_source, long long* host,
+                         void* stream);
+
 extern "C" {
 
 size_t iso_dc_dense_workspace_size(int nx, int ny, int nz, long long vertex_capacity, long long face_capacity) {
@@ -1600,9 +1612,44 @@ int iso_dc_dense_ex(const float* values, int nx, int ny, int nz, const float* aa
                     float level, float reg, float svd_tol, float* vertices, long long vertex_capacity, int* faces,
                     long long face_capacity, void* workspace, size_t workspace_bytes, long long* counts, int* status,
                     int* cell_ids, int* cell_offsets, int* vertex_source, void* stream) {
+    return dc_dense_impl(values, nx, ny, nz, aabb_min, aabb_max, level, reg, svd_tol, vertices, vertex_capacity, faces,
+                         face_capacity, workspace, workspace_bytes, counts, status, cell_ids, cell_offsets,
+                         vertex_source, nullptr, stream);
+}
+
+int iso_dc_dense_sync(const float* values, int nx, int ny, int nz, const float* aabb_min, const float* aabb_max,
+                      float level, float reg, float svd_tol, float* vertices, long long vertex_capacity, int* faces,
+                      long long face_capacity, void* workspace, size_t workspace_bytes, long long* sizes,
+                      void* stream) {
+    if (!sizes || vertex_capacity < 1) return iso::fail_code(ISO_ERR_ARG);
+    long long* host = iso::host_sizes();
+    if (!host) return iso::fail_code(ISO_ERR_CUDA);
+    const int rc = dc_dense_impl(values, nx, ny, nz, aabb_min, aabb_max, level, reg, svd_tol, vertices,
+                                 vertex_capacity, faces, face_capacity, workspace, workspace_bytes, nullptr, nullptr,
+                                 nullptr, nullptr, nullptr, host, stream);
+    return rc ? rc : iso::wait_sizes(host, 6, sizes, reinterpret_cast<cudaStream_t>(stream));
+}
+
+int iso_dc_dense(const float* values, int nx, int ny, int nz, const float* aabb_min, const float* aabb_max,
+                 float level, float reg, float svd_tol, float* vertices, long long vertex_capacity, int* faces,
+                 long long face_capacity, void* workspace, size_t workspace_bytes, long long* counts, int* status,
+                 void* stream) {
+    return iso_dc_dense_ex(values, nx, ny, nz, aabb_min, aabb_max, level, reg, svd_tol, vertices, vertex_capacity,
+                           faces, face_capacity, workspace, workspace_bytes, counts, status, nullptr, nullptr, nullptr,
+                           stream);
+}
+
+}  // extern "C"
+
+static int dc_dense_impl(const float* values, int nx, int ny, int nz, const float* aabb_min, const float* aabb_max,
+                         float level, float reg, float svd_tol, float* vertices, long long vertex_capacity, int* faces,
+                         long long face_capacity, void* workspace, size_t workspace_bytes, long long* counts,
+                         int* status, int* cell_ids, int* cell_offsets, int* vertex_source, long long* host,
+                         void* stream) {
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    if (!counts || !status || !aabb_min || !aabb_max || vertex_capacity < 0 || face_capacity < 0) return iso::fail_code(ISO_ERR_ARG);
+    if (((!counts || !status) && !host) || !aabb_min || !aabb_max || vertex_capacity < 0 || face_capacity < 0) return iso::fail_code(ISO_ERR_ARG);
     if ((long long)nx * ny * nz > 0x7fffffffll) return iso::fail_code(ISO_ERR_ARG);
+    if (host && (nx < 2 || ny < 2 || nz < 2)) return 0;  // the sizes are 0
     if (nx < 2 || ny < 2 || nz < 2)
         return cudaMemsetAsync(counts, 0, 5 * sizeof(long long), st) == cudaSuccess ? 0 : iso::fail_code(ISO_ERR_CUDA);
     if (!values || (vertex_capacity && !vertices) || (face_capacity && !faces)) return iso::fail_code(ISO_ERR_ARG);
@@ -1612,6 +1659,8 @@ int iso_dc_dense_ex(const float* values, int nx, int ny, int nz, const float* aa
     const DcDenseWs w = carve_dense(workspace, nx, ny, nz, capA);
     const Grid3 g = make_grid(nx, ny, nz, aabb_min, aabb_max);
     long long* eff = w.misc + 4;
+    if (!counts) counts = w.misc + 8;  // cleared by the sign pass
+    if (!status) status = reinterpret_cast<int*>(w.misc + 13);
     uint32_t* cells = cell_ids ? reinterpret_cast<uint32_t*>(cell_ids) : w.cells;
     {
         iso::ProfScope ps("mc_signs", st);
@@ -1656,19 +1705,9 @@ int iso_dc_dense_ex(const float* values, int nx, int ny, int nz, const float* aa
                             static_cast<const uint32_t*>(cells), static_cast<const uint32_t*>(w.qoff),
                             static_cast<const uint32_t*>(w.d.actm), static_cast<const uint32_t*>(w.d.offA),
                             static_cast<const float*>(w.dual), static_cast<const uint32_t*>(w.vmap),
-                            static_cast<const long long*>(eff), faces);
+                            static_cast<const long long*>(eff), faces, static_cast<const long long*>(counts),
+                            static_cast<const int*>(status), host);
         }
     }
     return cudaGetLastError() == cudaSuccess ? 0 : iso::fail_code(ISO_ERR_CUDA);
 }
-
-int iso_dc_dense(const float* values, int nx, int ny, int nz, const float* aabb_min, const float* aabb_max,
-                 float level, float reg, float svd_tol, float* vertices, long long vertex_capacity, int* faces,
-                 long long face_capacity, void* workspace, size_t workspace_bytes, long long* counts, int* status,
-                 void* stream) {
-    return iso_dc_dense_ex(values, nx, ny, nz, aabb_min, aabb_max, level, reg, svd_tol, vertices, vertex_capacity,
-                           faces, face_capacity, workspace, workspace_bytes, counts, status, nullptr, nullptr, nullptr,
-                           stream);
-}
-
-}  // extern "C"

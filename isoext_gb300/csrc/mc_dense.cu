@@ -97,9 +97,9 @@ struct McWs {
     unsigned long long* vlist;  // vertex entries [capV]: pw | axis << 32 | bit << 34 | slot << 39
     unsigned long long* clist;  // cell entries [capF]: pw | bit << 32 | the word's segment-local face offset << 37
     unsigned long long* blk2;   // blk of grids cut into more than nBlk segments
-    unsigned long long* ctr;    // [0] list size [1] snaps [4] V [5] F (before the fix-up) [6] count CTAs done [7] scan ticket
+    unsigned long long* ctr;    // [0] list size [1] snaps [2] V [3] F when the caller has no counts [4] V [5] F (before the fix-up) [6] count CTAs done [7] scan ticket
                                 // [8] merges [9] small hash full [10] cell entries [12] fix-up ticket
-                                // [13] fix-up tiles done; the rest unused
+                                // [13] fix-up tiles done [14] status when the caller has none; the rest unused
     unsigned long long* state;  // look-back state per segment (follows ctr; zeroed with it)
     uint32_t* small;            // SMALL_HC entries after the states (zeroed with them)
     float* gc;                  // grid coordinates [nx + ny + nz] (x, then y, then z)
@@ -936,8 +936,14 @@ struct FixArgs {
     long long* vedge;
     long long* counts;
     int* status;
+    long long* host;  // optional: the sizes and the status for the host
     long long capV, capF;
 };
+
+__device__ __forceinline__ void fix_fail(int* status, volatile long long* host, int code) {
+    atomicCAS(status, 0, code);
+    if (host) host[2] = code;
+}
 
 __device__ __forceinline__ bool bit_of(const uint32_t* bits, uint32_t i) { return (bits[i >> 5] >> (i & 31u)) & 1u; }
 __device__ __forceinline__ void set_bit(uint32_t* bits, uint32_t i) { atomicOr(&bits[i >> 5], 1u << (i & 31u)); }
@@ -956,7 +962,8 @@ __device__ __forceinline__ uint32_t fix_rep(const McWs& w, const float* vout, ui
 }
 
 // Candidate v into the position table; the smallest index wins.
-__device__ __forceinline__ void fix_insert(const McWs& w, const float* vout, uint32_t v, int* status) {
+__device__ __forceinline__ void fix_insert(const McWs& w, const float* vout, uint32_t v, int* status,
+                                           volatile long long* host) {
     const float p[3] = {__ldcg(vout + 3ll * v), __ldcg(vout + 3ll * v + 1), __ldcg(vout + 3ll * v + 2)};
     const uint32_t mask = w.HC - 1u;
     uint32_t h = phash(pbits(p[0]), pbits(p[1]), pbits(p[2])) & mask;
@@ -968,7 +975,7 @@ __device__ __forceinline__ void fix_insert(const McWs& w, const float* vout, uin
             return;
         }
     }
-    atomicCAS(status, 0, int(ISO_ERR_OVERFLOW));
+    fix_fail(status, host, int(ISO_ERR_OVERFLOW));
 }
 
 // Ordered compaction of a tile's kept rows (row k * FIX_THREADS + tid of the tile
@@ -1015,7 +1022,17 @@ __global__ void __launch_bounds__(FIX_THREADS, FIX_CTAS) mc_fix(const FixArgs a)
     const McWs& w = a.w;
     unsigned long long* ctr = w.ctr;
     const unsigned long long nsnap = min(ctr[1], (unsigned long long)a.capV);
-    if (nsnap == 0 || (ctr[8] == 0 && ctr[9] == 0)) return;
+    volatile long long* host = a.host;
+    const bool first = host && blockIdx.x == 0 && threadIdx.x == 0;
+    if (nsnap == 0 || (ctr[8] == 0 && ctr[9] == 0)) {
+        if (first) {
+            host[0] = a.counts[0];
+            host[1] = a.counts[1];
+            host[2] = *a.status;
+        }
+        return;
+    }
+    if (first && *a.status) host[2] = *a.status;  // the merge only ever adds a failure
     const bool big = ctr[9] != 0;
     const uint32_t V = uint32_t(ctr[4]), F = uint32_t(ctr[5]);
     const int tid = threadIdx.x;
@@ -1053,7 +1070,7 @@ __global__ void __launch_bounds__(FIX_THREADS, FIX_CTAS) mc_fix(const FixArgs a)
                 uint32_t spins = 0;
                 while (*(volatile unsigned long long*)(ctr + 13) < need) {
                     if (++spins > ISO_SPIN_LIMIT) {
-                        atomicCAS(a.status, 0, int(ISO_ERR_TIMEOUT));
+                        fix_fail(a.status, host, int(ISO_ERR_TIMEOUT));
                         ok = 0;
                         break;
                     }
@@ -1075,7 +1092,7 @@ __global__ void __launch_bounds__(FIX_THREADS, FIX_CTAS) mc_fix(const FixArgs a)
             for (unsigned long long i = b0 + tid; i < min(nsnap, b0 + FIX_TILE); i += FIX_THREADS) {
                 const uint32_t v = w.snaps[i];
                 if (insert) {
-                    fix_insert(w, a.vout, v, a.status);
+                    fix_insert(w, a.vout, v, a.status, host);
                 } else {
                     const uint32_t r = fix_rep(w, a.vout, v, big);
                     if (r != v) {
@@ -1143,6 +1160,11 @@ __global__ void __launch_bounds__(FIX_THREADS, FIX_CTAS) mc_fix(const FixArgs a)
             if (t == s[6] && tid == 0) {
                 a.counts[0] = ntV ? (long long)((__ldcg(vst + ntV - 1) >> 31) & LB_MASK31) : 0;
                 a.counts[1] = Fk;
+                if (host) {
+                    host[0] = a.counts[0];
+                    host[1] = Fk;
+                    if (*(volatile int*)a.status) host[2] = *(volatile int*)a.status;  // a look-back that gave up
+                }
             }
         } else {
             const uint32_t tile = uint32_t(t - s[5]);
@@ -1263,7 +1285,7 @@ int launch_emit(const McParams& p, const McGrid& g, const McWs& w, cudaStream_t 
     }
     {
         iso::ProfScope ps("mc_fix", st);
-        const FixArgs f{w, p.vout, p.fout, p.vedge, p.counts, p.status, p.capV, p.capF};
+        const FixArgs f{w, p.vout, p.fout, p.vedge, p.counts, p.status, p.host, p.capV, p.capF};
         const long long tiles = std::max<long long>(1, (std::max(p.capV, p.capF) + FIX_TILE - 1) / FIX_TILE);
         iso::launch_pdl(mc_fix, unsigned(std::min<long long>(tiles, (long long)sms * FIX_CTAS)), unsigned(FIX_THREADS), st, f);
         if (cudaGetLastError() != cudaSuccess) return iso::fail_code(ISO_ERR_CUDA);
@@ -1347,11 +1369,14 @@ size_t mc_workspace_bytes(int nx, int ny, int nz, long long capV, long long capF
     return carve(nx, ny, nz, capV, capF, nullptr).total;
 }
 
-int mc_launch(const McParams& p, void* ws, size_t ws_bytes, cudaStream_t st) {
+int mc_launch(const McParams& params, void* ws, size_t ws_bytes, cudaStream_t st) {
+    McParams p = params;
     const McWs w0 = carve(p.nx, p.ny, p.nz, p.capV, p.capF, nullptr);
     if (ws_bytes < w0.total) return iso::fail_code(ISO_ERR_WORKSPACE);
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(ws) + 255) & ~uintptr_t(255));
     McWs w = carve(p.nx, p.ny, p.nz, p.capV, p.capF, base);
+    if (!p.counts) p.counts = reinterpret_cast<long long*>(w.ctr + 2);  // cleared by the sign pass
+    if (!p.status) p.status = reinterpret_cast<int*>(w.ctr + 14);
     McGrid g;
     g.nx = p.nx; g.ny = p.ny; g.nz = p.nz;
     g.NW = (p.nz + 31) / 32;

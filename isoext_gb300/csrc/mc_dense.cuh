@@ -31,6 +31,8 @@ struct McParams {
     long long capV, capF;
     long long* counts;  // device [0] V, [1] F
     int* status;        // device status word
+    long long* host;    // optional: pinned [0] V [1] F [2] status, written by the last kernel; counts and
+                        // status may then be null (kept in the workspace)
     long long* vedge;   // optional [capV]: per vertex, 3 * (low endpoint's point id) + axis
 };
 

@@ -1066,15 +1066,21 @@ __global__ void sp_mc_sizes2(const long long* __restrict__ tot, long long capF, 
     counts[2] = F;
 }
 
-__global__ void sp_mc_finish(const long long* __restrict__ vtot, long long capV, long long* counts, int* status) {
+__global__ void sp_mc_finish(const long long* __restrict__ vtot, long long capV, long long* counts, int* status,
+                             long long* host) {
     const long long V = vtot[0];
     counts[0] = V;
     if (V > capV) atomicCAS(status, 0, int(ISO_ERR_OVERFLOW));
+    if (host) {  // the sizes and the status for the host
+        for (int k = 0; k < 3; ++k) host[k] = counts[k];
+        host[3] = *(volatile int*)status;
+    }
 }
 
 struct SpMcWs {
     void* blk;
-    long long* tot;  // [0..1] F, vertex-list entries  [4..7] eff  [8..9] V, 0
+    long long* tot;  // [0..1] F, vertex-list entries  [4..7] eff  [8..9] V, 0  [10..12] counts [13] status when
+                     // the caller has none
     float* soup;     // the vertex list (at most 3 F entries)
     int32_t* tri;    // the triangles' indices into it [3 F]
     uint16_t* clist;  // per chunk: crossed cells (SP2_CHUNK slots each)
@@ -1108,6 +1114,48 @@ SpMcWs sp_mc_carve(void* ws, long long n, long long capV, long long capF) {
     return w;
 }
 
+}  // namespace
+
+namespace {
+int sp_mc_launch(const int* ids, const float* vals, long long n, int nx, int ny, int nz, const float* amin,
+                  const float* amax, float level, int method, float* vertices, long long vertex_capacity, int* faces,
+                  long long face_capacity, void* workspace, size_t workspace_bytes, long long* counts, int* status,
+                  long long* host, void* stream) {
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    if (((!counts || !status) && !host) || !amin || !amax || n < 0 || vertex_capacity < 0 || face_capacity < 0) return iso::fail_code(ISO_ERR_ARG);
+    if (method != 0 && method != 1) return iso::fail_code(ISO_ERR_ARG);
+    if (n == 0 && host) return 0;  // the sizes are 0
+    if (n == 0) return cudaMemsetAsync(counts, 0, 24, st) == cudaSuccess ? 0 : iso::fail_code(ISO_ERR_CUDA);
+    if (!ids || !vals || (vertex_capacity && !vertices) || (face_capacity && !faces)) return iso::fail_code(ISO_ERR_ARG);
+    if (workspace_bytes < sp_mc_carve(nullptr, n, vertex_capacity, face_capacity).total) return iso::fail_code(ISO_ERR_WORKSPACE);
+    const SpMcWs w = sp_mc_carve(workspace, n, vertex_capacity, face_capacity);
+    const SpGrid g = mk(nx, ny, nz, amin, amax, level, method);
+    long long* eff = w.tot + 4;
+    if (!counts || !status) {
+        counts = w.tot + 10;
+        status = reinterpret_cast<int*>(w.tot + 13);
+        if (cudaMemsetAsync(counts, 0, 32, st) != cudaSuccess) return iso::fail_code(ISO_ERR_CUDA);
+    }
+    {
+        iso::ProfScope ps("sparse_mc", st, 4);
+        const unsigned chunks = nb(n, SP2_CHUNK);
+        sp_mc_count2<<<chunks, SP2_THREADS, 0, st>>>(g, ids, vals, n, (unsigned long long*)w.blk, w.clist, w.ccnt,
+                                                     w.cjy, w.clen);
+        iso_block_scan_launch((unsigned long long*)w.blk, chunks, w.tot, st);
+        sp_mc_sizes2<<<1, 1, 0, st>>>(w.tot, face_capacity, vertex_capacity, eff, counts, status);
+        sp_mc_emit2<<<chunks, SP2_THREADS, 0, st>>>(g, ids, vals, n, (const unsigned long long*)w.blk, w.clist,
+                                                    w.ccnt, w.cjy, w.clen, w.soup, w.tri, eff);
+    }
+    // the weld of the vertex list: its table holds vertex_capacity distinct
+    // positions; more report an overflow with a vertex count that fits on the rerun
+    weld_dev_launch(w.soup, 3 * face_capacity, std::max<long long>(vertex_capacity, 1), w.tri, 3 * face_capacity,
+                    eff, w.weld, vertices, faces, w.tot + 8, status, st, nullptr);
+    {
+        iso::ProfScope ps("sparse_mc", st);
+        sp_mc_finish<<<1, 1, 0, st>>>(w.tot + 8, vertex_capacity, counts, status, host);
+    }
+    return cudaGetLastError() == cudaSuccess ? 0 : iso::fail_code(ISO_ERR_CUDA);
+}
 }  // namespace
 
 extern "C" {
@@ -1246,34 +1294,20 @@ int iso_sparse_mc(const int* ids, const float* vals, long long n, int nx, int ny
                   const float* amax, float level, int method, float* vertices, long long vertex_capacity, int* faces,
                   long long face_capacity, void* workspace, size_t workspace_bytes, long long* counts, int* status,
                   void* stream) {
-    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    if (!counts || !status || !amin || !amax || n < 0 || vertex_capacity < 0 || face_capacity < 0) return iso::fail_code(ISO_ERR_ARG);
-    if (method != 0 && method != 1) return iso::fail_code(ISO_ERR_ARG);
-    if (n == 0) return cudaMemsetAsync(counts, 0, 24, st) == cudaSuccess ? 0 : iso::fail_code(ISO_ERR_CUDA);
-    if (!ids || !vals || (vertex_capacity && !vertices) || (face_capacity && !faces)) return iso::fail_code(ISO_ERR_ARG);
-    if (workspace_bytes < iso_sparse_mc_workspace_size(n, vertex_capacity, face_capacity)) return iso::fail_code(ISO_ERR_WORKSPACE);
-    const SpMcWs w = sp_mc_carve(workspace, n, vertex_capacity, face_capacity);
-    const SpGrid g = mk(nx, ny, nz, amin, amax, level, method);
-    long long* eff = w.tot + 4;
-    {
-        iso::ProfScope ps("sparse_mc", st, 4);
-        const unsigned chunks = nb(n, SP2_CHUNK);
-        sp_mc_count2<<<chunks, SP2_THREADS, 0, st>>>(g, ids, vals, n, (unsigned long long*)w.blk, w.clist, w.ccnt,
-                                                     w.cjy, w.clen);
-        iso_block_scan_launch((unsigned long long*)w.blk, chunks, w.tot, st);
-        sp_mc_sizes2<<<1, 1, 0, st>>>(w.tot, face_capacity, vertex_capacity, eff, counts, status);
-        sp_mc_emit2<<<chunks, SP2_THREADS, 0, st>>>(g, ids, vals, n, (const unsigned long long*)w.blk, w.clist,
-                                                    w.ccnt, w.cjy, w.clen, w.soup, w.tri, eff);
-    }
-    // the weld of the vertex list: its table holds vertex_capacity distinct
-    // positions; more report an overflow with a vertex count that fits on the rerun
-    weld_dev_launch(w.soup, 3 * face_capacity, std::max<long long>(vertex_capacity, 1), w.tri, 3 * face_capacity,
-                    eff, w.weld, vertices, faces, w.tot + 8, status, st, nullptr);
-    {
-        iso::ProfScope ps("sparse_mc", st);
-        sp_mc_finish<<<1, 1, 0, st>>>(w.tot + 8, vertex_capacity, counts, status);
-    }
-    return cudaGetLastError() == cudaSuccess ? 0 : iso::fail_code(ISO_ERR_CUDA);
+    return sp_mc_launch(ids, vals, n, nx, ny, nz, amin, amax, level, method, vertices, vertex_capacity, faces,
+                        face_capacity, workspace, workspace_bytes, counts, status, nullptr, stream);
+}
+
+int iso_sparse_mc_sync(const int* ids, const float* vals, long long n, int nx, int ny, int nz, const float* amin,
+                       const float* amax, float level, int method, float* vertices, long long vertex_capacity,
+                       int* faces, long long face_capacity, void* workspace, size_t workspace_bytes,
+                       long long* sizes, void* stream) {
+    if (!sizes) return iso::fail_code(ISO_ERR_ARG);
+    long long* host = iso::host_sizes();
+    if (!host) return iso::fail_code(ISO_ERR_CUDA);
+    const int rc = sp_mc_launch(ids, vals, n, nx, ny, nz, amin, amax, level, method, vertices, vertex_capacity, faces,
+                                face_capacity, workspace, workspace_bytes, nullptr, nullptr, host, stream);
+    return rc ? rc : iso::wait_sizes(host, 4, sizes, reinterpret_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

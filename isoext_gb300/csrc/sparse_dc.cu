@@ -39,7 +39,7 @@ void iso_block_scan_launch(unsigned long long* blk, long long nblk, long long* t
 namespace {
 
 constexpr int SD_THREADS = 256;
-constexpr int SD_ROUNDS = 16;                       // cells per thread of the first pass
+constexpr int SD_ROUNDS = 8;                        // cells per thread of the first pass
 constexpr int SD_TILE = SD_THREADS * SD_ROUNDS;     // cells per tile
 constexpr int SD_BLOCK = 512;                       // active cells per CTA (and per block sum)
 
@@ -55,7 +55,7 @@ __device__ __forceinline__ uint32_t case8(const float4& a, const float4& b, floa
 
 // Bound by HBM (32 bytes per cell): four rounds of two 16-byte loads in flight
 // per thread.  One pass with look-back instead of a count and a second read.
-__global__ void __launch_bounds__(SD_THREADS) sd_classify(const int* __restrict__ ids,
+__global__ void __launch_bounds__(SD_THREADS, 4) sd_classify(const int* __restrict__ ids,
                                                           const float* __restrict__ vals, uint32_t n, float level,
                                                           unsigned int* ticket, unsigned long long* state,
                                                           uint32_t* __restrict__ act, uint32_t* __restrict__ lat,
@@ -102,10 +102,12 @@ __global__ void __launch_bounds__(SD_THREADS) sd_classify(const int* __restrict_
     if (lane == 0) wk[warp] = nk;
     __syncthreads();
     if (warp == 0) {
-        // the 128 (round, warp) counts, four per lane in order: the tile's total
+        // the (round, warp) counts, PER per lane in order: prefixes and the tile's total
+        constexpr int WARPS = SD_THREADS / 32, PER = SD_ROUNDS * WARPS / 32;
+        static_assert(PER * 32 == SD_ROUNDS * WARPS && SD_ROUNDS <= 32, "every lane takes PER counts");
         uint32_t s = 0;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) s += wcnt[lane >> 1][4 * (lane & 1) + k];
+        for (int k = 0; k < PER; ++k) s += wcnt[(lane * PER + k) / WARPS][(lane * PER + k) % WARPS];
         uint32_t inc = s;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
@@ -115,9 +117,10 @@ __global__ void __launch_bounds__(SD_THREADS) sd_classify(const int* __restrict_
         const uint32_t total = __shfl_sync(~0u, inc, 31);
         uint32_t run = inc - s;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const uint32_t t = wcnt[lane >> 1][4 * (lane & 1) + k];
-            wcnt[lane >> 1][4 * (lane & 1) + k] = run;
+        for (int k = 0; k < PER; ++k) {
+            uint32_t& c = wcnt[(lane * PER + k) / WARPS][(lane * PER + k) % WARPS];
+            const uint32_t t = c;
+            c = run;
             run += t;
         }
         uint32_t ks = lane < SD_THREADS / 32 ? wk[lane] : 0u;
@@ -442,9 +445,15 @@ __global__ void __launch_bounds__(SD_BLOCK) sd_faces(Grid3 g, const uint8_t* __r
                                                      const long long* __restrict__ eff,
                                                      const unsigned long long* __restrict__ blk,
                                                      const long long* __restrict__ tot, long long capF,
-                                                     int32_t* __restrict__ faces) {
+                                                     int32_t* __restrict__ faces,
+                                                     const long long* __restrict__ counts,
+                                                     const int* __restrict__ status, long long* host) {
     __shared__ uint32_t ws[SD_BLOCK / 32];
     iso::grid_wait();
+    if (host && blockIdx.x == 0 && threadIdx.x == 0) {  // the sizes and the status for the host
+        for (int k = 0; k < 5; ++k) host[k] = counts[k];
+        host[5] = *status;
+    }
     const uint32_t A = uint32_t(eff[0]);
     if (2 * tot[0] > capF) return;
     const uint32_t a = blockIdx.x * SD_BLOCK + threadIdx.x;
@@ -486,9 +495,12 @@ __global__ void __launch_bounds__(SD_BLOCK) sd_faces(Grid3 g, const uint8_t* __r
 }
 
 struct SdWs {
-    unsigned long long* state;  // look-back states, then [0] eff, [1..2] totals, [3] ticket (zeroed together)
-    long long *eff, *tot;
+    // look-back states, then [0] eff, [1..2] totals, [3] ticket, [4..8] counts and [9] status for callers without
+    // their own (zeroed together)
+    unsigned long long* state;
+    long long *eff, *tot, *counts;
     unsigned int* ticket;
+    int* status;
     size_t zero_bytes;
     unsigned long long* blk;    // (quads, representatives) per block of active cells
     uint32_t *act, *lat, *vmap, *nbr;
@@ -509,11 +521,13 @@ SdWs carve_sd(void* ws, long long n, long long capA) {
     };
     const long long ntile = (n + SD_TILE - 1) / SD_TILE;
     w.nblk = (capA + SD_BLOCK - 1) / SD_BLOCK;
-    w.zero_bytes = size_t(ntile + 4) * 8;
+    w.zero_bytes = size_t(ntile + 10) * 8;
     w.state = reinterpret_cast<unsigned long long*>(take(w.zero_bytes));
     w.eff = reinterpret_cast<long long*>(w.state) + ntile;
     w.tot = w.eff + 1;
     w.ticket = reinterpret_cast<unsigned int*>(w.eff + 3);
+    w.counts = w.eff + 4;
+    w.status = reinterpret_cast<int*>(w.eff + 9);
     w.blk = reinterpret_cast<unsigned long long*>(take(size_t(w.nblk + 1) * 16));
     w.act = reinterpret_cast<uint32_t*>(take(size_t(capA) * 4));
     w.lat = reinterpret_cast<uint32_t*>(take(size_t(capA) * 4));
@@ -528,28 +542,24 @@ SdWs carve_sd(void* ws, long long n, long long capA) {
     return w;
 }
 
-}  // namespace
-
-extern "C" {
-
-size_t iso_sparse_dc_workspace_size(long long n, long long vertex_capacity, long long face_capacity) {
-    if (n < 0 || vertex_capacity < 0 || face_capacity < 0) return 0;
-    return carve_sd(nullptr, n, vertex_capacity).total;
+size_t sd_workspace(long long n, long long capA, long long capF) {
+    return n < 0 || capA < 0 || capF < 0 ? 0 : carve_sd(nullptr, n, capA).total;
 }
 
-int iso_sparse_dc(const int* ids, const float* values, long long n, int nx, int ny, int nz, const float* aabb_min,
-                  const float* aabb_max, float level, float reg, float svd_tol, float* vertices,
-                  long long vertex_capacity, int* faces, long long face_capacity, void* workspace,
-                  size_t workspace_bytes, long long* counts, int* status, void* stream) {
+int sd_launch(const int* ids, const float* values, long long n, int nx, int ny, int nz, const float* aabb_min,
+              const float* aabb_max, float level, float reg, float svd_tol, float* vertices,
+              long long vertex_capacity, int* faces, long long face_capacity, void* workspace, size_t workspace_bytes,
+              long long* counts, int* status, long long* host, void* stream) {
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    if (!counts || !status || !aabb_min || !aabb_max || vertex_capacity < 0 || face_capacity < 0 || n > 0x7fffffffll)
+    if (((!counts || !status) && !host) || !aabb_min || !aabb_max || vertex_capacity < 0 || face_capacity < 0 || n > 0x7fffffffll)
         return iso::fail_code(ISO_ERR_ARG);
+    if (n <= 0 && host) return 0;  // the sizes are 0
     if (n <= 0)
         return cudaMemsetAsync(counts, 0, 5 * sizeof(long long), st) == cudaSuccess ? 0 : iso::fail_code(ISO_ERR_CUDA);
     if (nx < 2 || ny < 2 || nz < 2 || !ids || !values || (reinterpret_cast<uintptr_t>(values) & 15) ||
         (vertex_capacity && !vertices) || (face_capacity && !faces))
         return iso::fail_code(ISO_ERR_ARG);
-    if (workspace_bytes < iso_sparse_dc_workspace_size(n, vertex_capacity, face_capacity))
+    if (workspace_bytes < sd_workspace(n, vertex_capacity, face_capacity))
         return iso::fail_code(ISO_ERR_WORKSPACE);
     const long long capA = vertex_capacity;
     const SdWs w = carve_sd(workspace, n, capA);
@@ -559,6 +569,8 @@ int iso_sparse_dc(const int* ids, const float* values, long long n, int nx, int 
     const long long *eff = w.eff, *tot = w.tot;
     const unsigned long long* blk = w.blk;
     const float* dual = w.dual;
+    if (!counts) counts = w.counts;
+    if (!status) status = w.status;
     {
         iso::ProfScope ps("sparse_its", st);
         if (cudaMemsetAsync(w.state, 0, w.zero_bytes, st) != cudaSuccess) return iso::fail_code(ISO_ERR_CUDA);
@@ -588,10 +600,40 @@ int iso_sparse_dc(const int* ids, const float* values, long long n, int nx, int 
         {
             iso::ProfScope ps("sparse_quads", st);
             iso::launch_pdl(sd_faces, nblk, unsigned(SD_BLOCK), st, g, qbits, nbr, capA, dual, vmap, eff, blk, tot,
-                            face_capacity, faces);
+                            face_capacity, faces, static_cast<const long long*>(counts),
+                            static_cast<const int*>(status), host);
         }
     }
     return cudaGetLastError() == cudaSuccess ? 0 : iso::fail_code(ISO_ERR_CUDA);
+}
+
+}  // namespace
+
+extern "C" {
+
+size_t iso_sparse_dc_workspace_size(long long n, long long vertex_capacity, long long face_capacity) {
+    return sd_workspace(n, vertex_capacity, face_capacity);
+}
+
+int iso_sparse_dc(const int* ids, const float* values, long long n, int nx, int ny, int nz, const float* aabb_min,
+                  const float* aabb_max, float level, float reg, float svd_tol, float* vertices,
+                  long long vertex_capacity, int* faces, long long face_capacity, void* workspace,
+                  size_t workspace_bytes, long long* counts, int* status, void* stream) {
+    return sd_launch(ids, values, n, nx, ny, nz, aabb_min, aabb_max, level, reg, svd_tol, vertices, vertex_capacity,
+                     faces, face_capacity, workspace, workspace_bytes, counts, status, nullptr, stream);
+}
+
+int iso_sparse_dc_sync(const int* ids, const float* values, long long n, int nx, int ny, int nz,
+                       const float* aabb_min, const float* aabb_max, float level, float reg, float svd_tol,
+                       float* vertices, long long vertex_capacity, int* faces, long long face_capacity,
+                       void* workspace, size_t workspace_bytes, long long* sizes, void* stream) {
+    if (!sizes || vertex_capacity < 1) return iso::fail_code(ISO_ERR_ARG);
+    long long* host = iso::host_sizes();
+    if (!host) return iso::fail_code(ISO_ERR_CUDA);
+    const int rc = sd_launch(ids, values, n, nx, ny, nz, aabb_min, aabb_max, level, reg, svd_tol, vertices,
+                             vertex_capacity, faces, face_capacity, workspace, workspace_bytes, nullptr, nullptr, host,
+                             stream);
+    return rc ? rc : iso::wait_sizes(host, 6, sizes, reinterpret_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

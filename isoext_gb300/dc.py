@@ -31,6 +31,8 @@ _ffi.register({
     "iso_dc_weld_write_src": ([_vp, _ll, _vp, _ll, _vp, _vp, _vp, _vp, _vp], _i),
     "iso_dc_intersect_solve": ([_vp, _i, _i, _i, _fa, _fa, _f, _vp, _ll, _ll, _vp, _vp, _f, _f, _vp, _vp], _i),
     "iso_dc_dense_workspace_size": ([_i, _i, _i, _ll, _ll], _sz),
+    "iso_dc_dense_sync": ([_vp, _i, _i, _i, _fa, _fa, _f, _f, _f, _vp, _ll, _vp, _ll, _vp, _sz, C.POINTER(_ll), _vp],
+                          _i),
     "iso_dc_dense": ([_vp, _i, _i, _i, _fa, _fa, _f, _f, _f, _vp, _ll, _vp, _ll, _vp, _sz, _vp, _vp, _vp], _i),
 })
 
@@ -170,28 +172,35 @@ def dc_workspace_bytes(shape, cap_v: int, cap_f: int) -> int:
 
 
 def _dc_one_call(grid: UniformGrid, level, reg, svd_tol):
-    """dual_contouring without a caller intersection: iso_dc_dense, one
-    synchronisation to read the sizes (a retry with exact capacities if the
-    buffers were too small)."""
+    """dual_contouring without a caller intersection: iso_dc_dense_sync, one call
+    that launches, waits and returns the sizes (a retry with exact capacities if
+    the buffers were too small)."""
     from .mc import _first_guess, _views
 
-    dev = grid._values.device
-    key = (tuple(grid.shape), float(level), tuple(grid.aabb_min), tuple(grid.aabb_max))
+    lib = _ffi.lib()
+    values = grid._values
+    dev = values.device
+    shape, lo, hi = tuple(grid.shape), tuple(grid.aabb_min), tuple(grid.aabb_max)
+    nx, ny, nz = values.shape
+    level = float(level)
+    key = (shape, level, lo, hi)
     if key in _dc_sizes:
         a, q = _dc_sizes[key]
         cap_v, cap_f = a + a // 10 + 1024, 2 * q + (2 * q) // 10 + 1024
     else:
-        cap_v, cap_f = _first_guess(grid.shape)
-    st = torch.cuda.current_stream(dev).cuda_stream
+        cap_v, cap_f = _first_guess(shape)
+    clo, chi, sizes = _ffi.fvec3(lo), _ffi.fvec3(hi), _ffi.Sizes6()
+    st = _ffi.raw_stream(dev)
     for _ in range(2):
+        ws_bytes = dc_workspace_bytes(shape, cap_v, cap_f)
         vout = torch.empty((cap_v, 3), dtype=torch.float32, device=dev)
         fout = torch.empty((cap_f, 3), dtype=torch.int32, device=dev)
-        ws = torch.empty(dc_workspace_bytes(grid.shape, cap_v, cap_f), dtype=torch.uint8, device=dev)
-        small = torch.zeros(8, dtype=torch.int64, device=dev)
-        _ffi.check(dc_dense_into(grid._values, grid.aabb_min, grid.aabb_max, level, reg, svd_tol, vout, fout, ws,
-                                 small, st))
-        h = small.cpu()
-        V, F, A, Q, status = int(h[0]), int(h[1]), int(h[2]), int(h[4]), int(h[6] & 0xFFFFFFFF)
+        ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
+        rc = lib.iso_dc_dense_sync(values.data_ptr(), nx, ny, nz, clo, chi, level, float(reg), float(svd_tol),
+                                   vout.data_ptr(), cap_v, fout.data_ptr(), cap_f, ws.data_ptr(), ws_bytes, sizes, st)
+        if rc:
+            _ffi.check(rc)
+        V, F, A, _, Q, status = sizes
         _dc_sizes[key] = (A, Q)
         if status == _ffi.ISO_ERR_OVERFLOW:
             cap_v, cap_f = A + 1024, 2 * Q + 1024

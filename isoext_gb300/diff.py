@@ -49,11 +49,11 @@ _sizes: dict[tuple, tuple[int, int]] = {}
 
 
 def _p(t):
-    return None if t is None else C.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()
 
 
 def _stream(dev):
-    return C.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
+    return _ffi.raw_stream(dev)
 
 
 def _vec3(v):
@@ -137,7 +137,7 @@ def _collect(launches, relaunch):
     too small are queued again with exact capacities (a second one)."""
     if not launches:
         return []
-    sizes = torch.stack([L.small for L in launches]).cpu()
+    sizes = torch.stack([L.small for L in launches]).tolist()
     finish = {"mc": _mc_finish, "dc": _dc_finish}
     out, again = [None] * len(launches), []
     for i, (L, h) in enumerate(zip(launches, sizes)):
@@ -147,7 +147,7 @@ def _collect(launches, relaunch):
         else:
             out[i] = res
     if again:
-        sizes = torch.stack([L.small for _, L in again]).cpu()
+        sizes = torch.stack([L.small for _, L in again]).tolist()
         for (i, L), h in zip(again, sizes):
             res, _ = finish[L.kind](L, h)
             if res is None:
@@ -160,6 +160,7 @@ class _MarchingCubes(torch.autograd.Function):
     @staticmethod
     def forward(ctx, values, res, box):
         v, f, e = res
+        ctx.set_materialize_grads(False)  # no zero gradients of faces
         ctx.save_for_backward(values, e)
         ctx.box = box
         ctx.mark_non_differentiable(f)
@@ -274,6 +275,7 @@ class _DualContouring(torch.autograd.Function):
     @staticmethod
     def forward(ctx, values, res, meta):
         v, f, cells, offs, src = res
+        ctx.set_materialize_grads(False)  # no zero gradients of faces
         ctx.save_for_backward(values, cells, offs, src)
         ctx.meta = meta
         ctx.mark_non_differentiable(f)

@@ -3,6 +3,7 @@
 from __future__ import annotations
 
 import ctypes as C
+import functools
 
 import numpy as np
 import torch
@@ -63,6 +64,11 @@ def workspace_bytes(shape, cap_v: int, cap_f: int) -> int:
 
 
 def coarse_float_grid(shape, aabb_min, aabb_max) -> bool:
+    return _coarse(tuple(shape), tuple(aabb_min), tuple(aabb_max))
+
+
+@functools.lru_cache(maxsize=256)
+def _coarse(shape, aabb_min, aabb_max) -> bool:
     """True when grid spacing is within 64 ulps of the coordinates' magnitude.
 
     Vertices are identified by grid key; isoext identifies them by exact
@@ -94,39 +100,53 @@ def weld_by_position(v: torch.Tensor, f: torch.Tensor):
 
 
 def _mc_uniform(grid: UniformGrid, level: float, method: int):
+    dev = grid._values.device
+    if torch.cuda.current_device() != dev.index:
+        with torch.cuda.device(dev):
+            return _mc_on_device(grid, level, method)
+    return _mc_on_device(grid, level, method)
+
+
+def _mc_on_device(grid: UniformGrid, level: float, method: int):
+    """iso_mc_dense_sync: one call that launches, waits and returns the sizes."""
+    lib = _ffi.lib()
     values = grid._values
     dev = values.device
-    key = (tuple(grid.shape), method, float(level), tuple(grid.aabb_min), tuple(grid.aabb_max))
+    shape, lo, hi = tuple(grid.shape), tuple(grid.aabb_min), tuple(grid.aabb_max)
+    nx, ny, nz = values.shape
+    level = float(level)
+    key = (shape, method, level, lo, hi)
     if key in _size_cache:
         nv, nf = _size_cache[key]
         cap_v, cap_f = nv + nv // 10 + 1024, nf + nf // 10 + 1024
     else:
-        cap_v, cap_f = _first_guess(grid.shape)
-    with torch.cuda.device(dev):
-        stream = torch.cuda.current_stream(dev).cuda_stream
-        need = None  # sizes before the snap fix-up shrank them, after a retry
-        for _attempt in range(2):
-            vout = torch.empty((cap_v, 3), dtype=torch.float32, device=dev)
-            fout = torch.empty((cap_f, 3), dtype=torch.int32, device=dev)
-            ws = torch.empty(workspace_bytes(grid.shape, cap_v, cap_f), dtype=torch.uint8, device=dev)
-            small = torch.zeros(4, dtype=torch.int64, device=dev)
-            _ffi.check(mc_dense_into(values, grid.aabb_min, grid.aabb_max, level, method, vout, fout,
-                                     ws, small, stream))
-            host = small.cpu()
-            nv, nf, status = int(host[0]), int(host[1]), int(host[2] & 0xffffffff)
-            if status == _ffi.ISO_ERR_OVERFLOW:
-                cap_v, cap_f = nv + 1024, nf + 1024
-                need = (nv, nf)
-                continue
-            if status != 0:
-                raise RuntimeError(f"isoext_gb300: device error {status} in marching_cubes")
-            # counts are final sizes; output buffers must hold the sizes before
-            # snapped vertices were merged, which a retry revealed
-            _size_cache[key] = need if need is not None else (nv, nf)
-            v, f = _views(vout, fout, nv, nf)
-            if v is not None and coarse_float_grid(grid.shape, grid.aabb_min, grid.aabb_max):
-                v, f = weld_by_position(v, f)
-            return v, f
+        cap_v, cap_f = _first_guess(shape)
+    clo, chi, sizes = _ffi.fvec3(lo), _ffi.fvec3(hi), _ffi.Sizes3()
+    stream = _ffi.raw_stream(dev)
+    need = None  # sizes before the snap fix-up shrank them, after a retry
+    for _attempt in range(2):
+        ws_bytes = workspace_bytes(shape, cap_v, cap_f)
+        vout = torch.empty((cap_v, 3), dtype=torch.float32, device=dev)
+        fout = torch.empty((cap_f, 3), dtype=torch.int32, device=dev)
+        ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
+        rc = lib.iso_mc_dense_sync(values.data_ptr(), nx, ny, nz, clo, chi, level, method, vout.data_ptr(), cap_v,
+                                   fout.data_ptr(), cap_f, ws.data_ptr(), ws_bytes, sizes, stream)
+        if rc:
+            _ffi.check(rc)
+        nv, nf, status = sizes
+        if status == _ffi.ISO_ERR_OVERFLOW:
+            cap_v, cap_f = nv + 1024, nf + 1024
+            need = (nv, nf)
+            continue
+        if status != 0:
+            raise RuntimeError(f"isoext_gb300: device error {status} in marching_cubes")
+        # counts are final sizes; output buffers must hold the sizes before
+        # snapped vertices were merged, which a retry revealed
+        _size_cache[key] = need if need is not None else (nv, nf)
+        v, f = _views(vout, fout, nv, nf)
+        if v is not None and _coarse(shape, lo, hi):
+            v, f = weld_by_position(v, f)
+        return v, f
     raise RuntimeError("isoext_gb300: marching_cubes output did not fit after resizing")
 
 

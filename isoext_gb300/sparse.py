@@ -36,6 +36,10 @@ _ffi.register({
     "iso_sparse_dc_workspace_size": ([_ll, _ll, _ll], _sz),
     "iso_sparse_dc": ([_vp, _vp, _ll, _i, _i, _i, _fa, _fa, _f, _f, _f, _vp, _ll, _vp, _ll, _vp, _sz, _vp, _vp, _vp],
                       _i),
+    "iso_sparse_dc_sync": ([_vp, _vp, _ll, _i, _i, _i, _fa, _fa, _f, _f, _f, _vp, _ll, _vp, _ll, _vp, _sz,
+                            C.POINTER(_ll), _vp], _i),
+    "iso_sparse_mc_sync": ([_vp, _vp, _ll, _i, _i, _i, _fa, _fa, _f, _i, _vp, _ll, _vp, _ll, _vp, _sz, C.POINTER(_ll),
+                            _vp], _i),
     "iso_sparse_mc_workspace_size": ([_ll, _ll, _ll], _sz),
     "iso_sparse_mc": ([_vp, _vp, _ll, _i, _i, _i, _fa, _fa, _f, _i, _vp, _ll, _vp, _ll, _vp, _sz, _vp, _vp, _vp], _i),
 })
@@ -297,8 +301,9 @@ class SparseGrid(SparseGridBase):
         n = self.get_num_cells()
         if n == 0:
             return None, None
-        st = _stream(dev)
+        st = _ffi.raw_stream(dev)
         sx, sy, sz, lo, hi = self._geom()
+        sizes = _ffi.Sizes4()
         key = (n, float(level), int(method))
         if getattr(self, "_mc_sizes", None) and key in self._mc_sizes:
             v, f = self._mc_sizes[key]
@@ -309,13 +314,14 @@ class SparseGrid(SparseGridBase):
         for _ in range(2):
             vout = torch.empty((cap_v, 3), dtype=torch.float32, device=dev)
             fout = torch.empty((cap_f, 3), dtype=torch.int32, device=dev)
-            ws = torch.empty(int(lib.iso_sparse_mc_workspace_size(n, cap_v, cap_f)), dtype=torch.uint8, device=dev)
-            small = torch.zeros(4, dtype=torch.int64, device=dev)
-            _ffi.check(lib.iso_sparse_mc(_p(self._ids), _p(self._values), n, sx, sy, sz, lo, hi, float(level),
-                                         int(method), _p(vout), cap_v, _p(fout), cap_f, _p(ws), ws.numel(),
-                                         _p(small), C.c_void_p(small.data_ptr() + 24), st))
-            h = small.cpu()
-            V, F, Fneed, status = int(h[0]), int(h[1]), int(h[2]), int(h[3] & 0xFFFFFFFF)
+            ws_bytes = int(lib.iso_sparse_mc_workspace_size(n, cap_v, cap_f))
+            ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
+            rc = lib.iso_sparse_mc_sync(self._ids.data_ptr(), self._values.data_ptr(), n, sx, sy, sz, lo, hi,
+                                        float(level), int(method), vout.data_ptr(), cap_v, fout.data_ptr(), cap_f,
+                                        ws.data_ptr(), ws_bytes, sizes, st)
+            if rc:
+                _ffi.check(rc)
+            V, F, Fneed, status = sizes
             if not getattr(self, "_mc_sizes", None):
                 self._mc_sizes = {}
             self._mc_sizes[key] = (max(V, 1), max(Fneed, 1))
@@ -364,8 +370,9 @@ class SparseGrid(SparseGridBase):
         lib = _ffi.lib()
         dev = self.device
         n = self.get_num_cells()
-        st = _stream(dev)
+        st = _ffi.raw_stream(dev)
         sx, sy, sz, lo, hi = self._geom()
+        sizes = _ffi.Sizes6()
         key = (n, float(level))
         if getattr(self, "_dc_sizes", None) and key in self._dc_sizes:
             a, q = self._dc_sizes[key]
@@ -374,16 +381,17 @@ class SparseGrid(SparseGridBase):
             # a band of a few cells on each side of the surface
             cap_v = min(n, n // 4 + 4096)
             cap_f = 2 * cap_v
-        for _ in range(3):
+        for _attempt in range(3):
             vout = torch.empty((cap_v, 3), dtype=torch.float32, device=dev)
             fout = torch.empty((cap_f, 3), dtype=torch.int32, device=dev)
-            ws = torch.empty(int(lib.iso_sparse_dc_workspace_size(n, cap_v, cap_f)), dtype=torch.uint8, device=dev)
-            small = torch.zeros(8, dtype=torch.int64, device=dev)
-            _ffi.check(lib.iso_sparse_dc(_p(self._ids), _p(self._values), n, sx, sy, sz, lo, hi, float(level),
-                                         float(reg), float(svd_tol), _p(vout), cap_v, _p(fout), cap_f, _p(ws),
-                                         ws.numel(), _p(small), C.c_void_p(small.data_ptr() + 48), st))
-            h = small.cpu()
-            V, F, A, Q, status = int(h[0]), int(h[1]), int(h[2]), int(h[4]), int(h[6] & 0xFFFFFFFF)
+            ws_bytes = int(lib.iso_sparse_dc_workspace_size(n, cap_v, cap_f))
+            ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
+            rc = lib.iso_sparse_dc_sync(self._ids.data_ptr(), self._values.data_ptr(), n, sx, sy, sz, lo, hi,
+                                        float(level), float(reg), float(svd_tol), vout.data_ptr(), cap_v,
+                                        fout.data_ptr(), cap_f, ws.data_ptr(), ws_bytes, sizes, st)
+            if rc:
+                _ffi.check(rc)
+            V, F, A, _, Q, status = sizes
             if status == _ffi.ISO_ERR_OVERFLOW:
                 cap_f = 2 * Q + 1024 if A <= cap_v else max(cap_f, 2 * A + 1024)
                 cap_v = max(cap_v, A + 1024)

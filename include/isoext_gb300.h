@@ -202,6 +202,23 @@ int iso_dc_dense_sync(const float *values, int nx, int ny, int nz, const float *
                       float level, float reg, float svd_tol, float *vertices, long long vertex_capacity, int *faces,
                       long long face_capacity, void *workspace, size_t workspace_bytes, long long *sizes,
                       void *stream);
+/* iso_dc_dense_sync with a caller's intersection (points, offsets and cell ids of A >= 1 active cells, as
+ * iso_dc_intersection_sync gives them; normals may be null: taken from the grid).  vertices [A, 3].  The
+ * device status is ISO_ERR_LOOKUP when the cells are not the grid's active cells at level (its values have
+ * changed since): nothing of the output is then valid. */
+int iso_dc_dense_its_sync(const float *values, int nx, int ny, int nz, const float *aabb_min, const float *aabb_max,
+                          float level, float reg, float svd_tol, const float *points, const float *normals,
+                          const int *cell_ids, const int *cell_offsets, long long A, float *vertices, int *faces,
+                          long long face_capacity, void *workspace, size_t workspace_bytes, long long *sizes,
+                          void *stream);
+/* The intersection in one call and a wait for the stream: points [point_capacity, 3], optional normals, cell ids
+ * [cell_capacity] and CSR offsets [cell_capacity + 1]; a workspace of
+ * iso_dc_dense_workspace_size(nx, ny, nz, cell_capacity, 0).  sizes (HOST long long[6]) <- (0, -, A, K, Q, device
+ * status): active cells, crossings, quads; status 6 when A or K exceed the capacities. */
+int iso_dc_intersection_sync(const float *values, int nx, int ny, int nz, const float *aabb_min,
+                             const float *aabb_max, float level, float *points, float *normals,
+                             long long point_capacity, int *cell_ids, int *cell_offsets, long long cell_capacity,
+                             void *workspace, size_t workspace_bytes, long long *sizes, void *stream);
 /* iso_dc_dense, and (each optional) the active cell ids [vertex_capacity] and
  * their crossing offsets [vertex_capacity + 1] (isoext's Intersection cells
  * and offsets), and the active cell each vertex came from [vertex_capacity]:

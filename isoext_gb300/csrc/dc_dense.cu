@@ -681,17 +681,18 @@ __global__ void dc_remap(const int32_t* __restrict__ tri, long long n, const uin
 
 
 // ---------------------------------------------------------------------------
-// One-call dual contouring: after the sign pass, eight kernels chained by
+// One-call dual contouring: after the sign pass, six or seven kernels chained by
 // programmatic dependent launch, with the sizes kept on the device.
 //
-//   dc_cells_count / _scan / _write
-//                  per point word: active cells, crossings, and the quads each
-//                  active cell owns.  A quad's owner is the cell whose lowest
-//                  corner is the low endpoint of the quad's edge, so the
-//                  reference's quad order (low endpoint, then z, y, x edge) is
-//                  the owners' order.  Counts per warp, one CTA scans them and
-//                  checks the sizes, then the words are written with offsets.
-//   dc_cell_solve  the QEF solve and whether faces use the cell.
+//   dc_cells (/ dc_cells_scan)
+//                  the active cells, their crossings, and the quads each of them
+//                  owns, per segment of point words.  A quad's owner is the cell
+//                  whose lowest corner is the low endpoint of the quad's edge, so
+//                  the reference's quad order (low endpoint, then z, y, x edge)
+//                  is the owners' order.  The segments' sums are scanned and
+//                  checked against the sizes.
+//   dc_solve_cells per entry: its cell's number, the QEF solve and whether faces
+//                  use the cell.
 //   dc_weld_flags / dc_block_scan / dc_weld_number
 //                  the exact-position weld.  A dual vertex is clipped to its
 //                  cell's closed box, and the boxes of different cells meet only
@@ -703,17 +704,62 @@ __global__ void dc_remap(const int32_t* __restrict__ tri, long long n, const uin
 //   dc_cell_quads  each active cell's quads with the final vertex numbers.
 
 // Crossed edges of one cell (bit b of a cell word): the 12 corner-sign XORs.
-__device__ __forceinline__ uint32_t cell_crossings(const uint32_t* ex, int b) {
+__device__ __forceinline__ uint32_t cell_crossings(const uint32_t* cw8, int b) {
     uint32_t n = 0;
 #pragma unroll
-    for (int e = 0; e < 12; ++e) n += (ex[e] >> b) & 1u;
+    for (int e = 0; e < 12; ++e) n += ((cw8[iso_edge_corner(2 * e)] ^ cw8[iso_edge_corner(2 * e + 1)]) >> b) & 1u;
     return n;
 }
 
-constexpr int CELLS_THREADS = 256;  // dc_cells: threads per CTA
-constexpr int CELLS_WPT = 4;        // point words per thread and round (one 16-byte load per row)
-constexpr int CELLS_ROUNDS = 2;
-constexpr int CELLS_TILE = CELLS_THREADS * CELLS_WPT * CELLS_ROUNDS;  // point words per CTA
+constexpr int CELLS_THREADS = 256;
+constexpr int CELLS_WARPS = CELLS_THREADS / 32;
+constexpr int CELLS_QUEUE = 512;      // cells a warp lays out at a time
+// Point words per thread: four, or one on grids whose CTAs of four words per
+// thread would leave SMs idle (256 x 256 x 128 points; the count of marching cubes
+// has the same rule).
+constexpr long long CELLS_FINE = 1ll << 18;
+// Segments that the last CTA of dc_cells scans itself; with more, the fence and
+// the atomic of every CTA cost more than the launch of dc_cells_scan.
+constexpr uint32_t CELLS_SCAN = 1024;
+
+// Geometry of the flat point-word bitmap and its segments (one CTA of dc_cells
+// each).
+struct PwGrid {
+    int NWg;
+    uint32_t syw, sxw, PW;  // row stride, plane stride, point words (< 2^32)
+    bool vec;               // rows start on 16-byte boundaries
+    int lgseg;              // log2 of the point words per segment
+    uint32_t nseg;
+};
+
+PwGrid pw_grid(const Grid3& g) {
+    PwGrid p;
+    p.NWg = (g.nz + 31) / 32;
+    p.syw = uint32_t(p.NWg);
+    p.sxw = uint32_t(g.ny) * p.syw;
+    p.PW = uint32_t(g.nx) * p.sxw;
+    p.vec = (p.NWg & 3) == 0;
+    p.lgseg = (long long)p.PW <= CELLS_FINE ? 8 : 10;
+    p.nseg = uint32_t(((unsigned long long)p.PW + (1ull << p.lgseg) - 1) >> p.lgseg);
+    return p;
+}
+
+// What dc_cells leaves for the other kernels.
+struct CellIndex {
+    PwGrid p;
+    uint32_t* actm;             // per point word: its active cells
+    uint32_t* offA;             // per word with active cells: their first's index within the segment
+    uint4* seg;                 // per segment: active cells, owned quads and crossings before it
+    unsigned long long* elist;  // per active cell, unordered: word | bit << 32 | quad bits << 37 | quad offset << 41
+    uint32_t* klist;            // per entry: its crossings' offset within the segment (only when asked for)
+};
+
+__device__ __forceinline__ void pw_xyw(const Grid3& g, const PwGrid& p, uint32_t pw, int& x, int& y, int& w) {
+    const uint32_t row = pw / p.syw;
+    w = int(pw - row * p.syw);
+    x = int(row / uint32_t(g.ny));
+    y = int(row - uint32_t(x) * uint32_t(g.ny));
+}
 
 // Owned quad edges of a cell word's active cells: corner 0 to corner 1 (z),
 // 2 (y), 4 (x); complete when the edge's other two coordinates are >= 1 (the
@@ -726,212 +772,18 @@ __device__ __forceinline__ void owned_quads(const Grid3& g, const uint32_t* cw8,
     qx = cy >= 1 ? (cw8[0] ^ cw8[4]) & act & zin : 0u;
 }
 
-// The sign words pw .. pw+3 of the rows (x, y), (x, y+1), (x+1, y), (x+1, y+1)
-// of point word pw (flat offsets 0, syw, sxw, sxw + syw), and each row's word
-// pw+4 (the next lane's first word, or a load).  All lanes call it.
-struct QuadRows {
-    uint32_t r[4][CELLS_WPT];  // row k = 2 dx + dy
-    uint32_t n4[4];
-};
-
-__device__ __forceinline__ void load_quad_rows(const uint32_t* __restrict__ S, uint32_t pw, uint32_t sxw,
-                                               uint32_t syw, uint32_t PW, bool vec, int lane, QuadRows& q) {
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const uint32_t o = pw + (k >> 1) * sxw + (k & 1) * syw;
-        if (vec && o + CELLS_WPT <= PW) {
-            const uint4 v4 = __ldg(reinterpret_cast<const uint4*>(S + o));
-            q.r[k][0] = v4.x; q.r[k][1] = v4.y; q.r[k][2] = v4.z; q.r[k][3] = v4.w;
-        } else {
-#pragma unroll
-            for (int j = 0; j < CELLS_WPT; ++j) q.r[k][j] = o + j < PW ? __ldg(S + o + j) : 0u;
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        q.n4[k] = __shfl_down_sync(~0u, q.r[k][0], 1);
-        if (lane == 31) {
-            const uint32_t o = pw + CELLS_WPT + (k >> 1) * sxw + (k & 1) * syw;
-            q.n4[k] = o < PW ? __ldg(S + o) : 0u;
-        }
-    }
-}
-
-// No cell of the lane's words can be active: all 20 words equal, all 0 or ~0.
-__device__ __forceinline__ bool quad_rows_quiet(const QuadRows& q) {
-    const uint32_t u = q.r[0][0];
-    uint32_t d = 0;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        d |= q.n4[k] ^ u;
-#pragma unroll
-        for (int j = 0; j < CELLS_WPT; ++j) d |= q.r[k][j] ^ u;
-    }
-    return (u == 0u || u == ~0u) && d == 0u;
-}
-
-// Corner words (cw8[2k]: dz 0, cw8[2k+1]: dz 1) and active cells of word j of
-// the lane, point word (x, y, w).
-__device__ __forceinline__ uint32_t quad_word_act(const Grid3& g, int nwg, int nwc, const QuadRows& q, int j, int x,
-                                                  int y, int w, uint32_t* cw8) {
-    const bool nxt = w + 1 < nwg;
-    uint32_t and8 = ~0u, or8 = 0u;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const uint32_t a = q.r[k][j];
-        const uint32_t nb = nxt ? (j + 1 < CELLS_WPT ? q.r[k][(j + 1) % CELLS_WPT] : q.n4[k]) : 0u;
-        const uint32_t b = __funnelshift_r(a, nb, 1);  // bit z <- z + 1
-        cw8[2 * k] = a;
-        cw8[2 * k + 1] = b;
-        and8 &= a & b;
-        or8 |= a | b;
-    }
-    if (x >= g.nx - 1 || y >= g.ny - 1 || w >= nwc) return 0u;
-    return (or8 & ~and8) & iso::range_mask(w, 0, g.nz - 2);
-}
-
-// Next point word in (x, y, w) order.
-__device__ __forceinline__ void next_point_word(const Grid3& g, int nwg, int& x, int& y, int& w) {
-    if (++w == nwg) {
-        w = 0;
-        if (++y == g.ny) { y = 0; ++x; }
-    }
-}
-
-// Geometry of the flat point-word bitmap, shared by the dc_cells kernels.
-struct PwGrid {
-    int NWg, NWc;
-    uint32_t syw, sxw, PW;  // row stride, plane stride, point words (< 2^32)
-    bool vec;               // rows start on 16-byte boundaries
-};
-
-__device__ __forceinline__ PwGrid pw_grid(const Grid3& g) {
-    PwGrid p;
-    p.NWg = (g.nz + 31) / 32;
-    p.NWc = (g.nz - 1 + 31) / 32;
-    p.syw = uint32_t(p.NWg);
-    p.sxw = uint32_t(g.ny) * p.syw;
-    p.PW = uint32_t(g.nx) * p.sxw;
-    p.vec = (p.NWg & 3) == 0;
-    return p;
-}
-
-// Round j of a lane of warp gw (over the grid): point words pw .. pw + 3.  A
-// warp's rounds are consecutive, so its words are too.
-__device__ __forceinline__ uint32_t cells_pw(uint32_t gw, int lane, int j) {
-    return gw * uint32_t(32 * CELLS_WPT * CELLS_ROUNDS) + uint32_t(j * 32 * CELLS_WPT) + uint32_t(lane * CELLS_WPT);
-}
-
-__device__ __forceinline__ void pw_xyw(const Grid3& g, const PwGrid& p, uint32_t pw, int& x, int& y, int& w) {
-    const uint32_t row = pw / p.syw;
-    w = int(pw - row * p.syw);
-    x = int(row / uint32_t(g.ny));
-    y = int(row - uint32_t(x) * uint32_t(g.ny));
-}
-
-// Per warp of 256 point words (flat bitmap order (x, y, w), which orders cells
-// as their ids do): the active masks (written here), and the counts of active
-// cells, owned quads and crossings.  A lane takes 4 consecutive words per
-// round: one 16-byte load per row, and a warp whose 128 words are all inside
-// or outside skips the rest.  wsum[warp] = the warp's exclusive prefix within
-// its CTA and its busy rounds; csum[CTA] = the CTA's sums.
-constexpr int CELLS_WARPS = CELLS_THREADS / 32;
-
-__device__ __forceinline__ void store_masks(uint32_t* __restrict__ m, uint32_t pw, uint32_t PW, const uint32_t* v) {
-    if (pw + CELLS_WPT <= PW) {
-        *reinterpret_cast<uint4*>(m + pw) = make_uint4(v[0], v[1], v[2], v[3]);
-    } else {
-        for (int k = 0; k < CELLS_WPT; ++k)
-            if (pw + k < PW) m[pw + k] = v[k];
-    }
-}
-
-__global__ void __launch_bounds__(CELLS_THREADS, 4) dc_cells_count(const uint32_t* __restrict__ S, Grid3 g,
-                                                                   uint32_t* __restrict__ actm,
-                                                                   uint32_t* __restrict__ wsum,
-                                                                   uint32_t* __restrict__ csum,
-                                                                   float* __restrict__ gc) {
-    __shared__ uint32_t ws[3][CELLS_WARPS];
-    iso::grid_wait();
-    // the grid's coordinates (x, then y, then z), read by the solve
-    for (uint32_t i = blockIdx.x * CELLS_THREADS + threadIdx.x; i < uint32_t(g.nx + g.ny + g.nz);
-         i += gridDim.x * CELLS_THREADS) {
-        const int axis = i < uint32_t(g.nx) ? 0 : (i < uint32_t(g.nx + g.ny) ? 1 : 2);
-        const uint32_t k = i - (axis > 0 ? uint32_t(g.nx) : 0u) - (axis > 1 ? uint32_t(g.ny) : 0u);
-        gc[i] = coord(g, axis, k);
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t gw = blockIdx.x * CELLS_WARPS + warp;
-    const PwGrid p = pw_grid(g);
-    uint32_t sa = 0, sq = 0, sk = 0, busy = 0;
-    for (int j = 0; j < CELLS_ROUNDS; ++j) {
-        const uint32_t pw = cells_pw(gw, lane, j);
-        QuadRows q;
-        load_quad_rows(S, pw, p.sxw, p.syw, p.PW, p.vec, lane, q);
-        uint32_t act[CELLS_WPT] = {0u, 0u, 0u, 0u};
-        if (!__all_sync(~0u, quad_rows_quiet(q) || pw >= p.PW)) {
-            busy |= 1u << j;
-            int x = 0, y = 0, w = 0;
-            if (pw < p.PW) pw_xyw(g, p, pw, x, y, w);
-#pragma unroll
-            for (int k = 0; k < CELLS_WPT; ++k) {
-                uint32_t cw8[8];
-                act[k] = pw + k < p.PW ? quad_word_act(g, p.NWg, p.NWc, q, k, x, y, w, cw8) : 0u;
-                if (act[k]) {
-                    uint32_t qz, qy, qx;
-                    owned_quads(g, cw8, act[k], x, y, w, qz, qy, qx);
-                    sa += __popc(act[k]);
-                    sq += __popc(qz) + __popc(qy) + __popc(qx);
-                    sk += word_crossings(cw8, act[k]);
-                }
-                next_point_word(g, p.NWg, x, y, w);
-            }
-        }
-        if (pw < p.PW) store_masks(actm, pw, p.PW, act);
-    }
-#pragma unroll
-    for (int d = 16; d >= 1; d >>= 1) {
-        sa += __shfl_xor_sync(~0u, sa, d);
-        sq += __shfl_xor_sync(~0u, sq, d);
-        sk += __shfl_xor_sync(~0u, sk, d);
-    }
-    if (lane == 0) { ws[0][warp] = sa; ws[1][warp] = sq; ws[2][warp] = sk; }
-    __syncthreads();
-    if (warp == 0) {
-        uint32_t e[3], t[3];
-#pragma unroll
-        for (int v = 0; v < 3; ++v) {
-            const uint32_t x = lane < CELLS_WARPS ? ws[v][lane] : 0u;
-            uint32_t incl = x;
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const uint32_t u = __shfl_up_sync(~0u, incl, d);
-                if (lane >= d) incl += u;
-            }
-            e[v] = incl - x;
-            t[v] = __shfl_sync(~0u, incl, 31);
-        }
-        if (lane < CELLS_WARPS) *reinterpret_cast<uint4*>(wsum + 4u * (blockIdx.x * CELLS_WARPS + lane)) =
-            make_uint4(e[0], e[1], e[2], 0u);
-        if (lane == 0) *reinterpret_cast<uint4*>(csum + 4u * blockIdx.x) = make_uint4(t[0], t[1], t[2], 0u);
-    }
-    __syncthreads();  // the record's busy word after warp 0's store of the prefixes
-    if (lane == 0) wsum[4u * gw + 3] = busy;
-}
-
-// One CTA: exclusive scan of the CTAs' (active, quads, crossings) sums in
-// place, the totals checked against the capacities.
-__global__ void __launch_bounds__(1024) dc_cells_scan(uint32_t* __restrict__ csum, long long ncta, long long capA,
-                                                      long long capQ, long long* eff, long long* counts,
-                                                      uint32_t* __restrict__ cell_off, int* status) {
-    __shared__ unsigned long long part[3][32], carry[3];
-    iso::grid_wait();
+// Exclusive scan of the segments' (active, quads, crossings) sums in place by
+// one CTA of T threads, and the totals against the capacities.
+template <int T>
+__device__ void scan_cells(uint4* seg, uint32_t nseg, long long capA, long long capQ, long long capK, long long* eff,
+                           long long* counts, uint32_t* __restrict__ cell_off, int* status) {
+    __shared__ unsigned long long part[3][T / 32], carry[3];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid < 3) carry[tid] = 0;
     __syncthreads();
-    for (long long base = 0; base < ncta; base += 1024) {
-        const long long i = base + tid;
-        const uint4 v = i < ncta ? *reinterpret_cast<const uint4*>(csum + 4 * i) : make_uint4(0u, 0u, 0u, 0u);
+    for (uint32_t base = 0; base < nseg; base += T) {
+        const uint32_t i = base + tid;
+        const uint4 v = i < nseg ? __ldcg(seg + i) : make_uint4(0u, 0u, 0u, 0u);
         const unsigned long long c[3] = {v.x, v.y, v.z};
         unsigned long long in[3] = {v.x, v.y, v.z};
 #pragma unroll
@@ -945,33 +797,26 @@ __global__ void __launch_bounds__(1024) dc_cells_scan(uint32_t* __restrict__ csu
 #pragma unroll
             for (int t = 0; t < 3; ++t) part[t][warp] = in[t];
         __syncthreads();
-        if (warp == 0) {
-#pragma unroll
-            for (int t = 0; t < 3; ++t) {
-                unsigned long long x = part[t][lane];
-#pragma unroll
-                for (int d = 1; d < 32; d <<= 1) {
-                    const unsigned long long u = __shfl_up_sync(~0u, x, d);
-                    if (lane >= d) x += u;
-                }
-                part[t][lane] = x;
-            }
-        }
-        __syncthreads();
-        if (i < ncta) {
+        if (i < nseg) {
             unsigned long long e[3];
 #pragma unroll
-            for (int t = 0; t < 3; ++t) e[t] = carry[t] + (warp ? part[t][warp - 1] : 0ull) + in[t] - c[t];
+            for (int t = 0; t < 3; ++t) {
+                e[t] = carry[t] + in[t] - c[t];
+#pragma unroll
+                for (int q = 0; q < T / 32; ++q) e[t] += q < warp ? part[t][q] : 0ull;
+            }
             // offsets past 2^32 only matter when the sizes overflow (then nothing is used)
-            *reinterpret_cast<uint4*>(csum + 4 * i) = make_uint4(uint32_t(e[0]), uint32_t(e[1]), uint32_t(e[2]), 0u);
+            seg[i] = make_uint4(uint32_t(e[0]), uint32_t(e[1]), uint32_t(e[2]), 0u);
         }
         __syncthreads();
-        if (tid < 3) carry[tid] += part[tid][31];
+        if (tid < 3)
+            for (int q = 0; q < T / 32; ++q) carry[tid] += part[tid][q];
         __syncthreads();
     }
     if (tid == 0) {
         const long long A = (long long)carry[0], Q = (long long)carry[1], K = (long long)carry[2];
-        const bool ok = A <= capA && Q <= capQ && A < 0x7fffffffll && K < 0x7fffffffll && 6 * Q < 0x7fffffffll;
+        const bool ok = A <= capA && Q <= capQ && K <= capK && A < 0x7fffffffll && K < 0x7fffffffll &&
+                        6 * Q < 0x7fffffffll;
         if (!ok) atomicCAS(status, 0, int(ISO_ERR_OVERFLOW));
         eff[0] = ok ? A : 0;
         eff[1] = ok ? K : 0;
@@ -986,116 +831,382 @@ __global__ void __launch_bounds__(1024) dc_cells_scan(uint32_t* __restrict__ csu
     }
 }
 
-// The busy rounds of dc_cells_count again, with each warp's offsets: active
-// prefixes per point word (rounds without an active cell have none to look
-// up), and per active cell its id, its first owned quad, its owned quad edges
-// (bits 0-2: z, y, x) with the sign of its lowest corner (bit 3), and (when
-// asked) its first crossing.
-__global__ void __launch_bounds__(CELLS_THREADS, 4) dc_cells_write(const uint32_t* __restrict__ S, Grid3 g,
-                                                                   const uint32_t* __restrict__ actm,
-                                                                   const uint32_t* __restrict__ wsum,
-                                                                   const uint32_t* __restrict__ csum,
-                                                                   uint32_t* __restrict__ offA,
-                                                                   uint32_t* __restrict__ cell_ids,
-                                                                   uint32_t* __restrict__ qoff,
-                                                                   uint8_t* __restrict__ qbits,
-                                                                   uint32_t* __restrict__ cell_off, long long capA) {
+struct CellsOut {
+    unsigned long long* ctr;  // [0] entries [1] CTAs done (cleared by the sign pass)
+    long long capA, capQ, capK;
+    long long *eff, *counts;
+    uint32_t* cell_off;
+    int* status;
+    float* gc;  // the grid's coordinates (x, then y, then z)
+};
+
+__global__ void __launch_bounds__(1024) dc_cells_scan(const CellIndex ix, const CellsOut o) {
     iso::grid_wait();
-    const int lane = threadIdx.x & 31;
-    const uint32_t gw = blockIdx.x * CELLS_WARPS + (threadIdx.x >> 5);
-    const PwGrid p = pw_grid(g);
-    const uint4 wo = *reinterpret_cast<const uint4*>(wsum + 4u * gw);
-    const uint4 co = *reinterpret_cast<const uint4*>(csum + 4u * blockIdx.x);
-    const uint32_t wbusy = wo.w;
-    if (!wbusy) return;
-    unsigned long long ra = (unsigned long long)co.x + wo.x, rq = (unsigned long long)co.y + wo.y,
-                       rk = (unsigned long long)co.z + wo.z;
-    const unsigned long long cap = (unsigned long long)capA;  // over capacity the caller reruns
-    const bool want_k = cell_off != nullptr;
-    for (int j = 0; j < CELLS_ROUNDS; ++j) {
-        if (!((wbusy >> j) & 1u)) continue;  // no active cell: nothing to number
-        const uint32_t pw = cells_pw(gw, lane, j);
-        uint32_t act[CELLS_WPT] = {0u, 0u, 0u, 0u};
-        if (pw + CELLS_WPT <= p.PW) {
-            const uint4 a4 = *reinterpret_cast<const uint4*>(actm + pw);
-            act[0] = a4.x; act[1] = a4.y; act[2] = a4.z; act[3] = a4.w;
+    scan_cells<1024>(ix.seg, ix.p.nseg, o.capA, o.capQ, o.capK, o.eff, o.counts, o.cell_off, o.status);
+}
+
+// The active cells of one segment of point words (whose flat order is the cells'
+// id order), from the bitmap alone.  As in the count of marching cubes the CTA
+// first lists its words that may hold a crossing, a thread then takes one of
+// them, and the cells of a warp's words are laid out in order in shared memory
+// and leave as entries in coalesced stores.  An entry finds its cell's index
+// through offA and seg, so no second pass numbers the cells: the kernel that
+// works on them does (the write pass that did, a lane walking up to 128 cells of
+// its words, took 12 us on a 41 x 57 x 48 grid, 29 us at 256^3 and 36 at 512^3).
+// KOFF: crossings' offsets are asked for.  Bound by latency.
+template <int WPT, bool KOFF>
+__global__ void __launch_bounds__(CELLS_THREADS, 4) dc_cells(const uint32_t* __restrict__ S, Grid3 g,
+                                                             const CellIndex ix, const CellsOut o) {
+    constexpr int T = CELLS_THREADS, NW = CELLS_WARPS;
+    constexpr uint32_t SEG = T * WPT;
+    __shared__ unsigned long long wsum[NW], base_s;
+    __shared__ uint32_t bsum[NW];
+    __shared__ uint16_t list[SEG];  // words that may hold a crossing
+    __shared__ uint32_t queue[NW][CELLS_QUEUE];
+    __shared__ uint32_t kqueue[KOFF ? NW : 1][KOFF ? CELLS_QUEUE : 1];
+    __shared__ int last_s;
+    iso::grid_wait();
+    const PwGrid& p = ix.p;
+    for (uint32_t i = blockIdx.x * T + threadIdx.x; i < uint32_t(g.nx + g.ny + g.nz); i += gridDim.x * T) {
+        const int axis = i < uint32_t(g.nx) ? 0 : (i < uint32_t(g.nx + g.ny) ? 1 : 2);
+        o.gc[i] = coord(g, axis, i - (axis > 0 ? uint32_t(g.nx) : 0u) - (axis > 1 ? uint32_t(g.ny) : 0u));
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t seg0 = blockIdx.x * SEG;
+    uint32_t nbusy = 0;
+    {
+        const uint32_t pw0 = seg0 + threadIdx.x * WPT;
+        // a word is quiet when the rows' words and the words after them are all 0 or
+        // all ~0 (conservative at the grid's edges)
+        uint32_t lo[WPT], hi[WPT], nlo = ~0u, nhi = 0u;
+#pragma unroll
+        for (int k = 0; k < WPT; ++k) { lo[k] = ~0u; hi[k] = 0u; }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint32_t a = pw0 + (q >> 1) * p.sxw + (q & 1) * p.syw;
+            uint32_t v[WPT];
+            if (WPT == 4 && p.vec && pw0 + WPT <= p.PW && a + WPT <= p.PW) {
+                const uint4 v4 = __ldg(reinterpret_cast<const uint4*>(S + a));
+                const uint32_t t[4] = {v4.x, v4.y, v4.z, v4.w};
+#pragma unroll
+                for (int k = 0; k < WPT; ++k) v[k] = t[k];
+            } else {
+#pragma unroll
+                for (int k = 0; k < WPT; ++k) v[k] = a + k < p.PW ? __ldg(S + a + k) : 0u;
+            }
+            uint32_t nx = __shfl_down_sync(~0u, v[0], 1);
+            if (lane == 31) nx = a + WPT < p.PW ? __ldg(S + a + WPT) : 0u;
+            nlo &= nx;
+            nhi |= nx;
+#pragma unroll
+            for (int k = 0; k < WPT; ++k) { lo[k] &= v[k]; hi[k] |= v[k]; }
+        }
+        uint32_t m = 0;
+#pragma unroll
+        for (int k = 0; k < WPT; ++k) {
+            const uint32_t l = lo[k] & (k + 1 < WPT ? lo[(k + 1) % WPT] : nlo);
+            const uint32_t h = hi[k] | (k + 1 < WPT ? hi[(k + 1) % WPT] : nhi);
+            if (l != ~0u && h != 0u && pw0 + k < p.PW) m |= 1u << k;
+        }
+        // quiet words have no active cell (the weld looks neighbours up)
+        if (WPT == 4 && !m && pw0 + WPT <= p.PW) {
+            *reinterpret_cast<uint4*>(ix.actm + pw0) = make_uint4(0u, 0u, 0u, 0u);
         } else {
 #pragma unroll
-            for (int k = 0; k < CELLS_WPT; ++k) act[k] = pw + k < p.PW ? actm[pw + k] : 0u;
+            for (int k = 0; k < WPT; ++k)
+                if (!((m >> k) & 1u) && pw0 + k < p.PW) ix.actm[pw0 + k] = 0u;
         }
-        QuadRows q;
-        load_quad_rows(S, pw, p.sxw, p.syw, p.PW, p.vec, lane, q);
-        int x = 0, y = 0, w = 0;
-        if (pw < p.PW) pw_xyw(g, p, pw, x, y, w);
-        const int x0 = x, y0 = y, w0 = w;
-        uint32_t la = 0, lq = 0, lk = 0;
-#pragma unroll
-        for (int k = 0; k < CELLS_WPT; ++k) {
-            if (act[k]) {
-                uint32_t cw8[8], qz, qy, qx;
-                quad_word_act(g, p.NWg, p.NWc, q, k, x, y, w, cw8);
-                owned_quads(g, cw8, act[k], x, y, w, qz, qy, qx);
-                la += __popc(act[k]);
-                lq += __popc(qz) + __popc(qy) + __popc(qx);
-                if (want_k) lk += word_crossings(cw8, act[k]);
-            }
-            next_point_word(g, p.NWg, x, y, w);
-        }
-        uint32_t ia = la, iq = lq, ik = lk;
+        const uint32_t mine = __popc(m);
+        uint32_t inc = mine;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t ta = __shfl_up_sync(~0u, ia, d), tq = __shfl_up_sync(~0u, iq, d),
-                           tk = __shfl_up_sync(~0u, ik, d);
-            if (lane >= d) { ia += ta; iq += tq; ik += tk; }
+            const uint32_t t = __shfl_up_sync(~0u, inc, d);
+            if (lane >= d) inc += t;
         }
-        unsigned long long a = ra + ia - la, qq = rq + iq - lq, kk = rk + ik - lk;
-        ra += __shfl_sync(~0u, ia, 31);
-        rq += __shfl_sync(~0u, iq, 31);
-        rk += __shfl_sync(~0u, ik, 31);
-        uint32_t offs[CELLS_WPT];
-        x = x0; y = y0; w = w0;
+        if (lane == 31) bsum[warp] = inc;
+        __syncthreads();
+        uint32_t at = inc - mine;
 #pragma unroll
-        for (int k = 0; k < CELLS_WPT; ++k) {
-            offs[k] = uint32_t(a);
-            if (act[k]) {
-                uint32_t cw8[8], qz, qy, qx;
-                quad_word_act(g, p.NWg, p.NWc, q, k, x, y, w, cw8);
-                owned_quads(g, cw8, act[k], x, y, w, qz, qy, qx);
-                uint32_t ex[12];
-                if (want_k) {
+        for (int q = 0; q < NW; ++q) {
+            at += q < warp ? bsum[q] : 0u;
+            nbusy += bsum[q];
+        }
+        for (; m; m &= m - 1) list[at++] = uint16_t(threadIdx.x * WPT + __ffs(m) - 1);
+    }
+    uint32_t sa = 0, sq = 0, sk = 0;  // active cells, quads and crossings of the rounds so far
+    for (uint32_t r0 = 0; r0 < nbusy; r0 += T) {
+        __syncthreads();  // the list; the shared arrays of the round before
+        const uint32_t i = r0 + threadIdx.x;
+        uint32_t cw8[8], act = 0, qz = 0, qy = 0, qx = 0, nk = 0, pw = 0;
+        if (i < nbusy) {
+            pw = seg0 + list[i];
+            int x, y, w;
+            pw_xyw(g, p, pw, x, y, w);
+            if (x < g.nx - 1 && y < g.ny - 1) {
+                const bool nxt = w + 1 < p.NWg;
+                uint32_t and8 = ~0u, or8 = 0u;
 #pragma unroll
-                    for (int e = 0; e < 12; ++e) ex[e] = cw8[iso_edge_corner(2 * e)] ^ cw8[iso_edge_corner(2 * e + 1)];
+                for (int k = 0; k < 4; ++k) {
+                    const uint32_t a = pw + (k >> 1) * p.sxw + (k & 1) * p.syw;
+                    const uint32_t lo = __ldg(S + a), hi = nxt ? __ldg(S + a + 1) : 0u;
+                    cw8[2 * k] = lo;
+                    cw8[2 * k + 1] = __funnelshift_r(lo, hi, 1);  // bit z <- z + 1
+                    and8 &= cw8[2 * k] & cw8[2 * k + 1];
+                    or8 |= cw8[2 * k] | cw8[2 * k + 1];
                 }
-                const uint32_t row = (uint32_t(x) * uint32_t(g.ny - 1) + uint32_t(y)) * uint32_t(g.nz - 1) + 32u * w;
-                uint32_t m = act[k];
-                while (m) {
+                act = (or8 & ~and8) & iso::range_mask(w, 0, g.nz - 2);
+                owned_quads(g, cw8, act, x, y, w, qz, qy, qx);
+                nk = word_crossings(cw8, act);
+            }
+            ix.actm[pw] = act;
+        }
+        const uint32_t na = __popc(act), nq = __popc(qz) + __popc(qy) + __popc(qx);
+        // active cells (at most 32 T), quads (from bit 20) and crossings (from 40)
+        const unsigned long long mine = (unsigned long long)na | ((unsigned long long)nq << 20) |
+                                        ((unsigned long long)nk << 40);
+        unsigned long long inc = mine;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const unsigned long long t = __shfl_up_sync(~0u, inc, d);
+            if (lane >= d) inc += t;
+        }
+        if (lane == 31) wsum[warp] = inc;
+        __syncthreads();
+        unsigned long long before = 0, all = 0;
+#pragma unroll
+        for (int q = 0; q < NW; ++q) {
+            before += q < warp ? wsum[q] : 0ull;
+            all += wsum[q];
+        }
+        const uint32_t ta = uint32_t(all) & 0xfffffu;
+        if (threadIdx.x == 0) base_s = ta ? atomicAdd(o.ctr, (unsigned long long)ta) : 0ull;
+        const unsigned long long ex = inc - mine;  // within the warp
+        if (act) ix.offA[pw] = sa + (uint32_t(before + ex) & 0xfffffu);
+        __syncthreads();  // the entries' block; from here to the next round warps go their own ways
+        const uint32_t n = uint32_t(__shfl_sync(~0u, inc, 31)) & 0xfffffu, c0 = uint32_t(ex) & 0xfffffu;
+        const unsigned long long base = base_s + (uint32_t(before) & 0xfffffu);
+        uint32_t* q = queue[warp];
+        for (uint32_t q0 = 0; q0 < n; q0 += CELLS_QUEUE) {
+            if (na && c0 < q0 + CELLS_QUEUE && c0 + na > q0) {
+                uint32_t j = c0 - q0;  // wraps below q0: not in this window
+                uint32_t qo = sq + (uint32_t((before + ex) >> 20) & 0xfffffu), ko = sk + uint32_t((before + ex) >> 40);
+                for (uint32_t m = act; m; m &= m - 1, ++j) {
                     const int b = __ffs(m) - 1;
-                    m &= m - 1;
                     const uint32_t oz = (qz >> b) & 1u, oy = (qy >> b) & 1u, ox = (qx >> b) & 1u;
-                    if (a < cap) {
-                        cell_ids[a] = row + b;
-                        qoff[a] = uint32_t(qq);
-                        qbits[a] = uint8_t(oz | (oy << 1) | (ox << 2) | (((cw8[0] >> b) & 1u) << 3));
-                        if (want_k) cell_off[a] = uint32_t(kk);
+                    if (j < uint32_t(CELLS_QUEUE)) {
+                        // bit, lane, quad bits (edges z, y, x; the low corner's sign), quad offset
+                        q[j] = uint32_t(b) | (uint32_t(lane) << 5) | (oz << 10) | (oy << 11) | (ox << 12) |
+                               (((cw8[0] >> b) & 1u) << 13) | (qo << 14);
+                        if (KOFF) kqueue[KOFF ? warp : 0][KOFF ? j : 0] = ko;
                     }
-                    qq += oz + oy + ox;
-                    if (want_k) kk += cell_crossings(ex, b);
-                    ++a;
+                    qo += oz + oy + ox;
+                    if (KOFF) ko += cell_crossings(cw8, b);
                 }
             }
-            next_point_word(g, p.NWg, x, y, w);
+            __syncwarp();
+            for (uint32_t j = lane; j < min(uint32_t(CELLS_QUEUE), n - q0); j += 32) {
+                const uint32_t it = q[j];
+                const unsigned long long e = base + q0 + j;
+                if ((long long)e < o.capA) {
+                    ix.elist[e] = (unsigned long long)(seg0 + list[r0 + warp * 32 + ((it >> 5) & 31u)]) |
+                                  ((unsigned long long)(it & 31u) << 32) | ((unsigned long long)(it >> 10) << 37);
+                    if (KOFF) ix.klist[e] = kqueue[KOFF ? warp : 0][KOFF ? j : 0];
+                }
+            }
+            __syncwarp();
         }
-        if (pw < p.PW) store_masks(offA, pw, p.PW, offs);
+        sa += ta;
+        sq += uint32_t(all >> 20) & 0xfffffu;
+        sk += uint32_t(all >> 40);
+    }
+    const bool scans = p.nseg <= CELLS_SCAN;
+    if (threadIdx.x == 0) {
+        ix.seg[blockIdx.x] = make_uint4(sa, sq, sk, 0u);
+        if (scans) {
+            __threadfence();
+            last_s = atomicAdd(o.ctr + 1, 1ull) == p.nseg - 1;
+            __threadfence();
+        }
+    }
+    if (!scans) return;
+    __syncthreads();
+    if (last_s) scan_cells<T>(ix.seg, p.nseg, o.capA, o.capQ, o.capK, o.eff, o.counts, o.cell_off, o.status);
+}
+
+// Launches dc_cells (and its scan) over the sign bitmap S.
+void launch_cells(const uint32_t* S, const Grid3& g, const CellIndex& ix, const CellsOut& o, cudaStream_t st) {
+    const bool fine = ix.p.lgseg == 8;
+    const auto kernel = o.cell_off ? (fine ? dc_cells<1, true> : dc_cells<4, true>)
+                                   : (fine ? dc_cells<1, false> : dc_cells<4, false>);
+    iso::launch_pdl(kernel, ix.p.nseg, unsigned(CELLS_THREADS), st, S, g, ix, o);
+    if (ix.p.nseg > CELLS_SCAN) iso::launch_pdl(dc_cells_scan, 1u, 1024u, st, ix, o);
+}
+
+// The active cell of entry e: its coordinates and index.
+struct ActiveCell {
+    int x, y, z;
+    uint32_t a, cid, qoff, qbits, kbase;
+};
+
+__device__ __forceinline__ ActiveCell entry_cell(const CellIndex& ix, const Grid3& g, unsigned long long e) {
+    ActiveCell c;
+    const uint32_t pw = uint32_t(e), b = uint32_t(e >> 32) & 31u;
+    const uint4 s = __ldg(ix.seg + (pw >> ix.p.lgseg));
+    const uint32_t m = __ldg(ix.actm + pw), off = __ldg(ix.offA + pw);
+    int w;
+    pw_xyw(g, ix.p, pw, c.x, c.y, w);
+    c.z = 32 * w + int(b);
+    c.a = s.x + off + __popc(m & ((1u << b) - 1u));
+    c.cid = (uint32_t(c.x) * uint32_t(g.ny - 1) + uint32_t(c.y)) * uint32_t(g.nz - 1) + uint32_t(c.z);
+    c.qbits = uint32_t(e >> 37) & 15u;
+    c.qoff = s.y + uint32_t(e >> 41);
+    c.kbase = s.z;
+    return c;
+}
+
+// What the solve of an active cell leaves for the weld and the quads.
+struct SolveOut {
+    uint32_t *cells, *qoff;
+    uint8_t *qbits, *used;  // used: 0 when no face uses the cell's vertex, else 1, or 3 when it lies on a face of its box
+    float* dual;
+    uint32_t* cell_off;     // optional: the first crossing
+};
+
+// A caller's intersection (GIVEN): points and normals of the crossings (normals
+// may be null: from the grid), its cells and offsets.
+struct Given {
+    const float *points, *normals;
+    const uint32_t *cells, *off;
+    long long A;
+    int* status;
+};
+
+// One thread per entry of dc_cells: the cell's number and records, and its dual
+// vertex: crossings, grid normals and the QEF in one pass (the arithmetic of
+// dc_points followed by dc_solve, nothing of it stored), or from a caller's
+// intersection.  F: the arithmetic reading (g.fma), a template argument so that
+// each reading compiles without the other's code.  Bound by FP32 issue (ten IEEE
+// divisions per crossing keep the normals the reference's).
+template <bool F, bool GIVEN>
+__global__ void __launch_bounds__(256) dc_solve_cells(const float* __restrict__ vals, Grid3 g, float level,
+                                                      const CellIndex ix, float reg, float svd_tol,
+                                                      const long long* __restrict__ eff,
+                                                      const float* __restrict__ gc, const SolveOut out,
+                                                      const Given in) {
+    iso::grid_wait();
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= eff[0]) return;
+    const ActiveCell c = entry_cell(ix, g, __ldg(ix.elist + i));
+    const long long a = c.a;
+    out.cells[a] = c.cid;
+    out.qoff[a] = c.qoff;
+    out.qbits[a] = uint8_t(c.qbits);
+    if (out.cell_off) out.cell_off[a] = c.kbase + ix.klist[i];
+    g.fma = F;
+    const bool inner = c.x >= 1 && c.x <= g.nx - 3 && c.y >= 1 && c.y <= g.ny - 3 && c.z >= 1 && c.z <= g.nz - 3;
+    CellCorners cc;
+    uint32_t est = 1;
+    if (!GIVEN || !in.normals || !inner) {
+        load_cell_table(vals, g, gc, c.x, c.y, c.z, cc);
+        uint32_t cs = 0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) cs |= uint32_t(iso::below(cc.v[j], level)) << j;
+        est = edge_status(cs);
+    } else {
+        cc.fma = F;
+        cc.p[0][0] = gc[c.x]; cc.p[7][0] = gc[c.x + 1];
+        cc.p[0][1] = gc[g.nx + c.y]; cc.p[7][1] = gc[g.nx + c.y + 1];
+        cc.p[0][2] = gc[g.nx + g.ny + c.z]; cc.p[7][2] = gc[g.nx + g.ny + c.z + 1];
+    }
+    const bool is_used = inner ? est != 0 : cell_used(g, c.x, c.y, c.z, est);
+    Qef Q;
+    qef_init(Q, F);
+    uint32_t K = 0;
+    if (GIVEN) {
+        // not this grid's intersection: the result is discarded, but every record is
+        // written, for the kernels that follow
+        const bool mine = eff[0] == in.A && in.cells[a] == c.cid;
+        if (!mine) atomicCAS(in.status, 0, int(ISO_ERR_LOOKUP));
+        const uint32_t k0 = mine ? in.off[a] : 0u;
+        K = mine ? in.off[a + 1] - k0 : 0u;
+        const float* pt = in.points + 3ll * k0;
+        for (uint32_t k = 0; k < K; ++k) {
+            const float p[3] = {pt[3 * k], pt[3 * k + 1], pt[3 * k + 2]};
+            float n[3];
+            if (in.normals) {
+#pragma unroll
+                for (int q = 0; q < 3; ++q) n[q] = in.normals[3ll * (k0 + k) + q];
+            } else {
+                cell_normal(cc, p, n);
+            }
+            qef_add(Q, p[0], p[1], p[2], n[0], n[1], n[2]);
+        }
+    } else {
+#pragma unroll 1
+        for (uint32_t em = est; em; em &= em - 1) {  // this lane's crossed edges, ascending
+            float p[3], n[3];
+            edge_cross(cc, level, __ffs(em) - 1, p);
+            cell_normal(cc, p, n);
+            qef_add(Q, p[0], p[1], p[2], n[0], n[1], n[2]);
+            ++K;
+        }
+    }
+    qef_finish(Q, K, reg, svd_tol);
+    bool face = false;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        const float lo = cc.p[0][q], hi = cc.p[7][q];  // the cell's box
+        const float x = fminf(fmaxf(float(Q.x[q]), lo), hi);
+        face |= x == lo || x == hi;
+        out.dual[3 * a + q] = x;
+    }
+    out.used[a] = is_used ? (face ? 3 : 1) : 0;
+}
+
+// The crossings' points (and normals) of each entry's cell, its id and its first
+// crossing: isoext's Intersection (src/its.cu:94-159, 186-268).
+__global__ void __launch_bounds__(256) dc_entry_points(const float* __restrict__ vals, Grid3 g, float level,
+                                                       const CellIndex ix, const long long* __restrict__ eff,
+                                                       const float* __restrict__ gc, uint32_t* __restrict__ cells,
+                                                       uint32_t* __restrict__ cell_off, float* __restrict__ points,
+                                                       float* __restrict__ normals,
+                                                       const long long* __restrict__ counts,
+                                                       const int* __restrict__ status, long long* host) {
+    iso::grid_wait();
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) {  // the sizes and the status for the host
+        for (int k = 0; k < 5; ++k) host[k] = counts[k];
+        host[5] = *status;
+    }
+    if (i >= eff[0]) return;
+    const ActiveCell c = entry_cell(ix, g, __ldg(ix.elist + i));
+    CellCorners cc;
+    load_cell_table(vals, g, gc, c.x, c.y, c.z, cc);
+    uint32_t cs = 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) cs |= uint32_t(iso::below(cc.v[j], level)) << j;
+    unsigned long long k = c.kbase + ix.klist[i];
+    cells[c.a] = c.cid;
+    cell_off[c.a] = uint32_t(k);
+#pragma unroll 1
+    for (uint32_t em = edge_status(cs); em; em &= em - 1, ++k) {  // this lane's crossed edges, ascending
+        float p[3];
+        edge_cross(cc, level, __ffs(em) - 1, p);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) points[3 * k + q] = p[q];
+        if (normals) {
+            float n[3];
+            cell_normal(cc, p, n);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) normals[3 * k + q] = n[q];
+        }
     }
 }
 
-// Active index of cell (cx, cy, cz) from the point-word masks and prefixes of
-// dc_cells.
-__device__ __forceinline__ uint32_t active_index_pw(const uint32_t* actm, const uint32_t* offA, const Grid3& g,
-                                                    int cx, int cy, int cz) {
-    const int NWg = (g.nz + 31) / 32;
-    const long long wi = ((long long)cx * g.ny + cy) * NWg + (cz >> 5);
-    return offA[wi] + __popc(actm[wi] & ((1u << (cz & 31)) - 1u));
+// Active index of active cell (cx, cy, cz).
+__device__ __forceinline__ uint32_t active_index_pw(const CellIndex& ix, const Grid3& g, int cx, int cy, int cz) {
+    const uint32_t wi = (uint32_t(cx) * uint32_t(g.ny) + uint32_t(cy)) * uint32_t(ix.p.NWg) + uint32_t(cz >> 5);
+    return ix.seg[wi >> ix.p.lgseg].x + ix.offA[wi] + __popc(ix.actm[wi] & ((1u << (cz & 31)) - 1u));
 }
 
 // Cells along one axis whose closed interval [coord(i), coord(i + 1)] holds v,
@@ -1113,7 +1224,7 @@ __device__ __forceinline__ void cells_holding(const Grid3& g, int axis, int c, f
 // smallest index among the used cells around that face with the same position.
 __device__ __noinline__ uint32_t face_rep(const Grid3& g, uint32_t a, uint32_t cid, float px, float py, float pz,
                                           const uint8_t* __restrict__ used, const float* __restrict__ dual,
-                                          const uint32_t* __restrict__ actm, const uint32_t* __restrict__ offA) {
+                                          const CellIndex& ix) {
     const float p[3] = {px, py, pz};
     const int cz = int(cid % uint32_t(g.nz - 1));
     const uint32_t rr = cid / uint32_t(g.nz - 1);
@@ -1122,17 +1233,16 @@ __device__ __noinline__ uint32_t face_rep(const Grid3& g, uint32_t a, uint32_t c
     cells_holding(g, 0, cx, p[0], x0, x1);
     cells_holding(g, 1, cy, p[1], y0, y1);
     cells_holding(g, 2, cz, p[2], z0, z1);
-    const int NWg = (g.nz + 31) / 32;
     const uint32_t k0 = pos_bits(p[0]), k1 = pos_bits(p[1]), k2 = pos_bits(p[2]);
     uint32_t rep = a;
     for (int x = x0; x <= x1; ++x)
         for (int y = y0; y <= y1; ++y)
             for (int z = z0; z <= z1; ++z) {
                 if (x == cx && y == cy && z == cz) continue;
-                const long long wi = ((long long)x * g.ny + y) * NWg + (z >> 5);  // point word
-                const uint32_t mw = actm[wi], bit = uint32_t(z & 31);
+                const uint32_t wi = (uint32_t(x) * uint32_t(g.ny) + uint32_t(y)) * uint32_t(ix.p.NWg) + uint32_t(z >> 5);
+                const uint32_t mw = ix.actm[wi], bit = uint32_t(z & 31);
                 if (!((mw >> bit) & 1u)) continue;
-                const uint32_t ib = offA[wi] + __popc(mw & ((1u << bit) - 1u));
+                const uint32_t ib = ix.seg[wi >> ix.p.lgseg].x + ix.offA[wi] + __popc(mw & ((1u << bit) - 1u));
                 if (ib < rep && used[ib] && pos_bits(dual[3ll * ib]) == k0 && pos_bits(dual[3ll * ib + 1]) == k1 &&
                     pos_bits(dual[3ll * ib + 2]) == k2)
                     rep = ib;
@@ -1146,9 +1256,7 @@ __device__ __noinline__ uint32_t face_rep(const Grid3& g, uint32_t a, uint32_t c
 // cells into blk.
 __global__ void __launch_bounds__(DC_BLOCK) dc_weld_flags(Grid3 g, const uint32_t* __restrict__ cell_ids,
                                                           const uint8_t* __restrict__ used,
-                                                          const float* __restrict__ dual,
-                                                          const uint32_t* __restrict__ actm,
-                                                          const uint32_t* __restrict__ offA,
+                                                          const float* __restrict__ dual, const CellIndex ix,
                                                           const long long* __restrict__ eff,
                                                           uint32_t* __restrict__ vmap,
                                                           unsigned long long* __restrict__ blk) {
@@ -1163,7 +1271,7 @@ __global__ void __launch_bounds__(DC_BLOCK) dc_weld_flags(Grid3 g, const uint32_
         if (u) {
             uint32_t rep = uint32_t(a);
             if (u & 2u) rep = face_rep(g, rep, cell_ids[a], dual[3 * a], dual[3 * a + 1], dual[3 * a + 2], used, dual,
-                                       actm, offA);
+                                       ix);
             is = rep == uint32_t(a) ? 1u : 0u;
             m = is ? 0u : (0x80000000u | rep);
         }
@@ -1214,9 +1322,7 @@ __device__ __forceinline__ int32_t vertex_of(const uint32_t* vmap, uint32_t i) {
 // of edge_neighbors_table (src/shared_luts.cu:78-81), the owner being o_0 = 0.
 __global__ void __launch_bounds__(256) dc_cell_quads(const uint8_t* __restrict__ qbits, Grid3 g,
                                                      const uint32_t* __restrict__ cell_ids,
-                                                     const uint32_t* __restrict__ qoff,
-                                                     const uint32_t* __restrict__ actm,
-                                                     const uint32_t* __restrict__ offA,
+                                                     const uint32_t* __restrict__ qoff, const CellIndex ix,
                                                      const float* __restrict__ dual,
                                                      const uint32_t* __restrict__ vmap,
                                                      const long long* __restrict__ eff, int32_t* __restrict__ faces,
@@ -1233,7 +1339,7 @@ __global__ void __launch_bounds__(256) dc_cell_quads(const uint8_t* __restrict__
     const int cz = int(cid % uint32_t(g.nz - 1));
     const uint32_t rr = cid / uint32_t(g.nz - 1);
     const int cy = int(rr % uint32_t(g.ny - 1)), cx = int(rr / uint32_t(g.ny - 1));
-    // owned edges (z, y, x) and the sign of the low corner, from dc_cells_write
+    // owned edges (z, y, x) and the sign of the low corner
     const uint32_t qb = qbits[a];
     const bool ez = qb & 1u, ey = qb & 2u, ex = qb & 4u;
     const uint32_t s0 = (qb >> 3) & 1u;
@@ -1259,7 +1365,7 @@ __global__ void __launch_bounds__(256) dc_cell_quads(const uint8_t* __restrict__
         qi[0] = uint32_t(a);
 #pragma unroll
         for (int u = 0; u < 3; ++u)
-            qi[u + 1] = active_index_pw(actm, offA, g, cx - o[u][0], cy - o[u][1], cz - o[u][2]);
+            qi[u + 1] = active_index_pw(ix, g, cx - o[u][0], cy - o[u][1], cz - o[u][2]);
         // is_out = v(p0) <= v(p1): for a crossed edge, p0 below the level
         if (!s0) {
             const uint32_t t0 = qi[0], t1 = qi[1];
@@ -1551,10 +1657,10 @@ struct DcDenseWs {
     DcWs d;
     unsigned long long* zero;  // cleared by the sign pass
     long long nzero;
-    long long* misc;           // [0..1] V  [4..7] eff  [8..12] counts [13] status when the caller has none
+    long long* misc;           // [0..1] V  [2..3] dc_cells: entries, CTAs done  [4..7] eff  [8..12] counts [13] status when the caller has none
     unsigned long long* wblk;  // weld: representatives per block of DC_BLOCK cells
-    uint32_t *wsum, *csum;     // dc_cells: 4 words per warp, per CTA
-    long long ntC, ntV;        // CTAs of the dc_cells kernels and of the weld
+    uint4* seg;                // dc_cells: a record per segment (of 256 point words at least)
+    long long ntV;             // CTAs of the weld
     uint32_t *cells, *qoff, *vmap;
     uint8_t *used, *qbits;
     float* dual;
@@ -1568,7 +1674,7 @@ DcDenseWs carve_dense(void* ws, int nx, int ny, int nz, long long capA) {
     uint8_t* b = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(ws) + 255) & ~uintptr_t(255));
     if (ws) w.d = carve(b, nx, ny, nz);
     const long long pwords = (long long)nx * ny * ((nz + 31) / 32);
-    w.ntC = (pwords + CELLS_TILE - 1) / CELLS_TILE;
+    const long long n2048 = (pwords + 2047) / 2048;
     w.ntV = (capA + DC_BLOCK - 1) / DC_BLOCK;
     size_t o = (base + 255) & ~size_t(255);
     auto take = [&](size_t bytes) {
@@ -1580,8 +1686,8 @@ DcDenseWs carve_dense(void* ws, int nx, int ny, int nz, long long capA) {
     w.zero = reinterpret_cast<unsigned long long*>(take(size_t(w.nzero) * 8));
     w.misc = reinterpret_cast<long long*>(w.zero);
     w.wblk = reinterpret_cast<unsigned long long*>(take(size_t(w.ntV + 1) * 16));
-    w.wsum = reinterpret_cast<uint32_t*>(take(size_t(w.ntC) * CELLS_WARPS * 16));
-    w.csum = reinterpret_cast<uint32_t*>(take(size_t(w.ntC) * 16));
+    w.seg = reinterpret_cast<uint4*>(take(size_t(n2048) * 128));
+    take(size_t(n2048) * 16);  // (the workspace's size is as it was)
     w.cells = reinterpret_cast<uint32_t*>(take(size_t(capA) * 4));
     w.qoff = reinterpret_cast<uint32_t*>(take(size_t(capA) * 4));
     w.vmap = reinterpret_cast<uint32_t*>(take(size_t(capA) * 4));
@@ -1592,13 +1698,18 @@ DcDenseWs carve_dense(void* ws, int nx, int ny, int nz, long long capA) {
     w.total = o + 256;
     return w;
 }
+
+CellIndex cell_index(const DcDenseWs& w, const Grid3& g, unsigned long long* elist) {
+    // the crossings' offsets of the entries live in vmap until the weld writes it
+    return CellIndex{pw_grid(g), w.d.actm, w.d.offA, w.seg, elist, w.vmap};
+}
 }  // namespace
 
 static int dc_dense_impl(const float* values, int nx, int ny, int nz, const float* aabb_min, const float* aabb_max,
                          float level, float reg, float svd_tol, float* vertices, long long vertex_capacity, int* faces,
                          long long face_capacity, void* workspace, size_t workspace_bytes, long long* counts,
                          int* status, int* cell_ids, int* cell_offsets, int* vertex_source, long long* host,
-                         void* stream);
+                         const Given* given, void* stream);
 
 extern "C" {
 
@@ -1614,7 +1725,7 @@ int iso_dc_dense_ex(const float* values, int nx, int ny, int nz, const float* aa
                     int* cell_ids, int* cell_offsets, int* vertex_source, void* stream) {
     return dc_dense_impl(values, nx, ny, nz, aabb_min, aabb_max, level, reg, svd_tol, vertices, vertex_capacity, faces,
                          face_capacity, workspace, workspace_bytes, counts, status, cell_ids, cell_offsets,
-                         vertex_source, nullptr, stream);
+                         vertex_source, nullptr, nullptr, stream);
 }
 
 int iso_dc_dense_sync(const float* values, int nx, int ny, int nz, const float* aabb_min, const float* aabb_max,
@@ -1626,8 +1737,61 @@ int iso_dc_dense_sync(const float* values, int nx, int ny, int nz, const float* 
     if (!host) return iso::fail_code(ISO_ERR_CUDA);
     const int rc = dc_dense_impl(values, nx, ny, nz, aabb_min, aabb_max, level, reg, svd_tol, vertices,
                                  vertex_capacity, faces, face_capacity, workspace, workspace_bytes, nullptr, nullptr,
-                                 nullptr, nullptr, nullptr, host, stream);
+                                 nullptr, nullptr, nullptr, host, nullptr, stream);
     return rc ? rc : iso::wait_sizes(host, 6, sizes, reinterpret_cast<cudaStream_t>(stream));
+}
+
+int iso_dc_dense_its_sync(const float* values, int nx, int ny, int nz, const float* aabb_min, const float* aabb_max,
+                          float level, float reg, float svd_tol, const float* points, const float* normals,
+                          const int* cell_ids, const int* cell_offsets, long long A, float* vertices, int* faces,
+                          long long face_capacity, void* workspace, size_t workspace_bytes, long long* sizes,
+                          void* stream) {
+    if (!sizes || A < 1 || !points || !cell_ids || !cell_offsets) return iso::fail_code(ISO_ERR_ARG);
+    long long* host = iso::host_sizes();
+    if (!host) return iso::fail_code(ISO_ERR_CUDA);
+    const Given in{points, normals, reinterpret_cast<const uint32_t*>(cell_ids),
+                   reinterpret_cast<const uint32_t*>(cell_offsets), A, nullptr};
+    const int rc = dc_dense_impl(values, nx, ny, nz, aabb_min, aabb_max, level, reg, svd_tol, vertices, A, faces,
+                                 face_capacity, workspace, workspace_bytes, nullptr, nullptr, nullptr, nullptr, nullptr,
+                                 host, &in, stream);
+    return rc ? rc : iso::wait_sizes(host, 6, sizes, reinterpret_cast<cudaStream_t>(stream));
+}
+
+int iso_dc_intersection_sync(const float* values, int nx, int ny, int nz, const float* aabb_min, const float* aabb_max,
+                             float level, float* points, float* normals, long long point_capacity, int* cell_ids,
+                             int* cell_offsets, long long cell_capacity, void* workspace, size_t workspace_bytes,
+                             long long* sizes, void* stream) {
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    if (!sizes || !aabb_min || !aabb_max || cell_capacity < 1 || point_capacity < 1 || nx < 2 || ny < 2 || nz < 2 ||
+        (long long)nx * ny * nz > 0x7fffffffll || !values || !points || !cell_ids || !cell_offsets)
+        return iso::fail_code(ISO_ERR_ARG);
+    if (workspace_bytes < iso_dc_dense_workspace_size(nx, ny, nz, cell_capacity, 0)) return iso::fail_code(ISO_ERR_WORKSPACE);
+    long long* host = iso::host_sizes();
+    if (!host) return iso::fail_code(ISO_ERR_CUDA);
+    const DcDenseWs w = carve_dense(workspace, nx, ny, nz, cell_capacity);
+    const Grid3 g = make_grid(nx, ny, nz, aabb_min, aabb_max);
+    long long *eff = w.misc + 4, *counts = w.misc + 8;
+    int* status = reinterpret_cast<int*>(w.misc + 13);
+    uint32_t *cells = reinterpret_cast<uint32_t*>(cell_ids), *off = reinterpret_cast<uint32_t*>(cell_offsets);
+    const CellIndex ix = cell_index(w, g, reinterpret_cast<unsigned long long*>(w.dual));
+    {
+        iso::ProfScope ps("mc_signs", st);
+        mc_signs_launch(values, nx, ny, nz, level, w.d.S, st, w.zero, w.nzero);
+    }
+    {
+        iso::ProfScope ps("dc_classify", st, ix.p.nseg > CELLS_SCAN ? 2 : 1);
+        const CellsOut co{w.zero + 2, cell_capacity, 0x7fffffffll, point_capacity, eff, counts, off, status, w.gc};
+        launch_cells(w.d.S, g, ix, co, st);
+    }
+    {
+        iso::ProfScope ps("dc_intersect", st);
+        const int bt = iso::tune_get(iso::TUNE_DC_CELL_THREADS);
+        iso::launch_pdl(dc_entry_points, blocks_for(cell_capacity, bt), unsigned(bt), st, values, g, level, ix,
+                        static_cast<const long long*>(eff), static_cast<const float*>(w.gc), cells, off, points,
+                        normals, static_cast<const long long*>(counts), static_cast<const int*>(status), host);
+    }
+    if (cudaGetLastError() != cudaSuccess) return iso::fail_code(ISO_ERR_CUDA);
+    return iso::wait_sizes(host, 6, sizes, st);
 }
 
 int iso_dc_dense(const float* values, int nx, int ny, int nz, const float* aabb_min, const float* aabb_max,
@@ -1645,7 +1809,7 @@ static int dc_dense_impl(const float* values, int nx, int ny, int nz, const floa
                          float level, float reg, float svd_tol, float* vertices, long long vertex_capacity, int* faces,
                          long long face_capacity, void* workspace, size_t workspace_bytes, long long* counts,
                          int* status, int* cell_ids, int* cell_offsets, int* vertex_source, long long* host,
-                         void* stream) {
+                         const Given* given, void* stream) {
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     if (((!counts || !status) && !host) || !aabb_min || !aabb_max || vertex_capacity < 0 || face_capacity < 0) return iso::fail_code(ISO_ERR_ARG);
     if ((long long)nx * ny * nz > 0x7fffffffll) return iso::fail_code(ISO_ERR_ARG);
@@ -1666,33 +1830,32 @@ static int dc_dense_impl(const float* values, int nx, int ny, int nz, const floa
         iso::ProfScope ps("mc_signs", st);
         mc_signs_launch(values, nx, ny, nz, level, w.d.S, st, w.zero, w.nzero);
     }
+    // the entries live in the vertex buffer until the weld writes it
+    const CellIndex ix = cell_index(w, g, reinterpret_cast<unsigned long long*>(
+                                              (reinterpret_cast<uintptr_t>(vertices) + 7) & ~uintptr_t(7)));
+    const CellsOut co{w.zero + 2, capA, capQ, 0x7fffffffll, eff, counts, reinterpret_cast<uint32_t*>(cell_offsets),
+                      status, w.gc};
     {
-        iso::ProfScope ps("dc_classify", st, 3);
-        const uint32_t* S = w.d.S;
-        iso::launch_pdl(dc_cells_count, unsigned(w.ntC), unsigned(CELLS_THREADS), st, S, g, w.d.actm, w.wsum,
-                        w.csum, w.gc);
-        iso::launch_pdl(dc_cells_scan, 1u, 1024u, st, w.csum, w.ntC, capA, capQ, eff, counts,
-                        reinterpret_cast<uint32_t*>(cell_offsets), status);
-        iso::launch_pdl(dc_cells_write, unsigned(w.ntC), unsigned(CELLS_THREADS), st, S, g,
-                        static_cast<const uint32_t*>(w.d.actm), static_cast<const uint32_t*>(w.wsum),
-                        static_cast<const uint32_t*>(w.csum), w.d.offA, cells, w.qoff, w.qbits,
-                        reinterpret_cast<uint32_t*>(cell_offsets), capA);
+        iso::ProfScope ps("dc_classify", st, ix.p.nseg > CELLS_SCAN ? 2 : 1);
+        launch_cells(w.d.S, g, ix, co, st);
     }
     if (capA > 0) {
         {
             iso::ProfScope ps("dc_solve", st);
             const int bt = iso::tune_get(iso::TUNE_DC_CELL_THREADS);
-            iso::launch_pdl(solve_kernel(g), blocks_for(capA, bt), unsigned(bt), st, values, g, level,
-                            static_cast<const uint32_t*>(cells), capA, reg, svd_tol, w.dual,
-                            static_cast<const long long*>(eff), w.used, static_cast<const float*>(w.gc));
+            const SolveOut so{cells, w.qoff, w.qbits, w.used, w.dual, co.cell_off};
+            const auto kernel = given ? (g.fma ? dc_solve_cells<true, true> : dc_solve_cells<false, true>)
+                                      : (g.fma ? dc_solve_cells<true, false> : dc_solve_cells<false, false>);
+            Given in = given ? *given : Given{};
+            in.status = status;
+            iso::launch_pdl(kernel, blocks_for(capA, bt), unsigned(bt), st, values, g, level, ix, reg, svd_tol,
+                            static_cast<const long long*>(eff), static_cast<const float*>(w.gc), so, in);
         }
         {
             iso::ProfScope ps("dc_weld", st, 3);
             iso::launch_pdl(dc_weld_flags, unsigned(w.ntV), unsigned(DC_BLOCK), st, g,
                             static_cast<const uint32_t*>(cells), static_cast<const uint8_t*>(w.used),
-                            static_cast<const float*>(w.dual), static_cast<const uint32_t*>(w.d.actm),
-                            static_cast<const uint32_t*>(w.d.offA), static_cast<const long long*>(eff), w.vmap,
-                            w.wblk);
+                            static_cast<const float*>(w.dual), ix, static_cast<const long long*>(eff), w.vmap, w.wblk);
             iso::launch_pdl(dc_block_scan, 1u, 1024u, st, w.wblk, w.ntV, w.misc);
             iso::launch_pdl(dc_weld_number, unsigned(w.ntV), unsigned(DC_BLOCK), st,
                             static_cast<const float*>(w.dual), static_cast<const long long*>(eff),
@@ -1702,8 +1865,7 @@ static int dc_dense_impl(const float* values, int nx, int ny, int nz, const floa
         {
             iso::ProfScope ps("dc_quads", st);
             iso::launch_pdl(dc_cell_quads, blocks_for(capA, 256), 256u, st, static_cast<const uint8_t*>(w.qbits), g,
-                            static_cast<const uint32_t*>(cells), static_cast<const uint32_t*>(w.qoff),
-                            static_cast<const uint32_t*>(w.d.actm), static_cast<const uint32_t*>(w.d.offA),
+                            static_cast<const uint32_t*>(cells), static_cast<const uint32_t*>(w.qoff), ix,
                             static_cast<const float*>(w.dual), static_cast<const uint32_t*>(w.vmap),
                             static_cast<const long long*>(eff), faces, static_cast<const long long*>(counts),
                             static_cast<const int*>(status), host);

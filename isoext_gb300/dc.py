@@ -31,6 +31,10 @@ _ffi.register({
     "iso_dc_weld_write_src": ([_vp, _ll, _vp, _ll, _vp, _vp, _vp, _vp, _vp], _i),
     "iso_dc_intersect_solve": ([_vp, _i, _i, _i, _fa, _fa, _f, _vp, _ll, _ll, _vp, _vp, _f, _f, _vp, _vp], _i),
     "iso_dc_dense_workspace_size": ([_i, _i, _i, _ll, _ll], _sz),
+    "iso_dc_dense_its_sync": ([_vp, _i, _i, _i, _fa, _fa, _f, _f, _f, _vp, _vp, _vp, _vp, _ll, _vp, _vp, _ll, _vp, _sz,
+                               C.POINTER(_ll), _vp], _i),
+    "iso_dc_intersection_sync": ([_vp, _i, _i, _i, _fa, _fa, _f, _vp, _vp, _ll, _vp, _vp, _ll, _vp, _sz,
+                                  C.POINTER(_ll), _vp], _i),
     "iso_dc_dense_sync": ([_vp, _i, _i, _i, _fa, _fa, _f, _f, _f, _vp, _ll, _vp, _ll, _vp, _sz, C.POINTER(_ll), _vp],
                           _i),
     "iso_dc_dense": ([_vp, _i, _i, _i, _fa, _fa, _f, _f, _f, _vp, _ll, _vp, _ll, _vp, _sz, _vp, _vp, _vp], _i),
@@ -39,6 +43,8 @@ _ffi.register({
 # Last seen (active cells, quads) per (shape, level, box): the next call sizes its
 # buffers from them (10% + a margin), so steady-state calls run once.
 _dc_sizes: dict[tuple, tuple[int, int]] = {}
+# The same of intersections: (active cells, crossings).
+_its_sizes: dict[tuple, tuple[int, int]] = {}
 
 
 def _p(t):
@@ -89,57 +95,134 @@ def _stream(dev):
     return C.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
 
 
-def _classify(grid: UniformGrid, level: float):
-    lib = _ffi.lib()
-    dev = grid._values.device
-    nx, ny, nz = grid.shape
-    ws = torch.empty(int(lib.iso_dc_workspace_size(nx, ny, nz)), dtype=torch.uint8, device=dev)
-    counts = torch.zeros(2, dtype=torch.int64, device=dev)
-    _ffi.check(lib.iso_dc_classify(_p(grid._values), nx, ny, nz, float(level), _p(ws), ws.numel(),
-                                   _p(counts), _stream(dev)))
-    A, K = (int(x) for x in counts.cpu())
-    return ws, A, K
+def _trimmed(t: torch.Tensor, n: int) -> torch.Tensor:
+    """The first n rows; storage of their own when the buffer is much larger."""
+    v = t[:n]
+    return v.clone() if t.shape[0] > 2 * n + 65536 else v
 
 
-def _intersect_uniform(grid: UniformGrid, level: float, compute_normals: bool):
+def _intersect_uniform(grid: UniformGrid, level: float, compute_normals: bool) -> Intersection:
+    """iso_dc_intersection_sync, sized from the last call (a retry with exact
+    capacities when they were small)."""
+    from .mc import _first_guess
+
     lib = _ffi.lib()
-    dev = grid._values.device
-    nx, ny, nz = grid.shape
-    ws, A, K = _classify(grid, level)
-    points = torch.empty((K, 3), dtype=torch.float32, device=dev)
-    normals = torch.empty((K, 3), dtype=torch.float32, device=dev) if compute_normals else None
-    cells = torch.empty(A, dtype=torch.int32, device=dev)
-    offs = torch.empty(A + 1, dtype=torch.int32, device=dev)
-    _ffi.check(lib.iso_dc_intersect(_p(grid._values), nx, ny, nz, _ffi.fvec3(grid.aabb_min),
-                                    _ffi.fvec3(grid.aabb_max), float(level), _p(ws), A, K, _p(points),
-                                    _p(normals), _p(cells), _p(offs), _stream(dev)))
-    its = Intersection(points, normals, cells, offs, level, _grid_key(grid))
-    return its, ws
+    values = grid._values
+    dev = values.device
+    shape, lo, hi = tuple(grid.shape), tuple(grid.aabb_min), tuple(grid.aabb_max)
+    if min(shape) < 2:  # no cells
+        def none(*s, dtype):
+            return torch.zeros(s, dtype=dtype, device=dev)
+
+        return Intersection(none(0, 3, dtype=torch.float32), none(0, 3, dtype=torch.float32) if compute_normals else None,
+                            none(0, dtype=torch.int32), none(1, dtype=torch.int32), level, _grid_key(grid))
+    nx, ny, nz = values.shape
+    key = (shape, float(level), lo, hi)
+    if key in _its_sizes:
+        a, k = _its_sizes[key]
+        cap_a, cap_k = a + a // 10 + 1024, k + k // 10 + 4096
+    else:
+        cap_a = _first_guess(shape)[0]
+        cap_k = 5 * cap_a
+    sizes = _ffi.Sizes6()
+    st = _ffi.raw_stream(dev)
+    for _ in range(2):
+        points = torch.empty((cap_k, 3), dtype=torch.float32, device=dev)
+        normals = torch.empty((cap_k, 3), dtype=torch.float32, device=dev) if compute_normals else None
+        cells = torch.empty(cap_a, dtype=torch.int32, device=dev)
+        offs = torch.empty(cap_a + 1, dtype=torch.int32, device=dev)
+        ws_bytes = dc_workspace_bytes(shape, cap_a, 0)
+        ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
+        rc = lib.iso_dc_intersection_sync(values.data_ptr(), nx, ny, nz, _ffi.fvec3(lo), _ffi.fvec3(hi), float(level),
+                                          points.data_ptr(), None if normals is None else normals.data_ptr(), cap_k,
+                                          cells.data_ptr(), offs.data_ptr(), cap_a, ws.data_ptr(), ws_bytes, sizes, st)
+        if rc:
+            _ffi.check(rc)
+        A, K, status = sizes[2], sizes[3], sizes[5]
+        _its_sizes[key] = (A, K)
+        if status == _ffi.ISO_ERR_OVERFLOW:
+            cap_a, cap_k = A + 1024, K + 1024
+            continue
+        if status:
+            raise RuntimeError(f"isoext_gb300: device error {status} in get_intersection")
+        return Intersection(_trimmed(points, K), None if normals is None else _trimmed(normals, K), _trimmed(cells, A),
+                            _trimmed(offs, A + 1), level, _grid_key(grid))
+    raise RuntimeError("isoext_gb300: get_intersection output did not fit after resizing")
 
 
 def get_intersection(grid, level: float = 0.0, compute_normals: bool = False) -> Intersection:
     """Crossings of the grid's edges with the iso-surface (isoext.get_intersection)."""
     if isinstance(grid, UniformGrid):
-        return _intersect_uniform(grid, level, compute_normals)[0]
+        return _intersect_uniform(grid, level, compute_normals)
     if isinstance(grid, SparseGridBase):
         return grid._get_intersection(level, compute_normals)
     raise TypeError("grid must be a UniformGrid or SparseGrid")
 
 
 def _dc_uniform(grid: UniformGrid, level, its: Intersection | None, reg, svd_tol):
+    if its is None:
+        return _dc_one_call(grid, level, reg, svd_tol)
+    if its._sparse is not None or its._grid_key[:3] != _grid_key(grid)[:3]:
+        raise RuntimeError("intersection was computed for a different grid")
+    if its._cells.numel() == 0 or min(grid.shape) < 2:
+        return None, None
+    out = _dc_given(grid, its, reg, svd_tol)
+    return out if out is not None else _dc_sequence(grid, its, reg, svd_tol)
+
+
+def _dc_given(grid: UniformGrid, its: Intersection, reg, svd_tol):
+    """dual_contouring with an intersection in one call (iso_dc_dense_its_sync);
+    the quads follow the intersection's crossings, i.e. its level.  None when the
+    intersection's cells are not the grid's (its values have changed since)."""
+    from .mc import _views
+
+    lib = _ffi.lib()
+    values = grid._values
+    dev = values.device
+    shape, lo, hi = tuple(grid.shape), tuple(grid.aabb_min), tuple(grid.aabb_max)
+    nx, ny, nz = values.shape
+    A = int(its._cells.numel())
+    key = (shape, its._level, lo, hi)
+    # a closed surface has about as many quads as active cells
+    q = max(_dc_sizes[key][1] if key in _dc_sizes else 0, A)
+    cap_f = 2 * q + q // 4 + 1024
+    sizes = _ffi.Sizes6()
+    st = _ffi.raw_stream(dev)
+    for _ in range(2):
+        vout = torch.empty((A, 3), dtype=torch.float32, device=dev)
+        fout = torch.empty((cap_f, 3), dtype=torch.int32, device=dev)
+        ws_bytes = dc_workspace_bytes(shape, A, cap_f)
+        ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
+        rc = lib.iso_dc_dense_its_sync(values.data_ptr(), nx, ny, nz, _ffi.fvec3(lo), _ffi.fvec3(hi), its._level,
+                                       float(reg), float(svd_tol), its._points.data_ptr(),
+                                       None if its._normals is None else its._normals.data_ptr(),
+                                       its._cells.data_ptr(), its._offsets.data_ptr(), A, vout.data_ptr(),
+                                       fout.data_ptr(), cap_f, ws.data_ptr(), ws_bytes, sizes, st)
+        if rc:
+            _ffi.check(rc)
+        V, F, grid_a, _, Q, status = sizes
+        if grid_a != A or status == _ffi.ISO_ERR_LOOKUP:
+            return None
+        _dc_sizes[key] = (A, Q)
+        if status == _ffi.ISO_ERR_OVERFLOW:
+            cap_f = 2 * Q + 1024
+            continue
+        if status:
+            raise RuntimeError(f"isoext_gb300: device error {status} in dual_contouring")
+        return _views(vout, fout, V, F)
+    raise RuntimeError("isoext_gb300: dual_contouring output did not fit after resizing")
+
+
+def _dc_sequence(grid: UniformGrid, its: Intersection, reg, svd_tol):
+    """The same as a sequence of calls, for an intersection whose cells are not
+    the grid's active cells any more."""
     lib = _ffi.lib()
     dev = grid._values.device
     nx, ny, nz = grid.shape
     amin, amax = _ffi.fvec3(grid.aabb_min), _ffi.fvec3(grid.aabb_max)
     st = _stream(dev)
-    if its is None:
-        return _dc_one_call(grid, level, reg, svd_tol)
-    else:
-        if its._sparse is not None or its._grid_key[:3] != _grid_key(grid)[:3]:
-            raise RuntimeError("intersection was computed for a different grid")
-        # the quads follow the intersection's crossings, i.e. its level
-        ws, (_, _, Q) = _classify_quads(grid, its._level)
-        _ffi.check(lib.iso_dc_cells(_p(grid._values), nx, ny, nz, its._level, _p(ws), st))
+    ws, (_, _, Q) = _classify_quads(grid, its._level)
+    _ffi.check(lib.iso_dc_cells(_p(grid._values), nx, ny, nz, its._level, _p(ws), st))
     A = int(its._cells.numel())
     normals = its._normals
     if normals is None:

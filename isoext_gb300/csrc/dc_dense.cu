@@ -23,6 +23,7 @@
 #define ISO_LUT_DECL static __constant__ const
 #include "luts.h"
 #include "dc_common.cuh"
+#include "lookback.cuh"
 #include "profile.cuh"
 
 namespace {
@@ -681,7 +682,7 @@ __global__ void dc_remap(const int32_t* __restrict__ tri, long long n, const uin
 
 
 // ---------------------------------------------------------------------------
-// One-call dual contouring: after the sign pass, six or seven kernels chained by
+// One-call dual contouring: after the sign pass, five or six kernels chained by
 // programmatic dependent launch, with the sizes kept on the device.
 //
 //   dc_cells (/ dc_cells_scan)
@@ -693,7 +694,7 @@ __global__ void dc_remap(const int32_t* __restrict__ tri, long long n, const uin
 //                  checked against the sizes.
 //   dc_solve_cells per entry: its cell's number, the QEF solve and whether faces
 //                  use the cell.
-//   dc_weld_flags / dc_block_scan / dc_weld_number
+//   dc_weld_faces / dc_weld_number
 //                  the exact-position weld.  A dual vertex is clipped to its
 //                  cell's closed box, and the boxes of different cells meet only
 //                  on shared faces, so a vertex strictly inside its box has a
@@ -797,20 +798,25 @@ __device__ void scan_cells(uint4* seg, uint32_t nseg, long long capA, long long 
 #pragma unroll
             for (int t = 0; t < 3; ++t) part[t][warp] = in[t];
         __syncthreads();
+        if (warp < 3) {  // warp t: inclusive sums over the warps
+            unsigned long long x = lane < T / 32 ? part[warp][lane] : 0ull;
+#pragma unroll
+            for (int d = 1; d < T / 32; d <<= 1) {
+                const unsigned long long u = __shfl_up_sync(~0u, x, d);
+                if (lane >= d) x += u;
+            }
+            if (lane < T / 32) part[warp][lane] = x;
+        }
+        __syncthreads();
         if (i < nseg) {
             unsigned long long e[3];
 #pragma unroll
-            for (int t = 0; t < 3; ++t) {
-                e[t] = carry[t] + in[t] - c[t];
-#pragma unroll
-                for (int q = 0; q < T / 32; ++q) e[t] += q < warp ? part[t][q] : 0ull;
-            }
+            for (int t = 0; t < 3; ++t) e[t] = carry[t] + (warp ? part[t][warp - 1] : 0ull) + in[t] - c[t];
             // offsets past 2^32 only matter when the sizes overflow (then nothing is used)
             seg[i] = make_uint4(uint32_t(e[0]), uint32_t(e[1]), uint32_t(e[2]), 0u);
         }
         __syncthreads();
-        if (tid < 3)
-            for (int q = 0; q < T / 32; ++q) carry[tid] += part[tid][q];
+        if (tid < 3) carry[tid] += part[tid][T / 32 - 1];
         __syncthreads();
     }
     if (tid == 0) {
@@ -838,6 +844,8 @@ struct CellsOut {
     uint32_t* cell_off;
     int* status;
     float* gc;  // the grid's coordinates (x, then y, then z)
+    unsigned long long* zero;  // to clear for the kernels that follow (the weld's look-back states)
+    long long nzero;
 };
 
 __global__ void __launch_bounds__(1024) dc_cells_scan(const CellIndex ix, const CellsOut o) {
@@ -871,6 +879,8 @@ __global__ void __launch_bounds__(CELLS_THREADS, 4) dc_cells(const uint32_t* __r
         const int axis = i < uint32_t(g.nx) ? 0 : (i < uint32_t(g.nx + g.ny) ? 1 : 2);
         o.gc[i] = coord(g, axis, i - (axis > 0 ? uint32_t(g.nx) : 0u) - (axis > 1 ? uint32_t(g.ny) : 0u));
     }
+    for (long long i = (long long)blockIdx.x * T + threadIdx.x; i < o.nzero; i += (long long)gridDim.x * T)
+        o.zero[i] = 0ull;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t seg0 = blockIdx.x * SEG;
     uint32_t nbusy = 0;
@@ -1070,6 +1080,9 @@ struct SolveOut {
     uint8_t *qbits, *used;  // used: 0 when no face uses the cell's vertex, else 1, or 3 when it lies on a face of its box
     float* dual;
     uint32_t* cell_off;     // optional: the first crossing
+    uint32_t* flist;        // the cells of used vertices on a face (FaceList)
+    unsigned long long* nface;
+    long long fcap;
 };
 
 // A caller's intersection (GIVEN): points and normals of the crossings (normals
@@ -1161,6 +1174,16 @@ __global__ void __launch_bounds__(256) dc_solve_cells(const float* __restrict__ 
         out.dual[3 * a + q] = x;
     }
     out.used[a] = is_used ? (face ? 3 : 1) : 0;
+    // list the vertex for the weld: one atomic per warp
+    const bool on = is_used && face;
+    const uint32_t m = __ballot_sync(__activemask(), on);
+    if (on) {
+        const int lane = threadIdx.x & 31, lead = __ffs(m) - 1;
+        unsigned long long base = 0;
+        if (lane == lead) base = atomicAdd(out.nface, (unsigned long long)__popc(m));
+        base = __shfl_sync(m, base, lead) + __popc(m & ((1u << lane) - 1u));
+        if ((long long)base < out.fcap) out.flist[base] = uint32_t(a);
+    }
 }
 
 // The crossings' points (and normals) of each entry's cell, its id and its first
@@ -1203,123 +1226,160 @@ __global__ void __launch_bounds__(256) dc_entry_points(const float* __restrict__
     }
 }
 
-// Active index of active cell (cx, cy, cz).
-__device__ __forceinline__ uint32_t active_index_pw(const CellIndex& ix, const Grid3& g, int cx, int cy, int cz) {
-    const uint32_t wi = (uint32_t(cx) * uint32_t(g.ny) + uint32_t(cy)) * uint32_t(ix.p.NWg) + uint32_t(cz >> 5);
-    return ix.seg[wi >> ix.p.lgseg].x + ix.offA[wi] + __popc(ix.actm[wi] & ((1u << (cz & 31)) - 1u));
-}
-
 // Cells along one axis whose closed interval [coord(i), coord(i + 1)] holds v,
 // for v in cell c's interval: [i0, i1] around c (wider than c +- 1 only when
-// grid coordinates repeat, on grids finer than FP32 resolves).
-__device__ __forceinline__ void cells_holding(const Grid3& g, int axis, int c, float v, int& i0, int& i1) {
-    const int n = axis == 0 ? g.nx : (axis == 1 ? g.ny : g.nz);
+// grid coordinates repeat, on grids finer than FP32 resolves).  t: the axis's
+// coordinates, n of them.
+__device__ __forceinline__ void cells_holding(const float* __restrict__ t, int n, int c, float v, int& i0, int& i1) {
     i0 = c;
     i1 = c;
-    while (i0 > 0 && coord(g, axis, uint32_t(i0)) == v) --i0;
-    while (i1 < n - 2 && coord(g, axis, uint32_t(i1 + 1)) == v) ++i1;
+    while (i0 > 0 && __ldg(t + i0) == v) --i0;
+    while (i1 < n - 2 && __ldg(t + i1 + 1) == v) ++i1;
 }
 
-// Representative of used cell a whose vertex p lies on a face of its box: the
-// smallest index among the used cells around that face with the same position.
-__device__ __noinline__ uint32_t face_rep(const Grid3& g, uint32_t a, uint32_t cid, float px, float py, float pz,
-                                          const uint8_t* __restrict__ used, const float* __restrict__ dual,
-                                          const CellIndex& ix) {
-    const float p[3] = {px, py, pz};
-    const int cz = int(cid % uint32_t(g.nz - 1));
-    const uint32_t rr = cid / uint32_t(g.nz - 1);
-    const int cy = int(rr % uint32_t(g.ny - 1)), cx = int(rr / uint32_t(g.ny - 1));
-    int x0, x1, y0, y1, z0, z1;
-    cells_holding(g, 0, cx, p[0], x0, x1);
-    cells_holding(g, 1, cy, p[1], y0, y1);
-    cells_holding(g, 2, cz, p[2], z0, z1);
-    const uint32_t k0 = pos_bits(p[0]), k1 = pos_bits(p[1]), k2 = pos_bits(p[2]);
-    uint32_t rep = a;
-    for (int x = x0; x <= x1; ++x)
-        for (int y = y0; y <= y1; ++y)
-            for (int z = z0; z <= z1; ++z) {
-                if (x == cx && y == cy && z == cz) continue;
-                const uint32_t wi = (uint32_t(x) * uint32_t(g.ny) + uint32_t(y)) * uint32_t(ix.p.NWg) + uint32_t(z >> 5);
-                const uint32_t mw = ix.actm[wi], bit = uint32_t(z & 31);
-                if (!((mw >> bit) & 1u)) continue;
-                const uint32_t ib = ix.seg[wi >> ix.p.lgseg].x + ix.offA[wi] + __popc(mw & ((1u << bit) - 1u));
-                if (ib < rep && used[ib] && pos_bits(dual[3ll * ib]) == k0 && pos_bits(dual[3ll * ib + 1]) == k1 &&
-                    pos_bits(dual[3ll * ib + 2]) == k2)
-                    rep = ib;
-            }
-    return rep;
-}
+// Where the solve lists the cells whose vertex lies on a face of their box.
+struct FaceList {
+    uint32_t* cells;          // active indices, unordered
+    unsigned long long* n;    // their number, past cap where the list had no room
+    long long cap;
+};
 
-// Weld, step 1 (one thread per active cell): vmap[a] = 0xffffffff when no face
-// uses the cell, 0 when its vertex is a representative (numbered in step 3),
-// else 0x80000000 | its representative; representatives per block of DC_BLOCK
-// cells into blk.
-__global__ void __launch_bounds__(DC_BLOCK) dc_weld_flags(Grid3 g, const uint32_t* __restrict__ cell_ids,
-                                                          const uint8_t* __restrict__ used,
-                                                          const float* __restrict__ dual, const CellIndex ix,
-                                                          const long long* __restrict__ eff,
-                                                          uint32_t* __restrict__ vmap,
-                                                          unsigned long long* __restrict__ blk) {
-    __shared__ uint32_t sm[66];
+// Weld, eight lanes per vertex on a face of its cell's box, a lane per cell around
+// that face, edge or corner (two per axis on which the vertex lies on a face; more
+// only where coordinates repeat): looks for the used ones with the same
+// position.  When one comes before the vertex's own, vmap[a] = 0x80000000 | the
+// first of them and used[a] gets bit 2.  Bound by the latency of six dependent
+// gathers; the list keeps every lane at it.  A pass over all cells waited in every
+// warp for its few such lanes and their cells one after another: 18 us at 512^3,
+// 8 on a 41 x 57 x 48 grid.
+__global__ void __launch_bounds__(128) dc_weld_faces(Grid3 g, const CellIndex ix, const float* __restrict__ gc,
+                                                     const FaceList list, const uint32_t* __restrict__ cells,
+                                                     uint8_t* used, const float* __restrict__ dual,
+                                                     const long long* __restrict__ eff,
+                                                     uint32_t* __restrict__ vmap) {
     iso::grid_wait();
-    const long long a = (long long)blockIdx.x * DC_BLOCK + threadIdx.x;
-    const long long A = eff[0];
-    uint32_t is = 0;
-    if (a < A) {
-        const uint32_t u = used[a];
-        uint32_t m = 0xffffffffu;
-        if (u) {
-            uint32_t rep = uint32_t(a);
-            if (u & 2u) rep = face_rep(g, rep, cell_ids[a], dual[3 * a], dual[3 * a + 1], dual[3 * a + 2], used, dual,
-                                       ix);
-            is = rep == uint32_t(a) ? 1u : 0u;
-            m = is ? 0u : (0x80000000u | rep);
+    const uint32_t A = uint32_t(eff[0]);
+    const bool listed = (long long)*list.n <= list.cap;  // else every cell is looked at
+    const uint32_t n = listed ? min(uint32_t(*list.n), A) : A;
+    const uint32_t k = threadIdx.x & 7u, group = (threadIdx.x & 31u) & ~7u;
+    const uint32_t step = gridDim.x * (blockDim.x / 8);
+    // a warp's four groups stay together (the shuffles name the group's lanes only)
+    for (uint32_t i = blockIdx.x * (blockDim.x / 8) + threadIdx.x / 8; i < n; i += step) {
+        const uint32_t a = listed ? list.cells[i] : i;
+        // (bit 0 is all that is read of another cell: the bits 2 that other threads
+        // set meanwhile do not matter)
+        if ((used[a] & 3u) != 3u) continue;
+        const float p[3] = {dual[3ll * a], dual[3ll * a + 1], dual[3ll * a + 2]};
+        const uint32_t cid = cells[a];
+        const int cz = int(cid % uint32_t(g.nz - 1));
+        const uint32_t rr = cid / uint32_t(g.nz - 1);
+        const int cy = int(rr % uint32_t(g.ny - 1)), cx = int(rr / uint32_t(g.ny - 1));
+        int x0, x1, y0, y1, z0, z1;
+        cells_holding(gc, g.nx, cx, p[0], x0, x1);
+        cells_holding(gc + g.nx, g.ny, cy, p[1], y0, y1);
+        cells_holding(gc + g.nx + g.ny, g.nz, cz, p[2], z0, z1);
+        const uint32_t k0 = pos_bits(p[0]), k1 = pos_bits(p[1]), k2 = pos_bits(p[2]);
+        const uint32_t ny = uint32_t(y1 - y0 + 1), nz = uint32_t(z1 - z0 + 1), count = uint32_t(x1 - x0 + 1) * ny * nz;
+        uint32_t rep = a;
+        for (uint32_t c = k; c < count; c += 8) {
+            const uint32_t z = uint32_t(z0) + c % nz, r = c / nz;
+            const uint32_t y = uint32_t(y0) + r % ny, x = uint32_t(x0) + r / ny;
+            const uint32_t wi = (x * uint32_t(g.ny) + y) * uint32_t(ix.p.NWg) + (z >> 5);
+            const uint32_t mw = ix.actm[wi], bit = z & 31u;
+            if (!((mw >> bit) & 1u)) continue;
+            const uint32_t ib = ix.seg[wi >> ix.p.lgseg].x + ix.offA[wi] + __popc(mw & ((1u << bit) - 1u));
+            if (ib >= rep) continue;
+            const uint32_t u = used[ib];
+            const float q0 = dual[3ll * ib], q1 = dual[3ll * ib + 1], q2 = dual[3ll * ib + 2];
+            if ((u & 1u) && pos_bits(q0) == k0 && pos_bits(q1) == k1 && pos_bits(q2) == k2) rep = ib;
         }
-        vmap[a] = m;
-    }
-    uint32_t e0, e1, t0, t1;
-    block_scan2(is, 0u, e0, e1, t0, t1, sm);
-    if (threadIdx.x == 0) {
-        blk[2 * blockIdx.x] = t0;
-        blk[2 * blockIdx.x + 1] = 0;
+        const uint32_t lanes = 0xffu << group;
+#pragma unroll
+        for (int d = 4; d >= 1; d >>= 1) rep = min(rep, __shfl_xor_sync(lanes, rep, d));
+        if (k == 0 && rep != a) {
+            vmap[a] = 0x80000000u | rep;
+            used[a] = 7;
+        }
     }
 }
 
-// Weld, step 3: representatives numbered in cell order (block offsets from the
-// scan of step 2), their positions (and source cells) written.
-__global__ void __launch_bounds__(DC_BLOCK) dc_weld_number(const float* __restrict__ dual,
-                                                           const long long* __restrict__ eff,
-                                                           const unsigned long long* __restrict__ blk,
-                                                           const long long* __restrict__ vtot,
-                                                           uint32_t* __restrict__ vmap, float* __restrict__ vout,
-                                                           uint32_t* __restrict__ vsrc, long long* counts) {
-    __shared__ uint32_t sm[66];
+// The used vertices that are their position's first, numbered in cell order and
+// written; vmap[a] = the number, or 0xffffffff where no face uses the cell.
+// Tiles of 1024 cells in ticket order, chained by look-back: the work of a tile
+// is the same everywhere, so no CTA waits long (a scan between two passes took
+// two more launches).
+constexpr int NUM_THREADS = 256, NUM_PER = 4;
+constexpr int NUM_TILE = NUM_THREADS * NUM_PER;
+
+__global__ void __launch_bounds__(NUM_THREADS) dc_weld_number(const float* __restrict__ dual,
+                                                              const long long* __restrict__ eff,
+                                                              const uint8_t* __restrict__ used,
+                                                              unsigned long long* state, unsigned long long* ticket,
+                                                              uint32_t* __restrict__ vmap, float* __restrict__ vout,
+                                                              uint32_t* __restrict__ vsrc, long long* counts,
+                                                              int* status) {
+    __shared__ uint32_t tile_s, wcnt[NUM_PER][NUM_THREADS / 32];
+    __shared__ unsigned long long pre_s;
     iso::grid_wait();
-    const long long a = (long long)blockIdx.x * DC_BLOCK + threadIdx.x;
-    const long long A = eff[0];
-    const uint32_t is = (a < A && vmap[a] == 0u) ? 1u : 0u;
-    uint32_t e0, e1, t0, t1;
-    block_scan2(is, 0u, e0, e1, t0, t1, sm);
-    if (blockIdx.x == 0 && threadIdx.x == 0) counts[0] = vtot[0];
-    if (!is) return;
-    const unsigned long long o = blk[2 * blockIdx.x] + e0;  // < V <= A: inside the vertex capacity
-    vmap[a] = uint32_t(o);
-    vout[3 * o] = dual[3 * a];
-    vout[3 * o + 1] = dual[3 * a + 1];
-    vout[3 * o + 2] = dual[3 * a + 2];
-    if (vsrc) vsrc[o] = uint32_t(a);
-}
-
-// Final vertex number of active cell i: its own, or its representative's.
-__device__ __forceinline__ int32_t vertex_of(const uint32_t* vmap, uint32_t i) {
-    uint32_t m = vmap[i];
-    if (m != 0xffffffffu && (m & 0x80000000u)) m = vmap[m & 0x7fffffffu];
-    return int32_t(m);
+    const uint32_t A = uint32_t(eff[0]);
+    if (threadIdx.x == 0) tile_s = uint32_t(atomicAdd(ticket, 1ull));
+    __syncthreads();
+    const uint32_t tile = tile_s;
+    if (tile * (unsigned long long)NUM_TILE >= A) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t u[NUM_PER], bal[NUM_PER];
+#pragma unroll
+    for (int k = 0; k < NUM_PER; ++k) {
+        const uint32_t a = tile * NUM_TILE + k * NUM_THREADS + threadIdx.x;
+        u[k] = a < A ? used[a] : 0u;
+    }
+#pragma unroll
+    for (int k = 0; k < NUM_PER; ++k) {
+        bal[k] = __ballot_sync(~0u, (u[k] & 5u) == 1u);
+        if (lane == 0) wcnt[k][warp] = __popc(bal[k]);
+    }
+    __syncthreads();
+    if (warp == 0) {  // the tile's 32 (round, warp) counts, one per lane, in order
+        static_assert(NUM_PER * (NUM_THREADS / 32) == 32, "one count per lane");
+        uint32_t& mine = wcnt[lane / (NUM_THREADS / 32)][lane % (NUM_THREADS / 32)];
+        const uint32_t c = mine;
+        uint32_t inc = c;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t t = __shfl_up_sync(~0u, inc, d);
+            if (lane >= d) inc += t;
+        }
+        mine = inc - c;
+        const uint32_t total = __shfl_sync(~0u, inc, 31);
+        unsigned long long e = 0, unused = 0;
+        lb_tile(state, tile, total, 0, e, unused, status);
+        if (lane == 0) {
+            pre_s = e;
+            if ((unsigned long long)(tile + 1) * NUM_TILE >= A) counts[0] = (long long)(e + total);
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < NUM_PER; ++k) {
+        const uint32_t a = tile * NUM_TILE + k * NUM_THREADS + threadIdx.x;
+        if (a >= A) continue;
+        if (!u[k]) vmap[a] = 0xffffffffu;
+        if ((u[k] & 5u) != 1u) continue;
+        const unsigned long long o = pre_s + wcnt[k][warp] + __popc(bal[k] & ((1u << lane) - 1u));  // < V <= A
+        vmap[a] = uint32_t(o);
+        vout[3 * o] = dual[3ll * a];
+        vout[3 * o + 1] = dual[3ll * a + 1];
+        vout[3 * o + 2] = dual[3ll * a + 2];
+        if (vsrc) vsrc[o] = a;
+    }
 }
 
 // The quads active cell a owns, in the reference's order and orientation
 // (src/dc.cu:101-157): the 4 cells around the edge are p - o_i with the offsets
 // of edge_neighbors_table (src/shared_luts.cu:78-81), the owner being o_0 = 0.
+// Bound by the latency of its gathers, so they go in two rounds: the index
+// records of the four words the neighbours lie in, then the vertices and numbers
+// of all neighbours that any of the quads uses.
 __global__ void __launch_bounds__(256) dc_cell_quads(const uint8_t* __restrict__ qbits, Grid3 g,
                                                      const uint32_t* __restrict__ cell_ids,
                                                      const uint32_t* __restrict__ qoff, const CellIndex ix,
@@ -1335,58 +1395,83 @@ __global__ void __launch_bounds__(256) dc_cell_quads(const uint8_t* __restrict__
     }
     const long long a = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= eff[0]) return;
+    // owned edges (z, y, x) and the sign of the low corner
+    const uint32_t qb = qbits[a];
+    if (!(qb & 7u)) return;
     const uint32_t cid = cell_ids[a];
+    unsigned long long q = qoff[a];
+    const bool s0 = (qb >> 3) & 1u;
     const int cz = int(cid % uint32_t(g.nz - 1));
     const uint32_t rr = cid / uint32_t(g.nz - 1);
     const int cy = int(rr % uint32_t(g.ny - 1)), cx = int(rr / uint32_t(g.ny - 1));
-    // owned edges (z, y, x) and the sign of the low corner
-    const uint32_t qb = qbits[a];
-    const bool ez = qb & 1u, ey = qb & 2u, ex = qb & 4u;
-    const uint32_t s0 = (qb >> 3) & 1u;
-    if (!(qb & 7u)) return;
-    unsigned long long q = qoff[a];
-    const float own[3] = {dual[3 * a], dual[3 * a + 1], dual[3 * a + 2]};
+    // cells 0 .. 6: itself, z-1, y-1, (y-1, z-1), x-1, (x-1, z-1), (x-1, y-1); those in use
+    const uint32_t use = 1u | ((qb & 1u) ? 0x54u : 0u) | ((qb & 2u) ? 0x32u : 0u) | ((qb & 4u) ? 0x0eu : 0u);
+    const uint32_t NWg = uint32_t(ix.p.NWg), b = uint32_t(cz & 31);
+    const uint32_t w0 = (uint32_t(cx) * uint32_t(g.ny) + uint32_t(cy)) * NWg + uint32_t(cz >> 5);
+    uint32_t idx[7];
+    idx[0] = uint32_t(a);
+    // rows (x, y), (x, y-1), (x-1, y), (x-1, y-1): the cells at z and at z - 1
+    uint32_t first[4], mask[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const uint32_t here = r ? 1u << (2 * r) : 0u, low = r < 3 ? 2u << (2 * r) : 0u;  // cells 2r and 2r + 1
+        first[r] = mask[r] = 0u;
+        if (!(use & (here | low))) continue;
+        const uint32_t wr = w0 - uint32_t(r & 1) * NWg - uint32_t(r >> 1) * uint32_t(g.ny) * NWg;
+        const uint32_t wl = wr - ((!(use & here) && b == 0u) ? 1u : 0u);  // only z - 1, in the word before
+        mask[r] = ix.actm[wl];
+        first[r] = ix.seg[wl >> ix.p.lgseg].x + ix.offA[wl];
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const uint32_t here = r ? 1u << (2 * r) : 0u, low = r < 3 ? 2u << (2 * r) : 0u;
+        if (r) idx[2 * r] = first[r] + __popc(mask[r] & ((1u << b) - 1u));
+        if (r < 3) {
+            if (b) {
+                idx[2 * r + 1] = first[r] + __popc(mask[r] & ((1u << (b - 1)) - 1u));
+            } else if (use & low) {
+                // z - 1 is the last cell of the word before
+                uint32_t m = mask[r], f = first[r];
+                if (use & here) {
+                    const uint32_t wl = w0 - uint32_t(r & 1) * NWg - uint32_t(r >> 1) * uint32_t(g.ny) * NWg - 1u;
+                    m = ix.actm[wl];
+                    f = ix.seg[wl >> ix.p.lgseg].x + ix.offA[wl];
+                }
+                idx[2 * r + 1] = f + __popc(m & 0x7fffffffu);
+            }
+        }
+    }
+    float v[7][3];
+    uint32_t f[7];
+#pragma unroll
+    for (int k = 0; k < 7; ++k) {
+        if (!((use >> k) & 1u)) continue;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) v[k][d] = dual[3ll * idx[k] + d];
+        f[k] = vmap[idx[k]];
+    }
+#pragma unroll
+    for (int k = 0; k < 7; ++k)
+        if (((use >> k) & 1u) && f[k] != 0xffffffffu && (f[k] & 0x80000000u)) f[k] = vmap[f[k] & 0x7fffffffu];
 #pragma unroll
     for (int ax = 2; ax >= 0; --ax) {
-        if (!(ax == 2 ? ez : (ax == 1 ? ey : ex))) continue;
-        // offsets o_1..o_3 of the other three cells
-        int o[3][3];
-        if (ax == 0) {
-            const int t[3][3] = {{0, 1, 0}, {0, 1, 1}, {0, 0, 1}};
-            for (int u = 0; u < 3; ++u) for (int d = 0; d < 3; ++d) o[u][d] = t[u][d];
-        } else if (ax == 1) {
-            const int t[3][3] = {{0, 0, 1}, {1, 0, 1}, {1, 0, 0}};
-            for (int u = 0; u < 3; ++u) for (int d = 0; d < 3; ++d) o[u][d] = t[u][d];
-        } else {
-            const int t[3][3] = {{1, 0, 0}, {1, 1, 0}, {0, 1, 0}};
-            for (int u = 0; u < 3; ++u) for (int d = 0; d < 3; ++d) o[u][d] = t[u][d];
-        }
-        uint32_t qi[4];
-        qi[0] = uint32_t(a);
-#pragma unroll
-        for (int u = 0; u < 3; ++u)
-            qi[u + 1] = active_index_pw(ix, g, cx - o[u][0], cy - o[u][1], cz - o[u][2]);
-        // is_out = v(p0) <= v(p1): for a crossed edge, p0 below the level
-        if (!s0) {
-            const uint32_t t0 = qi[0], t1 = qi[1];
-            qi[0] = qi[3]; qi[1] = qi[2]; qi[2] = t1; qi[3] = t0;
-        }
-        float v[4][3];
-#pragma unroll
-        for (int t = 0; t < 4; ++t)
-#pragma unroll
-            for (int d = 0; d < 3; ++d) v[t][d] = qi[t] == uint32_t(a) ? own[d] : dual[3ll * qi[t] + d];
-        int32_t f[4];
-#pragma unroll
-        for (int t = 0; t < 4; ++t) f[t] = vertex_of(vmap, qi[t]);
+        if (!((qb >> (2 - ax)) & 1u)) continue;
+        // the quad's cells 1 .. 3
+        const int c1 = ax == 0 ? 2 : (ax == 1 ? 1 : 4), c2 = ax == 0 ? 3 : (ax == 1 ? 5 : 6),
+                  c3 = ax == 0 ? 1 : (ax == 1 ? 4 : 2);
+        // is_out = v(p0) <= v(p1): for a crossed edge, p0 below the level; else the
+        // order is reversed, which swaps its ends and its middles
+        const bool second = dist3(s0 ? v[0] : v[c3], s0 ? v[c2] : v[c1], g.fma) >
+                            dist3(s0 ? v[c1] : v[c2], s0 ? v[c3] : v[0], g.fma);
+        const int32_t f0 = int32_t(s0 ? f[0] : f[c3]), f1 = int32_t(s0 ? f[c1] : f[c2]),
+                      f2 = int32_t(s0 ? f[c2] : f[c1]), f3 = int32_t(s0 ? f[c3] : f[0]);
         int32_t* o6 = faces + 6 * q;
-        if (dist3(v[0], v[2], g.fma) > dist3(v[1], v[3], g.fma)) {
-            o6[0] = f[1]; o6[1] = f[3]; o6[2] = f[0];
-            o6[3] = f[3]; o6[4] = f[1]; o6[5] = f[2];
-        } else {
-            o6[0] = f[2]; o6[1] = f[0]; o6[2] = f[1];
-            o6[3] = f[0]; o6[4] = f[2]; o6[5] = f[3];
-        }
+        o6[0] = second ? f1 : f2;
+        o6[1] = second ? f3 : f0;
+        o6[2] = second ? f0 : f1;
+        o6[3] = second ? f3 : f0;
+        o6[4] = second ? f1 : f2;
+        o6[5] = second ? f2 : f3;
         ++q;
     }
 }
@@ -1657,10 +1742,9 @@ struct DcDenseWs {
     DcWs d;
     unsigned long long* zero;  // cleared by the sign pass
     long long nzero;
-    long long* misc;           // [0..1] V  [2..3] dc_cells: entries, CTAs done  [4..7] eff  [8..12] counts [13] status when the caller has none
-    unsigned long long* wblk;  // weld: representatives per block of DC_BLOCK cells
+    long long* misc;           // [0..1] V  [2..3] dc_cells: entries, CTAs done  [4..7] eff  [8..12] counts [13] status when the caller has none  [14] numbering ticket  [15] vertices on faces
+    unsigned long long* wblk;  // weld: look-back states per NUM_TILE cells (room for two words each)
     uint4* seg;                // dc_cells: a record per segment (of 256 point words at least)
-    long long ntV;             // CTAs of the weld
     uint32_t *cells, *qoff, *vmap;
     uint8_t *used, *qbits;
     float* dual;
@@ -1675,7 +1759,7 @@ DcDenseWs carve_dense(void* ws, int nx, int ny, int nz, long long capA) {
     if (ws) w.d = carve(b, nx, ny, nz);
     const long long pwords = (long long)nx * ny * ((nz + 31) / 32);
     const long long n2048 = (pwords + 2047) / 2048;
-    w.ntV = (capA + DC_BLOCK - 1) / DC_BLOCK;
+    const long long ntV = (capA + NUM_TILE - 1) / NUM_TILE;
     size_t o = (base + 255) & ~size_t(255);
     auto take = [&](size_t bytes) {
         uint8_t* p = ws ? b + o : nullptr;
@@ -1685,7 +1769,7 @@ DcDenseWs carve_dense(void* ws, int nx, int ny, int nz, long long capA) {
     w.nzero = 16;
     w.zero = reinterpret_cast<unsigned long long*>(take(size_t(w.nzero) * 8));
     w.misc = reinterpret_cast<long long*>(w.zero);
-    w.wblk = reinterpret_cast<unsigned long long*>(take(size_t(w.ntV + 1) * 16));
+    w.wblk = reinterpret_cast<unsigned long long*>(take(size_t(ntV + 1) * 16));
     w.seg = reinterpret_cast<uint4*>(take(size_t(n2048) * 128));
     take(size_t(n2048) * 16);  // (the workspace's size is as it was)
     w.cells = reinterpret_cast<uint32_t*>(take(size_t(capA) * 4));
@@ -1780,7 +1864,8 @@ int iso_dc_intersection_sync(const float* values, int nx, int ny, int nz, const 
     }
     {
         iso::ProfScope ps("dc_classify", st, ix.p.nseg > CELLS_SCAN ? 2 : 1);
-        const CellsOut co{w.zero + 2, cell_capacity, 0x7fffffffll, point_capacity, eff, counts, off, status, w.gc};
+        const CellsOut co{w.zero + 2, cell_capacity, 0x7fffffffll, point_capacity, eff, counts, off, status, w.gc,
+                          nullptr, 0};
         launch_cells(w.d.S, g, ix, co, st);
     }
     {
@@ -1834,16 +1919,20 @@ static int dc_dense_impl(const float* values, int nx, int ny, int nz, const floa
     const CellIndex ix = cell_index(w, g, reinterpret_cast<unsigned long long*>(
                                               (reinterpret_cast<uintptr_t>(vertices) + 7) & ~uintptr_t(7)));
     const CellsOut co{w.zero + 2, capA, capQ, 0x7fffffffll, eff, counts, reinterpret_cast<uint32_t*>(cell_offsets),
-                      status, w.gc};
+                      status, w.gc, w.wblk, (capA + NUM_TILE - 1) / NUM_TILE};
     {
         iso::ProfScope ps("dc_classify", st, ix.p.nseg > CELLS_SCAN ? 2 : 1);
         launch_cells(w.d.S, g, ix, co, st);
     }
     if (capA > 0) {
+        // the list of vertices on faces follows the entries: room for all cells but at most one
+        const FaceList list{reinterpret_cast<uint32_t*>(ix.elist + capA), w.zero + 15,
+                            (reinterpret_cast<float*>(vertices) + 3 * capA) -
+                                reinterpret_cast<float*>(ix.elist + capA)};
         {
             iso::ProfScope ps("dc_solve", st);
             const int bt = iso::tune_get(iso::TUNE_DC_CELL_THREADS);
-            const SolveOut so{cells, w.qoff, w.qbits, w.used, w.dual, co.cell_off};
+            const SolveOut so{cells, w.qoff, w.qbits, w.used, w.dual, co.cell_off, list.cells, list.n, list.cap};
             const auto kernel = given ? (g.fma ? dc_solve_cells<true, true> : dc_solve_cells<false, true>)
                                       : (g.fma ? dc_solve_cells<true, false> : dc_solve_cells<false, false>);
             Given in = given ? *given : Given{};
@@ -1852,15 +1941,16 @@ static int dc_dense_impl(const float* values, int nx, int ny, int nz, const floa
                             static_cast<const long long*>(eff), static_cast<const float*>(w.gc), so, in);
         }
         {
-            iso::ProfScope ps("dc_weld", st, 3);
-            iso::launch_pdl(dc_weld_flags, unsigned(w.ntV), unsigned(DC_BLOCK), st, g,
-                            static_cast<const uint32_t*>(cells), static_cast<const uint8_t*>(w.used),
-                            static_cast<const float*>(w.dual), ix, static_cast<const long long*>(eff), w.vmap, w.wblk);
-            iso::launch_pdl(dc_block_scan, 1u, 1024u, st, w.wblk, w.ntV, w.misc);
-            iso::launch_pdl(dc_weld_number, unsigned(w.ntV), unsigned(DC_BLOCK), st,
+            iso::ProfScope ps("dc_weld", st, 2);
+            const uint32_t* cc = cells;
+            // (a few percent of the vertices lie on faces)
+            iso::launch_pdl(dc_weld_faces, std::min(blocks_for(capA, 16), 152u * 16u), 128u, st, g, ix,
+                            static_cast<const float*>(w.gc), list, cc, w.used, static_cast<const float*>(w.dual),
+                            static_cast<const long long*>(eff), w.vmap);
+            iso::launch_pdl(dc_weld_number, blocks_for(capA, NUM_TILE), unsigned(NUM_THREADS), st,
                             static_cast<const float*>(w.dual), static_cast<const long long*>(eff),
-                            static_cast<const unsigned long long*>(w.wblk), static_cast<const long long*>(w.misc),
-                            w.vmap, vertices, reinterpret_cast<uint32_t*>(vertex_source), counts);
+                            static_cast<const uint8_t*>(w.used), w.wblk, w.zero + 14, w.vmap, vertices,
+                            reinterpret_cast<uint32_t*>(vertex_source), counts, status);
         }
         {
             iso::ProfScope ps("dc_quads", st);

@@ -1,8 +1,8 @@
 // Dense-grid marching cubes on sm_103a.
 //
 // Five launches on one stream, nothing read back by the host:
-//   1. mc_signs   streams the grid once (one warp per row, 16 coalesced
-//                 128-byte loads in flight per warp) into a sign bitmap,
+//   1. mc_signs   streams the grid once (16 coalesced 128-byte loads in flight per
+//                 warp) into a sign bitmap,
 //                 1 bit per point.  This is the only pass over all values.
 //   2. mc_count   one CTA per segment of 256 to 1024 point words, from the bitmap
 //                 alone (16.8 MB at 512^3): the words near the surface, listed;
@@ -1205,42 +1205,77 @@ __global__ void __launch_bounds__(FIX_THREADS, FIX_CTAS) mc_fix(const FixArgs a)
 // 1. sign bitmap
 
 constexpr int SIGN_BLOCK = 256;
-constexpr int SIGN_UNROLL = 16;
 
-// Bit z % 32 of word [(x * ny + y) * NWg + z / 32] is (v - level < 0).  One warp
-// per grid row, all of the row's loads in flight before the ballots; lane w
-// keeps word w so each 32 words leave in one store.
-__global__ void __launch_bounds__(SIGN_BLOCK) mc_signs(const float* __restrict__ vals, long long rows,
-                                                       int nz, float level, uint32_t* __restrict__ out,
+// Bit z % 32 of word [(x * ny + y) * NW + z / 32] is (v - level < 0).  A warp has
+// 32 coalesced 128-byte loads in flight before their ballots, and lane w keeps
+// word w so that the words leave in one store.  Bound by HBM on large grids; a
+// warp per row, as before, had only a short row's loads in flight.
+// Both kernels clear `zero` (the counters, look-back states and small hash of
+// the call start at zero).
+
+// Rows that fill their words (nz a multiple of 32): 32 consecutive words are
+// 1024 consecutive values.  192^3: 17.4 us before, 11.7 now; 256^3 24.7 and 16.8;
+// 512^3 82.6 and 82.
+__global__ void __launch_bounds__(SIGN_BLOCK) mc_signs(const float* __restrict__ vals, unsigned long long PW,
+                                                       float level, uint32_t* __restrict__ out,
                                                        unsigned long long* __restrict__ zero, long long nzero) {
     iso::grid_wait();
-    // counters, look-back states and the small hash of the call start at zero
+    for (long long i = (long long)blockIdx.x * SIGN_BLOCK + threadIdx.x; i < nzero;
+         i += (long long)gridDim.x * SIGN_BLOCK)
+        zero[i] = 0ull;
+    const uint32_t lane = threadIdx.x & 31;
+    const unsigned long long step = (unsigned long long)gridDim.x * SIGN_BLOCK;  // 32 words per warp
+    for (unsigned long long base = ((unsigned long long)blockIdx.x * (SIGN_BLOCK / 32) + (threadIdx.x >> 5)) * 32;
+         base < PW; base += step) {
+        const float* q = vals + 32 * base + lane;
+        const uint32_t n = uint32_t(min(PW - base, 32ull));
+        float v[32];
+#pragma unroll
+        for (int u = 0; u < 32; ++u) v[u] = u < n ? __ldcs(q + 32 * u) : level;  // read once: evict first
+        uint32_t mine = 0;
+#pragma unroll
+        for (int u = 0; u < 32; ++u) {
+            const uint32_t b = __ballot_sync(~0u, iso::below(v[u], level));
+            if (uint32_t(u) == lane) mine = b;
+        }
+        if (lane < n) out[base + lane] = mine;
+    }
+}
+
+// Other rows: R of them at a time, W words of each (R * W = 32, W >= NW, or W = 32
+// and a row's words 32 at a time).  Carrying the place in the row from word to
+// word instead would keep all loads of short rows busy, but its address arithmetic
+// made it issue-bound on long ones (400 x 400 x 507: 77 us against 53).
+template <int R, int W>
+__global__ void __launch_bounds__(SIGN_BLOCK) mc_signs_rows(const float* __restrict__ vals, long long rows, int nz,
+                                                            int NW, float level, uint32_t* __restrict__ out,
+                                                            unsigned long long* __restrict__ zero, long long nzero) {
+    static_assert(R * W == 32, "a word per lane");
+    iso::grid_wait();
     for (long long i = (long long)blockIdx.x * SIGN_BLOCK + threadIdx.x; i < nzero;
          i += (long long)gridDim.x * SIGN_BLOCK)
         zero[i] = 0ull;
     const int lane = threadIdx.x & 31;
-    const int NWg = (nz + 31) / 32;
-    const long long warps = (long long)gridDim.x * (SIGN_BLOCK / 32);
-    for (long long row = (long long)blockIdx.x * (SIGN_BLOCK / 32) + (threadIdx.x >> 5); row < rows;
-         row += warps) {
-        const float* rp = vals + row * nz;
-        uint32_t* op = out + row * NWg;
-        for (int wb = 0; wb < NWg; wb += 32) {
-            uint32_t mine = 0;
-            for (int w0 = wb; w0 < min(NWg, wb + 32); w0 += SIGN_UNROLL) {
-                float v[SIGN_UNROLL];
+    const long long step = (long long)gridDim.x * (SIGN_BLOCK / 32) * R;
+    for (long long row = ((long long)blockIdx.x * (SIGN_BLOCK / 32) + (threadIdx.x >> 5)) * R; row < rows;
+         row += step) {
+        for (int wb = 0; wb < NW; wb += W) {
+            float v[32];
 #pragma unroll
-                for (int u = 0; u < SIGN_UNROLL; ++u) {
-                    const int z = 32 * (w0 + u) + lane;
-                    v[u] = (w0 + u < NWg && z < nz) ? __ldcs(rp + z) : level;  // read once: evict first
-                }
+            for (int r = 0; r < R; ++r) {
+                const float* q = vals + (row + r) * nz + 32 * wb + lane;
+                const int left = row + r < rows ? nz - 32 * wb - lane : 0;  // values of the row from the lane's on
 #pragma unroll
-                for (int u = 0; u < SIGN_UNROLL; ++u) {
-                    const uint32_t b = __ballot_sync(~0u, iso::below(v[u], level));
-                    if (((w0 + u) & 31) == lane) mine = b;
-                }
+                for (int w = 0; w < W; ++w) v[r * W + w] = 32 * w < left ? __ldcs(q + 32 * w) : level;
             }
-            if (wb + lane < NWg) op[wb + lane] = mine;
+            uint32_t mine = 0;
+#pragma unroll
+            for (int u = 0; u < 32; ++u) {
+                const uint32_t b = __ballot_sync(~0u, iso::below(v[u], level));
+                if (u == lane) mine = b;
+            }
+            const int r = lane / W, w = wb + lane % W;
+            if (row + r < rows && w < NW) out[(row + r) * NW + w] = mine;
         }
     }
 }
@@ -1336,11 +1371,22 @@ int mc_get_block() {
 
 void mc_signs_launch(const float* vals, int nx, int ny, int nz, float level, uint32_t* out,
                      cudaStream_t st, unsigned long long* zero, long long nzero) {
-    const long long rows = (long long)nx * ny;
-    const long long want = (rows + (SIGN_BLOCK / 32) - 1) / (SIGN_BLOCK / 32);
-    const long long per = iso::tune_get(iso::TUNE_MC_SIGN_CTAS);
-    const long long grid = std::max<long long>(1, std::min<long long>(want, (long long)sm_count() * per));
-    iso::launch_pdl(mc_signs, unsigned(grid), SIGN_BLOCK, st, vals, rows, nz, level, out, zero, nzero);
+    const int NW = (nz + 31) / 32;
+    const long long rows = (long long)nx * ny, most = (long long)sm_count() * iso::tune_get(iso::TUNE_MC_SIGN_CTAS);
+    const auto ctas = [&](long long warps) {
+        constexpr int per = SIGN_BLOCK / 32;
+        return unsigned(std::max<long long>(1, std::min<long long>((warps + per - 1) / per, most)));
+    };
+    if (nz % 32 == 0) {
+        const unsigned long long PW = (unsigned long long)rows * NW;
+        iso::launch_pdl(mc_signs, ctas((long long)((PW + 31) / 32)), SIGN_BLOCK, st, vals, PW, level, out, zero, nzero);
+        return;
+    }
+    const int R = NW <= 1 ? 32 : NW <= 2 ? 16 : NW <= 4 ? 8 : NW <= 8 ? 4 : NW <= 16 ? 2 : 1;
+    const auto kernel = R == 32 ? mc_signs_rows<32, 1> : R == 16 ? mc_signs_rows<16, 2>
+                        : R == 8 ? mc_signs_rows<8, 4> : R == 4 ? mc_signs_rows<4, 8>
+                        : R == 2 ? mc_signs_rows<2, 16> : mc_signs_rows<1, 32>;
+    iso::launch_pdl(kernel, ctas((rows + R - 1) / R), SIGN_BLOCK, st, vals, rows, nz, NW, level, out, zero, nzero);
 }
 
 // Bound on t for an edge vertex to land within a few ulps of an endpoint (the

@@ -16,8 +16,56 @@ namespace {
 
 constexpr int MAX_PRIMS = 32;
 
+// Union distances of Z points of a row, z = z0 + 32 j: a primitive's parameters
+// and everything of it that does not depend on z are taken once for all of them.
+// Every operation is rounded on its own, in the order of the formulas.
+template <int Z>
+__device__ __forceinline__ void union_points(const float (*pr)[7], int np, float px, float py, const float* pz,
+                                             float* d) {
+#pragma unroll
+    for (int j = 0; j < Z; ++j) d[j] = 3.402823466e38f;
+    for (int k = 0; k < np; ++k) {
+        const float dx = __fsub_rn(px, pr[k][1]), dy = __fsub_rn(py, pr[k][2]), cz = pr[k][3];
+        if (pr[k][0] == 0.0f) {
+            const float xy = __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), r = pr[k][4];
+#pragma unroll
+            for (int j = 0; j < Z; ++j) {
+                const float dz = __fsub_rn(pz[j], cz);
+                d[j] = fminf(d[j], __fsub_rn(__fsqrt_rn(__fadd_rn(xy, __fmul_rn(dz, dz))), r));
+            }
+        } else {
+            const float qx = __fsub_rn(fabsf(dx), pr[k][4]), qy = __fsub_rn(fabsf(dy), pr[k][5]), hz = pr[k][6];
+            const float ox = fmaxf(qx, 0.0f), oy = fmaxf(qy, 0.0f);
+            const float xy = __fadd_rn(__fmul_rn(ox, ox), __fmul_rn(oy, oy)), qxy = fmaxf(qx, qy);
+#pragma unroll
+            for (int j = 0; j < Z; ++j) {
+                const float qz = __fsub_rn(fabsf(__fsub_rn(pz[j], cz)), hz), oz = fmaxf(qz, 0.0f);
+                const float outside = __fsqrt_rn(__fadd_rn(xy, __fmul_rn(oz, oz)));
+                d[j] = fminf(d[j], __fadd_rn(outside, fminf(fmaxf(qxy, qz), 0.0f)));
+            }
+        }
+    }
+}
+
+template <int Z>
+__device__ __forceinline__ void union_run(const float (*pr)[7], int np, float px, float py, int z, int nz, float az,
+                                          float sz, bool fma, float* __restrict__ orow) {
+    float pz[Z], d[Z];
+#pragma unroll
+    for (int j = 0; j < Z; ++j) pz[j] = iso::grid_coord(uint32_t(min(z + 32 * j, nz - 1)), uint32_t(nz), az, sz, fma);
+    union_points<Z>(pr, np, px, py, pz, d);
+#pragma unroll
+    for (int j = 0; j < Z; ++j)
+        if (z + 32 * j < nz) orow[z + 32 * j] = d[j];
+}
+
 // prims: [0] = count (as a float), then count rows of 7 floats: kind (0 sphere,
 // 1 box), centre x y z, radius | half-extents x y z.
+// Bound by instruction issue.  Four points per lane share a primitive's shared
+// memory reads, its branch and its x and y terms: one point per lane issued some
+// 45 instructions per primitive and point.  Leaving out square roots that cannot
+// lower the minimum (compared squared) was slower: a warp takes the branch when
+// any of its lanes does.
 __global__ void __launch_bounds__(256) sdf_union_grid(const float* __restrict__ prims, int nx, int ny, int nz,
                                                       float ax, float ay, float az, float sx, float sy, float sz,
                                                       bool fma, float* __restrict__ out) {
@@ -38,28 +86,10 @@ __global__ void __launch_bounds__(256) sdf_union_grid(const float* __restrict__ 
         const float px = iso::grid_coord(uint32_t(x), uint32_t(nx), ax, sx, fma);
         const float py = iso::grid_coord(uint32_t(y), uint32_t(ny), ay, sy, fma);
         float* orow = out + row * nz;
-        for (int z = lane; z < nz; z += 32) {
-            const float pz = iso::grid_coord(uint32_t(z), uint32_t(nz), az, sz, fma);
-            float d = 3.402823466e38f;
-            for (int k = 0; k < np; ++k) {
-                const float dx = __fsub_rn(px, pr[k][1]), dy = __fsub_rn(py, pr[k][2]), dz = __fsub_rn(pz, pr[k][3]);
-                float dk;
-                if (pr[k][0] == 0.0f) {
-                    dk = __fsub_rn(__fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)),
-                                                        __fmul_rn(dz, dz))),
-                                   pr[k][4]);
-                } else {
-                    const float qx = __fsub_rn(fabsf(dx), pr[k][4]), qy = __fsub_rn(fabsf(dy), pr[k][5]),
-                                qz = __fsub_rn(fabsf(dz), pr[k][6]);
-                    const float ox = fmaxf(qx, 0.0f), oy = fmaxf(qy, 0.0f), oz = fmaxf(qz, 0.0f);
-                    const float outside =
-                        __fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(ox, ox), __fmul_rn(oy, oy)), __fmul_rn(oz, oz)));
-                    dk = __fadd_rn(outside, fminf(fmaxf(qx, fmaxf(qy, qz)), 0.0f));
-                }
-                d = fminf(d, dk);
-            }
-            orow[z] = d;
-        }
+        int z0 = 0;
+        for (; nz - z0 > 64; z0 += 128) union_run<4>(pr, np, px, py, z0 + lane, nz, az, sz, fma, orow);
+        if (nz - z0 > 32) union_run<2>(pr, np, px, py, z0 + lane, nz, az, sz, fma, orow);
+        else if (nz > z0) union_run<1>(pr, np, px, py, z0 + lane, nz, az, sz, fma, orow);
     }
 }
 

@@ -52,102 +52,83 @@ __global__ void __launch_bounds__(256) mc_backward(const float* __restrict__ val
     atomicAdd(gvals + ia + step, -gt * t / d);
 }
 
-// Trilinear weights at t and their derivatives along each axis (corner
-// j = 4x + 2y + z, the order of trilin()).
-__device__ __forceinline__ void tri_weights(const float t[3], float w[8], float dw[3][8]) {
+// Gradient of the grid normal at crossing point p (cell_normal) given dL/dn:
+// adds to the cell's corner values (gc) and to the point (gp).
+// The interpolant f is linear along each axis, so the stencil's difference along
+// axis a, (f(t + e_a) - f(t - e_a)) / width, is its derivative there whatever the
+// width (the clamps change the width only), and that derivative does not depend on
+// t_a.  With G_a = df/dt_a / size_a and n = G / |G|, the adjoint A_a = dL/dG_a / size_a
+// gives dL/dv_j = sum_a A_a dw_j/dt_a and dL/dt_b = sum_{a != b} A_a d2f/dt_a dt_b:
+// some 200 operations, where weights and their derivatives at all six samples of
+// the stencil took 850.
+__device__ __forceinline__ void normal_backward(const CellCorners& cc, const float* p, const float* gn, float* gp,
+                                                float* gc) {
+    float rsz[3], t[3], tin[3], o[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const float csz = __fsub_rn(cc.p[7][a], cc.p[0][a]);
+        const float r = __fdiv_rn(__fsub_rn(p[a], cc.p[0][a]), csz);
+        t[a] = fmaxf(0.01f, fminf(0.99f, r));
+        tin[a] = (r > 0.01f && r < 0.99f) ? 1.0f : 0.0f;
+        o[a] = 1.0f - t[a];
+        rsz[a] = 1.0f / csz;
+    }
+    const float* v = cc.v;  // corner 4x + 2y + z
+    // differences along z, then along y and x of them
+    const float z00 = v[1] - v[0], z01 = v[3] - v[2], z10 = v[5] - v[4], z11 = v[7] - v[6];
+    const float y00 = v[2] - v[0], y01 = v[3] - v[1], y10 = v[6] - v[4], y11 = v[7] - v[5];
+    const float x00 = v[4] - v[0], x01 = v[5] - v[1], x10 = v[6] - v[2], x11 = v[7] - v[3];
+    const float fx = o[1] * (o[2] * x00 + t[2] * x01) + t[1] * (o[2] * x10 + t[2] * x11);
+    const float fy = o[0] * (o[2] * y00 + t[2] * y01) + t[0] * (o[2] * y10 + t[2] * y11);
+    const float fz = o[0] * (o[1] * z00 + t[1] * z01) + t[0] * (o[1] * z10 + t[1] * z11);
+    const float fxy = o[2] * (x10 - x00) + t[2] * (x11 - x01);
+    const float fxz = o[1] * (x01 - x00) + t[1] * (x11 - x10);
+    const float fyz = o[0] * (y01 - y00) + t[0] * (y11 - y10);
+    const float G[3] = {fx * rsz[0], fy * rsz[1], fz * rsz[2]};
+    const float len = sqrtf(G[0] * G[0] + G[1] * G[1] + G[2] * G[2]);
+    if (!(len > 1e-8f)) return;  // the normal is the constant (0, 0, 1) there
+    const float rl = 1.0f / len;
+    const float n[3] = {G[0] * rl, G[1] * rl, G[2] * rl};
+    const float ng = n[0] * gn[0] + n[1] * gn[1] + n[2] * gn[2];
+    float A[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) A[a] = (gn[a] - n[a] * ng) * rl * rsz[a];
+    // dw_j/dt_a is the product of the other two axes' weights, signed by j's side of a
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
         const int bx = j >> 2, by = (j >> 1) & 1, bz = j & 1;
-        const float fx = bx ? t[0] : 1.0f - t[0], fy = by ? t[1] : 1.0f - t[1], fz = bz ? t[2] : 1.0f - t[2];
-        const float sx = bx ? 1.0f : -1.0f, sy = by ? 1.0f : -1.0f, sz = bz ? 1.0f : -1.0f;
-        w[j] = fx * fy * fz;
-        dw[0][j] = sx * fy * fz;
-        dw[1][j] = fx * sy * fz;
-        dw[2][j] = fx * fy * sz;
+        const float wx = bx ? t[0] : o[0], wy = by ? t[1] : o[1], wz = bz ? t[2] : o[2];
+        const float ax = bx ? A[0] : -A[0], ay = by ? A[1] : -A[1], az = bz ? A[2] : -A[2];
+        gc[j] += ax * (wy * wz) + ay * (wx * wz) + az * (wx * wy);
     }
-}
-
-// Gradient of the grid normal at crossing point p (cell_normal) given dL/dn:
-// adds to the cell's corner values (gc) and to the point (gp).
-__device__ __forceinline__ void normal_backward(const CellCorners& cc, const float* p, const float* gn, float* gp,
-                                                float* gc) {
-    const float eps = 0.02f;
-    float cmin[3], csz[3], t[3], tin[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        cmin[a] = cc.p[0][a];
-        csz[a] = __fsub_rn(cc.p[7][a], cc.p[0][a]);
-        const float r = __fdiv_rn(__fsub_rn(p[a], cmin[a]), csz[a]);
-        t[a] = fmaxf(0.01f, fminf(0.99f, r));
-        tin[a] = (r > 0.01f && r < 0.99f) ? 1.0f : 0.0f;
-    }
-    float d[3], den[3], fp[3], fm[3], sp[3], sm[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        float tp[3] = {t[0], t[1], t[2]}, tm[3] = {t[0], t[1], t[2]};
-        tp[a] = fminf(__fadd_rn(t[a], eps), 0.99f);
-        tm[a] = fmaxf(__fsub_rn(t[a], eps), 0.01f);
-        sp[a] = __fadd_rn(t[a], eps) < 0.99f ? 1.0f : 0.0f;
-        sm[a] = __fsub_rn(t[a], eps) > 0.01f ? 1.0f : 0.0f;
-        // the adjoint needs the stencil's values only to first order
-        fp[a] = iso::trilin_t<false, false>(cc.v, tp[0], tp[1], tp[2]);
-        fm[a] = iso::trilin_t<false, false>(cc.v, tm[0], tm[1], tm[2]);
-        den[a] = __fmul_rn(__fsub_rn(tp[a], tm[a]), csz[a]);
-        d[a] = __fdiv_rn(__fsub_rn(fp[a], fm[a]), den[a]);
-    }
-    const float len = sqrtf(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
-    if (!(len > 1e-8f)) return;  // the normal is the constant (0, 0, 1) there
-    const float n[3] = {d[0] / len, d[1] / len, d[2] / len};
-    const float ng = n[0] * gn[0] + n[1] * gn[1] + n[2] * gn[2];
-    float gd[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) gd[a] = (gn[a] - n[a] * ng) / len;
-    float gt[3] = {0.0f, 0.0f, 0.0f};
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        float tp[3] = {t[0], t[1], t[2]}, tm[3] = {t[0], t[1], t[2]};
-        tp[a] = fminf(t[a] + eps, 0.99f);
-        tm[a] = fmaxf(t[a] - eps, 0.01f);
-        float wp[8], wm[8], dwp[3][8], dwm[3][8];
-        tri_weights(tp, wp, dwp);
-        tri_weights(tm, wm, dwm);
-        const float s = gd[a] / den[a];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) gc[j] += s * (wp[j] - wm[j]);
-#pragma unroll
-        for (int b = 0; b < 3; ++b) {
-            float dfp = 0.0f, dfm = 0.0f;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                dfp += cc.v[j] * dwp[b][j];
-                dfm += cc.v[j] * dwm[b][j];
-            }
-            if (b == a) {
-                dfp *= sp[a];
-                dfm *= sm[a];
-            }
-            gt[b] += s * (dfp - dfm);
-        }
-        // the stencil's width (tp - tm) * csz changes where one side is clamped
-        gt[a] -= gd[a] * d[a] / den[a] * (sp[a] - sm[a]) * csz[a];
-    }
-#pragma unroll
-    for (int b = 0; b < 3; ++b) gp[b] += gt[b] * tin[b] / csz[b];
+    gp[0] += (A[1] * fxy + A[2] * fxz) * tin[0] * rsz[0];
+    gp[1] += (A[0] * fxy + A[2] * fyz) * tin[1] * rsz[1];
+    gp[2] += (A[0] * fxz + A[1] * fyz) * tin[2] * rsz[2];
 }
 
 // One thread per active cell.  The crossings, their normals and the QEF are
 // recomputed in the forward's order (the same bits), then the crossings are
 // walked again for the gradients; the cell's corners stay in registers (edge
-// corners are selected, not indexed).
-__global__ void __launch_bounds__(128) dc_backward(const float* __restrict__ vals, Grid3 g, float level,
+// corners are selected, not indexed), and the first crossings' points and normals
+// in shared memory between the two walks.  Bound by FP32 issue: spreading a
+// cell's crossings over two or four lanes, which shortens its chain, made it
+// slower (70 -> 105 and 98 us for 0.12 M cells before normal_backward's rewrite).
+// With it 42 us at 96 registers (five CTAs per SM: 942 CTAs are a wave and a
+// quarter), 35 at 72 with some spills (seven).
+constexpr int DCB_THREADS = 128;
+constexpr int DCB_KEEP = 6;  // crossings kept (a smooth surface's cells have three to six)
+
+__global__ void __launch_bounds__(DCB_THREADS, 7) dc_backward(const float* __restrict__ vals, Grid3 g, float level,
                                                    const uint32_t* __restrict__ cell_ids,
                                                    const uint32_t* __restrict__ cell_off, long long A,
                                                    float reg, float svd_tol,
                                                    const float* __restrict__ user_normals,
                                                    const float* __restrict__ gdual, float* gvals,
                                                    float* gnormals) {
+    __shared__ float kept[DCB_KEEP][7][DCB_THREADS];  // t, point, normal
     const long long a = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= A) return;
+    const int tid = threadIdx.x;
     float gx[3] = {gdual[3 * a], gdual[3 * a + 1], gdual[3 * a + 2]};
     const uint32_t cid = cell_ids[a];
     const int cz = int(cid % uint32_t(g.nz - 1));
@@ -168,20 +149,27 @@ __global__ void __launch_bounds__(128) dc_backward(const float* __restrict__ val
     for (uint32_t em = est; em; em &= em - 1, ++K) {
         const int e = __ffs(em) - 1;
         float p[3], n[3];
-        edge_cross(cc, level, e, p);
+        const float t = edge_cross(cc, level, e, p);
         if (user_normals) {
 #pragma unroll
             for (int q = 0; q < 3; ++q) n[q] = user_normals[3ll * (k0 + K) + q];
         } else {
             cell_normal(cc, p, n);
         }
+        if (K < uint32_t(DCB_KEEP)) {
+            kept[K][0][tid] = t;
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                kept[K][1 + q][tid] = p[q];
+                kept[K][4 + q][tid] = n[q];
+            }
+        }
         qef_add(Q, p[0], p[1], p[2], n[0], n[1], n[2]);
     }
     qef_finish(Q, K, reg, svd_tol);
-    const int ci[3] = {cx, cy, cz};
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
-        const float lo = coord(g, q, uint32_t(ci[q])), hi = coord(g, q, uint32_t(ci[q] + 1));
+        const float lo = cc.p[0][q], hi = cc.p[7][q];  // the cell's box
         const float xf = float(Q.x[q]);
         if (xf < lo || xf > hi) gx[q] = 0.0f;  // clipped: the output does not move
     }
@@ -194,13 +182,22 @@ __global__ void __launch_bounds__(128) dc_backward(const float* __restrict__ val
 #pragma unroll 1
     for (uint32_t em = est; em; em &= em - 1, ++k) {
         const int e = __ffs(em) - 1;
-        float p[3], n[3];
-        const float t = edge_cross(cc, level, e, p);
-        if (user_normals) {
+        float t, p[3], n[3];
+        if (k < uint32_t(DCB_KEEP)) {
+            t = kept[k][0][tid];
 #pragma unroll
-            for (int q = 0; q < 3; ++q) n[q] = user_normals[3ll * (k0 + k) + q];
+            for (int q = 0; q < 3; ++q) {
+                p[q] = kept[k][1 + q][tid];
+                n[q] = kept[k][4 + q][tid];
+            }
         } else {
-            cell_normal(cc, p, n);
+            t = edge_cross(cc, level, e, p);
+            if (user_normals) {
+#pragma unroll
+                for (int q = 0; q < 3; ++q) n[q] = user_normals[3ll * (k0 + k) + q];
+            } else {
+                cell_normal(cc, p, n);
+            }
         }
         float u[3], gn[3], gp[3];
 #pragma unroll
@@ -281,7 +278,7 @@ int iso_dc_backward(const float* values, int nx, int ny, int nz, const float* aa
     if (!values || !cell_ids || !cell_offsets || !grad_dual || !grad_values) return iso::fail_code(ISO_ERR_ARG);
     const Grid3 g = make_grid(nx, ny, nz, aabb_min, aabb_max);
     iso::ProfScope ps("dc_backward", st);
-    dc_backward<<<blocks_for(A, 128), 128, 0, st>>>(values, g, level, reinterpret_cast<const uint32_t*>(cell_ids),
+    dc_backward<<<blocks_for(A, DCB_THREADS), DCB_THREADS, 0, st>>>(values, g, level, reinterpret_cast<const uint32_t*>(cell_ids),
                                                     reinterpret_cast<const uint32_t*>(cell_offsets), A, reg,
                                                     svd_tol, normals, grad_dual, grad_values, grad_normals);
     return cudaGetLastError() == cudaSuccess ? 0 : iso::fail_code(ISO_ERR_CUDA);

@@ -139,42 +139,79 @@ __global__ void __launch_bounds__(DC_BLOCK) dc_cell_count(const uint32_t* __rest
     }
 }
 
-// Exclusive scan of block sums (one CTA; pairs of u64).
+// Exclusive scan of block sums (one CTA; pairs of u64).  A round is bound by its
+// chain of loads, shuffles and one barrier, so each takes 4096 pairs: a warp
+// scans four rows of 32 (14,676 pairs: 16 us, 22 at 1024 pairs a round).
+constexpr int BS_ROWS = 4;
+
+__device__ __forceinline__ void warp_scan2(unsigned long long& a, unsigned long long& b, int lane) {
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const unsigned long long x = __shfl_up_sync(~0u, a, d), y = __shfl_up_sync(~0u, b, d);
+        if (lane >= d) { a += x; b += y; }
+    }
+}
+
 __global__ void __launch_bounds__(1024) dc_block_scan(unsigned long long* blk, long long nblk,
                                                       long long* totals) {
-    __shared__ unsigned long long wa[32], wb[32], carry[2];
+    __shared__ unsigned long long wa[2][32], wb[2][32];
     iso::grid_wait();
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid == 0) { carry[0] = 0; carry[1] = 0; }
-    __syncthreads();
-    for (long long base = 0; base < nblk; base += 1024) {
-        const long long i = base + tid;
-        const unsigned long long a = i < nblk ? blk[2 * i] : 0ull, b = i < nblk ? blk[2 * i + 1] : 0ull;
-        unsigned long long ia = a, ib = b;
-        for (int d = 1; d < 32; d <<= 1) {
-            const unsigned long long x = __shfl_up_sync(~0u, ia, d), y = __shfl_up_sync(~0u, ib, d);
-            if (lane >= d) { ia += x; ib += y; }
-        }
-        if (lane == 31) { wa[warp] = ia; wb[warp] = ib; }
-        __syncthreads();
-        if (warp == 0) {
-            unsigned long long x = wa[lane], y = wb[lane];
-            for (int d = 1; d < 32; d <<= 1) {
-                const unsigned long long u = __shfl_up_sync(~0u, x, d), v = __shfl_up_sync(~0u, y, d);
-                if (lane >= d) { x += u; y += v; }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool wide = (reinterpret_cast<uintptr_t>(blk) & 15) == 0;
+    unsigned long long ca = 0, cb = 0;  // the rounds before
+    int buf = 0;
+    for (long long base = 0; base < nblk; base += 1024 * BS_ROWS, buf ^= 1) {
+        const long long i0 = base + warp * (32 * BS_ROWS) + lane;
+        unsigned long long a[BS_ROWS], b[BS_ROWS], ia[BS_ROWS], ib[BS_ROWS];
+#pragma unroll
+        for (int r = 0; r < BS_ROWS; ++r) {
+            const long long i = i0 + 32 * r;
+            a[r] = b[r] = 0;
+            if (i < nblk) {
+                if (wide) {
+                    const ulonglong2 p = reinterpret_cast<const ulonglong2*>(blk)[i];
+                    a[r] = p.x;
+                    b[r] = p.y;
+                } else {
+                    a[r] = blk[2 * i];
+                    b[r] = blk[2 * i + 1];
+                }
             }
-            wa[lane] = x;
-            wb[lane] = y;
         }
-        __syncthreads();
-        const unsigned long long ea = carry[0] + (warp ? wa[warp - 1] : 0ull) + ia - a;
-        const unsigned long long eb = carry[1] + (warp ? wb[warp - 1] : 0ull) + ib - b;
-        if (i < nblk) { blk[2 * i] = ea; blk[2 * i + 1] = eb; }
-        __syncthreads();
-        if (tid == 0) { carry[0] += wa[31]; carry[1] += wb[31]; }
-        __syncthreads();
+        unsigned long long ta = 0, tb = 0;  // the warp's rows before
+#pragma unroll
+        for (int r = 0; r < BS_ROWS; ++r) {
+            ia[r] = a[r];
+            ib[r] = b[r];
+            warp_scan2(ia[r], ib[r], lane);
+            const unsigned long long ra = __shfl_sync(~0u, ia[r], 31), rb = __shfl_sync(~0u, ib[r], 31);
+            ia[r] += ta - a[r];
+            ib[r] += tb - b[r];
+            ta += ra;
+            tb += rb;
+        }
+        if (lane == 0) { wa[buf][warp] = ta; wb[buf][warp] = tb; }
+        __syncthreads();  // the buffer's last reads are two rounds back
+        // every warp scans the warps' sums itself
+        unsigned long long x = wa[buf][lane], y = wb[buf][lane];
+        const unsigned long long ox = x, oy = y;
+        warp_scan2(x, y, lane);
+        const unsigned long long ea = ca + __shfl_sync(~0u, x - ox, warp), eb = cb + __shfl_sync(~0u, y - oy, warp);
+        ca += __shfl_sync(~0u, x, 31);
+        cb += __shfl_sync(~0u, y, 31);
+#pragma unroll
+        for (int r = 0; r < BS_ROWS; ++r) {
+            const long long i = i0 + 32 * r;
+            if (i >= nblk) continue;
+            if (wide) {
+                reinterpret_cast<ulonglong2*>(blk)[i] = make_ulonglong2(ea + ia[r], eb + ib[r]);
+            } else {
+                blk[2 * i] = ea + ia[r];
+                blk[2 * i + 1] = eb + ib[r];
+            }
+        }
     }
-    if (tid == 0) { totals[0] = (long long)carry[0]; totals[1] = (long long)carry[1]; }
+    if (threadIdx.x == 0) { totals[0] = (long long)ca; totals[1] = (long long)cb; }
 }
 
 // ---------------------------------------------------------------------------

@@ -567,9 +567,12 @@ __global__ void __launch_bounds__(SP2_THREADS) sp_mc_count2(SpGrid g, const int*
 
 // Output staging of one emit CTA: vertex-list entries and triangles up to
 // these counts go through shared memory and leave in coalesced stores; a CTA
-// with more (a dense patch of surface) writes the rest directly.
-constexpr int SP2_STAGE_V = 2048;
-constexpr int SP2_STAGE_F = 1024;
+// with more (a dense patch of surface) writes the rest directly.  A chunk of a
+// band ten cells deep has about 600 entries and 700 triangles; 768 each let
+// five CTAs be resident (371 -> 316 us for the band of a 1024^3 grid; 2048 and
+// 1024 hold four).
+constexpr int SP2_STAGE_V = 768;
+constexpr int SP2_STAGE_F = 768;
 
 struct SpStage {
     float* v;                  // [SP2_STAGE_V * 3]
@@ -624,7 +627,7 @@ __device__ __forceinline__ void sp_emit_near(const SpGrid& g, const Cell8& cc, u
 // offsets in list order.  A cell writes its used vertices in edge order and
 // its kept triangles as indices into the vertex list.  dn (device): nothing
 // is written when dn[0] == 0 (over capacity).
-__global__ void __launch_bounds__(SP2_THREADS) sp_mc_emit2(SpGrid g, const int* __restrict__ ids,
+__global__ void __launch_bounds__(SP2_THREADS, 5) sp_mc_emit2(SpGrid g, const int* __restrict__ ids,
                                                            const float* __restrict__ vals, long long n,
                                                            const unsigned long long* __restrict__ blk,
                                                            const uint16_t* __restrict__ clist,
@@ -638,9 +641,10 @@ __global__ void __launch_bounds__(SP2_THREADS) sp_mc_emit2(SpGrid g, const int* 
     __shared__ int32_t sf[SP2_STAGE_F * 3];
     __shared__ uint32_t wsum[2][SP2_THREADS / 32];
     __shared__ uint16_t slv[SP2_CHUNK];  // each listed cell's first own entry (CTA-local)
-    if (dn[0] == 0) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int i = threadIdx.x; i < 256; i += SP2_THREADS) tpk[i] = ISO_TRI_PACKED[g.method * 256 + i];
+    iso::grid_wait();
+    if (dn[0] == 0) return;
     const long long c0 = (long long)blockIdx.x * SP2_CHUNK;
     const uint32_t nl = clen[blockIdx.x];
     const uint16_t* gl = clist + (size_t)blockIdx.x * SP2_CHUNK;
@@ -1046,8 +1050,7 @@ void iso_block_scan_launch(unsigned long long* blk, long long nblk, long long* t
 size_t weld_dev_workspace(long long capA, long long capU);
 void weld_dev_launch(const float* pts, long long capA, long long capU, const int32_t* tri, long long capT,
                      const long long* eff,
-                     void* ws, float* vout, int32_t* fout, long long* vtot, int* status, cudaStream_t st,
-                     uint32_t* vsrc);
+                     void* ws, float* vout, int32_t* fout, long long* vtot, int* status, cudaStream_t st);
 
 namespace {
 
@@ -1055,6 +1058,7 @@ namespace {
 // entries, 0, 3 F, vertex capacity) for the weld, all 0 when they do not fit.
 __global__ void sp_mc_sizes2(const long long* __restrict__ tot, long long capF, long long capV, long long* eff,
                              long long* counts, int* status) {
+    iso::grid_wait();
     const long long F = tot[0], L = tot[1];
     const bool ok = F <= capF && L <= 3 * capF && 3 * F < 0x7fffffffll;
     if (!ok) atomicCAS(status, 0, int(ISO_ERR_OVERFLOW));
@@ -1068,6 +1072,7 @@ __global__ void sp_mc_sizes2(const long long* __restrict__ tot, long long capF, 
 
 __global__ void sp_mc_finish(const long long* __restrict__ vtot, long long capV, long long* counts, int* status,
                              long long* host) {
+    iso::grid_wait();
     const long long V = vtot[0];
     counts[0] = V;
     if (V > capV) atomicCAS(status, 0, int(ISO_ERR_OVERFLOW));
@@ -1142,17 +1147,17 @@ int sp_mc_launch(const int* ids, const float* vals, long long n, int nx, int ny,
         sp_mc_count2<<<chunks, SP2_THREADS, 0, st>>>(g, ids, vals, n, (unsigned long long*)w.blk, w.clist, w.ccnt,
                                                      w.cjy, w.clen);
         iso_block_scan_launch((unsigned long long*)w.blk, chunks, w.tot, st);
-        sp_mc_sizes2<<<1, 1, 0, st>>>(w.tot, face_capacity, vertex_capacity, eff, counts, status);
-        sp_mc_emit2<<<chunks, SP2_THREADS, 0, st>>>(g, ids, vals, n, (const unsigned long long*)w.blk, w.clist,
-                                                    w.ccnt, w.cjy, w.clen, w.soup, w.tri, eff);
+        iso::launch_pdl(sp_mc_sizes2, 1u, 1u, st, w.tot, face_capacity, vertex_capacity, eff, counts, status);
+        iso::launch_pdl(sp_mc_emit2, chunks, unsigned(SP2_THREADS), st, g, ids, vals, n,
+                        (const unsigned long long*)w.blk, w.clist, w.ccnt, w.cjy, w.clen, w.soup, w.tri, eff);
     }
     // the weld of the vertex list: its table holds vertex_capacity distinct
     // positions; more report an overflow with a vertex count that fits on the rerun
     weld_dev_launch(w.soup, 3 * face_capacity, std::max<long long>(vertex_capacity, 1), w.tri, 3 * face_capacity,
-                    eff, w.weld, vertices, faces, w.tot + 8, status, st, nullptr);
+                    eff, w.weld, vertices, faces, w.tot + 8, status, st);
     {
         iso::ProfScope ps("sparse_mc", st);
-        sp_mc_finish<<<1, 1, 0, st>>>(w.tot + 8, vertex_capacity, counts, status, host);
+        iso::launch_pdl(sp_mc_finish, 1u, 1u, st, w.tot + 8, vertex_capacity, counts, status, host);
     }
     return cudaGetLastError() == cudaSuccess ? 0 : iso::fail_code(ISO_ERR_CUDA);
 }

@@ -5,13 +5,17 @@
 // the first entry with its position.
 //
 //   weld_insert   hash table of positions: a slot keeps the smallest entry
-//                 with its position.  Two entries per thread, their probes in
-//                 flight together (the kernel is bound by the latency of
-//                 dependent atomics and gathers, not by bytes).
-//   weld_number   per tile of 512 entries: each entry's first entry (table
-//                 lookup), the tile's number of first entries, the exclusive
-//                 prefix over tiles by decoupled look-back, and the first
-//                 entries' new numbers and positions written out.
+//                 with its position, and every entry its slot.  Two entries per
+//                 thread, their probes in flight together (the kernel is bound
+//                 by the latency of dependent atomics and gathers, not by
+//                 bytes; a persistent grid or four entries are slower: 288 and
+//                 366 us against 174 for the band of a 1024^3 grid).
+//   weld_number   per tile of 1024 entries: each entry's first entry (one read
+//                 of its slot; hashing the position, reading the slot and
+//                 comparing the positions again took 217 us there, this 119 and
+//                 13 more in the insert), the tile's number of first entries,
+//                 the exclusive prefix over tiles by decoupled look-back, and
+//                 the first entries' new numbers and positions written out.
 //   weld_remap    triangle indices -> new numbers.
 #include <algorithm>
 #include <cstdint>
@@ -25,8 +29,10 @@
 namespace {
 
 constexpr int WELD_THREADS = 256;
-constexpr int WELD_PER = 2;                           // entries per thread (insert, numbering)
-constexpr int WELD_TILE = WELD_THREADS * WELD_PER;    // entries per CTA
+constexpr int WELD_PER = 2;                           // entries per thread of the insert
+constexpr int WELD_TILE = WELD_THREADS * WELD_PER;
+constexpr int NUM_PER = 4;                            // entries per thread of the numbering
+constexpr int NUM_TILE = WELD_THREADS * NUM_PER;
 constexpr int REMAP_PER = 4;                          // triangle indices per thread of the remap
 constexpr uint32_t WELD_EMPTY = 0xffffffffu;          // a free table slot
 constexpr uint32_t WELD_NEW = 0x80000000u;            // rep[a]: a is a first entry; low bits its new number
@@ -45,36 +51,29 @@ __device__ __forceinline__ Key key_of(const float* __restrict__ pts, long long a
 __device__ __forceinline__ bool same(const Key& a, const Key& b) { return a.x == b.x && a.y == b.y && a.z == b.z; }
 __device__ __forceinline__ uint32_t slot_of(const Key& k, uint32_t mask) { return pos_hash(k.x, k.y, k.z) & mask; }
 
-// The rest of an insert whose first probe met another position.
-__device__ __noinline__ void insert_probe(const float* __restrict__ pts, uint32_t* table, uint32_t mask, Key k,
-                                          uint32_t h, uint32_t a, int* status) {
-    if (*(volatile int*)status == int(ISO_ERR_OVERFLOW)) return;  // the output is discarded anyway
+// The rest of an insert whose first probe met another position: the slot, or
+// WELD_EMPTY (not placed: the status says overflow).
+__device__ __noinline__ uint32_t insert_probe(const float* __restrict__ pts, uint32_t* table, uint32_t mask, Key k,
+                                              uint32_t h, uint32_t a, int* status) {
+    if (*(volatile int*)status == int(ISO_ERR_OVERFLOW)) return WELD_EMPTY;  // the output is discarded anyway
     for (uint32_t p = 1; p <= mask && p < WELD_PROBES; ++p) {
         h = (h + 1) & mask;
         const uint32_t cur = atomicCAS(&table[h], WELD_EMPTY, a);
-        if (cur == WELD_EMPTY) return;
+        if (cur == WELD_EMPTY) return h;
         if (same(key_of(pts, cur), k)) {
             if (a < cur) atomicMin(&table[h], a);
-            return;
+            return h;
         }
     }
     atomicCAS(status, 0, int(ISO_ERR_OVERFLOW));
+    return WELD_EMPTY;
 }
 
-// The rest of a lookup whose first probe met another position.
-__device__ __noinline__ uint32_t lookup_probe(const float* __restrict__ pts, const uint32_t* table, uint32_t mask,
-                                              Key k, uint32_t h, uint32_t a) {
-    for (uint32_t p = 1; p <= mask && p < WELD_PROBES; ++p) {
-        h = (h + 1) & mask;
-        const uint32_t cur = table[h];
-        if (cur == WELD_EMPTY) break;
-        if (same(key_of(pts, cur), k)) return cur;
-    }
-    return a;  // not placed (the status says overflow)
-}
-
+// slot <- each entry's slot, so that the numbering reads the first
+// entry with its position from there instead of hashing and comparing again.
 __global__ void __launch_bounds__(WELD_THREADS) weld_insert(const float* __restrict__ pts, long long A,
-                                                            uint32_t* table, uint32_t mask, int* status,
+                                                            uint32_t* table, uint32_t mask,
+                                                            uint32_t* __restrict__ slot, int* status,
                                                             const long long* __restrict__ dn) {
     if (dn) A = dn[0];
     const long long base = (long long)blockIdx.x * WELD_TILE + threadIdx.x;
@@ -92,6 +91,7 @@ __global__ void __launch_bounds__(WELD_THREADS) weld_insert(const float* __restr
         if (live[e]) {
             h[e] = slot_of(k[e], mask);
             cur[e] = atomicCAS(&table[h[e]], WELD_EMPTY, uint32_t(base + e * WELD_THREADS));
+            slot[base + e * WELD_THREADS] = h[e];
         }
     Key o[WELD_PER];
 #pragma unroll
@@ -104,25 +104,26 @@ __global__ void __launch_bounds__(WELD_THREADS) weld_insert(const float* __restr
         if (same(o[e], k[e])) {
             if (a < cur[e]) atomicMin(&table[h[e]], a);
         } else {
-            insert_probe(pts, table, mask, k[e], h[e], a, status);
+            slot[a] = insert_probe(pts, table, mask, k[e], h[e], a, status);
         }
     }
 }
 
-// rep[a] <- WELD_NEW | new number for a first entry, else the first entry with
-// a's position; vout / vsrc <- the first
-// entries' positions and entries (up to capV); vtot[0] <- the number of
-// distinct positions.  Tiles are taken in ticket order (ctr) and chained by
-// look-back (state, one word per tile, zeroed by the caller).
+// rep[a], on entry the entry's slot, <- WELD_NEW | new number for a first
+// entry, else the first entry with a's position; vout <- the first entries'
+// positions (up to capV); vtot[0] <- the number of distinct positions.  Tiles
+// are taken in ticket order (ctr) and chained by look-back (state, one word per
+// tile, zeroed by the caller).
 __global__ void __launch_bounds__(WELD_THREADS) weld_number(const float* __restrict__ pts, long long A,
-                                                            const uint32_t* __restrict__ table, uint32_t mask,
+                                                            const uint32_t* __restrict__ table,
                                                             uint32_t* __restrict__ rep, unsigned long long* state,
                                                             unsigned int* ctr, float* __restrict__ vout,
-                                                            uint32_t* __restrict__ vsrc, long long* vtot, int* status,
+                                                            long long* vtot, int* status,
                                                             const long long* __restrict__ dn) {
     __shared__ uint32_t tile_s;
     __shared__ uint32_t wsum[WELD_THREADS / 32];
     __shared__ unsigned long long pre_s;
+    iso::grid_wait();
     long long capV = 0x7fffffffll;
     if (dn) {
         A = dn[0];
@@ -131,41 +132,27 @@ __global__ void __launch_bounds__(WELD_THREADS) weld_number(const float* __restr
     if (threadIdx.x == 0) tile_s = atomicAdd(ctr, 1u);
     __syncthreads();
     const uint32_t tile = tile_s;
-    const long long ntile = (A + WELD_TILE - 1) / WELD_TILE;
+    const long long ntile = (A + NUM_TILE - 1) / NUM_TILE;
     if ((long long)tile >= ntile) {
         if (tile == 0 && threadIdx.x == 0) { vtot[0] = 0; vtot[1] = 0; }  // no points
         return;
     }
-    // entries a0 .. a0 + 3 of this thread (consecutive: the prefix is in list order)
-    const long long a0 = (long long)tile * WELD_TILE + threadIdx.x * WELD_PER;
-    Key k[WELD_PER];
-    uint32_t h[WELD_PER], cur[WELD_PER], r[WELD_PER];
-    bool live[WELD_PER];
+    // this thread's entries, consecutive: the prefix is in list order
+    const long long a0 = (long long)tile * NUM_TILE + threadIdx.x * NUM_PER;
+    uint32_t r[NUM_PER];
+    const bool full = a0 + NUM_PER <= A;
+    if (full) {
+        const uint4 q = *reinterpret_cast<const uint4*>(rep + a0);
+        r[0] = q.x; r[1] = q.y; r[2] = q.z; r[3] = q.w;
+    } else {
 #pragma unroll
-    for (int e = 0; e < WELD_PER; ++e) {
-        live[e] = a0 + e < A;
-        r[e] = WELD_EMPTY;
-        if (live[e]) k[e] = key_of(pts, a0 + e);
+        for (int e = 0; e < NUM_PER; ++e) r[e] = a0 + e < A ? rep[a0 + e] : WELD_EMPTY;
     }
-#pragma unroll
-    for (int e = 0; e < WELD_PER; ++e)
-        if (live[e]) {
-            h[e] = slot_of(k[e], mask);
-            cur[e] = table[h[e]];
-        }
-    Key o[WELD_PER];
-#pragma unroll
-    for (int e = 0; e < WELD_PER; ++e)
-        if (live[e] && cur[e] != WELD_EMPTY) o[e] = key_of(pts, cur[e]);
     uint32_t cnt = 0;
 #pragma unroll
-    for (int e = 0; e < WELD_PER; ++e) {
-        if (!live[e]) continue;
-        const uint32_t a = uint32_t(a0 + e);
-        if (cur[e] != WELD_EMPTY && same(o[e], k[e])) r[e] = cur[e];
-        else r[e] = cur[e] == WELD_EMPTY ? a : lookup_probe(pts, table, mask, k[e], h[e], a);
-        cnt += r[e] == a ? 1u : 0u;
-    }
+    for (int e = 0; e < NUM_PER; ++e) r[e] = r[e] != WELD_EMPTY ? table[r[e]] : uint32_t(a0 + e);  // not placed: itself
+#pragma unroll
+    for (int e = 0; e < NUM_PER; ++e) cnt += a0 + e < A && r[e] == uint32_t(a0 + e) ? 1u : 0u;
     // exclusive prefix of first entries: in the tile, then over tiles
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t inc = cnt;
@@ -193,23 +180,33 @@ __global__ void __launch_bounds__(WELD_THREADS) weld_number(const float* __restr
             }
         }
     }
+    // the first entries' positions, while warp 0 looks back
+    float p[NUM_PER][3];
+#pragma unroll
+    for (int e = 0; e < NUM_PER; ++e)
+        if (a0 + e < A && r[e] == uint32_t(a0 + e)) {
+            const float* s = pts + 3 * (a0 + e);
+            p[e][0] = s[0]; p[e][1] = s[1]; p[e][2] = s[2];
+        }
     __syncthreads();
     unsigned long long no = pre_s + before + inc - cnt;
 #pragma unroll
-    for (int e = 0; e < WELD_PER; ++e) {
-        if (a0 + e >= A) break;
-        const uint32_t a = uint32_t(a0 + e);
-        if (r[e] == a) {
-            rep[a] = WELD_NEW | uint32_t(no);
+    for (int e = 0; e < NUM_PER; ++e) {
+        if (a0 + e < A && r[e] == uint32_t(a0 + e)) {
+            r[e] = WELD_NEW | uint32_t(no);
             if ((long long)no < capV) {  // past the capacity the caller sees V and retries
                 float* v = vout + 3 * no;
-                v[0] = pts[3ll * a]; v[1] = pts[3ll * a + 1]; v[2] = pts[3ll * a + 2];
-                if (vsrc) vsrc[no] = a;
+                v[0] = p[e][0]; v[1] = p[e][1]; v[2] = p[e][2];
             }
             ++no;
-        } else {
-            rep[a] = r[e];
         }
+    }
+    if (full) {
+        *reinterpret_cast<uint4*>(rep + a0) = make_uint4(r[0], r[1], r[2], r[3]);
+    } else {
+#pragma unroll
+        for (int e = 0; e < NUM_PER; ++e)
+            if (a0 + e < A) rep[a0 + e] = r[e];
     }
 }
 
@@ -217,6 +214,7 @@ __global__ void __launch_bounds__(WELD_THREADS) weld_number(const float* __restr
 __global__ void __launch_bounds__(WELD_THREADS) weld_remap(const int32_t* __restrict__ tri, long long n,
                                                            const uint32_t* __restrict__ rep, int32_t* fout,
                                                            const long long* __restrict__ dn) {
+    iso::grid_wait();
     if (dn) n = dn[2];
     const long long base = (long long)blockIdx.x * (WELD_THREADS * REMAP_PER) + threadIdx.x;
     uint32_t r[REMAP_PER];
@@ -273,7 +271,7 @@ size_t weld_dev_workspace(long long capA, long long capU) { return weld_dev_carv
 // eff[3] vertex capacity of vout.  vtot[0] <- V.
 void weld_dev_launch(const float* pts, long long capA, long long capU, const int32_t* tri, long long capT,
                      const long long* eff, void* ws, float* vout, int32_t* fout, long long* vtot, int* status,
-                     cudaStream_t st, uint32_t* vsrc) {
+                     cudaStream_t st) {
     const WeldDev w = weld_dev_carve(ws, capA, capU);
     iso::ProfScope ps("dc_weld", st, (capT > 0 ? 1 : 0) + (capA > 0 ? 2 : 0));
     if (capA > 0) {
@@ -281,16 +279,16 @@ void weld_dev_launch(const float* pts, long long capA, long long capU, const int
         unsigned int* ctr = reinterpret_cast<unsigned int*>(w.state + tiles);
         cudaMemsetAsync(w.table, 0xff, size_t(w.hcap) * 4, st);
         cudaMemsetAsync(w.state, 0, w.state_bytes, st);
-        weld_insert<<<tiles, WELD_THREADS, 0, st>>>(pts, capA, w.table, w.hcap - 1, status, eff);
-        weld_number<<<tiles, WELD_THREADS, 0, st>>>(pts, capA, w.table, w.hcap - 1, w.rep, w.state, ctr, vout, vsrc,
-                                                    vtot, status, eff);
+        weld_insert<<<tiles, WELD_THREADS, 0, st>>>(pts, capA, w.table, w.hcap - 1, w.rep, status, eff);
+        iso::launch_pdl(weld_number, unsigned((capA + NUM_TILE - 1) / NUM_TILE), unsigned(WELD_THREADS), st, pts, capA,
+                        w.table, w.rep, w.state, ctr, vout, vtot, status, eff);
     } else {
         cudaMemsetAsync(vtot, 0, 16, st);
     }
     if (capT > 0) {
         const long long per = (long long)WELD_THREADS * REMAP_PER;
-        weld_remap<<<unsigned(std::max<long long>((capT + per - 1) / per, 1)), WELD_THREADS, 0, st>>>(tri, capT,
-                                                                                                     w.rep, fout, eff);
+        iso::launch_pdl(weld_remap, unsigned(std::max<long long>((capT + per - 1) / per, 1)), unsigned(WELD_THREADS),
+                        st, tri, capT, w.rep, fout, eff);
     }
 }
 
@@ -305,16 +303,13 @@ void weld_dev_launch(const float* pts, long long capA, long long capU, const int
 
 namespace {
 
-__global__ void __launch_bounds__(WELD_THREADS) mesh_lookup(const float* __restrict__ pts, long long V,
-                                                            const uint32_t* __restrict__ table, uint32_t mask,
+// rep[a], on entry the vertex's slot, <- the first vertex with its position.
+__global__ void __launch_bounds__(WELD_THREADS) mesh_lookup(long long V, const uint32_t* __restrict__ table,
                                                             uint32_t* __restrict__ rep) {
     const long long a = (long long)blockIdx.x * WELD_THREADS + threadIdx.x;
     if (a >= V) return;
-    const Key k = key_of(pts, a);
-    uint32_t h = slot_of(k, mask);
-    const uint32_t cur = table[h];
-    if (cur != WELD_EMPTY && same(key_of(pts, cur), k)) rep[a] = cur;
-    else rep[a] = cur == WELD_EMPTY ? uint32_t(a) : lookup_probe(pts, table, mask, k, h, uint32_t(a));
+    const uint32_t h = rep[a];
+    rep[a] = h != WELD_EMPTY ? table[h] : uint32_t(a);
 }
 
 // Faces through rep; keep[i] = no two corners at one position; used[v] = 1
@@ -413,9 +408,8 @@ int iso_weld_mesh(const float* vertices, long long V, const int* faces, long lon
     iso::ProfScope ps("weld_mesh", st, 4);
     cudaMemsetAsync(w.table, 0xff, size_t(w.hcap) * 4, st);
     cudaMemsetAsync(w.used, 0, size_t(V) * 4, st);
-    weld_insert<<<tiles_for(V), WELD_THREADS, 0, st>>>(vertices, V, w.table, w.hcap - 1, status, nullptr);
-    mesh_lookup<<<unsigned((V + WELD_THREADS - 1) / WELD_THREADS), WELD_THREADS, 0, st>>>(vertices, V, w.table,
-                                                                                         w.hcap - 1, w.rep);
+    weld_insert<<<tiles_for(V), WELD_THREADS, 0, st>>>(vertices, V, w.table, w.hcap - 1, w.rep, status, nullptr);
+    mesh_lookup<<<unsigned((V + WELD_THREADS - 1) / WELD_THREADS), WELD_THREADS, 0, st>>>(V, w.table, w.rep);
     mesh_faces<<<unsigned((F + WELD_THREADS - 1) / WELD_THREADS), WELD_THREADS, 0, st>>>(
         reinterpret_cast<const int32_t*>(faces), F, w.rep, w.f2, w.keep, w.used);
     size_t tb = w.temp_bytes;

@@ -20,6 +20,7 @@
 #include "common.cuh"
 #define ISO_LUT_DECL static __constant__ const
 #include "luts.h"
+#include "dc_common.cuh"
 #include "mc_dense.cuh"
 #include "profile.cuh"
 
@@ -397,6 +398,26 @@ __device__ __forceinline__ uint32_t sp_pack(uint32_t f, uint32_t used, bool fast
 }
 __device__ __forceinline__ uint32_t sp_used(uint32_t pc) { return (pc >> 4) & 0xfffu; }
 
+// A list entry: the cell's place in its chunk, bit 15 set when its corner 0 is
+// below the level.
+__device__ __forceinline__ uint32_t sp_at(uint32_t entry) { return entry & 0x7fffu; }
+static_assert(SP2_CHUNK <= 0x8000, "a place fits 15 bits");
+
+// The case from the crossed edges and corner 0's sign: along the cube's edges
+// 0-1, 0-2, 2-3, 0-4, 4-5, 4-6, 6-7.
+constexpr bool sp_joins(int e, int a, int b) {
+    return iso_edge_corner(2 * e) + iso_edge_corner(2 * e + 1) == a + b &&
+           iso_edge_corner(2 * e) * iso_edge_corner(2 * e + 1) == a * b;
+}
+static_assert(sp_joins(0, 0, 1) && sp_joins(3, 0, 2) && sp_joins(2, 2, 3) && sp_joins(8, 0, 4) &&
+                  sp_joins(4, 4, 5) && sp_joins(7, 4, 6) && sp_joins(6, 6, 7), "the edges sp_case_of walks");
+__device__ __forceinline__ uint32_t sp_case_of(uint32_t est, uint32_t c0) {
+    const uint32_t c2 = c0 ^ (est >> 3), c4 = c0 ^ (est >> 8), c6 = c4 ^ (est >> 7);
+    const uint32_t c1 = c0 ^ est, c3 = c2 ^ (est >> 2), c5 = c4 ^ (est >> 4), c7 = c6 ^ (est >> 6);
+    return (c0 & 1u) | (c1 & 1u) << 1 | (c2 & 1u) << 2 | (c3 & 1u) << 3 | (c4 & 1u) << 4 | (c5 & 1u) << 5 |
+           (c6 & 1u) << 6 | (c7 & 1u) << 7;
+}
+
 // Edges whose vertex an earlier cell of the same x can make, in slot order:
 // 0, 3, 4, 7, 8, 9, 11.
 __host__ __device__ constexpr int sp_slot_edge(int s) {
@@ -486,11 +507,11 @@ __device__ __forceinline__ uint32_t sp_owners(const SpGrid& g, const float* vals
     }
     if (jz < 0 && jy < 0 && jyl < 0 && jyh < 0) return 0u;
     float d[8], vz[8], vy[8], vl[8], vh[8];
-    load8(vals, c0 + list[j], d);
-    if (jz >= 0) load8(vals, c0 + list[jz], vz);
-    if (jy >= 0) load8(vals, c0 + list[jy], vy);
-    if (jyl >= 0) load8(vals, c0 + list[jyl], vl);
-    if (jyh >= 0) load8(vals, c0 + list[jyh], vh);
+    load8(vals, c0 + sp_at(list[j]), d);
+    if (jz >= 0) load8(vals, c0 + sp_at(list[jz]), vz);
+    if (jy >= 0) load8(vals, c0 + sp_at(list[jy]), vy);
+    if (jyl >= 0) load8(vals, c0 + sp_at(list[jyl]), vl);
+    if (jyh >= 0) load8(vals, c0 + sp_at(list[jyh]), vh);
     // the neighbour's corner k' holds this cell's corner k: z (k | 1), y (k | 2)
     const bool z0 = jz >= 0 && same_bits(d[0], vz[1]), z2 = jz >= 0 && same_bits(d[2], vz[3]);
     const bool z4 = jz >= 0 && same_bits(d[4], vz[5]), z6 = jz >= 0 && same_bits(d[6], vz[7]);
@@ -543,6 +564,7 @@ __global__ void __launch_bounds__(SP2_THREADS) sp_mc_count2(SpGrid g, const int*
         bool fast;
         const uint32_t f = sp_cell_summary(g, ids, c, cc, cs, ev, used, fast);
         summ[j] = uint16_t(sp_pack(f, used, fast));
+        list[j] |= uint16_t((cs & 1u) << 15);
         cid[j] = uint32_t(__ldg(ids + c));
     }
     __syncthreads();
@@ -569,8 +591,8 @@ __global__ void __launch_bounds__(SP2_THREADS) sp_mc_count2(SpGrid g, const int*
 // these counts go through shared memory and leave in coalesced stores; a CTA
 // with more (a dense patch of surface) writes the rest directly.  A chunk of a
 // band ten cells deep has about 600 entries and 700 triangles; 768 each let
-// five CTAs be resident (371 -> 316 us for the band of a 1024^3 grid; 2048 and
-// 1024 hold four).
+// six CTAs be resident (for the band of a 1024^3 grid 371 us with 2048 and 1024,
+// which hold four, 302 with six CTAs, 336 with seven, whose registers spill).
 constexpr int SP2_STAGE_V = 768;
 constexpr int SP2_STAGE_F = 768;
 
@@ -599,6 +621,29 @@ __device__ __forceinline__ void stage_face(const SpStage& s, uint32_t k, uint32_
     }
 }
 
+// The vertex on edge q of sparse cell c: edge_point's values from the two
+// corners alone.
+__device__ __forceinline__ void sp_edge_point(const SpGrid& g, const int* ids, const float* vals, long long c, int q,
+                                              float* p) {
+    const int a = edge_ca(q), b = edge_cb(q);
+    const float va = __ldg(vals + 8 * c + a), vb = __ldg(vals + 8 * c + b);
+    int x, y, z;
+    cell_xyz(g, uint32_t(__ldg(ids + c)), x, y, z);
+    const int ax = __ffs(a ^ b) - 1;  // corner bits: 0 z, 1 y, 2 x
+    const float px = iso::grid_coord(x + (a >> 2), g.nx, g.amin[0], g.asize[0], g.fma);
+    const float py = iso::grid_coord(y + ((a >> 1) & 1), g.ny, g.amin[1], g.asize[1], g.fma);
+    const float pz = iso::grid_coord(z + (a & 1), g.nz, g.amin[2], g.asize[2], g.fma);
+    // the far corner's coordinate along the edge
+    const int i = ax == 2 ? x + (b >> 2) : (ax == 1 ? y + ((b >> 1) & 1) : z + (b & 1));
+    const float far = iso::grid_coord(i, ax == 2 ? g.nx : (ax == 1 ? g.ny : g.nz),
+                                      ax == 2 ? g.amin[0] : (ax == 1 ? g.amin[1] : g.amin[2]),
+                                      ax == 2 ? g.asize[0] : (ax == 1 ? g.asize[1] : g.asize[2]), g.fma);
+    const float t = iso::cross_t(g.level, va, vb);
+    p[0] = iso::lerp1(t, px, ax == 2 ? far : px, g.fma);
+    p[1] = iso::lerp1(t, py, ax == 1 ? far : py, g.fma);
+    p[2] = iso::lerp1(t, pz, ax == 0 ? far : pz, g.fma);
+}
+
 // A cell with a vertex near a corner: its triangles are kept by position
 // (as mc_cell does), so every crossed edge's position is needed.  Its
 // position array is indexed by the triangle table and lives in local memory;
@@ -624,10 +669,13 @@ __device__ __forceinline__ void sp_emit_near(const SpGrid& g, const Cell8& cc, u
 
 // Per CTA: its crossed cells in cell order (from the count pass), 256 per
 // round; a block scan of each round's (faces, vertices) gives every cell its
-// offsets in list order.  A cell writes its used vertices in edge order and
-// its kept triangles as indices into the vertex list.  dn (device): nothing
+// offsets in list order.  A cell lists its used vertices in edge order and
+// writes its kept triangles as indices into the vertex list; its case comes from
+// its summary, not from its values.  The listed vertices are computed after the
+// rounds, one edge per lane of full warps (twelve predicated edges per cell
+// before: 316 us, this 302).  dn (device): nothing
 // is written when dn[0] == 0 (over capacity).
-__global__ void __launch_bounds__(SP2_THREADS, 5) sp_mc_emit2(SpGrid g, const int* __restrict__ ids,
+__global__ void __launch_bounds__(SP2_THREADS, 6) sp_mc_emit2(SpGrid g, const int* __restrict__ ids,
                                                            const float* __restrict__ vals, long long n,
                                                            const unsigned long long* __restrict__ blk,
                                                            const uint16_t* __restrict__ clist,
@@ -638,6 +686,7 @@ __global__ void __launch_bounds__(SP2_THREADS, 5) sp_mc_emit2(SpGrid g, const in
                                                            const long long* __restrict__ dn) {
     __shared__ unsigned long long tpk[256];  // packed triangle lists of the cases
     __shared__ float sv[SP2_STAGE_V * 3];
+    __shared__ uint16_t sd[SP2_STAGE_V];  // staged entries to make: list position << 4 | edge (15: made)
     __shared__ int32_t sf[SP2_STAGE_F * 3];
     __shared__ uint32_t wsum[2][SP2_THREADS / 32];
     __shared__ uint16_t slv[SP2_CHUNK];  // each listed cell's first own entry (CTA-local)
@@ -685,21 +734,19 @@ __global__ void __launch_bounds__(SP2_THREADS, 5) sp_mc_emit2(SpGrid g, const in
         if (ok) slv[j] = uint16_t(lv);
         __syncthreads();  // first entries of this round's cells, for the cells that take them
         if (ok) {
-            const long long c = c0 + cl;
-            Cell8 cc;
-            const uint32_t cs = sp_case(g, vals, c, cc);
-            int x, y, z;
-            cell_xyz(g, uint32_t(ids[c]), x, y, z);
-            set_coords(g, x, y, z, cc);
-            const unsigned long long pk = tpk[cs];
             if (pc & 8u) {  // every triangle kept, every crossed edge used
-#pragma unroll
-                for (int q = 0; q < 12; ++q)
-                    if ((own >> q) & 1u) {
+                const unsigned long long pk = tpk[sp_case_of(used, cl >> 15)];
+                uint32_t k = lv;
+                for (uint32_t m = own; m; m &= m - 1, ++k) {  // made below, by full warps
+                    const int q = __ffs(m) - 1;
+                    if (k < uint32_t(SP2_STAGE_V)) {
+                        sd[k] = uint16_t(j << 4 | uint32_t(q));
+                    } else {
                         float p[3];
-                        edge_point(cc, q, g.level, p);
-                        stage_vertex(s, lv + __popc(own & ((1u << q) - 1u)), p[0], p[1], p[2]);
+                        sp_edge_point(g, ids, vals, c0 + sp_at(cl), q, p);
+                        stage_vertex(s, k, p[0], p[1], p[2]);
                     }
+                }
                 // entry of each edge: the cell's own, or its owner's (an earlier
                 // listed cell: first entry from slv, rank among the owner's own edges)
                 const uint32_t codes = pc >> 16;
@@ -746,11 +793,26 @@ __global__ void __launch_bounds__(SP2_THREADS, 5) sp_mc_emit2(SpGrid g, const in
                     stage_face(s, lf + k, v3[0], v3[1], v3[2]);
                 }
             } else {
-                sp_emit_near(g, cc, cs, used, pk, s, lv, lf);
+                const long long c = c0 + sp_at(cl);
+                Cell8 cc;
+                const uint32_t cs = sp_case(g, vals, c, cc);
+                int x, y, z;
+                cell_xyz(g, uint32_t(ids[c]), x, y, z);
+                set_coords(g, x, y, z, cc);
+                sp_emit_near(g, cc, cs, used, tpk[cs], s, lv, lf);
+                for (uint32_t k = lv; k < min(lv + __popc(used), uint32_t(SP2_STAGE_V)); ++k) sd[k] = 15;
             }
         }
         accf += all & 0xffffu;
         accv += all >> 16;
+    }
+    __syncthreads();
+    for (uint32_t k = threadIdx.x; k < min(accv, uint32_t(SP2_STAGE_V)); k += SP2_THREADS) {
+        const uint32_t d = sd[k];
+        if ((d & 15u) == 15u) continue;
+        float p[3];
+        sp_edge_point(g, ids, vals, c0 + sp_at(gl[d >> 4]), int(d & 15u), p);
+        sv[3 * k] = p[0]; sv[3 * k + 1] = p[1]; sv[3 * k + 2] = p[2];
     }
     __syncthreads();
     const uint32_t nv = 3 * min(accv, uint32_t(SP2_STAGE_V)), nf = 3 * min(accf, uint32_t(SP2_STAGE_F));

@@ -350,20 +350,14 @@ __device__ __forceinline__ bool cell_used(const Grid3& g, int cx, int cy, int cz
 
 // Crossings, grid normals and the QEF solve of each active cell in one pass,
 // when nobody asked for the intersection: the same arithmetic as dc_points
-// followed by dc_solve, without writing points and normals.  used (optional):
-// per cell, 0 when no face uses its dual vertex, else 1, or 3 when the vertex
-// lies on a face of the cell's box.  F: the arithmetic reading (g.fma), a
-// template argument so that each reading compiles without the other's code.
-// gc (optional): the grid's coordinates (x, y, z).
+// followed by dc_solve, without writing points and normals.  F: the arithmetic
+// reading (g.fma), a template argument so that each reading compiles without
+// the other's code.
 template <bool F>
 __global__ void __launch_bounds__(256) dc_cell_solve(const float* __restrict__ vals, Grid3 g, float level,
                                                      const uint32_t* __restrict__ cell_ids, long long A, float reg,
-                                                     float svd_tol, float* __restrict__ dual,
-                                                     const long long* __restrict__ dn,
-                                                     uint8_t* __restrict__ used, const float* __restrict__ gc) {
-    iso::grid_wait();
+                                                     float svd_tol, float* __restrict__ dual) {
     const long long a = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (dn) A = dn[0];
     if (a >= A) return;
     const uint32_t cid = cell_ids[a];
     const int cz = int(cid % uint32_t(g.nz - 1));
@@ -371,13 +365,11 @@ __global__ void __launch_bounds__(256) dc_cell_solve(const float* __restrict__ v
     const int cy = int(rr % uint32_t(g.ny - 1)), cx = int(rr / uint32_t(g.ny - 1));
     g.fma = F;
     CellCorners cc;
-    if (gc) load_cell_table(vals, g, gc, cx, cy, cz, cc);
-    else load_cell(vals, g, cx, cy, cz, cc);
+    load_cell(vals, g, cx, cy, cz, cc);
     uint32_t cs = 0;
 #pragma unroll
     for (int j = 0; j < 8; ++j) cs |= uint32_t(iso::below(cc.v[j], level)) << j;
     const uint32_t est = edge_status(cs);
-    const bool is_used = used && cell_used(g, cx, cy, cz, est);
     Qef Q;
     qef_init(Q, g.fma);
     uint32_t K = 0;
@@ -391,20 +383,13 @@ __global__ void __launch_bounds__(256) dc_cell_solve(const float* __restrict__ v
         ++K;
     }
     qef_finish(Q, K, reg, svd_tol);
-    bool face = false;
 #pragma unroll
-    for (int q = 0; q < 3; ++q) {
-        const float lo = cc.p[0][q], hi = cc.p[7][q];  // the cell's box
-        const float x = fminf(fmaxf(float(Q.x[q]), lo), hi);
-        face |= x == lo || x == hi;
-        dual[3 * a + q] = x;
-    }
-    if (used) used[a] = is_used ? (face ? 3 : 1) : 0;  // bit 1: on a face of its cell's box
+    for (int q = 0; q < 3; ++q)  // clipped to the cell's box
+        dual[3 * a + q] = fminf(fmaxf(float(Q.x[q]), cc.p[0][q]), cc.p[7][q]);
 }
 
 // The solve for the call's arithmetic reading.
-using SolveFn = void (*)(const float*, Grid3, float, const uint32_t*, long long, float, float, float*,
-                         const long long*, uint8_t*, const float*);
+using SolveFn = void (*)(const float*, Grid3, float, const uint32_t*, long long, float, float, float*);
 SolveFn solve_kernel(const Grid3& g) { return g.fma ? dc_cell_solve<true> : dc_cell_solve<false>; }
 
 // Lane whose inclusive prefix first exceeds j (prefixes nondecreasing, j < total).
@@ -1633,7 +1618,7 @@ int iso_dc_intersect_solve(const float* values, int nx, int ny, int nz, const fl
     iso::ProfScope ps("dc_solve", st);
     const int bt = iso::tune_get(iso::TUNE_DC_CELL_THREADS);
     solve_kernel(g)<<<blocks_for(A, bt), bt, 0, st>>>(values, g, level, reinterpret_cast<uint32_t*>(cell_ids), A, reg,
-                                                    svd_tol, dual, nullptr, nullptr, nullptr);
+                                                    svd_tol, dual);
     return cudaGetLastError() == cudaSuccess ? 0 : iso::fail_code(ISO_ERR_CUDA);
 }
 

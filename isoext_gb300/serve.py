@@ -78,11 +78,11 @@ def prims_buffer(prims: np.ndarray) -> np.ndarray:
     return out
 
 
-# Kernels of this library one request launches: marching cubes = grid evaluation
-# + mc_signs, mc_count, mc_scan, mc_emit, mc_fix; dual contouring = grid evaluation +
-# mc_signs, cell count, scan and write, solve, weld flags, scan and numbering,
-# quads.
-KERNELS_PER_REQUEST = {"mc": 6, "dc": 10}
+# Kernels of this library one request launches, at least (grids above 2^20 point
+# words take a scan more): marching cubes = grid evaluation + mc_signs, mc_count,
+# mc_emit, mc_fix; dual contouring = grid evaluation + mc_signs, cell numbering,
+# solve, face weld, vertex numbering, quads.
+KERNELS_PER_REQUEST = {"mc": 5, "dc": 7}
 
 
 # ---------------------------------------------------------------------------

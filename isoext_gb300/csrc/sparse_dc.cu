@@ -14,7 +14,7 @@
 //   sd_flags      which dual vertices are representatives of their position.  A
 //                 vertex is clipped to its cell's box, so only one on a face of
 //                 the box can equal another cell's (see dc_dense.cu).
-//   (block scan of the quads and the representatives)
+//                 Its last CTA scans the blocks' quads and representatives.
 //   sd_number     vertices in cell order.
 //   sd_faces      the quads as two triangles each.
 //
@@ -331,53 +331,104 @@ __device__ __forceinline__ void cells_holding(const Grid3& g, int axis, int c, f
     while (i1 < n - 2 && coord(g, axis, uint32_t(i1 + 1)) == v) ++i1;
 }
 
-// Smallest used active cell with the position of used cell a's vertex, which
-// lies on a face of its box.
-__device__ __noinline__ uint32_t face_rep(const Grid3& g, uint32_t a, uint32_t A, const uint32_t* __restrict__ lat,
-                                          const uint8_t* __restrict__ used, const float* __restrict__ dual) {
-    int x, y, z, x0, x1, y0, y1, z0, z1;
-    lat_xyz(g, lat[a], x, y, z);
-    cells_holding(g, 0, x, dual[3ll * a], x0, x1);
-    cells_holding(g, 1, y, dual[3ll * a + 1], y0, y1);
-    cells_holding(g, 2, z, dual[3ll * a + 2], z0, z1);
-    const uint32_t k0 = pos_bits(dual[3ll * a]), k1 = pos_bits(dual[3ll * a + 1]), k2 = pos_bits(dual[3ll * a + 2]);
-    // ids ascend with (x, y, z): the first match is the smallest; cells from a on
-    // cannot come before it
-    for (int i = x0; i <= x1; ++i)
-        for (int j = y0; j <= y1; ++j) {
-            const uint32_t key = (uint32_t(i) * uint32_t(g.ny - 1) + uint32_t(j)) * uint32_t(g.nz - 1);
-            for (uint32_t b = lower(lat, 0u, a, key + uint32_t(z0)); b < a && lat[b] <= key + uint32_t(z1); ++b)
-                if (used[b] && pos_bits(dual[3ll * b]) == k0 && pos_bits(dual[3ll * b + 1]) == k1 &&
-                    pos_bits(dual[3ll * b + 2]) == k2)
-                    return b;
-        }
-    return a;
-}
-
 // vmap[a] = NONE when no quad uses the cell, 0 when its vertex is a
-// representative, else 0x80000000 | its representative; representatives per
-// block into blk.
+// representative, else 0x80000000 | its representative, the smallest used cell
+// with its position; representatives per block into blk.  Only a vertex on a face
+// of its box can have one (face): a CTA lists those and takes each with four
+// lanes, a lane per column (x, y) of the cells around the face, edge or corner.
+// Bound by the latency of a column's binary search.  The last CTA turns blk's
+// pairs into offsets (scan): 16 us with that for 0.22 M cells, where a thread per
+// cell, searching its columns one after another, and the scan's launch took 16 + 5.
+constexpr int SD_LANES = 4;
+constexpr uint32_t SD_SCAN = 2 * SD_BLOCK;  // blocks the last CTA scans, two per thread
+
 __global__ void __launch_bounds__(SD_BLOCK) sd_flags(Grid3 g, const uint32_t* __restrict__ lat,
                                                      const uint8_t* __restrict__ used,
                                                      const uint8_t* __restrict__ face,
                                                      const float* __restrict__ dual,
                                                      const long long* __restrict__ eff, uint32_t* __restrict__ vmap,
-                                                     unsigned long long* blk) {
+                                                     unsigned long long* blk, bool scan, unsigned int* done,
+                                                     long long* tot) {
+    __shared__ uint16_t list[SD_BLOCK];
+    __shared__ uint32_t listed, merged;
+    __shared__ bool last;
     iso::grid_wait();
     const uint32_t A = uint32_t(eff[0]);
-    const uint32_t a = blockIdx.x * SD_BLOCK + threadIdx.x;
-    bool is = false;
-    if (a < A) {
-        uint32_t m = NONE;
-        if (used[a]) {
-            const uint32_t r = face[a] ? face_rep(g, a, A, lat, used, dual) : a;
-            is = r == a;
-            m = is ? 0u : 0x80000000u | r;
+    const uint32_t b0 = blockIdx.x * SD_BLOCK, a0 = b0 + threadIdx.x;
+    if (threadIdx.x == 0) { listed = 0; merged = 0; }
+    __syncthreads();
+    const bool on = a0 < A && used[a0];
+    if (a0 < A) vmap[a0] = on ? 0u : NONE;
+    if (on && face[a0]) list[atomicAdd(&listed, 1u)] = uint16_t(threadIdx.x);  // in any order
+    const uint32_t reps = uint32_t(__syncthreads_count(on));
+    const uint32_t k = threadIdx.x % SD_LANES;
+    const uint32_t lanes = ((1u << SD_LANES) - 1u) << (threadIdx.x & 31u & ~uint32_t(SD_LANES - 1));
+    for (uint32_t i = threadIdx.x / SD_LANES; i < listed; i += SD_BLOCK / SD_LANES) {
+        const uint32_t a = b0 + list[i];
+        const float p[3] = {dual[3ll * a], dual[3ll * a + 1], dual[3ll * a + 2]};
+        int x, y, z, x0, x1, y0, y1, z0, z1;
+        lat_xyz(g, lat[a], x, y, z);
+        cells_holding(g, 0, x, p[0], x0, x1);
+        cells_holding(g, 1, y, p[1], y0, y1);
+        cells_holding(g, 2, z, p[2], z0, z1);
+        const uint32_t k0 = pos_bits(p[0]), k1 = pos_bits(p[1]), k2 = pos_bits(p[2]);
+        const uint32_t cy = uint32_t(y1 - y0 + 1), columns = uint32_t(x1 - x0 + 1) * cy;
+        uint32_t first = a;  // cells from a on cannot come before it
+        for (uint32_t c = k; c < columns; c += SD_LANES) {
+            const uint32_t key = (uint32_t(x0) + c / cy) * uint32_t(g.ny - 1) + uint32_t(y0) + c % cy;
+            const uint32_t zend = key * uint32_t(g.nz - 1) + uint32_t(z1);
+            for (uint32_t b = lower(lat, 0u, first, key * uint32_t(g.nz - 1) + uint32_t(z0)); b < first && lat[b] <= zend; ++b)
+                if (used[b] && pos_bits(dual[3ll * b]) == k0 && pos_bits(dual[3ll * b + 1]) == k1 &&
+                    pos_bits(dual[3ll * b + 2]) == k2)
+                    first = b;
         }
-        vmap[a] = m;
+#pragma unroll
+        for (int d = SD_LANES / 2; d >= 1; d >>= 1) first = min(first, __shfl_xor_sync(lanes, first, d));
+        if (k == 0 && first != a) {
+            vmap[a] = 0x80000000u | first;
+            atomicAdd(&merged, 1u);
+        }
     }
-    const int t = __syncthreads_count(is);
-    if (threadIdx.x == 0) blk[2 * blockIdx.x + 1] = (unsigned long long)t;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        blk[2 * blockIdx.x + 1] = (unsigned long long)(reps - merged);
+        if (scan) {
+            __threadfence();
+            last = atomicAdd(done, 1u) == gridDim.x - 1;
+        }
+    }
+    if (!scan) return;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    __shared__ unsigned long long wa[SD_BLOCK / 32], wb[SD_BLOCK / 32];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, i0 = 2 * threadIdx.x;
+    unsigned long long va[2], vb[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const bool in = i0 + j < gridDim.x;
+        va[j] = in ? __ldcg(blk + 2 * (i0 + j)) : 0ull;
+        vb[j] = in ? __ldcg(blk + 2 * (i0 + j) + 1) : 0ull;
+    }
+    unsigned long long ia = va[0] + va[1], ib = vb[0] + vb[1];
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const unsigned long long ta = __shfl_up_sync(~0u, ia, d), tb = __shfl_up_sync(~0u, ib, d);
+        if (lane >= uint32_t(d)) { ia += ta; ib += tb; }
+    }
+    if (lane == 31) { wa[warp] = ia; wb[warp] = ib; }
+    __syncthreads();
+    unsigned long long ea = ia - va[0] - va[1], eb = ib - vb[0] - vb[1];
+#pragma unroll
+    for (uint32_t q = 0; q < SD_BLOCK / 32; ++q)
+        if (q < warp) { ea += wa[q]; eb += wb[q]; }
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        if (i0 + j < gridDim.x) { blk[2 * (i0 + j)] = ea; blk[2 * (i0 + j) + 1] = eb; }
+        ea += va[j];
+        eb += vb[j];
+    }
+    if (threadIdx.x == SD_BLOCK - 1) { tot[0] = (long long)ea; tot[1] = (long long)eb; }
 }
 
 // Exclusive position of `mine` items of each thread within the CTA.
@@ -495,8 +546,8 @@ __global__ void __launch_bounds__(SD_BLOCK) sd_faces(Grid3 g, const uint8_t* __r
 }
 
 struct SdWs {
-    // look-back states, then [0] eff, [1..2] totals, [3] ticket, [4..8] counts and [9] status for callers without
-    // their own (zeroed together)
+    // look-back states, then [0] eff, [1..2] totals, [3] ticket and blocks done, [4..8] counts and [9] status for
+    // callers without their own (zeroed together)
     unsigned long long* state;
     long long *eff, *tot, *counts;
     unsigned int* ticket;
@@ -591,9 +642,11 @@ int sd_launch(const int* ids, const float* values, long long n, int nx, int ny, 
                             w.blk);
         }
         {
-            iso::ProfScope ps("dc_weld", st, 3);
-            iso::launch_pdl(sd_flags, nblk, unsigned(SD_BLOCK), st, g, lat, used, face, dual, eff, w.vmap, w.blk);
-            iso_block_scan_launch(w.blk, w.nblk, w.tot, st);
+            const bool scan = nblk <= SD_SCAN;
+            iso::ProfScope ps("dc_weld", st, scan ? 2 : 3);
+            iso::launch_pdl(sd_flags, nblk, unsigned(SD_BLOCK), st, g, lat, used, face, dual, eff, w.vmap, w.blk, scan,
+                            w.ticket + 1, w.tot);
+            if (!scan) iso_block_scan_launch(w.blk, w.nblk, w.tot, st);
             iso::launch_pdl(sd_number, nblk, unsigned(SD_BLOCK), st, dual, eff, blk, tot, face_capacity, w.vmap,
                             vertices, counts, status);
         }

@@ -100,3 +100,16 @@ def test_retries_reach_the_sizes():
 def test_no_active_cell_gives_none():
     g = _grid(sphere((12, 12, 12), 0.5), np.arange(30))
     assert iso.dual_contouring(g, level=50.0) == (None, None)
+
+
+@pytest.mark.parametrize("active", [511, 512, 513, 1023 * 512 + 1, 1024 * 512, 1024 * 512 + 1, 700_000])
+def test_block_counts(active):
+    """One block of active cells and up to the 1024 that the weld's last CTA scans
+    by itself, and more (a launch of its own): noise, where every cell is active."""
+    n = 100
+    vals = noise((n, n, n), seed=active, zero_frac=0.02)
+    corners = [vals[i:n - 1 + i, j:n - 1 + j, k:n - 1 + k] < 0 for i in (0, 1) for j in (0, 1) for k in (0, 1)]
+    neg = sum(c.astype(np.int32) for c in corners).ravel()
+    ids = np.flatnonzero((neg > 0) & (neg < 8))[:active]
+    assert len(ids) == active
+    assert _both(_grid(vals, ids)) > 0

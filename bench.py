@@ -167,6 +167,7 @@ def kernel_bytes(kind: str, n: int, nv: int, nf: int) -> dict:
         "mc_count": 4 * words + 4 * words,         # bitmap once, per-word entries once
         "mc_scan": 32 * segs,                      # segment sums read, offsets written
         "mc_emit": 16 * nv + 12 * nv + 8 * nf + 12 * nf,  # entries and endpoint values; vertices, faces
+        "mc_fix": 32,                              # the counters, when no vertices coincide
     }
 
 

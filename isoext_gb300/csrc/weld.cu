@@ -12,8 +12,9 @@
 //                 366 us against 174 for the band of a 1024^3 grid).
 //   weld_number   per tile of 1024 entries: each entry's first entry (one read
 //                 of its slot; hashing the position, reading the slot and
-//                 comparing the positions again took 217 us there, this 119 and
-//                 13 more in the insert), the tile's number of first entries,
+//                 comparing the positions again took 217 us there, this 119;
+//                 the insert, which keeps the slots, takes 174 either way at eight
+//                 CTAs per SM, 187 at six), the tile's number of first entries,
 //                 the exclusive prefix over tiles by decoupled look-back, and
 //                 the first entries' new numbers and positions written out.
 //   weld_remap    triangle indices -> new numbers.
@@ -71,7 +72,7 @@ __device__ __noinline__ uint32_t insert_probe(const float* __restrict__ pts, uin
 
 // slot <- each entry's slot, so that the numbering reads the first
 // entry with its position from there instead of hashing and comparing again.
-__global__ void __launch_bounds__(WELD_THREADS) weld_insert(const float* __restrict__ pts, long long A,
+__global__ void __launch_bounds__(WELD_THREADS, 8) weld_insert(const float* __restrict__ pts, long long A,
                                                             uint32_t* table, uint32_t mask,
                                                             uint32_t* __restrict__ slot, int* status,
                                                             const long long* __restrict__ dn) {

@@ -1591,11 +1591,11 @@ int iso_dc_intersect(const float* values, int nx, int ny, int nz, const float* a
         values, w.S, g, level, w.cwords, w.blkC, w.actm, w.offA, points, normals,
         reinterpret_cast<uint32_t*>(cell_ids), reinterpret_cast<uint32_t*>(cell_offsets), A, K, nullptr);
     if (A == 0 && cell_offsets) cudaMemsetAsync(cell_offsets, 0, 4, st);
-    if (A > 0 && points)
-        dc_points<<<blocks_for(A, iso::tune_get(iso::TUNE_DC_CELL_THREADS)), iso::tune_get(iso::TUNE_DC_CELL_THREADS), 0,
-                    st>>>(values, g, level, reinterpret_cast<uint32_t*>(cell_ids),
-                                                      reinterpret_cast<uint32_t*>(cell_offsets), A, points,
-                                                      normals);
+    if (A > 0 && points) {
+        const int bt = iso::tune_get(iso::TUNE_DC_CELL_THREADS);  // read once: another thread may set it meanwhile
+        dc_points<<<blocks_for(A, bt), bt, 0, st>>>(values, g, level, reinterpret_cast<uint32_t*>(cell_ids),
+                                                    reinterpret_cast<uint32_t*>(cell_offsets), A, points, normals);
+    }
     return cudaGetLastError() == cudaSuccess ? 0 : iso::fail_code(ISO_ERR_CUDA);
 }
 

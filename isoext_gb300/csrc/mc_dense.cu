@@ -1328,9 +1328,9 @@ int launch_emit(const McParams& p, const McGrid& g, const McWs& w, cudaStream_t 
     return 0;
 }
 
-int launch_count_emit(const McParams& p, const McGrid& g, const McWs& w, cudaStream_t st) {
+// ct: the threads of a count CTA that g.lgseg was made from.
+int launch_count_emit(const McParams& p, const McGrid& g, const McWs& w, int ct, cudaStream_t st) {
     const int sms = sm_count();
-    const int ct = count_threads();
     const uint32_t nseg = uint32_t((g.PW + (1ll << g.lgseg) - 1) >> g.lgseg);
     {
         iso::ProfScope ps("mc_count", st);
@@ -1434,7 +1434,8 @@ int mc_launch(const McParams& params, void* ws, size_t ws_bytes, cudaStream_t st
     g.tau = snap_tau(p);
     g.fma = iso::arith_fma();
     const bool fine = g.PW <= FINE_PW;
-    g.lgseg = (count_threads() == 128 ? 7 : 8) + (fine ? 0 : 2);
+    const int ct = count_threads();  // read once: another thread may set it while this one launches
+    g.lgseg = (ct == 128 ? 7 : 8) + (fine ? 0 : 2);
     if (fine) w.blk = w.blk2;
     g.gc = w.gc;
     if (g.PW > 0xffffffffll) return iso::fail_code(ISO_ERR_ARG);
@@ -1443,7 +1444,7 @@ int mc_launch(const McParams& params, void* ws, size_t ws_bytes, cudaStream_t st
         mc_signs_launch(p.vals, p.nx, p.ny, p.nz, p.level, w.S, st, w.ctr, (long long)(zeroed_bytes(w.nBlk) / 8));
         if (cudaGetLastError() != cudaSuccess) return iso::fail_code(ISO_ERR_CUDA);
     }
-    const int rc = launch_count_emit(p, g, w, st);
+    const int rc = launch_count_emit(p, g, w, ct, st);
     if (rc) return rc;
     return 0;
 }

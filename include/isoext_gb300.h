@@ -122,7 +122,10 @@ int iso_mc_dense(const float *values, int nx, int ny, int nz, const float *aabb_
                  long long vertex_capacity, int *faces, long long face_capacity, void *workspace,
                  size_t workspace_bytes, long long *counts, int *status, void *stream);
 /* iso_mc_dense and a wait for the stream: sizes (HOST long long[3]) <- (V, F, device
- * status).  The device counts and status are kept in the workspace. */
+ * status).  The device counts and status are kept in the workspace.  This and the
+ * other iso_*_sync calls take the sizes through a small record of pinned memory of
+ * the CUDA context current on the calling thread, from a pool that all threads
+ * share; a context made after a cudaDeviceReset gets records of its own. */
 int iso_mc_dense_sync(const float *values, int nx, int ny, int nz, const float *aabb_min, const float *aabb_max,
                       float level, int method, float *vertices, long long vertex_capacity, int *faces,
                       long long face_capacity, void *workspace, size_t workspace_bytes, long long *sizes,

@@ -11,6 +11,7 @@
 
 #include "common.cuh"
 #include "mc_dense.cuh"
+#include "size_pool.h"
 
 namespace {
 thread_local std::string g_err;
@@ -44,29 +45,57 @@ int fail_code(int code) {
 }
 
 namespace {
-struct Pinned {
-    long long* p = nullptr;
-    ~Pinned() {
-        if (p) cudaFreeHost(p);
-    }
-};
-}  // namespace
-
-long long* host_sizes() {
-    thread_local Pinned t;
-    if (!t.p && cudaHostAlloc(reinterpret_cast<void**>(&t.p), 16 * sizeof(long long), cudaHostAllocPortable) != cudaSuccess)
-        t.p = nullptr;
-    if (t.p) std::memset(t.p, 0, 16 * sizeof(long long));
-    return t.p;
+// Never destroyed: threads may still be in a call when the process's statics go.
+SizePool& size_pool() {
+    static SizePool* p = new SizePool;
+    return *p;
 }
 
-int wait_sizes(const long long* pinned, int n, long long* out, cudaStream_t st) {
-    const cudaError_t e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) {
-        g_err = std::string("CUDA error: ") + cudaGetErrorString(e);
-        return ISO_ERR_CUDA;
+// The id of the context current on this thread, which the runtime makes when there
+// is none (or it was reset).
+bool context_id(unsigned long long* id) {
+    using GetId = int (*)(void*, unsigned long long*);  // cuCtxGetId
+    static const GetId get = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult r = cudaDriverEntryPointSymbolNotFound;
+        const cudaError_t e = cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &r);
+        return e == cudaSuccess && r == cudaDriverEntryPointSuccess ? reinterpret_cast<GetId>(f) : nullptr;
+    }();
+    if (!get) return false;
+    if (get(nullptr, id) == 0) return true;
+    int dev = 0;
+    return cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess && get(nullptr, id) == 0;
+}
+
+// What failed, as this thread's message; the runtime's last error is cleared, so
+// that the next call does not take it for its own.
+int sizes_failed(const char* what, cudaError_t e) {
+    g_err = std::string(what) + ": " + cudaGetErrorString(e);
+    cudaGetLastError();
+    return ISO_ERR_CUDA;
+}
+}  // namespace
+
+HostSizes::HostSizes() {
+    cudaError_t e = cudaErrorDeviceUninitialized;
+    if (context_id(&ctx_)) {
+        p_ = size_pool().lease(ctx_, [&](size_t bytes) -> void* {
+            void* slab = nullptr;
+            e = cudaHostAlloc(&slab, bytes, cudaHostAllocDefault);
+            return e == cudaSuccess ? slab : nullptr;
+        });
     }
-    for (int i = 0; i < n; ++i) out[i] = const_cast<const volatile long long*>(pinned)[i];
+    if (!p_) sizes_failed("no pinned memory for the sizes", e);
+}
+
+HostSizes::~HostSizes() {
+    if (p_) size_pool().release(ctx_, p_);
+}
+
+int HostSizes::wait(int n, long long* out, cudaStream_t st) {
+    const cudaError_t e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return sizes_failed("CUDA error", e);
+    for (int i = 0; i < n; ++i) out[i] = const_cast<const volatile long long*>(p_)[i];
     return ISO_OK;
 }
 
@@ -232,12 +261,12 @@ int iso_mc_dense_sync(const float* values, int nx, int ny, int nz, const float* 
                       long long face_capacity, void* workspace, size_t workspace_bytes, long long* sizes,
                       void* stream) {
     if (!sizes) return fail(ISO_ERR_ARG, "sizes is null");
-    long long* host = iso::host_sizes();
-    if (!host) return fail(ISO_ERR_CUDA, "cudaHostAlloc failed");
+    iso::HostSizes host;
+    if (!host.words()) return ISO_ERR_CUDA;
     const int rc = mc_dense_impl(values, nx, ny, nz, aabb_min, aabb_max, level, method, vertices, vertex_capacity,
                                  faces, face_capacity, workspace, workspace_bytes, nullptr, nullptr, nullptr, stream,
-                                 host);
-    return rc ? rc : iso::wait_sizes(host, 3, sizes, reinterpret_cast<cudaStream_t>(stream));
+                                 host.words());
+    return rc ? rc : host.wait(3, sizes, reinterpret_cast<cudaStream_t>(stream));
 }
 
 int iso_mc_dense_edges(const float* values, int nx, int ny, int nz, const float* aabb_min,

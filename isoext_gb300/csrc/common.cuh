@@ -201,11 +201,23 @@ int tune_get(int key);
 // true = the reference's CUDA build (fused), false = its host build.
 bool arith_fma();
 
-// Sizes that a call's last kernel writes for the host (iso_*_sync): 16 words of
-// pinned memory per host thread, cleared; nullptr when there is none to be had.
-// wait_sizes waits for the stream and copies the first n words to out.
-long long* host_sizes();
-int wait_sizes(const long long* pinned, int n, long long* out, cudaStream_t st);
+// Sizes that a call's last kernel writes for the host (iso_*_sync): words() is a
+// cleared record of 16 words of pinned memory, this call's own until the object
+// goes (size_pool.h); nullptr, with the message set, when there is none to be had.
+// wait() waits for the stream and copies the first n words to out.
+class HostSizes {
+public:
+    HostSizes();
+    ~HostSizes();
+    HostSizes(const HostSizes&) = delete;
+    HostSizes& operator=(const HostSizes&) = delete;
+    long long* words() const { return p_; }
+    int wait(int n, long long* out, cudaStream_t st);
+
+private:
+    long long* p_ = nullptr;
+    unsigned long long ctx_ = 0;
+};
 
 // An entry point's failure: sets the message iso_last_error returns on this
 // thread to the plain meaning of `code` (with CUDA's error text for

@@ -1839,12 +1839,12 @@ int iso_dc_dense_sync(const float* values, int nx, int ny, int nz, const float* 
                       long long face_capacity, void* workspace, size_t workspace_bytes, long long* sizes,
                       void* stream) {
     if (!sizes || vertex_capacity < 1) return iso::fail_code(ISO_ERR_ARG);
-    long long* host = iso::host_sizes();
-    if (!host) return iso::fail_code(ISO_ERR_CUDA);
+    iso::HostSizes host;
+    if (!host.words()) return ISO_ERR_CUDA;
     const int rc = dc_dense_impl(values, nx, ny, nz, aabb_min, aabb_max, level, reg, svd_tol, vertices,
                                  vertex_capacity, faces, face_capacity, workspace, workspace_bytes, nullptr, nullptr,
-                                 nullptr, nullptr, nullptr, host, nullptr, stream);
-    return rc ? rc : iso::wait_sizes(host, 6, sizes, reinterpret_cast<cudaStream_t>(stream));
+                                 nullptr, nullptr, nullptr, host.words(), nullptr, stream);
+    return rc ? rc : host.wait(6, sizes, reinterpret_cast<cudaStream_t>(stream));
 }
 
 int iso_dc_dense_its_sync(const float* values, int nx, int ny, int nz, const float* aabb_min, const float* aabb_max,
@@ -1853,14 +1853,14 @@ int iso_dc_dense_its_sync(const float* values, int nx, int ny, int nz, const flo
                           long long face_capacity, void* workspace, size_t workspace_bytes, long long* sizes,
                           void* stream) {
     if (!sizes || A < 1 || !points || !cell_ids || !cell_offsets) return iso::fail_code(ISO_ERR_ARG);
-    long long* host = iso::host_sizes();
-    if (!host) return iso::fail_code(ISO_ERR_CUDA);
+    iso::HostSizes host;
+    if (!host.words()) return ISO_ERR_CUDA;
     const Given in{points, normals, reinterpret_cast<const uint32_t*>(cell_ids),
                    reinterpret_cast<const uint32_t*>(cell_offsets), A, nullptr};
     const int rc = dc_dense_impl(values, nx, ny, nz, aabb_min, aabb_max, level, reg, svd_tol, vertices, A, faces,
                                  face_capacity, workspace, workspace_bytes, nullptr, nullptr, nullptr, nullptr, nullptr,
-                                 host, &in, stream);
-    return rc ? rc : iso::wait_sizes(host, 6, sizes, reinterpret_cast<cudaStream_t>(stream));
+                                 host.words(), &in, stream);
+    return rc ? rc : host.wait(6, sizes, reinterpret_cast<cudaStream_t>(stream));
 }
 
 int iso_dc_intersection_sync(const float* values, int nx, int ny, int nz, const float* aabb_min, const float* aabb_max,
@@ -1872,8 +1872,8 @@ int iso_dc_intersection_sync(const float* values, int nx, int ny, int nz, const 
         (long long)nx * ny * nz > 0x7fffffffll || !values || !points || !cell_ids || !cell_offsets)
         return iso::fail_code(ISO_ERR_ARG);
     if (workspace_bytes < iso_dc_dense_workspace_size(nx, ny, nz, cell_capacity, 0)) return iso::fail_code(ISO_ERR_WORKSPACE);
-    long long* host = iso::host_sizes();
-    if (!host) return iso::fail_code(ISO_ERR_CUDA);
+    iso::HostSizes host;
+    if (!host.words()) return ISO_ERR_CUDA;
     const DcDenseWs w = carve_dense(workspace, nx, ny, nz, cell_capacity);
     const Grid3 g = make_grid(nx, ny, nz, aabb_min, aabb_max);
     long long *eff = w.misc + 4, *counts = w.misc + 8;
@@ -1895,10 +1895,11 @@ int iso_dc_intersection_sync(const float* values, int nx, int ny, int nz, const 
         const int bt = iso::tune_get(iso::TUNE_DC_CELL_THREADS);
         iso::launch_pdl(dc_entry_points, blocks_for(cell_capacity, bt), unsigned(bt), st, values, g, level, ix,
                         static_cast<const long long*>(eff), static_cast<const float*>(w.gc), cells, off, points,
-                        normals, static_cast<const long long*>(counts), static_cast<const int*>(status), host);
+                        normals, static_cast<const long long*>(counts), static_cast<const int*>(status),
+                        host.words());
     }
     if (cudaGetLastError() != cudaSuccess) return iso::fail_code(ISO_ERR_CUDA);
-    return iso::wait_sizes(host, 6, sizes, st);
+    return host.wait(6, sizes, st);
 }
 
 int iso_dc_dense(const float* values, int nx, int ny, int nz, const float* aabb_min, const float* aabb_max,

@@ -1370,11 +1370,11 @@ int iso_sparse_mc_sync(const int* ids, const float* vals, long long n, int nx, i
                        int* faces, long long face_capacity, void* workspace, size_t workspace_bytes,
                        long long* sizes, void* stream) {
     if (!sizes) return iso::fail_code(ISO_ERR_ARG);
-    long long* host = iso::host_sizes();
-    if (!host) return iso::fail_code(ISO_ERR_CUDA);
+    iso::HostSizes host;
+    if (!host.words()) return ISO_ERR_CUDA;
     const int rc = sp_mc_launch(ids, vals, n, nx, ny, nz, amin, amax, level, method, vertices, vertex_capacity, faces,
-                                face_capacity, workspace, workspace_bytes, nullptr, nullptr, host, stream);
-    return rc ? rc : iso::wait_sizes(host, 4, sizes, reinterpret_cast<cudaStream_t>(stream));
+                                face_capacity, workspace, workspace_bytes, nullptr, nullptr, host.words(), stream);
+    return rc ? rc : host.wait(4, sizes, reinterpret_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

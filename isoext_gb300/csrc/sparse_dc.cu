@@ -681,12 +681,12 @@ int iso_sparse_dc_sync(const int* ids, const float* values, long long n, int nx,
                        float* vertices, long long vertex_capacity, int* faces, long long face_capacity,
                        void* workspace, size_t workspace_bytes, long long* sizes, void* stream) {
     if (!sizes || vertex_capacity < 1) return iso::fail_code(ISO_ERR_ARG);
-    long long* host = iso::host_sizes();
-    if (!host) return iso::fail_code(ISO_ERR_CUDA);
+    iso::HostSizes host;
+    if (!host.words()) return ISO_ERR_CUDA;
     const int rc = sd_launch(ids, values, n, nx, ny, nz, aabb_min, aabb_max, level, reg, svd_tol, vertices,
-                             vertex_capacity, faces, face_capacity, workspace, workspace_bytes, nullptr, nullptr, host,
-                             stream);
-    return rc ? rc : iso::wait_sizes(host, 6, sizes, reinterpret_cast<cudaStream_t>(stream));
+                             vertex_capacity, faces, face_capacity, workspace, workspace_bytes, nullptr, nullptr,
+                             host.words(), stream);
+    return rc ? rc : host.wait(6, sizes, reinterpret_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

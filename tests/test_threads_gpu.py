@@ -46,3 +46,36 @@ def test_count_threads_set_during_calls(vals):
         done.set()
         t.join()
         tune.set("mc.count_threads", old)
+
+
+# Every call that waits for its sizes, from eight threads with a stream each, new
+# threads every round.
+def test_threads_and_streams():
+    g = _grid(sphere((61, 70, 83), 0.6))
+    h = _grid(noise((20, 21, 33), 5, 0.1))
+    sp = iso.SparseGrid([48, 48, 48])
+    sp.populate(lambda p: p.norm(dim=-1) - 0.7)
+    its = iso.get_intersection(h, 0.0, True)
+    calls = [lambda: iso.marching_cubes(g), lambda: iso.dual_contouring(h), lambda: iso.marching_cubes(sp),
+             lambda: iso.dual_contouring(sp), lambda: iso.dual_contouring(h, 0.0, its),
+             lambda: (iso.get_intersection(g).get_points(),), lambda: iso.marching_cubes(h, method="lorensen"),
+             lambda: iso.dual_contouring(g)]
+    want = [[t.clone() for t in c()] for c in calls]
+    torch.cuda.synchronize()
+    bad = []
+
+    def work(k):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for i in range(24):
+                j = (k + i) % len(calls)
+                got = calls[j]()
+                if not all(torch.equal(a, b) for a, b in zip(got, want[j])):
+                    bad.append((k, j))
+
+    for _ in range(3):
+        ts = [threading.Thread(target=work, args=(k,)) for k in range(8)]
+        for t in ts:
+            t.start()
+        for t in ts:
+            t.join()
+    assert not bad, bad

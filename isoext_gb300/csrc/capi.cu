@@ -92,11 +92,13 @@ HostSizes::~HostSizes() {
     if (p_) size_pool().release(ctx_, p_);
 }
 
-int HostSizes::wait(int n, long long* out, cudaStream_t st) {
-    const cudaError_t e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return sizes_failed("CUDA error", e);
-    for (int i = 0; i < n; ++i) out[i] = const_cast<const volatile long long*>(p_)[i];
-    return ISO_OK;
+int HostSizes::wait(int rc, int n, long long* out, cudaStream_t st) {
+    return finish_sizes(rc, ISO_ERR_CUDA, p_, n, out, [&] {
+        const cudaError_t e = cudaStreamSynchronize(st);
+        if (e == cudaSuccess) return true;
+        if (!rc) sizes_failed("CUDA error", e);  // else the launch's message stays
+        return false;
+    });
 }
 
 // Tunables: sign-pass CTAs per SM (MC and DC sign bitmaps), threads per block of
@@ -266,7 +268,7 @@ int iso_mc_dense_sync(const float* values, int nx, int ny, int nz, const float* 
     const int rc = mc_dense_impl(values, nx, ny, nz, aabb_min, aabb_max, level, method, vertices, vertex_capacity,
                                  faces, face_capacity, workspace, workspace_bytes, nullptr, nullptr, nullptr, stream,
                                  host.words());
-    return rc ? rc : host.wait(3, sizes, reinterpret_cast<cudaStream_t>(stream));
+    return host.wait(rc, 3, sizes, reinterpret_cast<cudaStream_t>(stream));
 }
 
 int iso_mc_dense_edges(const float* values, int nx, int ny, int nz, const float* aabb_min,

@@ -204,7 +204,9 @@ bool arith_fma();
 // Sizes that a call's last kernel writes for the host (iso_*_sync): words() is a
 // cleared record of 16 words of pinned memory, this call's own until the object
 // goes (size_pool.h); nullptr, with the message set, when there is none to be had.
-// wait() waits for the stream and copies the first n words to out.
+// wait(rc) ends the call: the launches' result rc when they failed (their kernels
+// waited for, see finish_sizes), else it waits for the stream and copies the first
+// n words to out.
 class HostSizes {
 public:
     HostSizes();
@@ -212,7 +214,7 @@ public:
     HostSizes(const HostSizes&) = delete;
     HostSizes& operator=(const HostSizes&) = delete;
     long long* words() const { return p_; }
-    int wait(int n, long long* out, cudaStream_t st);
+    int wait(int rc, int n, long long* out, cudaStream_t st);
 
 private:
     long long* p_ = nullptr;

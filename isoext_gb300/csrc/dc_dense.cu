@@ -1844,7 +1844,7 @@ int iso_dc_dense_sync(const float* values, int nx, int ny, int nz, const float* 
     const int rc = dc_dense_impl(values, nx, ny, nz, aabb_min, aabb_max, level, reg, svd_tol, vertices,
                                  vertex_capacity, faces, face_capacity, workspace, workspace_bytes, nullptr, nullptr,
                                  nullptr, nullptr, nullptr, host.words(), nullptr, stream);
-    return rc ? rc : host.wait(6, sizes, reinterpret_cast<cudaStream_t>(stream));
+    return host.wait(rc, 6, sizes, reinterpret_cast<cudaStream_t>(stream));
 }
 
 int iso_dc_dense_its_sync(const float* values, int nx, int ny, int nz, const float* aabb_min, const float* aabb_max,
@@ -1860,7 +1860,7 @@ int iso_dc_dense_its_sync(const float* values, int nx, int ny, int nz, const flo
     const int rc = dc_dense_impl(values, nx, ny, nz, aabb_min, aabb_max, level, reg, svd_tol, vertices, A, faces,
                                  face_capacity, workspace, workspace_bytes, nullptr, nullptr, nullptr, nullptr, nullptr,
                                  host.words(), &in, stream);
-    return rc ? rc : host.wait(6, sizes, reinterpret_cast<cudaStream_t>(stream));
+    return host.wait(rc, 6, sizes, reinterpret_cast<cudaStream_t>(stream));
 }
 
 int iso_dc_intersection_sync(const float* values, int nx, int ny, int nz, const float* aabb_min, const float* aabb_max,
@@ -1898,8 +1898,8 @@ int iso_dc_intersection_sync(const float* values, int nx, int ny, int nz, const 
                         normals, static_cast<const long long*>(counts), static_cast<const int*>(status),
                         host.words());
     }
-    if (cudaGetLastError() != cudaSuccess) return iso::fail_code(ISO_ERR_CUDA);
-    return host.wait(6, sizes, st);
+    const int rc = cudaGetLastError() == cudaSuccess ? 0 : iso::fail_code(ISO_ERR_CUDA);
+    return host.wait(rc, 6, sizes, st);
 }
 
 int iso_dc_dense(const float* values, int nx, int ny, int nz, const float* aabb_min, const float* aabb_max,

@@ -82,4 +82,20 @@ private:
     std::vector<Context> contexts_;
 };
 
+// Ends a waiting call whose launches returned rc: failed launches (rc ==
+// launch_failed) can have kernels before them still queued, on the caller's
+// buffers and on the record, so those are waited for before anyone uses either
+// again; other failures launched nothing.  sync() -> whether the wait succeeded;
+// the first n words are then copied to out.
+template <typename Sync>
+int finish_sizes(int rc, int launch_failed, const long long* words, int n, long long* out, Sync sync) {
+    if (rc) {
+        if (rc == launch_failed) sync();
+        return rc;
+    }
+    if (!sync()) return launch_failed;
+    for (int i = 0; i < n; ++i) out[i] = static_cast<const volatile long long*>(words)[i];
+    return 0;
+}
+
 }  // namespace iso

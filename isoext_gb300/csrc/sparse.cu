@@ -1374,7 +1374,7 @@ int iso_sparse_mc_sync(const int* ids, const float* vals, long long n, int nx, i
     if (!host.words()) return ISO_ERR_CUDA;
     const int rc = sp_mc_launch(ids, vals, n, nx, ny, nz, amin, amax, level, method, vertices, vertex_capacity, faces,
                                 face_capacity, workspace, workspace_bytes, nullptr, nullptr, host.words(), stream);
-    return rc ? rc : host.wait(4, sizes, reinterpret_cast<cudaStream_t>(stream));
+    return host.wait(rc, 4, sizes, reinterpret_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

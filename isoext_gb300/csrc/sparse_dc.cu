@@ -686,7 +686,7 @@ int iso_sparse_dc_sync(const int* ids, const float* values, long long n, int nx,
     const int rc = sd_launch(ids, values, n, nx, ny, nz, aabb_min, aabb_max, level, reg, svd_tol, vertices,
                              vertex_capacity, faces, face_capacity, workspace, workspace_bytes, nullptr, nullptr,
                              host.words(), stream);
-    return rc ? rc : host.wait(6, sizes, reinterpret_cast<cudaStream_t>(stream));
+    return host.wait(rc, 6, sizes, reinterpret_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

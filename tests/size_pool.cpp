@@ -78,6 +78,18 @@ int main() {
         for (std::thread& t : ts) t.join();
         CHECK(slabs <= 8);  // a slab by each that found the pool empty at the start
     }
+    {  // the end of a call: what is waited for, and what it returns
+        long long words[4] = {5, 6, 7, 8}, out[4] = {};
+        int waits = 0;
+        bool good = true;
+        const auto sync = [&] { ++waits; return good; };
+        CHECK(iso::finish_sizes(0, 2, words, 3, out, sync) == 0 && waits == 1 && out[2] == 7 && out[3] == 0);
+        out[0] = 0;
+        CHECK(iso::finish_sizes(1, 2, words, 3, out, sync) == 1 && waits == 1);  // refused: nothing was launched
+        CHECK(iso::finish_sizes(2, 2, words, 3, out, sync) == 2 && waits == 2);  // a launch failed: the rest waited for
+        good = false;
+        CHECK(iso::finish_sizes(0, 2, words, 3, out, sync) == 2 && waits == 3 && out[0] == 0);
+    }
     std::printf("ok\n");
     return 0;
 }

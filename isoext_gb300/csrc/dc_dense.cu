@@ -843,8 +843,7 @@ __device__ void scan_cells(uint4* seg, uint32_t nseg, long long capA, long long 
     }
     if (tid == 0) {
         const long long A = (long long)carry[0], Q = (long long)carry[1], K = (long long)carry[2];
-        const bool ok = A <= capA && Q <= capQ && K <= capK && A < 0x7fffffffll && K < 0x7fffffffll &&
-                        6 * Q < 0x7fffffffll;
+        const bool ok = A <= capA && Q <= capQ && K <= capK && A < 0x7fffffffll && Q < 0x7fffffffll && K < 0x7fffffffll;
         if (!ok) atomicCAS(status, 0, int(ISO_ERR_OVERFLOW));
         eff[0] = ok ? A : 0;
         eff[1] = ok ? K : 0;
@@ -1925,7 +1924,9 @@ static int dc_dense_impl(const float* values, int nx, int ny, int nz, const floa
     if (nx < 2 || ny < 2 || nz < 2)
         return cudaMemsetAsync(counts, 0, 5 * sizeof(long long), st) == cudaSuccess ? 0 : iso::fail_code(ISO_ERR_CUDA);
     if (!values || (vertex_capacity && !vertices) || (face_capacity && !faces)) return iso::fail_code(ISO_ERR_ARG);
-    const long long capA = vertex_capacity, capQ = face_capacity / 2;
+    // without a caller's intersection 6 Q face indices stay below 2^31
+    const long long capA = vertex_capacity,
+                    capQ = given ? face_capacity / 2 : std::min(face_capacity / 2, 0x7ffffffell / 6);
     if (workspace_bytes < iso_dc_dense_workspace_size(nx, ny, nz, vertex_capacity, face_capacity))
         return iso::fail_code(ISO_ERR_WORKSPACE);
     const DcDenseWs w = carve_dense(workspace, nx, ny, nz, capA);

@@ -463,7 +463,7 @@ __global__ void __launch_bounds__(SD_BLOCK) sd_number(const float* __restrict__ 
     const uint32_t e = block_before(is ? 1u : 0u, ws);
     if (blockIdx.x == 0 && threadIdx.x == 0 && A) {
         const long long Q = tot[0];
-        if (2 * Q > capF || 6 * Q >= 0x7fffffffll) atomicCAS(status, 0, int(ISO_ERR_OVERFLOW));
+        if (2 * Q > capF) atomicCAS(status, 0, int(ISO_ERR_OVERFLOW));
         counts[0] = tot[1];
         counts[1] = 2 * Q;
         counts[4] = Q;

@@ -32,6 +32,7 @@
 #include "dc_common.cuh"
 #include "lookback.cuh"
 #include "profile.cuh"
+#include "weld_table.cuh"
 
 // (dc_dense.cu) exclusive scan of pairs of block sums in place, totals -> totals[0..1]
 void iso_block_scan_launch(unsigned long long* blk, long long nblk, long long* totals, cudaStream_t st);
@@ -42,8 +43,6 @@ constexpr int SD_THREADS = 256;
 constexpr int SD_ROUNDS = 8;                        // cells per thread of the first pass
 constexpr int SD_TILE = SD_THREADS * SD_ROUNDS;     // cells per tile
 constexpr int SD_BLOCK = 512;                       // active cells per CTA (and per block sum)
-
-using iso::pos_bits;
 
 __device__ __forceinline__ uint32_t case8(const float4& a, const float4& b, float level) {
     const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
@@ -321,25 +320,25 @@ __global__ void __launch_bounds__(SD_BLOCK) sd_quads(Grid3 g, const uint32_t* __
     }
 }
 
-// Cells along one axis whose closed interval holds v, around cell c (wider than
-// c +- 1 only where grid coordinates repeat).
+// Cells along one axis whose closed interval holds v, in cell c's: c alone, or c
+// and the cell on the side where v is the common coordinate (neighbouring
+// coordinates are distinct here).
 __device__ __forceinline__ void cells_holding(const Grid3& g, int axis, int c, float v, int& i0, int& i1) {
     const int n = axis == 0 ? g.nx : (axis == 1 ? g.ny : g.nz);
-    i0 = c;
-    i1 = c;
-    while (i0 > 0 && coord(g, axis, uint32_t(i0)) == v) --i0;
-    while (i1 < n - 2 && coord(g, axis, uint32_t(i1 + 1)) == v) ++i1;
+    i0 = c - (c > 0 && coord(g, axis, uint32_t(c)) == v ? 1 : 0);
+    i1 = c + (c < n - 2 && coord(g, axis, uint32_t(c + 1)) == v ? 1 : 0);
 }
 
 // vmap[a] = NONE when no quad uses the cell, 0 when its vertex is a
 // representative, else 0x80000000 | its representative, the smallest used cell
 // with its position; representatives per block into blk.  Only a vertex on a face
 // of its box can have one (face): a CTA lists those and takes each with four
-// lanes, a lane per column (x, y) of the cells around the face, edge or corner.
+// lanes, a lane per column (x, y) of the cells around the face, edge or corner;
+// where coordinates may repeat it reads their table instead (weld_table.cuh).
 // Bound by the latency of a column's binary search.  The last CTA turns blk's
 // pairs into offsets (scan): 16 us with that for 0.22 M cells, where a thread per
 // cell, searching its columns one after another, and the scan's launch took 16 + 5.
-constexpr int SD_LANES = 4;
+constexpr int SD_LANES = 4;                 // at most four columns meet at an edge
 constexpr uint32_t SD_SCAN = 2 * SD_BLOCK;  // blocks the last CTA scans, two per thread
 
 __global__ void __launch_bounds__(SD_BLOCK) sd_flags(Grid3 g, const uint32_t* __restrict__ lat,
@@ -348,7 +347,7 @@ __global__ void __launch_bounds__(SD_BLOCK) sd_flags(Grid3 g, const uint32_t* __
                                                      const float* __restrict__ dual,
                                                      const long long* __restrict__ eff, uint32_t* __restrict__ vmap,
                                                      unsigned long long* blk, bool scan, unsigned int* done,
-                                                     long long* tot) {
+                                                     long long* tot, const WeldTable table) {
     __shared__ uint16_t list[SD_BLOCK];
     __shared__ uint32_t listed, merged;
     __shared__ bool last;
@@ -365,22 +364,23 @@ __global__ void __launch_bounds__(SD_BLOCK) sd_flags(Grid3 g, const uint32_t* __
     const uint32_t lanes = ((1u << SD_LANES) - 1u) << (threadIdx.x & 31u & ~uint32_t(SD_LANES - 1));
     for (uint32_t i = threadIdx.x / SD_LANES; i < listed; i += SD_BLOCK / SD_LANES) {
         const uint32_t a = b0 + list[i];
-        const float p[3] = {dual[3ll * a], dual[3ll * a + 1], dual[3ll * a + 2]};
-        int x, y, z, x0, x1, y0, y1, z0, z1;
-        lat_xyz(g, lat[a], x, y, z);
-        cells_holding(g, 0, x, p[0], x0, x1);
-        cells_holding(g, 1, y, p[1], y0, y1);
-        cells_holding(g, 2, z, p[2], z0, z1);
-        const uint32_t k0 = pos_bits(p[0]), k1 = pos_bits(p[1]), k2 = pos_bits(p[2]);
-        const uint32_t cy = uint32_t(y1 - y0 + 1), columns = uint32_t(x1 - x0 + 1) * cy;
         uint32_t first = a;  // cells from a on cannot come before it
-        for (uint32_t c = k; c < columns; c += SD_LANES) {
-            const uint32_t key = (uint32_t(x0) + c / cy) * uint32_t(g.ny - 1) + uint32_t(y0) + c % cy;
-            const uint32_t zend = key * uint32_t(g.nz - 1) + uint32_t(z1);
-            for (uint32_t b = lower(lat, 0u, first, key * uint32_t(g.nz - 1) + uint32_t(z0)); b < first && lat[b] <= zend; ++b)
-                if (used[b] && pos_bits(dual[3ll * b]) == k0 && pos_bits(dual[3ll * b + 1]) == k1 &&
-                    pos_bits(dual[3ll * b + 2]) == k2)
-                    first = b;
+        if (table.slot) {
+            if (k == 0) first = table_first(table, dual, a);
+        } else {
+            const float p[3] = {dual[3ll * a], dual[3ll * a + 1], dual[3ll * a + 2]};
+            int x, y, z, x0, x1, y0, y1, z0, z1;
+            lat_xyz(g, lat[a], x, y, z);
+            cells_holding(g, 0, x, p[0], x0, x1);
+            cells_holding(g, 1, y, p[1], y0, y1);
+            cells_holding(g, 2, z, p[2], z0, z1);
+            const uint32_t cy = uint32_t(y1 - y0 + 1), columns = uint32_t(x1 - x0 + 1) * cy;  // at most SD_LANES
+            if (k < columns) {
+                const uint32_t key = (uint32_t(x0) + k / cy) * uint32_t(g.ny - 1) + uint32_t(y0) + k % cy;
+                const uint32_t zend = key * uint32_t(g.nz - 1) + uint32_t(z1);
+                for (uint32_t b = lower(lat, 0u, first, key * uint32_t(g.nz - 1) + uint32_t(z0)); b < first && lat[b] <= zend; ++b)
+                    if (used[b] && same_position(dual, a, b)) first = b;
+            }
         }
 #pragma unroll
         for (int d = SD_LANES / 2; d >= 1; d >>= 1) first = min(first, __shfl_xor_sync(lanes, first, d));
@@ -643,9 +643,14 @@ int sd_launch(const int* ids, const float* values, long long n, int nx, int ny, 
         }
         {
             const bool scan = nblk <= SD_SCAN;
-            iso::ProfScope ps("dc_weld", st, scan ? 2 : 3);
+            // the table, where one is needed, lies in the vertices until sd_number writes them
+            const bool hash = coords_may_repeat(g);
+            const WeldTable table{hash ? reinterpret_cast<uint32_t*>(vertices) : nullptr, weld_table_size(capA)};
+            iso::ProfScope ps("dc_weld", st, (scan ? 2 : 3) + (hash ? 1 : 0));
+            if (hash && launch_weld_table(table, dual, used, 1u, face, eff, capA, st) != cudaSuccess)
+                return iso::fail_code(ISO_ERR_CUDA);
             iso::launch_pdl(sd_flags, nblk, unsigned(SD_BLOCK), st, g, lat, used, face, dual, eff, w.vmap, w.blk, scan,
-                            w.ticket + 1, w.tot);
+                            w.ticket + 1, w.tot, table);
             if (!scan) iso_block_scan_launch(w.blk, w.nblk, w.tot, st);
             iso::launch_pdl(sd_number, nblk, unsigned(SD_BLOCK), st, dual, eff, blk, tot, face_capacity, w.vmap,
                             vertices, counts, status);

@@ -25,6 +25,7 @@
 #include "dc_common.cuh"
 #include "lookback.cuh"
 #include "profile.cuh"
+#include "weld_table.cuh"
 
 namespace {
 
@@ -1247,15 +1248,13 @@ __global__ void __launch_bounds__(256) dc_entry_points(const float* __restrict__
     }
 }
 
-// Cells along one axis whose closed interval [coord(i), coord(i + 1)] holds v,
-// for v in cell c's interval: [i0, i1] around c (wider than c +- 1 only when
-// grid coordinates repeat, on grids finer than FP32 resolves).  t: the axis's
+// Cells along one axis whose closed interval [coord(i), coord(i + 1)] holds v, in
+// cell c's: c alone, or c and the cell on the side where v is the common
+// coordinate (neighbouring coordinates are distinct here).  t: the axis's
 // coordinates, n of them.
 __device__ __forceinline__ void cells_holding(const float* __restrict__ t, int n, int c, float v, int& i0, int& i1) {
-    i0 = c;
-    i1 = c;
-    while (i0 > 0 && __ldg(t + i0) == v) --i0;
-    while (i1 < n - 2 && __ldg(t + i1 + 1) == v) ++i1;
+    i0 = c - (c > 0 && __ldg(t + c) == v ? 1 : 0);
+    i1 = c + (c < n - 2 && __ldg(t + c + 1) == v ? 1 : 0);
 }
 
 // Where the solve lists the cells whose vertex lies on a face of their box.
@@ -1266,9 +1265,9 @@ struct FaceList {
 };
 
 // Weld, eight lanes per vertex on a face of its cell's box, a lane per cell around
-// that face, edge or corner (two per axis on which the vertex lies on a face; more
-// only where coordinates repeat): looks for the used ones with the same
-// position.  When one comes before the vertex's own, vmap[a] = 0x80000000 | the
+// that face, edge or corner (two per axis on which the vertex lies on a face):
+// looks for the used ones with the same position; where coordinates may repeat it
+// reads their table instead (weld_table.cuh).  When one comes before the vertex's own, vmap[a] = 0x80000000 | the
 // first of them and used[a] gets bit 2.  Bound by the latency of six dependent
 // gathers; the list keeps every lane at it.  A pass over all cells waited in every
 // warp for its few such lanes and their cells one after another: 18 us at 512^3,
@@ -1277,7 +1276,7 @@ __global__ void __launch_bounds__(128) dc_weld_faces(Grid3 g, const CellIndex ix
                                                      const FaceList list, const uint32_t* __restrict__ cells,
                                                      uint8_t* used, const float* __restrict__ dual,
                                                      const long long* __restrict__ eff,
-                                                     uint32_t* __restrict__ vmap) {
+                                                     uint32_t* __restrict__ vmap, const WeldTable table) {
     iso::grid_wait();
     const uint32_t A = uint32_t(eff[0]);
     const bool listed = (long long)*list.n <= list.cap;  // else every cell is looked at
@@ -1290,29 +1289,31 @@ __global__ void __launch_bounds__(128) dc_weld_faces(Grid3 g, const CellIndex ix
         // (bit 0 is all that is read of another cell: the bits 2 that other threads
         // set meanwhile do not matter)
         if ((used[a] & 3u) != 3u) continue;
-        const float p[3] = {dual[3ll * a], dual[3ll * a + 1], dual[3ll * a + 2]};
-        const uint32_t cid = cells[a];
-        const int cz = int(cid % uint32_t(g.nz - 1));
-        const uint32_t rr = cid / uint32_t(g.nz - 1);
-        const int cy = int(rr % uint32_t(g.ny - 1)), cx = int(rr / uint32_t(g.ny - 1));
-        int x0, x1, y0, y1, z0, z1;
-        cells_holding(gc, g.nx, cx, p[0], x0, x1);
-        cells_holding(gc + g.nx, g.ny, cy, p[1], y0, y1);
-        cells_holding(gc + g.nx + g.ny, g.nz, cz, p[2], z0, z1);
-        const uint32_t k0 = pos_bits(p[0]), k1 = pos_bits(p[1]), k2 = pos_bits(p[2]);
-        const uint32_t ny = uint32_t(y1 - y0 + 1), nz = uint32_t(z1 - z0 + 1), count = uint32_t(x1 - x0 + 1) * ny * nz;
         uint32_t rep = a;
-        for (uint32_t c = k; c < count; c += 8) {
-            const uint32_t z = uint32_t(z0) + c % nz, r = c / nz;
-            const uint32_t y = uint32_t(y0) + r % ny, x = uint32_t(x0) + r / ny;
-            const uint32_t wi = (x * uint32_t(g.ny) + y) * uint32_t(ix.p.NWg) + (z >> 5);
-            const uint32_t mw = ix.actm[wi], bit = z & 31u;
-            if (!((mw >> bit) & 1u)) continue;
-            const uint32_t ib = ix.seg[wi >> ix.p.lgseg].x + ix.offA[wi] + __popc(mw & ((1u << bit) - 1u));
-            if (ib >= rep) continue;
-            const uint32_t u = used[ib];
-            const float q0 = dual[3ll * ib], q1 = dual[3ll * ib + 1], q2 = dual[3ll * ib + 2];
-            if ((u & 1u) && pos_bits(q0) == k0 && pos_bits(q1) == k1 && pos_bits(q2) == k2) rep = ib;
+        if (table.slot) {
+            if (k == 0) rep = table_first(table, dual, a);
+        } else {
+            const float p[3] = {dual[3ll * a], dual[3ll * a + 1], dual[3ll * a + 2]};
+            const uint32_t cid = cells[a];
+            const int cz = int(cid % uint32_t(g.nz - 1));
+            const uint32_t rr = cid / uint32_t(g.nz - 1);
+            const int cy = int(rr % uint32_t(g.ny - 1)), cx = int(rr / uint32_t(g.ny - 1));
+            int x0, x1, y0, y1, z0, z1;
+            cells_holding(gc, g.nx, cx, p[0], x0, x1);
+            cells_holding(gc + g.nx, g.ny, cy, p[1], y0, y1);
+            cells_holding(gc + g.nx + g.ny, g.nz, cz, p[2], z0, z1);
+            const uint32_t ny = uint32_t(y1 - y0 + 1), nz = uint32_t(z1 - z0 + 1),
+                           count = uint32_t(x1 - x0 + 1) * ny * nz;  // at most 8
+            if (k < count) {
+                const uint32_t z = uint32_t(z0) + k % nz, r = k / nz;
+                const uint32_t y = uint32_t(y0) + r % ny, x = uint32_t(x0) + r / ny;
+                const uint32_t wi = (x * uint32_t(g.ny) + y) * uint32_t(ix.p.NWg) + (z >> 5);
+                const uint32_t mw = ix.actm[wi], bit = z & 31u;
+                if ((mw >> bit) & 1u) {
+                    const uint32_t ib = ix.seg[wi >> ix.p.lgseg].x + ix.offA[wi] + __popc(mw & ((1u << bit) - 1u));
+                    if (ib < a && (used[ib] & 1u) && same_position(dual, a, ib)) rep = ib;
+                }
+            }
         }
         const uint32_t lanes = 0xffu << group;
 #pragma unroll
@@ -1965,12 +1966,17 @@ static int dc_dense_impl(const float* values, int nx, int ny, int nz, const floa
                             static_cast<const long long*>(eff), static_cast<const float*>(w.gc), so, in);
         }
         {
-            iso::ProfScope ps("dc_weld", st, 2);
+            // the table, where one is needed, takes the place of the entries, which the solve was the last to read
+            const bool hash = coords_may_repeat(g);
+            const WeldTable table{hash ? reinterpret_cast<uint32_t*>(ix.elist) : nullptr, weld_table_size(capA)};
+            iso::ProfScope ps("dc_weld", st, hash ? 3 : 2);
+            if (hash && launch_weld_table(table, w.dual, w.used, 3u, nullptr, eff, capA, st) != cudaSuccess)
+                return iso::fail_code(ISO_ERR_CUDA);
             const uint32_t* cc = cells;
             // (a few percent of the vertices lie on faces)
             iso::launch_pdl(dc_weld_faces, std::min(blocks_for(capA, 16), 152u * 16u), 128u, st, g, ix,
                             static_cast<const float*>(w.gc), list, cc, w.used, static_cast<const float*>(w.dual),
-                            static_cast<const long long*>(eff), w.vmap);
+                            static_cast<const long long*>(eff), w.vmap, table);
             iso::launch_pdl(dc_weld_number, blocks_for(capA, NUM_TILE), unsigned(NUM_THREADS), st,
                             static_cast<const float*>(w.dual), static_cast<const long long*>(eff),
                             static_cast<const uint8_t*>(w.used), w.wblk, w.zero + 14, w.vmap, vertices,

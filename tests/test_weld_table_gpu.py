@@ -12,6 +12,7 @@ pytestmark = pytest.mark.gpu
 
 import isoext_gb300 as iso  # noqa: E402
 from helpers import noise, sphere  # noqa: E402
+from isoext_gb300 import dc, diff  # noqa: E402
 from isoext_gb300.grids import grid_positions  # noqa: E402
 
 BOXES = {
@@ -49,6 +50,21 @@ def test_sparse(box, kind):
     a, f = iso.dual_contouring(g)
     b, h = iso.dual_contouring(g, intersection=iso.get_intersection(g, compute_normals=True))
     assert f.numel() and _same(a, b) and torch.equal(f, h)
+
+
+@pytest.mark.parametrize("kind", ["sphere", "noise"])
+@pytest.mark.parametrize("box", list(BOXES))
+def test_dense(box, kind):
+    """The call without an intersection and the one with it against the sequence;
+    the differentiable one has the same mesh."""
+    vals = _values(kind)
+    g = iso.UniformGrid(vals.shape, *BOXES[box])
+    g.set_values(torch.from_numpy(vals).cuda())
+    its = iso.get_intersection(g, compute_normals=True)
+    b, h = dc._dc_sequence(g, its, 1e-2, 1e-6)
+    for a, f in (iso.dual_contouring(g), iso.dual_contouring(g, intersection=its),
+                 diff.dual_contouring(g.get_values(), *BOXES[box])):
+        assert f.numel() and _same(a, b) and torch.equal(f, h)
 
 
 # Spacings just above the rule's line, 2^-20 of the box's magnitude: no coordinate repeats.

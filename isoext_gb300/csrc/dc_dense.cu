@@ -1208,33 +1208,84 @@ __global__ void __launch_bounds__(256) dc_solve_cells(const float* __restrict__ 
     }
 }
 
-// The crossings' points (and normals) of each entry's cell, its id and its first
-// crossing: isoext's Intersection (src/its.cu:94-159, 186-268).
-__global__ void __launch_bounds__(256) dc_entry_points(const float* __restrict__ vals, Grid3 g, float level,
-                                                       const CellIndex ix, const long long* __restrict__ eff,
-                                                       const float* __restrict__ gc, uint32_t* __restrict__ cells,
-                                                       uint32_t* __restrict__ cell_off, float* __restrict__ points,
-                                                       float* __restrict__ normals,
-                                                       const long long* __restrict__ counts,
-                                                       const int* __restrict__ status, long long* host) {
+// The crossings' points (and normals) of the entries' cells, their ids and first
+// crossings: isoext's Intersection (src/its.cu:94-159, 186-268).  A warp reads 32
+// entries' cells, a lane each, into shared memory, and then takes their crossings
+// one per lane: these are mostly consecutive rows of the output, so the stores
+// coalesce, and no lane waits for a cell with more crossings.  A lane that walked
+// its own cell's crossings stored rows 12 bytes wide some 70 apart, and the
+// store queue bound it: for the 99.5 M crossings of 256^3 noise 2.50 ms with normals
+// and 1.14 without, where this takes 1.61 and 0.80.
+constexpr int ENTRY_THREADS = 256;  // at most
+
+__global__ void __launch_bounds__(ENTRY_THREADS) dc_entry_points(
+    const float* __restrict__ vals, Grid3 g, float level, const CellIndex ix, const long long* __restrict__ eff,
+    const float* __restrict__ gc, uint32_t* __restrict__ cells, uint32_t* __restrict__ cell_off,
+    float* __restrict__ points, float* __restrict__ normals, const long long* __restrict__ counts,
+    const int* __restrict__ status, long long* host) {
+    __shared__ float cell_s[ENTRY_THREADS / 32][14][32];   // corner values, low and high corner
+    __shared__ uint32_t edge_s[ENTRY_THREADS / 32][3][32];  // crossed edges, crossings up to the cell's end, first crossing
     iso::grid_wait();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0) {  // the sizes and the status for the host
         for (int k = 0; k < 5; ++k) host[k] = counts[k];
         host[5] = *status;
     }
-    if (i >= eff[0]) return;
-    const ActiveCell c = entry_cell(ix, g, __ldg(ix.elist + i));
-    CellCorners cc;
-    load_cell_table(vals, g, gc, c.x, c.y, c.z, cc);
-    uint32_t cs = 0;
+    const int lane = threadIdx.x & 31;
+    if (i - lane >= eff[0]) return;
+    float(*cell)[32] = cell_s[threadIdx.x >> 5];
+    uint32_t(*edge)[32] = edge_s[threadIdx.x >> 5];
+    uint32_t est = 0, first = 0;
+    if (i < eff[0]) {
+        const ActiveCell c = entry_cell(ix, g, __ldg(ix.elist + i));
+        first = c.kbase + ix.klist[i];
+        cells[c.a] = c.cid;
+        cell_off[c.a] = first;
+        CellCorners cc;
+        load_cell_table(vals, g, gc, c.x, c.y, c.z, cc);
+        uint32_t cs = 0;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) cs |= uint32_t(iso::below(cc.v[j], level)) << j;
-    unsigned long long k = c.kbase + ix.klist[i];
-    cells[c.a] = c.cid;
-    cell_off[c.a] = uint32_t(k);
+        for (int j = 0; j < 8; ++j) {
+            cs |= uint32_t(iso::below(cc.v[j], level)) << j;
+            cell[j][lane] = cc.v[j];
+        }
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            cell[8 + q][lane] = cc.p[0][q];
+            cell[11 + q][lane] = cc.p[7][q];
+        }
+        est = edge_status(cs);
+    }
+    uint32_t end = __popc(est);
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t t = __shfl_up_sync(~0u, end, d);
+        if (lane >= d) end += t;
+    }
+    edge[0][lane] = est;
+    edge[1][lane] = end;
+    edge[2][lane] = first;
+    __syncwarp();
+    const uint32_t total = edge[1][31];
 #pragma unroll 1
-    for (uint32_t em = edge_status(cs); em; em &= em - 1, ++k) {  // this lane's crossed edges, ascending
+    for (uint32_t j = lane; j < total; j += 32) {
+        int o = 0;  // the first cell that ends past j
+#pragma unroll
+        for (int s = 16; s >= 1; s >>= 1)
+            if (edge[1][o + s - 1] <= j) o += s;
+        uint32_t em = edge[0][o];
+        const uint32_t r = j - (edge[1][o] - __popc(em));
+        const unsigned long long k = edge[2][o] + r;
+        for (uint32_t q = 0; q < r; ++q) em &= em - 1;
+        CellCorners cc;
+        cc.fma = g.fma;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            cc.v[q] = cell[q][o];
+            cc.p[q][0] = cell[(q >> 2) ? 11 : 8][o];
+            cc.p[q][1] = cell[((q >> 1) & 1) ? 12 : 9][o];
+            cc.p[q][2] = cell[(q & 1) ? 13 : 10][o];
+        }
         float p[3];
         edge_cross(cc, level, __ffs(em) - 1, p);
 #pragma unroll

@@ -141,3 +141,28 @@ def test_intersection_retries_reach_the_sizes():
     v, f = iso.dual_contouring(g, intersection=its)
     w, h = dc._dc_sequence(g, its, 1e-2, 1e-6)
     assert _same(v, w) and torch.equal(f, h)
+
+
+# Points below the level in a corner, on an edge, on a face and inside the grid (one,
+# two, four and eight active cells each): the last warp of the crossings full, short
+# and of one cell.
+@pytest.mark.parametrize("corner, edge, face, inner",
+                         [(1, 0, 0, 0), (1, 1, 1, 3), (0, 0, 0, 4), (1, 0, 0, 4), (1, 1, 1, 7), (1, 0, 0, 8),
+                          (0, 0, 0, 32), (1, 0, 0, 32)])
+def test_few_cells(corner, edge, face, inner):
+    vals = np.full((13, 12, 40), 1.0, np.float32)
+    if corner:
+        vals[0, 0, 0] = -0.3
+    if edge:
+        vals[0, 0, 20] = -0.2
+    if face:
+        vals[0, 6, 10] = -0.7
+    at = [(x, y, z) for x in (3, 6, 9) for y in (3, 6, 9) for z in (3, 6, 9, 31, 34, 37)][:inner]
+    for i, (x, y, z) in enumerate(at):
+        vals[x, y, z] = -0.1 - 0.05 * i
+    g = _grid(vals)
+    its = iso.get_intersection(g, compute_normals=True)
+    want = _reference_intersection(g, 0.0)
+    assert its._cells.numel() == corner + 2 * edge + 4 * face + 8 * inner
+    assert all(_same(x, y) for x, y in zip((its.get_points(), its.get_normals(), its._cells, its._offsets), want))
+    assert _same(iso.get_intersection(g).get_points(), want[0])

@@ -191,6 +191,14 @@ cudaError_t launch_pdl(void (*kernel)(Params...), unsigned grid, unsigned block,
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
 }
 
+// SMs of the current device.
+inline int sm_count() {
+    int dev = 0, sms = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+
 // ---------------------------------------------------------------------------
 // Launch parameters the autotuner may change (process-wide; iso_tune_set).
 

@@ -278,6 +278,12 @@ __device__ __forceinline__ float edge_cross(const CellCorners& cc, float level, 
     return t;
 }
 
+// |a - b| (norm(v0 - v2) of src/dc.cu:139), in the grid's arithmetic reading.
+__device__ __forceinline__ float dist3(const float* a, const float* b, bool fma) {
+    const float dx = __fsub_rn(a[0], b[0]), dy = __fsub_rn(a[1], b[1]), dz = __fsub_rn(a[2], b[2]);
+    return iso::norm3f(dx, dy, dz, fma);
+}
+
 Grid3 make_grid(int nx, int ny, int nz, const float* amin, const float* amax) {
     Grid3 g;
     g.nx = nx; g.ny = ny; g.nz = nz;

@@ -219,20 +219,12 @@ __global__ void __launch_bounds__(1024) dc_block_scan(unsigned long long* blk, l
 // intersect: crossing points / normals, active cells, CSR offsets; also the
 // per-word active mask and exclusive active-cell prefix used by the quads.
 
-__global__ void __launch_bounds__(DC_BLOCK) dc_intersect(const float* __restrict__ vals,
-                                                         const uint32_t* __restrict__ S, Grid3 g,
-                                                         float level, long long nwords,
+__global__ void __launch_bounds__(DC_BLOCK) dc_intersect(const uint32_t* __restrict__ S, Grid3 g, long long nwords,
                                                          const unsigned long long* __restrict__ blk,
                                                          uint32_t* __restrict__ actm,
-                                                         uint32_t* __restrict__ offA, float* points,
-                                                         float* normals, uint32_t* cell_ids,
-                                                         uint32_t* cell_off, long long A, long long K,
-                                                         const long long* __restrict__ dn) {
+                                                         uint32_t* __restrict__ offA, uint32_t* cell_ids,
+                                                         uint32_t* cell_off, long long A, long long K) {
     __shared__ uint32_t sm[66];
-    if (dn) {  // the sizes on the device (A, K); 0 when they exceeded the capacities
-        A = dn[0];
-        K = dn[1];
-    }
     const long long i = (long long)blockIdx.x * DC_BLOCK + threadIdx.x;
     const int NWc = (g.nz - 1 + 31) / 32;
     uint32_t act = 0, na = 0, nk = 0;
@@ -482,12 +474,6 @@ __device__ __forceinline__ uint32_t active_index(const uint32_t* actm, const uin
     return offA[wi] + __popc(actm[wi] & ((1u << (cz & 31)) - 1u));
 }
 
-// |a - b| (norm(v0 - v2) of src/dc.cu:139), in the grid's arithmetic reading.
-__device__ __forceinline__ float dist3(const float* a, const float* b, bool fma) {
-    const float dx = __fsub_rn(a[0], b[0]), dy = __fsub_rn(a[1], b[1]), dz = __fsub_rn(a[2], b[2]);
-    return iso::norm3f(dx, dy, dz, fma);
-}
-
 // The k-th quad of a point word in the reference's order: by bit (low endpoint
 // z) ascending, then the bit's z, y, x edges.
 __device__ __forceinline__ void kth_quad(uint32_t mz, uint32_t my, uint32_t mx, uint32_t k, int& b, int& ax) {
@@ -518,14 +504,11 @@ __global__ void __launch_bounds__(DC_BLOCK) dc_quad_emit(const uint32_t* __restr
                                                          const uint32_t* __restrict__ actm,
                                                          const uint32_t* __restrict__ offA,
                                                          const float* __restrict__ dual,
-                                                         int32_t* __restrict__ tri,
-                                                         const long long* __restrict__ dn) {
+                                                         int32_t* __restrict__ tri) {
     __shared__ uint32_t sm[66];
     const long long i = (long long)blockIdx.x * DC_BLOCK + threadIdx.x;
     const int NWg = (g.nz + 31) / 32;
     const int lane = threadIdx.x & 31;
-    // dn: the triangle indices the output holds (6 Q, or 0 over capacity)
-    const unsigned long long qmax = dn ? (unsigned long long)(dn[2] / 6) : ~0ull;
     uint32_t mz = 0, my = 0, mx = 0, sw = 0;
     int x = 0, y = 0, w = 0;
     if (i < nwords) {
@@ -557,7 +540,6 @@ __global__ void __launch_bounds__(DC_BLOCK) dc_quad_emit(const uint32_t* __restr
         if (j >= total) continue;
         const uint32_t k = j - oexcl;
         const unsigned long long q = qb + oeq + k;
-        if (q >= qmax) continue;
         int b, ax;
         kth_quad(omz, omy, omx, k, b, ax);
         const int z = 32 * ow + b;
@@ -605,11 +587,9 @@ __global__ void __launch_bounds__(DC_BLOCK) dc_quad_emit(const uint32_t* __restr
 using iso::pos_bits;
 using iso::pos_hash;
 
-__global__ void dc_mark_used(const int32_t* __restrict__ tri, long long n, uint32_t* used,
-                             const long long* __restrict__ dn) {
+__global__ void dc_mark_used(const int32_t* __restrict__ tri, long long n, uint32_t* used) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (dn) n = dn[2];
-    if (i < n) used[tri ? tri[i] : int32_t(i)] = 1u;  // tri == nullptr: triangle i is point i
+    if (i < n) used[tri ? tri[i] : int32_t(i)] = 1u;  // tri == nullptr: triangle i is point i (a soup)
 }
 
 // Probes before an insert gives up (the table is at most half full when the
@@ -618,14 +598,11 @@ __global__ void dc_mark_used(const int32_t* __restrict__ tri, long long n, uint3
 // overflow, later threads skip their probes: the call's output is discarded.
 constexpr uint32_t HASH_PROBES = 512;
 
-// Insert used vertices (used == nullptr: all); a slot keeps the smallest index
-// with its position.
+// Insert used vertices; a slot keeps the smallest index with its position.
 __global__ void dc_hash_insert(const float* __restrict__ dual, const uint32_t* __restrict__ used,
-                               long long A, uint32_t* table, uint32_t mask, int* status,
-                               const long long* __restrict__ dn) {
+                               long long A, uint32_t* table, uint32_t mask, int* status) {
     const long long a = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (dn) A = dn[0];
-    if (a >= A || (used && !used[a])) return;
+    if (a >= A || !used[a]) return;
     if (status && *(volatile int*)status == int(ISO_ERR_OVERFLOW)) return;
     const uint32_t k0 = pos_bits(dual[3 * a]), k1 = pos_bits(dual[3 * a + 1]), k2 = pos_bits(dual[3 * a + 2]);
     uint32_t h = pos_hash(k0, k1, k2) & mask;
@@ -645,11 +622,10 @@ __global__ void dc_hash_insert(const float* __restrict__ dual, const uint32_t* _
 // rep[a] = smallest index with the same position (for used vertices).
 __global__ void dc_hash_lookup(const float* __restrict__ dual, const uint32_t* __restrict__ used,
                                long long A, const uint32_t* __restrict__ table, uint32_t mask,
-                               uint32_t* rep, const long long* __restrict__ dn) {
+                               uint32_t* rep) {
     const long long a = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (dn) A = dn[0];
     if (a >= A) return;
-    if (used && !used[a]) { rep[a] = 0xffffffffu; return; }
+    if (!used[a]) { rep[a] = 0xffffffffu; return; }
     const uint32_t k0 = pos_bits(dual[3 * a]), k1 = pos_bits(dual[3 * a + 1]), k2 = pos_bits(dual[3 * a + 2]);
     uint32_t h = pos_hash(k0, k1, k2) & mask;
     for (uint32_t probe = 0; probe <= mask && probe < HASH_PROBES; ++probe, h = (h + 1) & mask) {
@@ -666,10 +642,9 @@ __global__ void dc_hash_lookup(const float* __restrict__ dual, const uint32_t* _
 
 // Per block of 1024 dual vertices: number of representatives (rep[a] == a).
 __global__ void __launch_bounds__(DC_BLOCK) dc_rep_count(const uint32_t* __restrict__ rep, long long A,
-                                                         unsigned long long* blk, const long long* __restrict__ dn) {
+                                                         unsigned long long* blk) {
     __shared__ uint32_t sm[66];
     const long long a = (long long)blockIdx.x * DC_BLOCK + threadIdx.x;
-    if (dn) A = dn[0];
     const uint32_t is = (a < A && rep[a] == uint32_t(a)) ? 1u : 0u;
     uint32_t e0, e1, t0, t1;
     block_scan2(is, 0u, e0, e1, t0, t1, sm);
@@ -679,17 +654,15 @@ __global__ void __launch_bounds__(DC_BLOCK) dc_rep_count(const uint32_t* __restr
 __global__ void __launch_bounds__(DC_BLOCK) dc_rep_write(const uint32_t* __restrict__ rep, long long A,
                                                          const unsigned long long* __restrict__ blk,
                                                          const float* __restrict__ dual, uint32_t* newidx,
-                                                         float* vout, uint32_t* vsrc, const long long* __restrict__ dn) {
+                                                         float* vout, uint32_t* vsrc) {
     __shared__ uint32_t sm[66];
     const long long a = (long long)blockIdx.x * DC_BLOCK + threadIdx.x;
-    if (dn) A = dn[0];
     const uint32_t is = (a < A && rep[a] == uint32_t(a)) ? 1u : 0u;
     uint32_t e0, e1, t0, t1;
     block_scan2(is, 0u, e0, e1, t0, t1, sm);
     if (!is) return;
     const unsigned long long o = blk[2 * blockIdx.x] + e0;
     newidx[a] = uint32_t(o);
-    if (dn && (long long)o >= dn[3]) return;  // past the vertex capacity: the caller sees V and retries
     if (vsrc) vsrc[o] = uint32_t(a);
     vout[3 * o] = dual[3 * a];
     vout[3 * o + 1] = dual[3 * a + 1];
@@ -697,12 +670,10 @@ __global__ void __launch_bounds__(DC_BLOCK) dc_rep_write(const uint32_t* __restr
 }
 
 __global__ void dc_remap(const int32_t* __restrict__ tri, long long n, const uint32_t* __restrict__ rep,
-                         const uint32_t* __restrict__ newidx, int32_t* fout, const long long* __restrict__ dn) {
+                         const uint32_t* __restrict__ newidx, int32_t* fout) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (dn) n = dn[2];
     if (i < n) fout[i] = int32_t(newidx[rep[tri ? tri[i] : int32_t(i)]]);
 }
-
 
 // ---------------------------------------------------------------------------
 // One-call dual contouring: after the sign pass, five or six kernels chained by
@@ -1639,8 +1610,8 @@ int iso_dc_intersect(const float* values, int nx, int ny, int nz, const float* a
     Grid3 g = make_grid(nx, ny, nz, aabb_min, aabb_max);
     iso::ProfScope ps("dc_intersect", st, A > 0 && points ? 2 : 1);
     dc_intersect<<<blocks_for(w.cwords, DC_BLOCK), DC_BLOCK, 0, st>>>(
-        values, w.S, g, level, w.cwords, w.blkC, w.actm, w.offA, points, normals,
-        reinterpret_cast<uint32_t*>(cell_ids), reinterpret_cast<uint32_t*>(cell_offsets), A, K, nullptr);
+        w.S, g, w.cwords, w.blkC, w.actm, w.offA, reinterpret_cast<uint32_t*>(cell_ids),
+        reinterpret_cast<uint32_t*>(cell_offsets), A, K);
     if (A == 0 && cell_offsets) cudaMemsetAsync(cell_offsets, 0, 4, st);
     if (A > 0 && points) {
         const int bt = iso::tune_get(iso::TUNE_DC_CELL_THREADS);  // read once: another thread may set it meanwhile
@@ -1663,8 +1634,8 @@ int iso_dc_intersect_solve(const float* values, int nx, int ny, int nz, const fl
     {
         iso::ProfScope ps("dc_intersect", st);
         dc_intersect<<<blocks_for(w.cwords, DC_BLOCK), DC_BLOCK, 0, st>>>(
-            values, w.S, g, level, w.cwords, w.blkC, w.actm, w.offA, nullptr, nullptr,
-            reinterpret_cast<uint32_t*>(cell_ids), reinterpret_cast<uint32_t*>(cell_offsets), A, K, nullptr);
+            w.S, g, w.cwords, w.blkC, w.actm, w.offA, reinterpret_cast<uint32_t*>(cell_ids),
+            reinterpret_cast<uint32_t*>(cell_offsets), A, K);
     }
     iso::ProfScope ps("dc_solve", st);
     const int bt = iso::tune_get(iso::TUNE_DC_CELL_THREADS);
@@ -1710,7 +1681,7 @@ int iso_dc_cells(const float* values, int nx, int ny, int nz, float level, void*
     Grid3 g = make_grid(nx, ny, nz, amin, amax);
     iso::ProfScope ps("dc_intersect", st);
     dc_intersect<<<blocks_for(w.cwords, DC_BLOCK), DC_BLOCK, 0, st>>>(
-        values, w.S, g, level, w.cwords, w.blkC, w.actm, w.offA, nullptr, nullptr, nullptr, nullptr, -1, 0, nullptr);
+        w.S, g, w.cwords, w.blkC, w.actm, w.offA, nullptr, nullptr, -1, 0);
     return cudaGetLastError() == cudaSuccess ? 0 : iso::fail_code(ISO_ERR_CUDA);
 }
 
@@ -1734,7 +1705,7 @@ int iso_dc_quads_emit(int nx, int ny, int nz, void* ws, const float* dual, int* 
     Grid3 g = make_grid(nx, ny, nz, amin, amax);
     iso::ProfScope ps("dc_quads", st);
     dc_quad_emit<<<blocks_for(w.pwords, DC_BLOCK), DC_BLOCK, 0, st>>>(w.S, g, w.pwords, w.blkQ, w.actm,
-                                                                     w.offA, dual, tri, nullptr);
+                                                                     w.offA, dual, tri);
     return cudaGetLastError() == cudaSuccess ? 0 : iso::fail_code(ISO_ERR_CUDA);
 }
 
@@ -1763,11 +1734,11 @@ int iso_dc_weld_count(const float* dual, long long A, const int* tri, long long 
     iso::ProfScope ps("dc_weld", st, (ntri > 0 ? 1 : 0) + (A > 0 ? 4 : 0));
     cudaMemsetAsync(used, 0, size_t(A) * 4, st);
     cudaMemsetAsync(table, 0xff, size_t(cap) * 4, st);
-    if (ntri > 0) dc_mark_used<<<blocks_for(ntri, 256), 256, 0, st>>>(tri, ntri, used, nullptr);
+    if (ntri > 0) dc_mark_used<<<blocks_for(ntri, 256), 256, 0, st>>>(tri, ntri, used);
     if (A > 0) {
-        dc_hash_insert<<<blocks_for(A, 256), 256, 0, st>>>(dual, used, A, table, cap - 1, status, nullptr);
-        dc_hash_lookup<<<blocks_for(A, 256), 256, 0, st>>>(dual, used, A, table, cap - 1, rep, nullptr);
-        dc_rep_count<<<unsigned(nblk), DC_BLOCK, 0, st>>>(rep, A, blk, nullptr);
+        dc_hash_insert<<<blocks_for(A, 256), 256, 0, st>>>(dual, used, A, table, cap - 1, status);
+        dc_hash_lookup<<<blocks_for(A, 256), 256, 0, st>>>(dual, used, A, table, cap - 1, rep);
+        dc_rep_count<<<unsigned(nblk), DC_BLOCK, 0, st>>>(rep, A, blk);
         dc_block_scan<<<1, 1024, 0, st>>>(blk, nblk, counts);
     } else {
         cudaMemsetAsync(counts, 0, 16, st);
@@ -1793,8 +1764,8 @@ int iso_dc_weld_write_src(const float* dual, long long A, const int* tri, long l
     iso::ProfScope ps("dc_weld", st, (A > 0 ? 1 : 0) + (ntri > 0 ? 1 : 0));
     if (A > 0)
         dc_rep_write<<<unsigned(nblk), DC_BLOCK, 0, st>>>(rep, A, blk, dual, newidx, vout,
-                                                           reinterpret_cast<uint32_t*>(vertex_source), nullptr);
-    if (ntri > 0) dc_remap<<<blocks_for(ntri, 256), 256, 0, st>>>(tri, ntri, rep, newidx, fout, nullptr);
+                                                           reinterpret_cast<uint32_t*>(vertex_source));
+    if (ntri > 0) dc_remap<<<blocks_for(ntri, 256), 256, 0, st>>>(tri, ntri, rep, newidx, fout);
     return cudaGetLastError() == cudaSuccess ? 0 : iso::fail_code(ISO_ERR_CUDA);
 }
 
@@ -2025,7 +1996,7 @@ static int dc_dense_impl(const float* values, int nx, int ny, int nz, const floa
                 return iso::fail_code(ISO_ERR_CUDA);
             const uint32_t* cc = cells;
             // (a few percent of the vertices lie on faces)
-            iso::launch_pdl(dc_weld_faces, std::min(blocks_for(capA, 16), 152u * 16u), 128u, st, g, ix,
+            iso::launch_pdl(dc_weld_faces, std::min(blocks_for(capA, 16), 16u * unsigned(iso::sm_count())), 128u, st, g, ix,
                             static_cast<const float*>(w.gc), list, cc, w.used, static_cast<const float*>(w.dual),
                             static_cast<const long long*>(eff), w.vmap, table);
             iso::launch_pdl(dc_weld_number, blocks_for(capA, NUM_TILE), unsigned(NUM_THREADS), st,

@@ -359,6 +359,7 @@ __device__ __forceinline__ void mc_totals(unsigned long long V, unsigned long lo
 // segments this saves the launch of mc_scan (4 us); the count's CTAs then each
 // take a fence and an atomic on one counter before they end, which costs more
 // than the launch from 2048 segments on (15 -> 22 us at 2048, 48 -> 60 us at 4096).
+// Their sums fit 32 bits (1024 segments of 1024 words, each below 2^18).
 constexpr int SCAN_LAST = 4;
 
 template <int T>
@@ -376,28 +377,9 @@ __device__ void scan_segments(unsigned long long* blk, uint32_t nseg, unsigned l
         sa += a[k];
         sb += b[k];
     }
-    // totals beyond 32 bits: summed in 64 (the offsets then are not used)
-    unsigned long long wa = sa, wb = sb;
-#pragma unroll
-    for (int d = 16; d >= 1; d >>= 1) {
-        wa += __shfl_xor_sync(~0u, wa, d);
-        wb += __shfl_xor_sync(~0u, wb, d);
-    }
-    __shared__ unsigned long long tot[2][T / 32];
-    if ((threadIdx.x & 31) == 0) {
-        tot[0][threadIdx.x >> 5] = wa;
-        tot[1][threadIdx.x >> 5] = wb;
-    }
     uint32_t ea, eb, ta, tb;
     block_scan2<T>(sa, sb, ea, eb, ta, tb, sm);
-    if (threadIdx.x == 0) {
-        unsigned long long V = 0, F = 0;
-        for (int q = 0; q < T / 32; ++q) {
-            V += tot[0][q];
-            F += tot[1][q];
-        }
-        mc_totals(V, F, ctr, counts, status, capV, capF);
-    }
+    if (threadIdx.x == 0) mc_totals(ta, tb, ctr, counts, status, capV, capF);
 #pragma unroll
     for (int k = 0; k < SCAN_LAST; ++k) {
         if (k < per && s0 + k < nseg)
@@ -1283,13 +1265,6 @@ __global__ void __launch_bounds__(SIGN_BLOCK) mc_signs_rows(const float* __restr
 std::mutex g_mu;
 int g_block = 256;
 
-int sm_count() {
-    int dev = 0, sms = 1;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return sms;
-}
-
 // Threads of a count CTA.
 int count_threads() { return iso::tune_get(iso::TUNE_MC_COUNT_THREADS) == 128 ? 128 : 256; }
 
@@ -1330,7 +1305,7 @@ int launch_emit(const McParams& p, const McGrid& g, const McWs& w, cudaStream_t 
 
 // ct: the threads of a count CTA that g.lgseg was made from.
 int launch_count_emit(const McParams& p, const McGrid& g, const McWs& w, int ct, cudaStream_t st) {
-    const int sms = sm_count();
+    const int sms = iso::sm_count();
     const uint32_t nseg = uint32_t((g.PW + (1ll << g.lgseg) - 1) >> g.lgseg);
     {
         iso::ProfScope ps("mc_count", st);
@@ -1372,7 +1347,7 @@ int mc_get_block() {
 void mc_signs_launch(const float* vals, int nx, int ny, int nz, float level, uint32_t* out,
                      cudaStream_t st, unsigned long long* zero, long long nzero) {
     const int NW = (nz + 31) / 32;
-    const long long rows = (long long)nx * ny, most = (long long)sm_count() * iso::tune_get(iso::TUNE_MC_SIGN_CTAS);
+    const long long rows = (long long)nx * ny, most = (long long)iso::sm_count() * iso::tune_get(iso::TUNE_MC_SIGN_CTAS);
     const auto ctas = [&](long long warps) {
         constexpr int per = SIGN_BLOCK / 32;
         return unsigned(std::max<long long>(1, std::min<long long>((warps + per - 1) / per, most)));

@@ -214,11 +214,8 @@ int iso_sdf_union_grid(const float* prims, int nx, int ny, int nz, const float* 
             prims, nx, ny, nz, aabb_min[0], aabb_min[1], aabb_min[2], aabb_max[0] - aabb_min[0],
             aabb_max[1] - aabb_min[1], aabb_max[2] - aabb_min[2], iso::arith_fma(), out);
     } else {
-        int dev = 0, sms = 1;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         const long long rows = (long long)nx * ny;  // a warp each, 8 per CTA
-        const long long grid = std::max<long long>(1, std::min<long long>((rows + 7) / 8, (long long)sms * 8));
+        const long long grid = std::max<long long>(1, std::min<long long>((rows + 7) / 8, (long long)iso::sm_count() * 8));
         sdf_union_grid<<<unsigned(grid), 256, 0, st>>>(prims, nx, ny, nz, aabb_min[0], aabb_min[1], aabb_min[2],
                                                        aabb_max[0] - aabb_min[0], aabb_max[1] - aabb_min[1],
                                                        aabb_max[2] - aabb_min[2], iso::arith_fma(), out);

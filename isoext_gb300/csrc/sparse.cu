@@ -992,12 +992,6 @@ __global__ void __launch_bounds__(SP_BLOCK) sp_quad_count(SpGrid g, const int* _
     if (threadIdx.x == 0) { blk[2 * blockIdx.x] = t; blk[2 * blockIdx.x + 1] = 0; }
 }
 
-// |a - b| (norm(v0 - v2) of src/dc.cu:139), in the grid's arithmetic reading.
-__device__ __forceinline__ float dist3(const float* a, const float* b, bool fma) {
-    const float dx = __fsub_rn(a[0], b[0]), dy = __fsub_rn(a[1], b[1]), dz = __fsub_rn(a[2], b[2]);
-    return iso::norm3f(dx, dy, dz, fma);
-}
-
 __global__ void __launch_bounds__(SP_BLOCK) sp_quad_emit(SpGrid g, const int* __restrict__ ids,
                                                          const float* __restrict__ vals, long long n,
                                                          const uint32_t* __restrict__ rank,

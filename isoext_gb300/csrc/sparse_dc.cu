@@ -482,11 +482,6 @@ __device__ __forceinline__ int32_t vertex_of(const uint32_t* vmap, uint32_t i) {
     return int32_t(m);
 }
 
-// |a - b| (norm(v0 - v2) of src/dc.cu:139), in the grid's arithmetic reading.
-__device__ __forceinline__ float dist3(const float* a, const float* b, bool fma) {
-    return iso::norm3f(__fsub_rn(a[0], b[0]), __fsub_rn(a[1], b[1]), __fsub_rn(a[2], b[2]), fma);
-}
-
 // The quads in owner order, z, y, x edge within an owner, split along the shorter
 // diagonal (src/dc.cu:101-157).
 __global__ void __launch_bounds__(SD_BLOCK) sd_faces(Grid3 g, const uint8_t* __restrict__ qbits,

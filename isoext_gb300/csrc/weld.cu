@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(WELD_THREADS, 8) weld_insert(const float* __re
 // positions (up to capV); vtot[0] <- the number of distinct positions.  Tiles
 // are taken in ticket order (ctr) and chained by look-back (state, one word per
 // tile, zeroed by the caller).
-__global__ void __launch_bounds__(WELD_THREADS) weld_number(const float* __restrict__ pts, long long A,
+__global__ void __launch_bounds__(WELD_THREADS) weld_number(const float* __restrict__ pts,
                                                             const uint32_t* __restrict__ table,
                                                             uint32_t* __restrict__ rep, unsigned long long* state,
                                                             unsigned int* ctr, float* __restrict__ vout,
@@ -125,11 +125,7 @@ __global__ void __launch_bounds__(WELD_THREADS) weld_number(const float* __restr
     __shared__ uint32_t wsum[WELD_THREADS / 32];
     __shared__ unsigned long long pre_s;
     iso::grid_wait();
-    long long capV = 0x7fffffffll;
-    if (dn) {
-        A = dn[0];
-        capV = dn[3];
-    }
+    const long long A = dn[0], capV = dn[3];
     if (threadIdx.x == 0) tile_s = atomicAdd(ctr, 1u);
     __syncthreads();
     const uint32_t tile = tile_s;
@@ -212,17 +208,17 @@ __global__ void __launch_bounds__(WELD_THREADS) weld_number(const float* __restr
 }
 
 // fout[i] <- the new number of triangle index tri[i]'s position.
-__global__ void __launch_bounds__(WELD_THREADS) weld_remap(const int32_t* __restrict__ tri, long long n,
+__global__ void __launch_bounds__(WELD_THREADS) weld_remap(const int32_t* __restrict__ tri,
                                                            const uint32_t* __restrict__ rep, int32_t* fout,
                                                            const long long* __restrict__ dn) {
     iso::grid_wait();
-    if (dn) n = dn[2];
+    const long long n = dn[2];
     const long long base = (long long)blockIdx.x * (WELD_THREADS * REMAP_PER) + threadIdx.x;
     uint32_t r[REMAP_PER];
 #pragma unroll
     for (int e = 0; e < REMAP_PER; ++e) {
         const long long i = base + e * WELD_THREADS;
-        r[e] = i < n ? rep[tri ? tri[i] : int32_t(i)] : WELD_NEW;
+        r[e] = i < n ? rep[tri[i]] : WELD_NEW;
     }
 #pragma unroll
     for (int e = 0; e < REMAP_PER; ++e)
@@ -268,7 +264,7 @@ WeldDev weld_dev_carve(void* ws, long long capA, long long capU) {
 size_t weld_dev_workspace(long long capA, long long capU) { return weld_dev_carve(nullptr, capA, capU).total; }
 
 // The weld of eff[0] points (at most capA) whose distinct positions fit capU:
-// eff[2] triangle indices (tri == nullptr: index i is point i; at most capT),
+// eff[2] triangle indices (at most capT),
 // eff[3] vertex capacity of vout.  vtot[0] <- V.
 void weld_dev_launch(const float* pts, long long capA, long long capU, const int32_t* tri, long long capT,
                      const long long* eff, void* ws, float* vout, int32_t* fout, long long* vtot, int* status,
@@ -281,7 +277,7 @@ void weld_dev_launch(const float* pts, long long capA, long long capU, const int
         cudaMemsetAsync(w.table, 0xff, size_t(w.hcap) * 4, st);
         cudaMemsetAsync(w.state, 0, w.state_bytes, st);
         weld_insert<<<tiles, WELD_THREADS, 0, st>>>(pts, capA, w.table, w.hcap - 1, w.rep, status, eff);
-        iso::launch_pdl(weld_number, unsigned((capA + NUM_TILE - 1) / NUM_TILE), unsigned(WELD_THREADS), st, pts, capA,
+        iso::launch_pdl(weld_number, unsigned((capA + NUM_TILE - 1) / NUM_TILE), unsigned(WELD_THREADS), st, pts,
                         w.table, w.rep, w.state, ctr, vout, vtot, status, eff);
     } else {
         cudaMemsetAsync(vtot, 0, 16, st);
@@ -289,7 +285,7 @@ void weld_dev_launch(const float* pts, long long capA, long long capU, const int
     if (capT > 0) {
         const long long per = (long long)WELD_THREADS * REMAP_PER;
         iso::launch_pdl(weld_remap, unsigned(std::max<long long>((capT + per - 1) / per, 1)), unsigned(WELD_THREADS),
-                        st, tri, capT, w.rep, fout, eff);
+                        st, tri, w.rep, fout, eff);
     }
 }
 

@@ -221,9 +221,11 @@ def _dc_sequence(grid: UniformGrid, its: Intersection, reg, svd_tol):
     nx, ny, nz = grid.shape
     amin, amax = _ffi.fvec3(grid.aabb_min), _ffi.fvec3(grid.aabb_max)
     st = _stream(dev)
-    ws, (_, _, Q) = _classify_quads(grid, its._level)
-    _ffi.check(lib.iso_dc_cells(_p(grid._values), nx, ny, nz, its._level, _p(ws), st))
+    ws, (cells, _, Q) = _classify_quads(grid, its._level)
     A = int(its._cells.numel())
+    if cells > A:  # quads would name dual vertices that the intersection does not have
+        raise RuntimeError("the grid's values changed: they cross more cells than the intersection has")
+    _ffi.check(lib.iso_dc_cells(_p(grid._values), nx, ny, nz, its._level, _p(ws), st))
     normals = its._normals
     if normals is None:
         normals = torch.empty_like(its._points)

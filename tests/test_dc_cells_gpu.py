@@ -166,3 +166,23 @@ def test_few_cells(corner, edge, face, inner):
     assert its._cells.numel() == corner + 2 * edge + 4 * face + 8 * inner
     assert all(_same(x, y) for x, y in zip((its.get_points(), its.get_normals(), its._cells, its._offsets), want))
     assert _same(iso.get_intersection(g).get_points(), want[0])
+
+
+def test_the_mesh_after_the_values_changed():
+    """As many active cells elsewhere, the same cells with the signs swapped, and
+    fewer cells: the mesh is the sequence's, bit for bit.  More cells than the
+    intersection has dual vertices are refused."""
+    vals = sphere((30, 31, 32), 0.5, center=(0.2, 0.0, 0.0))
+    g = _grid(vals)
+    for normals in (True, False):
+        for other in (vals[::-1], -vals, sphere(vals.shape, 0.3)):
+            g.set_values(torch.from_numpy(vals).cuda())
+            its = iso.get_intersection(g, compute_normals=normals)
+            g.set_values(torch.from_numpy(np.ascontiguousarray(other)).cuda())
+            assert iso.get_intersection(g)._cells.numel() <= its._cells.numel()
+            w, h = dc._dc_sequence(g, its, 1e-2, 1e-6)
+            v, f = iso.dual_contouring(g, intersection=its)
+            assert len(h) and _same(v, w) and torch.equal(f, h)
+        g.set_values(torch.from_numpy(sphere(vals.shape, 0.7)).cuda())
+        with pytest.raises(RuntimeError, match="more cells"):
+            iso.dual_contouring(g, intersection=its)

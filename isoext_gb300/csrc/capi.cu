@@ -76,7 +76,7 @@ int sizes_failed(const char* what, cudaError_t e) {
 }
 }  // namespace
 
-HostSizes::HostSizes() {
+long long* HostSizes::lease() {
     cudaError_t e = cudaErrorDeviceUninitialized;
     if (context_id(&ctx_)) {
         p_ = size_pool().lease(ctx_, [&](size_t bytes) -> void* {
@@ -86,6 +86,7 @@ HostSizes::HostSizes() {
         });
     }
     if (!p_) sizes_failed("no pinned memory for the sizes", e);
+    return p_;
 }
 
 HostSizes::~HostSizes() {
@@ -93,7 +94,8 @@ HostSizes::~HostSizes() {
 }
 
 int HostSizes::wait(int rc, int n, long long* out, cudaStream_t st) {
-    return finish_sizes(rc, ISO_ERR_CUDA, p_, n, out, [&] {
+    static const long long none[SizePool::WORDS] = {};
+    return finish_sizes(rc, ISO_ERR_CUDA, p_ ? p_ : none, n, out, [&] {
         const cudaError_t e = cudaStreamSynchronize(st);
         if (e == cudaSuccess) return true;
         if (!rc) sizes_failed("CUDA error", e);  // else the launch's message stays
@@ -200,7 +202,7 @@ namespace {
 int mc_dense_impl(const float* values, int nx, int ny, int nz, const float* aabb_min, const float* aabb_max,
                   float level, int method, float* vertices, long long vertex_capacity, int* faces,
                   long long face_capacity, void* workspace, size_t workspace_bytes, long long* counts,
-                  int* status, long long* vertex_edges, void* stream, long long* host = nullptr) {
+                  int* status, long long* vertex_edges, void* stream, iso::HostSizes* host = nullptr) {
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     if (!grid_ok(nx, ny, nz))
         return fail(ISO_ERR_ARG, "Number of points exceeds maximum value 2147483647 (max int)");
@@ -236,7 +238,11 @@ int mc_dense_impl(const float* values, int nx, int ny, int nz, const float* aabb
     p.capF = face_capacity;
     p.counts = counts;
     p.vedge = vertex_edges;
-    p.host = host;
+    if (host) {
+        if (workspace_bytes < mc_workspace_bytes(nx, ny, nz, vertex_capacity, face_capacity))
+            return fail(ISO_ERR_WORKSPACE, "workspace too small");
+        if (!(p.host = host->lease())) return ISO_ERR_CUDA;
+    }
     int rc = mc_launch(p, workspace, workspace_bytes, st);
     if (rc == ISO_ERR_WORKSPACE) return fail(rc, "workspace too small");
     if (rc) {
@@ -264,10 +270,9 @@ int iso_mc_dense_sync(const float* values, int nx, int ny, int nz, const float* 
                       void* stream) {
     if (!sizes) return fail(ISO_ERR_ARG, "sizes is null");
     iso::HostSizes host;
-    if (!host.words()) return ISO_ERR_CUDA;
     const int rc = mc_dense_impl(values, nx, ny, nz, aabb_min, aabb_max, level, method, vertices, vertex_capacity,
                                  faces, face_capacity, workspace, workspace_bytes, nullptr, nullptr, nullptr, stream,
-                                 host.words());
+                                 &host);
     return host.wait(rc, 3, sizes, reinterpret_cast<cudaStream_t>(stream));
 }
 

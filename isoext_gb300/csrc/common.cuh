@@ -209,19 +209,20 @@ int tune_get(int key);
 // true = the reference's CUDA build (fused), false = its host build.
 bool arith_fma();
 
-// Sizes that a call's last kernel writes for the host (iso_*_sync): words() is a
-// cleared record of 16 words of pinned memory, this call's own until the object
-// goes (size_pool.h); nullptr, with the message set, when there is none to be had.
-// wait(rc) ends the call: the launches' result rc when they failed (their kernels
-// waited for, see finish_sizes), else it waits for the stream and copies the first
-// n words to out.
+// Sizes that a call's last kernel writes for the host (iso_*_sync).  lease(), called
+// once the arguments have been checked, gives a cleared record of 16 words of
+// pinned memory, the call's own until the object goes (size_pool.h); nullptr, with
+// the message set, when there is none to be had.  wait(rc) ends the call: the
+// launches' result rc when they failed (their kernels waited for, see
+// finish_sizes), else it waits for the stream and copies the first n words to out
+// (zeros when nothing was leased: an empty grid).
 class HostSizes {
 public:
-    HostSizes();
+    HostSizes() = default;
     ~HostSizes();
     HostSizes(const HostSizes&) = delete;
     HostSizes& operator=(const HostSizes&) = delete;
-    long long* words() const { return p_; }
+    long long* lease();
     int wait(int rc, int n, long long* out, cudaStream_t st);
 
 private:

@@ -1836,7 +1836,7 @@ CellIndex cell_index(const DcDenseWs& w, const Grid3& g, unsigned long long* eli
 static int dc_dense_impl(const float* values, int nx, int ny, int nz, const float* aabb_min, const float* aabb_max,
                          float level, float reg, float svd_tol, float* vertices, long long vertex_capacity, int* faces,
                          long long face_capacity, void* workspace, size_t workspace_bytes, long long* counts,
-                         int* status, int* cell_ids, int* cell_offsets, int* vertex_source, long long* host,
+                         int* status, int* cell_ids, int* cell_offsets, int* vertex_source, iso::HostSizes* host,
                          const Given* given, void* stream);
 
 extern "C" {
@@ -1862,10 +1862,9 @@ int iso_dc_dense_sync(const float* values, int nx, int ny, int nz, const float* 
                       void* stream) {
     if (!sizes || vertex_capacity < 1) return iso::fail_code(ISO_ERR_ARG);
     iso::HostSizes host;
-    if (!host.words()) return ISO_ERR_CUDA;
     const int rc = dc_dense_impl(values, nx, ny, nz, aabb_min, aabb_max, level, reg, svd_tol, vertices,
                                  vertex_capacity, faces, face_capacity, workspace, workspace_bytes, nullptr, nullptr,
-                                 nullptr, nullptr, nullptr, host.words(), nullptr, stream);
+                                 nullptr, nullptr, nullptr, &host, nullptr, stream);
     return host.wait(rc, 6, sizes, reinterpret_cast<cudaStream_t>(stream));
 }
 
@@ -1876,12 +1875,11 @@ int iso_dc_dense_its_sync(const float* values, int nx, int ny, int nz, const flo
                           void* stream) {
     if (!sizes || A < 1 || !points || !cell_ids || !cell_offsets) return iso::fail_code(ISO_ERR_ARG);
     iso::HostSizes host;
-    if (!host.words()) return ISO_ERR_CUDA;
     const Given in{points, normals, reinterpret_cast<const uint32_t*>(cell_ids),
                    reinterpret_cast<const uint32_t*>(cell_offsets), A, nullptr};
     const int rc = dc_dense_impl(values, nx, ny, nz, aabb_min, aabb_max, level, reg, svd_tol, vertices, A, faces,
                                  face_capacity, workspace, workspace_bytes, nullptr, nullptr, nullptr, nullptr, nullptr,
-                                 host.words(), &in, stream);
+                                 &host, &in, stream);
     return host.wait(rc, 6, sizes, reinterpret_cast<cudaStream_t>(stream));
 }
 
@@ -1895,7 +1893,8 @@ int iso_dc_intersection_sync(const float* values, int nx, int ny, int nz, const 
         return iso::fail_code(ISO_ERR_ARG);
     if (workspace_bytes < iso_dc_dense_workspace_size(nx, ny, nz, cell_capacity, 0)) return iso::fail_code(ISO_ERR_WORKSPACE);
     iso::HostSizes host;
-    if (!host.words()) return ISO_ERR_CUDA;
+    long long* const words = host.lease();
+    if (!words) return ISO_ERR_CUDA;
     const DcDenseWs w = carve_dense(workspace, nx, ny, nz, cell_capacity);
     const Grid3 g = make_grid(nx, ny, nz, aabb_min, aabb_max);
     long long *eff = w.misc + 4, *counts = w.misc + 8;
@@ -1918,7 +1917,7 @@ int iso_dc_intersection_sync(const float* values, int nx, int ny, int nz, const 
         iso::launch_pdl(dc_entry_points, blocks_for(cell_capacity, bt), unsigned(bt), st, values, g, level, ix,
                         static_cast<const long long*>(eff), static_cast<const float*>(w.gc), cells, off, points,
                         normals, static_cast<const long long*>(counts), static_cast<const int*>(status),
-                        host.words());
+                        words);
     }
     const int rc = cudaGetLastError() == cudaSuccess ? 0 : iso::fail_code(ISO_ERR_CUDA);
     return host.wait(rc, 6, sizes, st);
@@ -1938,7 +1937,7 @@ int iso_dc_dense(const float* values, int nx, int ny, int nz, const float* aabb_
 static int dc_dense_impl(const float* values, int nx, int ny, int nz, const float* aabb_min, const float* aabb_max,
                          float level, float reg, float svd_tol, float* vertices, long long vertex_capacity, int* faces,
                          long long face_capacity, void* workspace, size_t workspace_bytes, long long* counts,
-                         int* status, int* cell_ids, int* cell_offsets, int* vertex_source, long long* host,
+                         int* status, int* cell_ids, int* cell_offsets, int* vertex_source, iso::HostSizes* host,
                          const Given* given, void* stream) {
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     if (((!counts || !status) && !host) || !aabb_min || !aabb_max || vertex_capacity < 0 || face_capacity < 0) return iso::fail_code(ISO_ERR_ARG);
@@ -1952,6 +1951,8 @@ static int dc_dense_impl(const float* values, int nx, int ny, int nz, const floa
                     capQ = given ? face_capacity / 2 : std::min(face_capacity / 2, 0x7ffffffell / 6);
     if (workspace_bytes < iso_dc_dense_workspace_size(nx, ny, nz, vertex_capacity, face_capacity))
         return iso::fail_code(ISO_ERR_WORKSPACE);
+    long long* const words = host ? host->lease() : nullptr;
+    if (host && !words) return ISO_ERR_CUDA;
     const DcDenseWs w = carve_dense(workspace, nx, ny, nz, capA);
     const Grid3 g = make_grid(nx, ny, nz, aabb_min, aabb_max);
     long long* eff = w.misc + 4;
@@ -2010,7 +2011,7 @@ static int dc_dense_impl(const float* values, int nx, int ny, int nz, const floa
                             static_cast<const uint32_t*>(cells), static_cast<const uint32_t*>(w.qoff), ix,
                             static_cast<const float*>(w.dual), static_cast<const uint32_t*>(w.vmap),
                             static_cast<const long long*>(eff), faces, static_cast<const long long*>(counts),
-                            static_cast<const int*>(status), host);
+                            static_cast<const int*>(status), words);
         }
     }
     return cudaGetLastError() == cudaSuccess ? 0 : iso::fail_code(ISO_ERR_CUDA);

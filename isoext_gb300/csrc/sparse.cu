@@ -1181,7 +1181,7 @@ namespace {
 int sp_mc_launch(const int* ids, const float* vals, long long n, int nx, int ny, int nz, const float* amin,
                   const float* amax, float level, int method, float* vertices, long long vertex_capacity, int* faces,
                   long long face_capacity, void* workspace, size_t workspace_bytes, long long* counts, int* status,
-                  long long* host, void* stream) {
+                  iso::HostSizes* host, void* stream) {
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     if (((!counts || !status) && !host) || !amin || !amax || n < 0 || vertex_capacity < 0 || face_capacity < 0) return iso::fail_code(ISO_ERR_ARG);
     if (method != 0 && method != 1) return iso::fail_code(ISO_ERR_ARG);
@@ -1189,6 +1189,8 @@ int sp_mc_launch(const int* ids, const float* vals, long long n, int nx, int ny,
     if (n == 0) return cudaMemsetAsync(counts, 0, 24, st) == cudaSuccess ? 0 : iso::fail_code(ISO_ERR_CUDA);
     if (!ids || !vals || (vertex_capacity && !vertices) || (face_capacity && !faces)) return iso::fail_code(ISO_ERR_ARG);
     if (workspace_bytes < sp_mc_carve(nullptr, n, vertex_capacity, face_capacity).total) return iso::fail_code(ISO_ERR_WORKSPACE);
+    long long* const words = host ? host->lease() : nullptr;
+    if (host && !words) return ISO_ERR_CUDA;
     const SpMcWs w = sp_mc_carve(workspace, n, vertex_capacity, face_capacity);
     const SpGrid g = mk(nx, ny, nz, amin, amax, level, method);
     long long* eff = w.tot + 4;
@@ -1213,7 +1215,7 @@ int sp_mc_launch(const int* ids, const float* vals, long long n, int nx, int ny,
                     eff, w.weld, vertices, faces, w.tot + 8, status, st);
     {
         iso::ProfScope ps("sparse_mc", st);
-        iso::launch_pdl(sp_mc_finish, 1u, 1u, st, w.tot + 8, vertex_capacity, counts, status, host);
+        iso::launch_pdl(sp_mc_finish, 1u, 1u, st, w.tot + 8, vertex_capacity, counts, status, words);
     }
     return cudaGetLastError() == cudaSuccess ? 0 : iso::fail_code(ISO_ERR_CUDA);
 }
@@ -1365,9 +1367,8 @@ int iso_sparse_mc_sync(const int* ids, const float* vals, long long n, int nx, i
                        long long* sizes, void* stream) {
     if (!sizes) return iso::fail_code(ISO_ERR_ARG);
     iso::HostSizes host;
-    if (!host.words()) return ISO_ERR_CUDA;
     const int rc = sp_mc_launch(ids, vals, n, nx, ny, nz, amin, amax, level, method, vertices, vertex_capacity, faces,
-                                face_capacity, workspace, workspace_bytes, nullptr, nullptr, host.words(), stream);
+                                face_capacity, workspace, workspace_bytes, nullptr, nullptr, &host, stream);
     return host.wait(rc, 4, sizes, reinterpret_cast<cudaStream_t>(stream));
 }
 

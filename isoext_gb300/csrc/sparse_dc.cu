@@ -595,7 +595,7 @@ size_t sd_workspace(long long n, long long capA, long long capF) {
 int sd_launch(const int* ids, const float* values, long long n, int nx, int ny, int nz, const float* aabb_min,
               const float* aabb_max, float level, float reg, float svd_tol, float* vertices,
               long long vertex_capacity, int* faces, long long face_capacity, void* workspace, size_t workspace_bytes,
-              long long* counts, int* status, long long* host, void* stream) {
+              long long* counts, int* status, iso::HostSizes* host, void* stream) {
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     if (((!counts || !status) && !host) || !aabb_min || !aabb_max || vertex_capacity < 0 || face_capacity < 0 || n > 0x7fffffffll)
         return iso::fail_code(ISO_ERR_ARG);
@@ -607,6 +607,8 @@ int sd_launch(const int* ids, const float* values, long long n, int nx, int ny, 
         return iso::fail_code(ISO_ERR_ARG);
     if (workspace_bytes < sd_workspace(n, vertex_capacity, face_capacity))
         return iso::fail_code(ISO_ERR_WORKSPACE);
+    long long* const words = host ? host->lease() : nullptr;
+    if (host && !words) return ISO_ERR_CUDA;
     const long long capA = vertex_capacity;
     const SdWs w = carve_sd(workspace, n, capA);
     const Grid3 g = make_grid(nx, ny, nz, aabb_min, aabb_max);
@@ -654,7 +656,7 @@ int sd_launch(const int* ids, const float* values, long long n, int nx, int ny, 
             iso::ProfScope ps("sparse_quads", st);
             iso::launch_pdl(sd_faces, nblk, unsigned(SD_BLOCK), st, g, qbits, nbr, capA, dual, vmap, eff, blk, tot,
                             face_capacity, faces, static_cast<const long long*>(counts),
-                            static_cast<const int*>(status), host);
+                            static_cast<const int*>(status), words);
         }
     }
     return cudaGetLastError() == cudaSuccess ? 0 : iso::fail_code(ISO_ERR_CUDA);
@@ -682,10 +684,9 @@ int iso_sparse_dc_sync(const int* ids, const float* values, long long n, int nx,
                        void* workspace, size_t workspace_bytes, long long* sizes, void* stream) {
     if (!sizes || vertex_capacity < 1) return iso::fail_code(ISO_ERR_ARG);
     iso::HostSizes host;
-    if (!host.words()) return ISO_ERR_CUDA;
     const int rc = sd_launch(ids, values, n, nx, ny, nz, aabb_min, aabb_max, level, reg, svd_tol, vertices,
                              vertex_capacity, faces, face_capacity, workspace, workspace_bytes, nullptr, nullptr,
-                             host.words(), stream);
+                             &host, stream);
     return host.wait(rc, 6, sizes, reinterpret_cast<cudaStream_t>(stream));
 }
 

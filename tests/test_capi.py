@@ -199,3 +199,51 @@ def test_failures_leave_a_message_of_their_own():
     assert lib.iso_serve_set_bucket(None, 2) == 1 and _ffi.last_error() == "invalid argument"
     stale()
     assert lib.iso_serve_set_capacity_scale(None, 0.5) == 1 and _ffi.last_error() == "invalid argument"
+
+
+def test_waiting_calls_check_their_arguments_first():
+    """The iso_*_sync calls fail on their arguments and workspace sizes before they
+    take a record for the sizes or queue anything, and leave the sizes alone."""
+    import importlib
+
+    from isoext_gb300 import _ffi
+
+    for mod in ("mc", "dc", "sparse"):
+        importlib.import_module(f"isoext_gb300.{mod}")
+    lib = _ffi.lib()
+    _ffi._apply(lib, _ffi._EXTRA)
+    lo, hi = (ctypes.c_float * 3)(-1, -1, -1), (ctypes.c_float * 3)(1, 1, 1)
+    P, big = 1 << 20, 1 << 30  # a placeholder device address, never dereferenced
+    sizes = (ctypes.c_longlong * 6)(*[7] * 6)
+
+    def mc(n=8, method=0, cap=16, ws=0, out=sizes):
+        return lib.iso_mc_dense_sync(P, n, 8, 8, lo, hi, 0.0, method, P, cap, P, cap, P, ws, out, None)
+
+    def dc(n=8, values=P, cap=16, ws=0, out=sizes):
+        return lib.iso_dc_dense_sync(values, n, 8, 8, lo, hi, 0.0, 1e-2, 1e-6, P, cap, P, 16, P, ws, out, None)
+
+    def given(points=P, cells=P, A=4, ws=0, out=sizes):
+        return lib.iso_dc_dense_its_sync(P, 8, 8, 8, lo, hi, 0.0, 1e-2, 1e-6, points, None, cells, P, A, P, P, 16, P,
+                                         ws, out, None)
+
+    def its(n=8, points=P, cap=16, ws=0, out=sizes):
+        return lib.iso_dc_intersection_sync(P, n, 8, 8, lo, hi, 0.0, points, None, cap, P, P, cap, P, ws, out, None)
+
+    def sp_mc(n=4, method=0, cap=16, ws=0, out=sizes):
+        return lib.iso_sparse_mc_sync(P, P, n, 8, 8, 8, lo, hi, 0.0, method, P, cap, P, cap, P, ws, out, None)
+
+    def sp_dc(values=P, cap=16, ws=0, out=sizes):
+        return lib.iso_sparse_dc_sync(P, values, 4, 8, 8, 8, lo, hi, 0.0, 1e-2, 1e-6, P, cap, P, 16, P, ws, out, None)
+
+    bad = [lambda: mc(method=2), lambda: mc(cap=-1), lambda: mc(n=big), lambda: mc(out=None), lambda: dc(n=big),
+           lambda: dc(values=None), lambda: dc(cap=0), lambda: dc(out=None), lambda: given(points=None),
+           lambda: given(cells=None), lambda: given(A=0), lambda: given(out=None), lambda: its(n=1),
+           lambda: its(points=None), lambda: its(cap=0), lambda: its(out=None), lambda: sp_mc(n=-1),
+           lambda: sp_mc(method=7), lambda: sp_mc(out=None), lambda: sp_dc(values=None), lambda: sp_dc(values=P + 4),
+           lambda: sp_dc(cap=0), lambda: sp_dc(out=None)]
+    for i, call in enumerate(bad):
+        assert lib.iso_mc_set_config(100) == 1
+        assert call() == 1 and _ffi.last_error() and "threads must be" not in _ffi.last_error(), i
+    for call in (mc, dc, given, its, sp_mc, sp_dc):
+        assert call() == 5 and _ffi.last_error() == "workspace too small"
+    assert list(sizes) == [7] * 6

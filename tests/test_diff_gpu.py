@@ -150,3 +150,26 @@ def test_batched_extraction_equals_one_by_one():
         assert torch.equal(vm, vm1) and torch.equal(fm, fm1) and torch.equal(vd, vd1) and torch.equal(fd, fd1)
         # atomics make the summation order vary: equal to FP32 rounding
         assert torch.allclose(x.grad, y.grad, rtol=1e-5, atol=1e-7 * float(y.grad.abs().max()))
+
+
+class _NoGradient(torch.autograd.Function):
+    """Hands no gradient back to its input."""
+
+    @staticmethod
+    def forward(ctx, x):
+        return x.clone()
+
+    @staticmethod
+    def backward(ctx, g):
+        return None
+
+
+@pytest.mark.parametrize("name", ["marching_cubes", "dual_contouring"])
+def test_undefined_vertex_gradient_gives_zeros(name):
+    from isoext_gb300 import diff
+
+    vals, lo, hi = _crop()
+    x = torch.from_numpy(vals).cuda().requires_grad_(True)
+    v, f = getattr(diff, name)(x, lo, hi)
+    (_NoGradient.apply(v).sum() + 0.0 * x.sum()).backward()
+    assert len(v) and x.grad is not None and not x.grad.any()

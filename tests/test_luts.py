@@ -67,3 +67,22 @@ def test_packed_triangle_lists_match_tables():
             edges = [(v >> (4 * i)) & 15 for i in range(3 * n)]
             row = [e for e in flat[c * width:(c + 1) * width] if e >= 0]
             assert edges == row and n == len(cases[c])
+
+
+def test_one_polygon_cells_have_two_triangles_less_than_crossed_edges():
+    """The MC count's rule (word_faces): outside the cases with a face whose diagonal
+    corners pair up, or two opposite corners against the other six, both tables
+    have (crossed edges - 2) triangles."""
+    edges = [(a, a | d) for a in range(8) for d in (1, 2, 4) if not a & d]
+    faces = [(0, 1, 3, 2), (4, 5, 7, 6), (0, 1, 5, 4), (2, 3, 7, 6), (0, 2, 6, 4), (1, 3, 7, 5)]
+    checked = 0
+    for table, reflect in ((gen_luts.NAGAE, False), (gen_luts.LORENSEN, True)):
+        for cs, tris in enumerate(gen_luts.expand(table, reflect)):
+            c = [(cs >> k) & 1 for k in range(8)]
+            many = any(c[a] == c[d] and c[b] == c[e] and c[a] != c[b] for a, b, d, e in faces)
+            many |= any(c[i] == c[7 - i] and all(c[k] != c[i] for k in range(8) if k not in (i, 7 - i)) for i in range(4))
+            if cs in (0, 255) or many:
+                continue
+            assert len(tris) == sum(c[a] != c[b] for a, b in edges) - 2, cs
+            checked += 1
+    assert checked > 200

@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 import isoext_gb300 as iso  # noqa: E402
 from helpers import noise, sphere  # noqa: E402
-from isoext_gb300 import dc, diff  # noqa: E402
+from isoext_gb300 import _ffi, dc, diff  # noqa: E402
 from isoext_gb300.grids import grid_positions  # noqa: E402
 
 BOXES = {
@@ -65,6 +65,54 @@ def test_dense(box, kind):
     for a, f in (iso.dual_contouring(g), iso.dual_contouring(g, intersection=its),
                  diff.dual_contouring(g.get_values(), *BOXES[box])):
         assert f.numel() and _same(a, b) and torch.equal(f, h)
+
+
+# In a captured graph, replayed on other values, and with the vertices 4 bytes off
+# the 8-byte boundary that the entries (then the table) need: the room for the list
+# of vertices on faces is one short, and on these boxes every vertex lies on one.
+# "mirrored" has distinct coordinates: the local search over all cells.
+@pytest.mark.parametrize("box", ["point", "reversed", "mirrored"])
+def test_capture_and_a_full_face_list(box):
+    lo, hi = BOXES.get(box, ((1.0,) * 3, (-1.0,) * 3))
+    lib = _ffi.lib()
+    fields = [torch.from_numpy(noise((21, 22, 35), seed, 0.1)).cuda() for seed in (1, 2)]
+    want = []
+    for x in fields:
+        g = iso.UniformGrid(x.shape, lo, hi)
+        g.set_values(x)
+        its = iso.get_intersection(g, compute_normals=True)
+        want.append((*dc._dc_sequence(g, its, 1e-2, 1e-6), its._cells.numel()))
+    values = fields[0].clone()
+    for capA, offset in ((want[0][2], 1), (1 << 15, 0)):
+        ws = torch.empty(dc.dc_workspace_bytes(values.shape, capA, 1 << 17), dtype=torch.uint8, device="cuda")
+        vout = torch.empty(3 * capA + offset, device="cuda")[offset:]
+        fout = torch.empty((1 << 17, 3), dtype=torch.int32, device="cuda")
+        small = torch.zeros(8, dtype=torch.int64, device="cuda")
+        assert vout.data_ptr() % 8 == 4 * offset
+
+        def call():
+            small.zero_()
+            _ffi.check(dc.dc_dense_into(values, lo, hi, 0.0, 1e-2, 1e-6, vout.view(-1, 3), fout, ws, small,
+                                        torch.cuda.current_stream().cuda_stream))
+
+        def check(k):
+            V, F, status = int(small[0]), int(small[1]), int(small[6]) & 0xffffffff
+            assert status == 0 and V == len(want[k][0]) and F == len(want[k][1])
+            assert _same(vout[:3 * V].view(-1, 3), want[k][0]) and torch.equal(fout[:F], want[k][1])
+
+        values.copy_(fields[0])
+        call()
+        check(0)
+        if offset:
+            continue
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            call()
+        for k in (1, 0):
+            values.copy_(fields[k])
+            graph.replay()
+            torch.cuda.synchronize()
+            check(k)
 
 
 # Spacings just above the rule's line, 2^-20 of the box's magnitude: no coordinate repeats.

@@ -164,9 +164,11 @@ def kernel_bytes(kind: str, n: int, nv: int, nf: int) -> dict:
     segs = (words + 1023) // 1024
     return {
         "mc_signs": 4 * pts + 4 * words,           # values once, sign bitmap once
-        "mc_count": 4 * words + 4 * words,         # bitmap once, per-word entries once
+        # bitmap once, vertex and cell entries (two triangles a cell); the offsets of the
+        # words with crossings, a few percent of them, are left out
+        "mc_count": 4 * words + 8 * nv + 8 * (nf // 2),
         "mc_scan": 32 * segs,                      # segment sums read, offsets written
-        "mc_emit": 16 * nv + 12 * nv + 8 * nf + 12 * nf,  # entries and endpoint values; vertices, faces
+        "mc_emit": 16 * nv + 12 * nv + 8 * (nf // 2) + 12 * nf,  # entries and endpoint values; vertices, faces
         "mc_fix": 32,                              # the counters, when no vertices coincide
     }
 

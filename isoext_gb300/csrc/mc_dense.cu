@@ -1,10 +1,11 @@
 // Dense-grid marching cubes on sm_103a.
 //
-// Five launches on one stream, nothing read back by the host:
-//   1. mc_signs   streams the grid once (16 coalesced 128-byte loads in flight per
+// Four launches on one stream (five on grids of more than 1024 segments), nothing
+// read back by the host:
+//   1. mc_signs   streams the grid once (32 coalesced 128-byte loads in flight per
 //                 warp) into a sign bitmap,
 //                 1 bit per point.  This is the only pass over all values.
-//   2. mc_count   one CTA per segment of 256 to 1024 point words, from the bitmap
+//   2. mc_count   one CTA per segment of 128 to 1024 point words, from the bitmap
 //                 alone (16.8 MB at 512^3): the words near the surface, listed;
 //                 their crossed-edge masks, active cells and triangle counts,
 //                 bit-parallel; vertex and cell entry lists.  On grids of few
@@ -96,7 +97,7 @@ struct McWs {
     unsigned long long* blk;    // per segment of words: (V, F) sums, then exclusive offsets
     unsigned long long* vlist;  // vertex entries [capV]: pw | axis << 32 | bit << 34 | slot << 39
     unsigned long long* clist;  // cell entries [capF]: pw | bit << 32 | the word's segment-local face offset << 37
-    unsigned long long* blk2;   // blk of grids cut into more than nBlk segments
+    unsigned long long* blk2;   // blk of grids of one word per count thread, cut into more than nBlk segments
     unsigned long long* ctr;    // [0] list size [1] snaps [2] V [3] F when the caller has no counts [4] V [5] F (before the fix-up) [6] count CTAs done [7] scan ticket
                                 // [8] merges [9] small hash full [10] cell entries [12] fix-up ticket
                                 // [13] fix-up tiles done [14] status when the caller has none; the rest unused
@@ -110,7 +111,7 @@ struct McWs {
     unsigned long long* fstate; // fix-up: look-back states of its face tiles (region of capF * 12 bytes)
     uint32_t* vbits;            // fix-up: two more bitmaps, then the look-back states of its vertex tiles
                                 // (region of capV * 12 bytes)
-    long long nBlk;             // segments at most (SEG_MIN point words each)
+    long long nBlk;             // segments of SEG_MIN point words: as many as four words per count thread make, at most
     uint32_t HC;
     size_t total;
 };
@@ -140,7 +141,7 @@ McWs carve(int nx, int ny, int nz, long long capV, long long capF, uint8_t* base
     McWs w{};
     const long long NW = (nz + 31) / 32;
     const long long PW = (long long)nx * ny * NW;
-    w.nBlk = (PW + SEG_MIN - 1) / SEG_MIN;  // segments at most (the smallest count CTA)
+    w.nBlk = (PW + SEG_MIN - 1) / SEG_MIN;
     w.HC = hash_cap(capV);
     size_t o = 0;
     auto take = [&](size_t bytes) {

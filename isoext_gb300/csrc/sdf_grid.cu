@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(256) sdf_union_tiles(const float* __restrict__
     const int np = load_prims(prims, pr, &np_s);
     const int lane = threadIdx.x & 31, lz = lane & 7, ly = lane >> 3;
     const uint32_t tz = uint32_t(nz + 31) / 32u, ty = uint32_t(ny + 3) / 4u, tx = uint32_t(nx + TILE_X - 1) / TILE_X;
-    const uint32_t tiles = tx * ty * tz;  // at least 68 points each: below 2^32 for any grid that fits
+    const uint32_t tiles = tx * ty * tz;  // a few dozen points each at least (ny >= 4, nz >= 17): below 2^32 for any grid that fits
     const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
     for (uint32_t t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < tiles; t += nwarps) {
         const int z0 = int(t % tz) * 32, y0 = int((t / tz) % ty) * 4, x0 = int(t / tz / ty) * TILE_X;

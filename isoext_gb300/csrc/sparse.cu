@@ -593,6 +593,9 @@ __global__ void __launch_bounds__(SP2_THREADS) sp_mc_count2(SpGrid g, const int*
 // band ten cells deep has about 600 entries and 700 triangles; 768 each let
 // six CTAs be resident (for the band of a 1024^3 grid 371 us with 2048 and 1024,
 // which hold four, 302 with six CTAs, 336 with seven, whose registers spill).
+// Grids of crossed cells only have thousands of both per chunk; their calls got
+// faster all the same (a 1024^3 sphere's 2.4 M cells 630 -> 505 us, a 512^3
+// gyroid's 4.9 M 1025 -> 925).
 constexpr int SP2_STAGE_V = 768;
 constexpr int SP2_STAGE_F = 768;
 
@@ -687,6 +690,7 @@ __global__ void __launch_bounds__(SP2_THREADS, 6) sp_mc_emit2(SpGrid g, const in
     __shared__ unsigned long long tpk[256];  // packed triangle lists of the cases
     __shared__ float sv[SP2_STAGE_V * 3];
     __shared__ uint16_t sd[SP2_STAGE_V];  // staged entries to make: list position << 4 | edge (15: made)
+    static_assert(SP2_CHUNK <= 0x1000, "a list position fits 12 bits");
     __shared__ int32_t sf[SP2_STAGE_F * 3];
     __shared__ uint32_t wsum[2][SP2_THREADS / 32];
     __shared__ uint16_t slv[SP2_CHUNK];  // each listed cell's first own entry (CTA-local)

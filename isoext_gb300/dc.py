@@ -1,8 +1,10 @@
 """get_intersection / dual_contouring / Intersection with isoext's API
 (src/isoext_ext.cu:305-378) on the CUDA path (csrc/dc_dense.cu).
 
-The steps run asynchronously on the current stream; the host synchronises only
-to size the next buffers (active cells and crossings, quads, welded vertices).
+Usually one native call on the current stream that launches, waits and returns
+the sizes, its buffers sized from the call before (a second one where they were
+too small).  An intersection whose cells are not the grid's any more takes a
+sequence of calls, the host synchronising to size the next buffers.
 """
 
 from __future__ import annotations

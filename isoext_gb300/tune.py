@@ -8,7 +8,8 @@ The knobs (C ABI iso_tune_set) change launch shapes only, never results:
   "mc.emit_threads"     threads per CTA of the MC emit kernel
   "mc.sign_ctas_per_sm" CTAs per SM of the sign pass
   "mc.count_threads"    threads per CTA of the MC count kernel (and so the
-                        scan's segment: 4 point words per thread)
+                        scan's segment: 4 point words per thread, 1 on
+                        grids of up to 2^18 words)
   "dc.cell_threads"     threads per CTA of the per-active-cell DC kernels
 Each knob is timed in turn (coordinate descent) with CUDA events over the
 extraction it affects, on the caller's grid, the others held at their current
